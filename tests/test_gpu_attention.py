@@ -42,6 +42,28 @@ def test_attention_fwd_bwd(shape, causal):
     assert err < 0.15 and rel < 2e-2, (err, rel)
 
 
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("shape", [(5, 384, 61), (2, 1280, 40), (37, 128, 4), (149, 128, 1)])
+def test_attention_forward_items(shape, causal):
+    """More items than SMs (running CTAs take the rest over), an odd number of tiles (an item of one tile), and the
+    two sides of the rule that gives a CTA one or two tiles.  P and the result are rounded to bf16 (2^-9 each, of
+    values that are averages of |v| <= 5.5): 0.022, and 1e-3 for the fp32 sums and exponentials."""
+    from meshslice_b200 import _native
+    from meshslice_b200.ops import functional as F
+    batch, seq, heads = shape
+    g = torch.Generator(device="cuda").manual_seed(batch)
+    qkv = torch.randn(batch * seq, heads * 3 * 128, device="cuda", generator=g).bfloat16()
+    out, lse = F.attention_fwd(qkv, batch, seq, heads, causal)
+    _native.check_status()
+    q, k, v = (qkv.view(batch, seq, heads, 3, 128)[:, :, :, i].transpose(1, 2).float() for i in range(3))
+    s = q @ k.transpose(-1, -2) / math.sqrt(128)
+    if causal:
+        s.masked_fill_(torch.ones(seq, seq, dtype=torch.bool, device="cuda").triu(1), float("-inf"))
+    ref = (torch.softmax(s, -1) @ v).transpose(1, 2).reshape(batch * seq, heads * 128)
+    assert (out.float() - ref).abs().max().item() < 0.023
+    assert (lse - torch.logsumexp(s, -1)).abs().max().item() < 0.02
+
+
 def test_attention_large_scores_exercise_rescaling():
     """Scores that grow along the keys force the running maximum (and O) to be rescaled."""
     from meshslice_b200 import _native
