@@ -193,10 +193,10 @@ cudaError_t launch_sm100_gemm(const CUtensorMap& tma_a, const CUtensorMap& tma_b
 cudaError_t launch_sm100_gemm2(const CUtensorMap& tma_a, const CUtensorMap& tma_b,
                                const GemmArgs& args, int grid, cudaStream_t stream);
 
-// Builds a 2-D bf16 tensor map with 128-byte swizzle.  `inner` is the contiguous extent,
+// Builds a 2-D bf16 tensor map with a swizzle of 128 (or 64) bytes.  `inner` is the contiguous extent,
 // `outer` the number of rows, `pitch_bytes` the row pitch.  Returns 0 on success.
 int make_tensor_map_2d(CUtensorMap* map, const void* base, uint64_t inner, uint64_t outer,
-                       uint64_t pitch_bytes, uint32_t box_inner, uint32_t box_outer);
+                       uint64_t pitch_bytes, uint32_t box_inner, uint32_t box_outer, int swizzle_bytes = 128);
 
 // Tensor map of an MN-major operand (stored [k_rows, mn_extent] row-major, mn_extent % 64 == 0) as
 // {64 elements, k_rows, mn_extent / 64 blocks}: one box of {64, kBK, blocks_per_box} fills the

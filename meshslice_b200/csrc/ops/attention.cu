@@ -5,8 +5,8 @@
 //   into TMEM, online softmax in the log2 domain with lazy rescaling of O (only when the running
 //   maximum grows by more than 2^8), P written back over S as packed bf16 and read by O += P V as
 //   the TMEM operand.
-// Backward (attn_bwd2_kernel<key-major>, <query-major>): dK / dV are accumulated by the CTA that owns
-//   128 keys, dQ by the CTA that owns 128 queries; both recompute S and dP, keep P and dS in TMEM,
+// Backward (attn_bwd2_kernel<key-major>, <query-major>): dK / dV are accumulated by the CTA that works on
+//   128 keys, dQ by the CTA that works on 128 queries; both recompute S and dP, keep P and dS in TMEM,
 //   and never add to global memory: the gradients are bit-identical from run to run.
 // All waits are bounded; a timeout records a code in `status` and the CTA leaves.
 #include "attention.h"
@@ -36,10 +36,7 @@ constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kLn2 = 0.6931471805599453f;
 
 struct AttnArgs {
-  void* out;          // fwd: out;  bwd: dqkv
   float* lse;
-  float* dq_acc;      // bwd
-  const float* delta; // bwd
   int batch, seq, heads, causal;
   int tiles_per_item; // fwd: query tiles that a CTA works on at a time (1 or 2)
   float scale;
@@ -55,13 +52,9 @@ __device__ __forceinline__ void report(uint32_t* status, uint32_t code, uint32_t
   }
 }
 
-// Bounded wait that the whole warp follows: lane 0 polls, the verdict is broadcast.
+// Bounded wait of a whole warp: the lanes poll together (one transaction), the verdict is common.
 __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, uint64_t tmo) {
-  int ok = 1;
-  if ((threadIdx.x & 31) == 0) ok = mbar_wait(bar, parity, tmo) ? 1 : 0;
-  ok = __shfl_sync(0xffffffffu, ok, 0);
-  if (ok) mbar_wait(bar, parity, tmo);  // already complete: orders this lane's later reads
-  return ok != 0;
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, tmo));
 }
 
 // 2^x on the special-function unit in one instruction (relative error 2^-22, denormal results
@@ -113,14 +106,15 @@ __device__ __forceinline__ void load_tile(uint8_t* dst, const CUtensorMap* map, 
 // the next scores are there (768 of MMAs, the rest is latency of the hand-over).  Issue order keeps the two tiles
 // apart, so that one's softmax runs under the other's products; two steps take about 3800 cycles.  Two CTAs per SM
 // with a tile each and the same softmax fall into step instead, because the tensor pipe and the SFU then serve
-// both at once: 298 us against 253 for 16 heads x 8192, causal (361 with two passes over S in tensor memory).
+// both at once: 298 us against 253 for 16 heads x 8192, causal (321 with two passes over S in tensor memory).
 // A row of S is read once, into 128 registers; maxima take three inputs and multiply-adds and sums two lanes per
 // instruction; P is handed over in two parts, so that six of the eight k-steps of P V run under the last quarter's
 // exponentials, and half of the row's sum waits until P is on its way.  An item's output and the next item's first
 // scores overlap: the roles only meet at the barriers.  Tried without gain: two threads per row (264 us, more
 // barriers for the same tensor-memory traffic), a quarter to three eighths of the exponentials as a polynomial on
 // the FMA pipe (263-289 us: the registers spill and the warp's issue slots are the limit).
-// Batch 4 x 2048, 32 heads, causal: 202 -> 155 us (890 TFLOP/s), full 252 us (1090).
+// With outputs as TMA stores and one poll per wait: 230 us (1196 TFLOP/s) for 16 heads x 8192, causal; batch 4 x 2048,
+// 32 heads: causal 202 -> 148 us (930), full 330 -> 233 us (1180).
 constexpr int kFwdWarpStage = 32 * 128;   // output staging per softmax warp: 32 rows x 64 columns
 constexpr size_t kFwd2Smem = 6 * kTile + 8 * kFwdWarpStage + 256 + 1024;
 constexpr int kFwd2Threads = 384;
@@ -166,6 +160,31 @@ __device__ __forceinline__ void tmem_st_32x16(uint32_t taddr, const uint32_t (&r
       : "memory");
 }
 
+__device__ __forceinline__ void tmem_st_32x8(uint32_t taddr, const uint32_t (&r)[8]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+               ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+               : "memory");
+}
+// shared -> global, one box of a tensor map; tracked by bulk groups
+__device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, const void* smem_src, int32_t x, int32_t y) {
+  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];"
+               ::"l"(map), "r"(smem_u32(smem_src)), "r"(x), "r"(y) : "memory");
+}
+// A warp's staged box on its way: every lane's writes are visible to the copy engine before lane 0 starts it.
+__device__ __forceinline__ void warp_store_box(const CUtensorMap* map, const void* stage, int32_t x, int32_t y) {
+  fence_proxy_async_smem();
+  __syncwarp();
+  if ((threadIdx.x & 31) == 0) {
+    tma_store_2d(map, stage, x, y);
+    bulk_commit();
+  }
+}
+// The staging area may be written again: the copy engine has read it.
+__device__ __forceinline__ void warp_stage_free() {
+  if ((threadIdx.x & 31) == 0) bulk_wait_read<0>();
+  __syncwarp();
+}
+
 // Two fp32 lanes in one 64-bit register: fma / add / mul of both in one issue slot (same rounding as the scalar forms).
 __device__ __forceinline__ uint64_t f32x2(float lo, float hi) {
   uint64_t d;
@@ -183,6 +202,11 @@ __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
 __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
   uint64_t d;
   asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
   return d;
 }
 __device__ __forceinline__ float max3(float a, float b, float c) {
@@ -207,7 +231,8 @@ __device__ __forceinline__ FwdItem fwd_item(const AttnArgs& a, uint32_t x, uint3
 }
 
 __global__ void __launch_bounds__(kFwd2Threads, 1)
-attn_fwd2_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constant__ AttnArgs a) {
+attn_fwd2_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constant__ CUtensorMap tm_out,
+                 const __grid_constant__ AttnArgs a) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
@@ -519,35 +544,27 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_consta
       if (n_kv > 0) {
         tc_fence_after_sync();
         const float inv = 1.0f / l;
-        // The warp's 32 rows go through shared memory, 64 columns at a time, so that a store instruction writes four
-        // whole 128-byte lines instead of 16 bytes of 32 rows.
-        __nv_bfloat16* orow = reinterpret_cast<__nv_bfloat16*>(a.out) +
-                              ((int64_t)w.b * a.seq + i_blk * kBlk + q4 * 32) * (a.heads * kD) + w.h * kD;
+        // The warp's 32 rows leave through shared memory, 64 columns at a time, as TMA stores: nothing here waits for
+        // the memory system (with plain stores a warp stalls when all SMs write their items at the same time).
 #pragma unroll 1
         for (int half = 0; half < 2; ++half) {
+          uint32_t o[2][32];
+          tmem_ld_32x32(to + half * 64, o[0]);
+          tmem_ld_32x32(to + half * 64 + 32, o[1]);
+          warp_stage_free();
+          tmem_ld_wait();
 #pragma unroll
-          for (int c = 0; c < 2; ++c) {
-            uint32_t o[32];
-            tmem_ld_32x32(to + half * 64 + c * 32, o);
-            tmem_ld_wait();
+          for (int c = 0; c < 2; ++c)
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
               uint4 u;
-              u.x = pack_bf16(__uint_as_float(o[q * 8 + 0]) * inv, __uint_as_float(o[q * 8 + 1]) * inv);
-              u.y = pack_bf16(__uint_as_float(o[q * 8 + 2]) * inv, __uint_as_float(o[q * 8 + 3]) * inv);
-              u.z = pack_bf16(__uint_as_float(o[q * 8 + 4]) * inv, __uint_as_float(o[q * 8 + 5]) * inv);
-              u.w = pack_bf16(__uint_as_float(o[q * 8 + 6]) * inv, __uint_as_float(o[q * 8 + 7]) * inv);
-              *reinterpret_cast<uint4*>(stage + lane * 128 + (((c * 4 + q) ^ (lane & 7)) << 4)) = u;
+              u.x = pack_bf16(__uint_as_float(o[c][q * 8 + 0]) * inv, __uint_as_float(o[c][q * 8 + 1]) * inv);
+              u.y = pack_bf16(__uint_as_float(o[c][q * 8 + 2]) * inv, __uint_as_float(o[c][q * 8 + 3]) * inv);
+              u.z = pack_bf16(__uint_as_float(o[c][q * 8 + 4]) * inv, __uint_as_float(o[c][q * 8 + 5]) * inv);
+              u.w = pack_bf16(__uint_as_float(o[c][q * 8 + 6]) * inv, __uint_as_float(o[c][q * 8 + 7]) * inv);
+              *reinterpret_cast<uint4*>(stage + lane * 128 + (((c * 4 + q) ^ (lane & 7)) << 4)) = u;   // 128-byte swizzle
             }
-          }
-          __syncwarp();
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const int rr = i * 4 + (lane >> 3), ch = lane & 7;
-            const uint4 u = *reinterpret_cast<const uint4*>(stage + rr * 128 + ((ch ^ (rr & 7)) << 4));
-            *reinterpret_cast<uint4*>(orow + (int64_t)rr * (a.heads * kD) + half * 64 + ch * 8) = u;
-          }
-          __syncwarp();
+          warp_store_box(&tm_out, stage, w.h * kD + half * 64, w.b * a.seq + i_blk * kBlk + q4 * 32);
         }
         a.lse[((int64_t)w.b * a.heads + w.h) * a.seq + i_blk * kBlk + row] = m_used * kLn2 + logf(l);
       }
@@ -555,6 +572,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_consta
       __syncwarp();                              // every lane has read the response
       if (lane == 0) mbar_arrive(clc_empty);
     }
+    if (lane == 0) bulk_wait_all<0>();
   }
   tc_fence_before_sync();
   __syncthreads();
@@ -565,32 +583,58 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_consta
 // ==========================================================================================
 // backward
 // ==========================================================================================
-// delta[b, h, s] = rowsum(dO * O) * scale and lse2[b, h, s] = lse * log2(e): pre-scaled so that the
-// element-wise passes of the backward kernels need one fused multiply-add each for the exponent and
-// for dP * scale - delta.
-__global__ void attn_delta_kernel(const __nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict__ dout,
-                                  float* __restrict__ delta, int batch, int seq, int heads,
-                                  const float* __restrict__ lse, float* __restrict__ lse2, float scale) {
-  // one warp per (token, head): delta = sum_d out * dout
-  const int64_t w = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  const int64_t total = (int64_t)batch * seq * heads;
-  if (w >= total) return;
-  const int64_t t = w / heads;
-  const int h = (int)(w - t * heads);
-  const uint2 o = *reinterpret_cast<const uint2*>(out + t * heads * kD + h * kD + lane * 4);
-  const uint2 d = *reinterpret_cast<const uint2*>(dout + t * heads * kD + h * kD + lane * 4);
-  float s = __uint_as_float(o.x << 16) * __uint_as_float(d.x << 16) +
-            __uint_as_float(o.x & 0xffff0000u) * __uint_as_float(d.x & 0xffff0000u) +
-            __uint_as_float(o.y << 16) * __uint_as_float(d.y << 16) +
-            __uint_as_float(o.y & 0xffff0000u) * __uint_as_float(d.y & 0xffff0000u);
+// delta[b, h, s] = -rowsum(dO * O) * scale and lse2[b, h, s] = -lse * log2(e): scaled and negated so that the
+// element-wise passes of the backward kernels need one multiply-add each for the exponent and for dP * scale - delta.
+// Bound by HBM (it reads O and dO once): 16 lanes with a 16-byte vector each take one head of kDeltaRows consecutive
+// tokens, all loads requested before the first sum, and write neighbouring statistics.  33.5 M elements, cold: 52 us
+// with a warp per (token, head) and 8 bytes per lane, 26 us so.
+// kWide: `out` is 16-byte aligned (dout always is: the tensor map asks for it).
+constexpr int kDeltaRows = 4;
+static_assert(kBlk % kDeltaRows == 0, "sequences are whole groups of rows");
+template <bool kWide>
+__global__ void __launch_bounds__(256)
+attn_delta_kernel(const uint4* __restrict__ out, const uint4* __restrict__ dout, float* __restrict__ delta,
+                  uint32_t groups, uint32_t seq, uint32_t heads, const float* __restrict__ lse, float* __restrict__ lse2,
+                  float scale) {
+  const uint32_t sub = threadIdx.x & 15;
+  const uint32_t w = blockIdx.x * (blockDim.x >> 4) + (threadIdx.x >> 4);   // (group of tokens, head)
+  const bool live = w < groups;
+  const uint32_t tg = w / heads, h = w - tg * heads;
+  const int64_t t0 = (int64_t)tg * kDeltaRows;
+  uint4 o[kDeltaRows], d[kDeltaRows];
 #pragma unroll
-  for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-  if (lane == 0) {
-    const int64_t bq = t / seq, sq = t - bq * seq;
-    const int64_t idx = (bq * heads + h) * seq + sq;
-    delta[idx] = s * scale;
-    lse2[idx] = lse[idx] * kLog2e;
+  for (int i = 0; i < kDeltaRows; ++i) {
+    o[i] = d[i] = make_uint4(0u, 0u, 0u, 0u);
+    if (live) {
+      const int64_t at = ((t0 + i) * heads + h) * 16 + sub;
+      if (kWide) {
+        o[i] = __ldcs(out + at);
+      } else {
+        const uint2* p = reinterpret_cast<const uint2*>(out) + at * 2;
+        const uint2 lo = __ldcs(p), hi = __ldcs(p + 1);
+        o[i] = make_uint4(lo.x, lo.y, hi.x, hi.y);
+      }
+      d[i] = __ldcs(dout + at);
+    }
+  }
+  float mine = 0.f;                      // the sum of row `sub`
+#pragma unroll
+  for (int i = 0; i < kDeltaRows; ++i) {
+    const uint32_t ov[4] = {o[i].x, o[i].y, o[i].z, o[i].w}, dv[4] = {d[i].x, d[i].y, d[i].z, d[i].w};
+    float s = 0.f;
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      s += __uint_as_float(ov[k] << 16) * __uint_as_float(dv[k] << 16) +
+           __uint_as_float(ov[k] & 0xffff0000u) * __uint_as_float(dv[k] & 0xffff0000u);
+#pragma unroll
+    for (int off = 8; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
+    if (sub == i) mine = s;
+  }
+  if (live && sub < kDeltaRows) {
+    const uint32_t b = tg / (seq / kDeltaRows);
+    const int64_t idx = ((int64_t)b * heads + h) * seq + (t0 - (int64_t)b * seq) + sub;
+    delta[idx] = -mine * scale;
+    lse2[idx] = -lse[idx] * kLog2e;
   }
 }
 
@@ -598,91 +642,139 @@ __global__ void attn_delta_kernel(const __nv_bfloat16* __restrict__ out, const _
 // backward: two deterministic kernels, P / dS stay in tensor memory
 // ==========================================================================================
 // The gradient is split by who accumulates it:
-//   attn_bwd2_kernel<true>   one CTA per 128 KEYS walks the query blocks and accumulates dV, dK in TMEM
-//   attn_bwd2_kernel<false>  one CTA per 128 QUERIES walks the key blocks and accumulates dQ in TMEM
+//   attn_bwd2_kernel<true>   an item is 128 KEYS, whose CTA walks the query blocks and accumulates dV, dK in TMEM
+//   attn_bwd2_kernel<false>  an item is 128 QUERIES, whose CTA walks the key blocks and accumulates dQ in TMEM
 // Both recompute S and dP (7 products per block pair instead of 5), but nothing is ever added to
 // global memory: no fp32 dQ buffer, no memset, no atomics, and the result is bit-identical from run
 // to run.  P and dS are written back over S and dP as packed bf16 and feed the gradient products
 // as the TMEM (A) operand: they never touch shared memory.
 //
-// An MMA of M = 128 occupies the tensor pipe for about 92-105 cycles whatever its N up to 128, so
-// the products use full 128-wide blocks (eight instructions each) and the kernels are organised
-// around keeping that one pipe fed: the element-wise work is split in two phases (P from S; dS from
+// The products use full 128-wide blocks (eight instructions of 64 cycles each) and the kernels are organised
+// around keeping the tensor pipe fed: the element-wise work is split in two phases (P from S; dS from
 // dP and P) and the MMA warp issues the next block's S (and dP) between the gradient products of the
 // current block, so each phase runs under products that do not depend on it:
 //   key-major    S(i) dP(i) | P(i)? dV(i) S(i+1) | dS(i)? dK(i) dP(i+1) | P(i+1)? ...
 //   query-major  S(j) dP(j) S(j+1) | dS(j)? dQ(j) dP(j+1) S(j+2) | ...          (two S buffers)
 //
-//   warp 0      TMA: the two resident 128-row tiles once, then a two-stage ring of 128-row tile pairs
-//   warp 1      MMA issuer (all operand descriptors are built once, outside the loops)
-//   warps 2-9   element-wise: two threads per TMEM lane, 64 of the 128 columns each
-constexpr int kRing = 2;
-constexpr size_t kBwd2Smem = 2 * kTile + kRing * 2 * kTile + 256 + 1024;
-constexpr int kBwd2Threads = 64 + 32 * 8;
+//   warp 0      TMA: the two resident 128-row tiles, a two-stage ring of 128-row tile pairs and, key-major, the
+//               statistics of the streamed queries; asks for the next item (cluster launch control, as in forward)
+//   warp 1      MMA issuer
+//   warps 2-17  element-wise: four threads per TMEM lane, 32 of the 128 columns each
+//
+// What bounds it: the chain S -> P -> dV, S' and dP -> dS -> dK, dP'.  Per block pair the products take 2048
+// (key-major) and 1536 cycles, the exponentials 1024 of the SFU; measured 3350 and 2150, of which 350-450 cycles go
+// into every hand-over from the tensor pipe to the warps and back.  So sixteen warps share a phase, each thread reads its
+// 32 columns with one load and keeps P in fp32 registers for dS; P^T is handed over in two parts; the key-major
+// statistics come through shared memory (broadcast loads of them from global memory cost 7 L1 wavefronts each and a
+// miss per block); the rings are split by operand, because a shared stage of K and V was only free after dQ and the
+// products waited for the next one (query-major 3300 cycles a pair).  CTAs are persistent: the next item's tiles, S and
+// dP arrive while this item's accumulators leave as TMA stores (9000 cycles between items with 16-byte stores per
+// lane, 4000 staged through shared memory, as all SMs write at once).
+// Batch 4 x 2048, 32 heads, causal: key-major 424 -> 232 us, query-major 306 -> 179 us.
+constexpr int kStatBytes = 2 * kBlk * 4;   // lse2 and delta of 128 queries
+constexpr int kBwdWarps = 16;               // element-wise warps
+constexpr int kBwdCols = kBlk * 4 / kBwdWarps;   // columns of a row per element-wise thread
+constexpr int kBwdStage = 32 * kBwdCols * 2;     // output staging per element-wise warp
+constexpr int kBwdAlignSlack = 512;
+constexpr size_t kBwd2Smem = 6 * kTile + kBwdWarps * kBwdStage + 2 * kStatBytes + 256 + kBwdAlignSlack;
+static_assert(kBwd2Smem <= 232448, "shared memory of a CTA");
+constexpr int kBwd2Threads = 64 + 32 * kBwdWarps;
 
 struct Bwd2Args {
-  void* dqkv;
-  const float* lse2;    // lse * log2(e)          (written by attn_delta_kernel)
-  const float* delta;   // rowsum(dO * O) * scale (written by attn_delta_kernel)
+  const float* lse2;    // -lse * log2(e)          (written by attn_delta_kernel)
+  const float* delta;   // -rowsum(dO * O) * scale (written by attn_delta_kernel)
   int batch, seq, heads, causal;
   float scale;
   uint32_t* status;
   uint64_t timeout_ns;
 };
 
-// kKeyMajor = true:  resident tiles K, V (this CTA's 128 keys), streamed Q, dO; accumulators dV, dK.
+struct BwdItem {
+  int b, h, blk, i0, n_it;   // sequence, head, owned block, first streamed block, streamed blocks
+};
+template <bool kKeyMajor>
+__device__ __forceinline__ BwdItem bwd_item(const Bwd2Args& a, uint32_t x, uint32_t y, uint32_t z, int group) {
+  BwdItem w;
+  const int bh = (int)z * group + (int)x, nblk = a.seq / kBlk;
+  w.b = bh / a.heads;
+  w.h = bh - w.b * a.heads;
+  // same block order as the forward kernel: per group of batch-heads the longest tiles first (key block 0 / the
+  // last query block stream the most); queries i0 .. nblk-1 for a key block, keys 0 .. blk for a query block
+  w.blk = kKeyMajor ? (int)y : (a.causal ? nblk - 1 - (int)y : (int)y);
+  w.i0 = kKeyMajor && a.causal ? w.blk : 0;
+  w.n_it = kKeyMajor ? nblk - w.i0 : (a.causal ? w.blk + 1 : nblk);
+  return w;
+}
+
+// kKeyMajor = true:  resident tiles K, V (this item's 128 keys), streamed Q, dO; accumulators dV, dK.
 //                    TMEM lanes = keys, columns = queries: lse / delta vary along the columns.
-// kKeyMajor = false: resident tiles Q, dO (this CTA's 128 queries), streamed K, V; accumulator dQ.
+// kKeyMajor = false: resident tiles Q, dO (this item's 128 queries), streamed K, V; accumulator dQ.
 //                    TMEM lanes = queries, columns = keys: lse / delta are per thread.
 template <bool kKeyMajor>
 __global__ void __launch_bounds__(kBwd2Threads, 1)
 attn_bwd2_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constant__ CUtensorMap tm_do,
-                 const __grid_constant__ Bwd2Args a) {
+                 const __grid_constant__ CUtensorMap tm_dqkv, const __grid_constant__ Bwd2Args a) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
+  // the base is 1024-byte aligned in practice; there is no room for the full slack of an arbitrary one
+  if (smem - smem_raw > kBwdAlignSlack) {
+    if (threadIdx.x == 0) report(a.status, kErrAttn + 10, 0, 0);
+    return;
+  }
   uint8_t* sR0 = smem;                      // resident: K (key-major) or Q
   uint8_t* sR1 = smem + kTile;              // resident: V (key-major) or dO
-  uint8_t* sS0 = smem + 2 * kTile;          // ring of streamed tiles: Q or K
-  uint8_t* sS1 = sS0 + kRing * kTile;       //                          dO or V
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sS1 + kRing * kTile);
-  uint64_t* res_full = bars;
-  uint64_t* ring_full = bars + 1;           // [kRing]
-  uint64_t* ring_empty = bars + 3;          // [kRing]
-  uint64_t* s_full = bars + 5;              // [2] (key-major uses [0] only)
-  uint64_t* dp_full = bars + 7;
-  uint64_t* p_ready = bars + 8;             // key-major: P^T is in TMEM
-  uint64_t* ds_ready = bars + 9;            // dS is in TMEM
-  uint64_t* acc_done = bars + 10;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 11);
+  // Streamed tiles, a ring each.  Q / K is read by the first and the last product of a block, dO (key-major) by the
+  // second and third, V (query-major) by the second alone: four tiles are 2 + 2 stages or 3 + 1.
+  constexpr uint32_t kRing0 = kKeyMajor ? 2 : 3, kRing1 = kKeyMajor ? 2 : 1;
+  uint8_t* sS0 = smem + 2 * kTile;          // Q or K
+  uint8_t* sS1 = sS0 + kRing0 * kTile;      // dO or V
+  uint8_t* sO = smem + 6 * kTile;           // output staging
+  float* sStat = reinterpret_cast<float*>(sO + kBwdWarps * kBwdStage);   // key-major: [2][lse2 | delta][128], with dO
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sO + kBwdWarps * kBwdStage + 2 * kStatBytes);
+  uint8_t* clc_resp = reinterpret_cast<uint8_t*>(bars);   // 16 bytes
+  uint64_t* clc_full = bars + 2;
+  uint64_t* clc_empty = bars + 3;
+  uint64_t* res_full = bars + 4;
+  uint64_t* res_empty = bars + 5;
+  uint64_t* full0 = bars + 6;               // [3] rings
+  uint64_t* empty0 = bars + 9;              // [3]
+  uint64_t* full1 = bars + 12;              // [2]
+  uint64_t* empty1 = bars + 14;             // [2]
+  uint64_t* s_full = bars + 16;             // [2] (key-major uses [0] only)
+  uint64_t* dp_full = bars + 18;
+  uint64_t* p_ready = bars + 19;            // [2] key-major: the first / second 16 columns of every warp's P^T
+  uint64_t* ds_ready = bars + 21;           // dS is in TMEM
+  uint64_t* acc_done = bars + 22;           // [2] key-major: dV / dK; query-major: [1] dQ
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 24);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nblk = a.seq / kBlk;
-  // same block order as the forward kernel: per group of batch-heads the longest tiles first (key block 0 / the
-  // last query block stream the most)
-  const int blk = kKeyMajor ? (int)blockIdx.y : (a.causal ? nblk - 1 - (int)blockIdx.y : (int)blockIdx.y);
-  const int bh = blockIdx.z * gridDim.x + blockIdx.x;
-  const int h = bh % a.heads, b = bh / a.heads;
-  // streamed blocks: queries i0 .. nblk-1 for a key block, keys 0 .. blk for a query block
-  const int i0 = kKeyMajor && a.causal ? blk : 0;
-  const int n_it = kKeyMajor ? nblk - i0 : (a.causal ? blk + 1 : nblk);
-  const int colq = h * 3 * kD;
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+  const int group = gridDim.x;
   const uint64_t tmo = a.timeout_ns;
 
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tm_qkv);
     tma_prefetch_desc(&tm_do);
+    mbar_init(clc_full, 1);
+    mbar_init(clc_empty, 2 + kBwdWarps);    // producer and MMA thread, element-wise warps
     mbar_init(res_full, 1);
-    for (int i = 0; i < kRing; ++i) {
-      mbar_init(ring_full + i, 1);
-      mbar_init(ring_empty + i, 1);
+    mbar_init(res_empty, 1);
+    for (int i = 0; i < 3; ++i) {
+      mbar_init(full0 + i, 1);
+      mbar_init(empty0 + i, 1);
+    }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(full1 + i, 1);
+      mbar_init(empty1 + i, 1);
     }
     mbar_init(s_full, 1);
     mbar_init(s_full + 1, 1);
     mbar_init(dp_full, 1);
-    mbar_init(p_ready, 256);
-    mbar_init(ds_ready, 256);
+    mbar_init(p_ready, kBwdWarps);
+    mbar_init(p_ready + 1, kBwdWarps);
+    mbar_init(ds_ready, kBwdWarps);
     mbar_init(acc_done, 1);
+    mbar_init(acc_done + 1, 1);
     mbar_fence_init();
   }
   if (warp == 1) {
@@ -698,274 +790,283 @@ attn_bwd2_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_consta
   const uint32_t t_dp = tmem + (kKeyMajor ? 128 : 256);
   const uint32_t t_acc0 = tmem + (kKeyMajor ? 256 : 384), t_acc1 = tmem + 384;
 
+  BwdItem w = bwd_item<kKeyMajor>(a, blockIdx.x, blockIdx.y, blockIdx.z, group);
+  // The next item as the producer got it: false when there is none (or on a timeout).
+  uint32_t items = 0;                       // items finished by this thread
+  auto next_item = [&]() -> bool {
+    uint32_t x, y, z;
+    if (!mbar_wait(clc_full, items & 1, 8 * tmo)) {
+      report(a.status, kErrAttn + 18, items, 0);
+      return false;
+    }
+    ++items;
+    const bool more = clc_read(clc_resp, x, y, z);
+    fence_proxy_async_smem();               // this read before the next response overwrites it
+    if (more) w = bwd_item<kKeyMajor>(a, x, y, z, group);
+    return more;
+  };
+  uint32_t g = 0;                           // streamed blocks so far: stages and phases of the rings and the hand-overs
+
   if (warp == 0) {
-    if (lane == 0) {
-      const int rrow = b * a.seq + blk * kBlk;
-      mbar_expect_tx(res_full, 2 * kTile);
-      if (kKeyMajor) {
-        load_tile(sR0, &tm_qkv, res_full, colq + kD, rrow);        // K
-        load_tile(sR1, &tm_qkv, res_full, colq + 2 * kD, rrow);    // V
-      } else {
-        load_tile(sR0, &tm_qkv, res_full, colq, rrow);             // Q
-        load_tile(sR1, &tm_do, res_full, h * kD, rrow);            // dO
-      }
-      for (int it = 0; it < n_it; ++it) {
-        const int st = it & 1;
-        if (!mbar_wait(ring_empty + st, ((it >> 1) & 1) ^ 1, 6 * tmo)) {
-          report(a.status, kErrAttn + 11, it, 0);
-          break;
+    if (elect_one()) {
+      bool ok = true, more = true;
+      while (ok && more) {
+        const int colq = w.h * 3 * kD, seq0 = w.b * a.seq, rrow = seq0 + w.blk * kBlk;
+        const int64_t stat0 = ((int64_t)w.b * a.heads + w.h) * a.seq;
+        if ((ok = mbar_wait(res_empty, (items & 1) ^ 1, 8 * tmo))) {
+          mbar_expect_tx(res_full, 2 * kTile);
+          if (kKeyMajor) {
+            load_tile(sR0, &tm_qkv, res_full, colq + kD, rrow);        // K
+            load_tile(sR1, &tm_qkv, res_full, colq + 2 * kD, rrow);    // V
+          } else {
+            load_tile(sR0, &tm_qkv, res_full, colq, rrow);             // Q
+            load_tile(sR1, &tm_do, res_full, w.h * kD, rrow);          // dO
+          }
         }
-        const int srow = b * a.seq + (i0 + it) * kBlk;
-        mbar_expect_tx(ring_full + st, 2 * kTile);
-        if (kKeyMajor) {
-          load_tile(sS0 + st * kTile, &tm_qkv, ring_full + st, colq, srow);            // Q
-          load_tile(sS1 + st * kTile, &tm_do, ring_full + st, h * kD, srow);           // dO
-        } else {
-          load_tile(sS0 + st * kTile, &tm_qkv, ring_full + st, colq + kD, srow);       // K
-          load_tile(sS1 + st * kTile, &tm_qkv, ring_full + st, colq + 2 * kD, srow);   // V
+        for (int it = 0; it < w.n_it && ok; ++it, ++g) {
+          const uint32_t st0 = g % kRing0, st1 = g % kRing1;
+          const int srow = (w.i0 + it) * kBlk;
+          if (!(ok = mbar_wait(empty0 + st0, ((g / kRing0) & 1) ^ 1, 8 * tmo))) break;
+          mbar_expect_tx(full0 + st0, kTile);
+          load_tile(sS0 + st0 * kTile, &tm_qkv, full0 + st0, kKeyMajor ? colq : colq + kD, seq0 + srow);   // Q or K
+          if (!(ok = mbar_wait(empty1 + st1, ((g / kRing1) & 1) ^ 1, 8 * tmo))) break;
+          mbar_expect_tx(full1 + st1, kTile + (kKeyMajor ? kStatBytes : 0));
+          if (kKeyMajor) {
+            load_tile(sS1 + st1 * kTile, &tm_do, full1 + st1, w.h * kD, seq0 + srow);                      // dO
+            bulk_g2s(sStat + st1 * 2 * kBlk, a.lse2 + stat0 + srow, kBlk * 4, full1 + st1);
+            bulk_g2s(sStat + st1 * 2 * kBlk + kBlk, a.delta + stat0 + srow, kBlk * 4, full1 + st1);
+          } else {
+            load_tile(sS1 + st1 * kTile, &tm_qkv, full1 + st1, colq + 2 * kD, seq0 + srow);                // V
+          }
         }
+        if (ok && (ok = mbar_wait(clc_empty, (items & 1) ^ 1, 8 * tmo))) {
+          mbar_expect_tx(clc_full, 16);
+          clc_try_cancel(clc_resp, clc_full);
+          more = next_item();
+          mbar_arrive(clc_empty);
+        }
+        if (!ok) report(a.status, kErrAttn + 11, w.blk, g);
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t id_s = make_idesc_bf16(128, 128, 0, 0);      // A K-major (smem) * B K-major
       const uint32_t id_g = make_idesc_bf16(128, 128, 0, 1);      // A (TMEM) * B MN-major
-      // all operand descriptors, once: resident tiles; ring stage 0 (stage 1 = + kTile >> 4 in the
-      // start-address field)
-      uint64_t dr0[8], dr1[8], ds0k[8], ds1k[8], ds0m[8], ds1m[8];
-      {
-        const uint32_t r0 = smem_u32(sR0), r1 = smem_u32(sR1), b0 = smem_u32(sS0), b1 = smem_u32(sS1);
+      // descriptors of the first k-step of each operand; the others are these plus constants
+      const uint64_t dr0 = desc_kmajor(smem_u32(sR0), 0), dr1 = desc_kmajor(smem_u32(sR1), 0);
+      const uint64_t ds0k = desc_kmajor(smem_u32(sS0), 0), ds1k = desc_kmajor(smem_u32(sS1), 0);
+      const uint64_t ds0m = desc_mnmajor(smem_u32(sS0), 0), ds1m = desc_mnmajor(smem_u32(sS1), 0);
+      constexpr uint64_t kStageOff = (uint64_t)(kTile >> 4);
+      bool ok = true, more = true;
+      auto wait = [&](uint64_t* bar, uint32_t parity, uint32_t code) -> bool {
+        if (mbar_wait(bar, parity, 8 * tmo)) {
+          tc_fence_after_sync();
+          return true;
+        }
+        report(a.status, kErrAttn + code, g, items);
+        return false;
+      };
+      // S (or S^T) / dP (or dP^T) of streamed block number q, once its tile is there
+      auto issue_s = [&](uint32_t q) -> bool {
+        const uint32_t st = q % kRing0;
+        if (!wait(full0 + st, (q / kRing0) & 1, 13)) return false;
+        const uint64_t tile = ds0k + st * kStageOff;
+        const int buf = kKeyMajor ? 0 : (q & 1);
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
-          dr0[k] = desc_kmajor(r0, k);
-          dr1[k] = desc_kmajor(r1, k);
-          ds0k[k] = desc_kmajor(b0, k);
-          ds1k[k] = desc_kmajor(b1, k);
-          ds0m[k] = desc_mnmajor(b0, k);
-          ds1m[k] = desc_mnmajor(b1, k);
+          const uint64_t off = (uint64_t)(((k >> 2) * kHalf + (k & 3) * 32) >> 4);
+          umma_f16(tmem + buf * 128, dr0 + off, tile + off, id_s, k != 0);
         }
-      }
-      constexpr uint64_t kStageOff = (uint64_t)(kTile >> 4);
-      bool ok = mbar_wait(res_full, 0, 2 * tmo);
-      if (!ok) report(a.status, kErrAttn + 12, 0, 0);
-      auto wait_ring = [&](int it) -> bool {
-        if (mbar_wait(ring_full + (it & 1), (it >> 1) & 1, 4 * tmo)) {
-          tc_fence_after_sync();
-          return true;
-        }
-        report(a.status, kErrAttn + 13, it, 0);
-        return false;
-      };
-      auto wait_ew = [&](uint64_t* bar, int it, uint32_t code) -> bool {
-        if (mbar_wait(bar, it & 1, 8 * tmo)) {
-          tc_fence_after_sync();
-          return true;
-        }
-        report(a.status, code, it, 0);
-        return false;
-      };
-      // S (or S^T) of block `it` into score buffer `buf`; dP (or dP^T) of block `it`
-      auto issue_s = [&](int it, int buf) {
-        const uint64_t so = (it & 1) ? kStageOff : 0;
-#pragma unroll
-        for (int k = 0; k < 8; ++k) umma_f16(tmem + buf * 128, dr0[k], ds0k[k] + so, id_s, k != 0);
         umma_commit(s_full + buf);
+        return true;
       };
-      auto issue_dp = [&](int it) {
-        const uint64_t so = (it & 1) ? kStageOff : 0;
+      auto issue_dp = [&](uint32_t q) -> bool {
+        const uint32_t st = q % kRing1;
+        if (!wait(full1 + st, (q / kRing1) & 1, 13)) return false;
+        const uint64_t tile = ds1k + st * kStageOff;
 #pragma unroll
-        for (int k = 0; k < 8; ++k) umma_f16(t_dp, dr1[k], ds1k[k] + so, id_s, k != 0);
+        for (int k = 0; k < 8; ++k) {
+          const uint64_t off = (uint64_t)(((k >> 2) * kHalf + (k & 3) * 32) >> 4);
+          umma_f16(t_dp, dr1 + off, tile + off, id_s, k != 0);
+        }
         umma_commit(dp_full);
+        if (!kKeyMajor) umma_commit(empty1 + st);         // V has no other reader
+        return true;
       };
-      if (ok && n_it > 0) {
-        ok = wait_ring(0);
+      // acc += (P or dS in TMEM at `src`: a warp's columns packed from its first column) * streamed tile; the k-steps
+      // of the first / second 16 columns of every warp
+      auto issue_grad = [&](uint32_t acc, uint32_t src, uint64_t tile, int part, bool first) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          umma_f16_ts(acc, src + i * kBwdCols + part * 8, tile + (uint64_t)(((2 * i + part) * 2048) >> 4), id_g,
+                      !(first && i == 0));
+      };
+      while (ok && more) {
+        const int n = w.n_it;
+        if (!(ok = wait(res_full, items & 1, 12) && issue_s(g) && issue_dp(g))) break;
+        if (n == 1) umma_commit(res_empty);
+        for (int it = 0; it < n && ok; ++it, ++g) {
+          const bool next = it + 1 < n;
+          const uint32_t st0 = g % kRing0, st1 = g % kRing1;
+          if (kKeyMajor) {
+            // dV += P^T dO (contraction over the queries)
+            if (!(ok = wait(p_ready, g & 1, 14))) break;
+            issue_grad(t_acc0, tmem, ds1m + st1 * kStageOff, 0, it == 0);
+            if (!(ok = wait(p_ready + 1, g & 1, 14))) break;
+            issue_grad(t_acc0, tmem, ds1m + st1 * kStageOff, 1, false);
+            umma_commit(empty1 + st1);
+            if (!next) umma_commit(acc_done);
+          }
+          // key-major: P^T(it) is read by the products just issued; query-major: the other S buffer
+          if (next && !(ok = issue_s(g + 1))) break;
+          if (!(ok = wait(ds_ready, g & 1, 14))) break;
+          issue_grad(kKeyMajor ? t_acc1 : t_acc0, t_dp, ds0m + st0 * kStageOff, 0, it == 0);   // dK += dS^T Q / dQ += dS K
+          issue_grad(kKeyMajor ? t_acc1 : t_acc0, t_dp, ds0m + st0 * kStageOff, 1, false);
+          umma_commit(empty0 + st0);
+          if (!next) umma_commit(acc_done + 1);
+          if (next && !(ok = issue_dp(g + 1))) break;
+          if (it + 2 == n) umma_commit(res_empty);
+        }
         if (ok) {
-          issue_s(0, 0);
-          issue_dp(0);
+          more = next_item();
+          mbar_arrive(clc_empty);
         }
       }
-      for (int it = 0; it < n_it && ok; ++it) {
-        const uint64_t so = (it & 1) ? kStageOff : 0;
-        const bool more = it + 1 < n_it;
-        if (kKeyMajor) {
-          if (!(ok = wait_ew(p_ready, it, kErrAttn + 14))) break;
-#pragma unroll
-          for (int k = 0; k < 8; ++k)   // dV += P^T dO   (contraction over the 128 queries)
-            umma_f16_ts(t_acc0, tmem + (k >> 2) * 64 + (k & 3) * 8, ds1m[k] + so, id_g, (it | k) != 0);
-          if (more) {
-            if (!(ok = wait_ring(it + 1))) break;
-            issue_s(it + 1, 0);         // S^T region: P^T(it) was read by the products just issued
-          }
-          if (!(ok = wait_ew(ds_ready, it, kErrAttn + 14))) break;
-#pragma unroll
-          for (int k = 0; k < 8; ++k)   // dK += dS^T Q
-            umma_f16_ts(t_acc1, t_dp + (k >> 2) * 64 + (k & 3) * 8, ds0m[k] + so, id_g, (it | k) != 0);
-          umma_commit(ring_empty + (it & 1));
-          if (more) issue_dp(it + 1);
-        } else {
-          if (more) {
-            if (!(ok = wait_ring(it + 1))) break;
-            issue_s(it + 1, (it + 1) & 1);
-          }
-          if (!(ok = wait_ew(ds_ready, it, kErrAttn + 14))) break;
-#pragma unroll
-          for (int k = 0; k < 8; ++k)   // dQ += dS K     (contraction over the 128 keys)
-            umma_f16_ts(t_acc0, t_dp + (k >> 2) * 64 + (k & 3) * 8, ds0m[k] + so, id_g, (it | k) != 0);
-          umma_commit(ring_empty + (it & 1));
-          if (more) issue_dp(it + 1);
-        }
-      }
-      if (ok) umma_commit(acc_done);
     }
   } else {
     const int q4 = warp & 3;
-    const int half = (warp - 2) >> 2;                     // which 64 of the 128 columns
+    const int part = (warp - 2) >> 2;                     // which kBwdCols of the 128 columns
     const int row = q4 * 32 + lane;                       // TMEM lane: key (key-major) or query
     const uint32_t lane_off = static_cast<uint32_t>(q4 * 32) << 16;
-    const float sl2 = a.scale * kLog2e;
-    const int64_t stat0 = ((int64_t)b * a.heads + h) * a.seq;
-    float my_lse2 = 0.f, my_delta = 0.f;
-    if (!kKeyMajor) {
-      my_lse2 = a.lse2[stat0 + blk * kBlk + row];
-      my_delta = a.delta[stat0 + blk * kBlk + row];
-    }
-    const int me = blk * kBlk + row;                      // this lane's key (key-major) or query index
-    bool ok = true;
-    for (int it = 0; it < n_it; ++it) {
-      const int sb = kKeyMajor ? 0 : (it & 1);
-      const uint32_t ts = tmem + lane_off + sb * 128 + half * 64;
-      const uint32_t tdp = t_dp + lane_off + half * 64;
-      const int c0 = (i0 + it) * kBlk + half * 64;        // first streamed index of this thread's columns
-      // causal: a score survives when key <= query; only blocks that touch the diagonal pay for it
-      const bool masked = a.causal && (kKeyMajor ? (c0 < me) : (c0 + 63 > me));
-      uint32_t pk[32];                                    // P of this thread's 64 columns, packed bf16
-      // ---- phase 1: P = exp2(S * scale * log2(e) - lse2) ----
-      if (!warp_wait(s_full + sb, kKeyMajor ? (it & 1) : ((it >> 1) & 1), 8 * tmo)) {
-        if (lane == 0) report(a.status, kErrAttn + 15, it, 0);
-        ok = false;
-        break;
+    const uint32_t tdp = t_dp + lane_off + part * kBwdCols;
+    const uint64_t sl2 = f32x2(a.scale * kLog2e, a.scale * kLog2e), sc2 = f32x2(a.scale, a.scale);
+    uint8_t* stage = sO + (warp - 2) * kBwdStage;
+    bool ok = true, more = true;
+    while (more) {
+      const int me = w.blk * kBlk + row;                  // this lane's key (key-major) or query index
+      uint64_t my_lse2 = 0, my_delta = 0;
+      if (!kKeyMajor) {
+        const int64_t at = ((int64_t)w.b * a.heads + w.h) * a.seq + me;
+        my_lse2 = f32x2(a.lse2[at], a.lse2[at]);
+        my_delta = f32x2(a.delta[at], a.delta[at]);
       }
-      tc_fence_after_sync();
-#pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        uint32_t rs[32];
-        tmem_ld_32x32(ts + c * 32, rs);
-        float ls[32];
-        if (kKeyMajor) {   // one address per warp: broadcast loads of 16 bytes
-          const float4* lp = reinterpret_cast<const float4*>(a.lse2 + stat0 + c0 + c * 32);
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const float4 x = __ldg(lp + i);
-            ls[4 * i] = x.x; ls[4 * i + 1] = x.y; ls[4 * i + 2] = x.z; ls[4 * i + 3] = x.w;
-          }
+      for (int it = 0; it < w.n_it; ++it, ++g) {
+        const int sb = kKeyMajor ? 0 : (g & 1);
+        const uint32_t ts = tmem + lane_off + sb * 128 + part * kBwdCols;
+        const int c0 = (w.i0 + it) * kBlk + part * kBwdCols;   // first streamed index of this thread's columns
+        const ulonglong2* stat = reinterpret_cast<const ulonglong2*>(sStat + (g & 1) * 2 * kBlk + part * kBwdCols);
+        // causal: a score survives when key <= query; only blocks that touch the diagonal pay for it
+        const bool masked = a.causal && (kKeyMajor ? (c0 < me) : (c0 + kBwdCols - 1 > me));
+        float e[kBwdCols];                                // P of this thread's columns
+        // ---- phase 1: P = exp2(S * scale * log2(e) - lse2) ----
+        // (key-major: the statistics come with dO, whose barrier orders them for this thread)
+        if (!warp_wait(s_full + sb, kKeyMajor ? (g & 1) : ((g >> 1) & 1), 8 * tmo) ||
+            (kKeyMajor && !warp_wait(full1 + (g & 1), (g >> 1) & 1, 8 * tmo))) {
+          if (lane == 0) report(a.status, kErrAttn + 15, it, 0);
+          ok = false;
+          break;
         }
-        tmem_ld_wait();
-        if (!masked) {
-#pragma unroll
-          for (int i = 0; i < 32; i += 2) {
-            const float e0 = fast_exp2(fmaf(__uint_as_float(rs[i]), sl2, -(kKeyMajor ? ls[i] : my_lse2)));
-            const float e1 = fast_exp2(fmaf(__uint_as_float(rs[i + 1]), sl2, -(kKeyMajor ? ls[i + 1] : my_lse2)));
-            pk[c * 16 + (i >> 1)] = pack_bf16(e0, e1);
-          }
-        } else {
-#pragma unroll
-          for (int i = 0; i < 32; i += 2) {
-            float e0 = fast_exp2(fmaf(__uint_as_float(rs[i]), sl2, -(kKeyMajor ? ls[i] : my_lse2)));
-            float e1 = fast_exp2(fmaf(__uint_as_float(rs[i + 1]), sl2, -(kKeyMajor ? ls[i + 1] : my_lse2)));
-            const int q0 = c0 + c * 32 + i;
-            if (!(kKeyMajor ? (me <= q0) : (q0 <= me))) e0 = 0.f;
-            if (!(kKeyMajor ? (me <= q0 + 1) : (q0 + 1 <= me))) e1 = 0.f;
-            pk[c * 16 + (i >> 1)] = pack_bf16(e0, e1);
-          }
-        }
-      }
-      if (kKeyMajor) {
-        // P^T over this thread's own S^T columns: 64 bf16 = 32 TMEM columns from the half's first column
-        uint32_t lo[16], hi[16];
-#pragma unroll
-        for (int i = 0; i < 16; ++i) { lo[i] = pk[i]; hi[i] = pk[16 + i]; }
-        tmem_st_32x16(ts, lo);
-        tmem_st_32x16(ts + 16, hi);
-        tmem_st_wait();
-        tc_fence_before_sync();
-        mbar_arrive(p_ready);
-      }
-      // ---- phase 2: dS = P * (dP * scale - delta * scale) ----
-      if (!warp_wait(dp_full, it & 1, 8 * tmo)) {
-        if (lane == 0) report(a.status, kErrAttn + 16, it, 0);
-        ok = false;
-        break;
-      }
-      tc_fence_after_sync();
-      uint32_t dk[32];
-#pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        uint32_t rp[32];
-        tmem_ld_32x32(tdp + c * 32, rp);
-        float dl[32];
-        if (kKeyMajor) {
-          const float4* dp = reinterpret_cast<const float4*>(a.delta + stat0 + c0 + c * 32);
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const float4 y = __ldg(dp + i);
-            dl[4 * i] = y.x; dl[4 * i + 1] = y.y; dl[4 * i + 2] = y.z; dl[4 * i + 3] = y.w;
-          }
-        }
-        tmem_ld_wait();
-#pragma unroll
-        for (int i = 0; i < 32; i += 2) {
-          const uint32_t pp = pk[c * 16 + (i >> 1)];
-          const float e0 = __uint_as_float(pp << 16), e1 = __uint_as_float(pp & 0xffff0000u);
-          const float g0 = e0 * fmaf(__uint_as_float(rp[i]), a.scale, -(kKeyMajor ? dl[i] : my_delta));
-          const float g1 = e1 * fmaf(__uint_as_float(rp[i + 1]), a.scale, -(kKeyMajor ? dl[i + 1] : my_delta));
-          dk[c * 16 + (i >> 1)] = pack_bf16(g0, g1);
-        }
-      }
-      {
-        uint32_t lo[16], hi[16];
-#pragma unroll
-        for (int i = 0; i < 16; ++i) { lo[i] = dk[i]; hi[i] = dk[16 + i]; }
-        tmem_st_32x16(tdp, lo);       // dS over this thread's own dP columns
-        tmem_st_32x16(tdp + 16, hi);
-        tmem_st_wait();
-        tc_fence_before_sync();
-        mbar_arrive(ds_ready);
-      }
-    }
-    if (ok) {
-      if (!warp_wait(acc_done, 0, 8 * tmo)) {
-        if (lane == 0) report(a.status, kErrAttn + 17, 0, 0);
-        ok = false;
-      }
-    }
-    if (ok) {
-      tc_fence_after_sync();
-      // accumulators -> bf16 rows of dqkv; the two threads of a lane take 64 columns each
-      __nv_bfloat16* base = reinterpret_cast<__nv_bfloat16*>(a.dqkv) +
-                            ((int64_t)b * a.seq + blk * kBlk + row) * (a.heads * 3 * kD) + colq;
-      const int n_acc = kKeyMajor ? 2 : 1;
-#pragma unroll 1
-      for (int which = 0; which < n_acc; ++which) {
-        // key-major: acc0 = dV, acc1 = dK;  query-major: acc0 = dQ
-        const uint32_t t = (which == 0 ? t_acc0 : t_acc1) + lane_off + half * 64;
-        __nv_bfloat16* dst = base + (kKeyMajor ? (which == 0 ? 2 * kD : kD) : 0) + half * 64;
-#pragma unroll 1
-        for (int c = 0; c < 2; ++c) {
-          uint32_t r[32];
-          tmem_ld_32x32(t + c * 32, r);
+        tc_fence_after_sync();
+        {
+          uint32_t rs[kBwdCols];
+          tmem_ld_32x32(ts, rs);
           tmem_ld_wait();
 #pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            uint4 v;
-            v.x = pack_bf16(__uint_as_float(r[q * 8 + 0]), __uint_as_float(r[q * 8 + 1]));
-            v.y = pack_bf16(__uint_as_float(r[q * 8 + 2]), __uint_as_float(r[q * 8 + 3]));
-            v.z = pack_bf16(__uint_as_float(r[q * 8 + 4]), __uint_as_float(r[q * 8 + 5]));
-            v.w = pack_bf16(__uint_as_float(r[q * 8 + 6]), __uint_as_float(r[q * 8 + 7]));
-            *reinterpret_cast<uint4*>(dst + c * 32 + q * 8) = v;
+          for (int hp = 0; hp < 2; ++hp) {
+#pragma unroll
+            for (int k = hp * 16; k < hp * 16 + 16; k += 4) {
+              ulonglong2 st = make_ulonglong2(my_lse2, my_lse2);
+              if (kKeyMajor) st = stat[k >> 2];
+              split(fma2(f32x2(__uint_as_float(rs[k]), __uint_as_float(rs[k + 1])), sl2, st.x), e[k], e[k + 1]);
+              split(fma2(f32x2(__uint_as_float(rs[k + 2]), __uint_as_float(rs[k + 3])), sl2, st.y), e[k + 2], e[k + 3]);
+#pragma unroll
+              for (int u = 0; u < 4; ++u) e[k + u] = fast_exp2(e[k + u]);
+            }
+            if (masked) {
+#pragma unroll
+              for (int k = hp * 16; k < hp * 16 + 16; ++k)
+                if (!(kKeyMajor ? (me <= c0 + k) : (c0 + k <= me))) e[k] = 0.f;
+            }
+            if (kKeyMajor) {
+              // P^T over this thread's own S^T columns, packed from the first: the products that read the first 16
+              // run under the exponentials of the second
+              uint32_t pk[8];
+#pragma unroll
+              for (int i = 0; i < 8; ++i) pk[i] = pack_bf16(e[hp * 16 + 2 * i], e[hp * 16 + 2 * i + 1]);
+              tmem_st_32x8(ts + hp * 8, pk);
+              tmem_st_wait();
+              tc_fence_before_sync();
+              __syncwarp();
+              if (lane == 0) mbar_arrive(p_ready + hp);
+            }
           }
         }
+        // ---- phase 2: dS = P * (dP * scale - delta * scale) ----
+        if (!warp_wait(dp_full, g & 1, 8 * tmo)) {
+          if (lane == 0) report(a.status, kErrAttn + 16, it, 0);
+          ok = false;
+          break;
+        }
+        tc_fence_after_sync();
+        {
+          uint32_t rp[kBwdCols], dk[16];
+          tmem_ld_32x32(tdp, rp);
+          tmem_ld_wait();
+#pragma unroll
+          for (int k = 0; k < kBwdCols; k += 4) {
+            ulonglong2 st = make_ulonglong2(my_delta, my_delta);
+            if (kKeyMajor) st = stat[kBlk / 4 + (k >> 2)];
+            float g0, g1;
+            split(mul2(f32x2(e[k], e[k + 1]),
+                       fma2(f32x2(__uint_as_float(rp[k]), __uint_as_float(rp[k + 1])), sc2, st.x)), g0, g1);
+            dk[k >> 1] = pack_bf16(g0, g1);
+            split(mul2(f32x2(e[k + 2], e[k + 3]),
+                       fma2(f32x2(__uint_as_float(rp[k + 2]), __uint_as_float(rp[k + 3])), sc2, st.y)), g0, g1);
+            dk[(k >> 1) + 1] = pack_bf16(g0, g1);
+          }
+          tmem_st_32x16(tdp, dk);               // dS over this thread's own dP columns
+          tmem_st_wait();
+          tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(ds_ready);
+        }
       }
+      if (!ok) break;
+      // Accumulators -> bf16 rows of dqkv: a warp's 32 rows x kBwdCols columns leave through shared memory as a TMA store
+      // (with plain stores the warps stall for 4000 cycles when all SMs write their items at the same time).
+      const int col = w.h * 3 * kD + part * kBwdCols, orow = w.b * a.seq + w.blk * kBlk + q4 * 32;
+      const uint32_t phase = items & 1;
+      more = next_item();                        // w is the next item's from here on
+#pragma unroll 1
+      for (int which = kKeyMajor ? 0 : 1; which < 2; ++which) {
+        if (!warp_wait(acc_done + which, phase, 8 * tmo)) {
+          if (lane == 0) report(a.status, kErrAttn + 17, which, 0);
+          ok = false;
+          break;
+        }
+        tc_fence_after_sync();
+        // key-major: acc0 = dV, acc1 = dK;  query-major: acc0 = dQ
+        uint32_t r[kBwdCols];
+        tmem_ld_32x32((kKeyMajor && which ? t_acc1 : t_acc0) + lane_off + part * kBwdCols, r);
+        warp_stage_free();
+        tmem_ld_wait();
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          uint4 v;
+          v.x = pack_bf16(__uint_as_float(r[q * 8 + 0]), __uint_as_float(r[q * 8 + 1]));
+          v.y = pack_bf16(__uint_as_float(r[q * 8 + 2]), __uint_as_float(r[q * 8 + 3]));
+          v.z = pack_bf16(__uint_as_float(r[q * 8 + 4]), __uint_as_float(r[q * 8 + 5]));
+          v.w = pack_bf16(__uint_as_float(r[q * 8 + 6]), __uint_as_float(r[q * 8 + 7]));
+          *reinterpret_cast<uint4*>(stage + lane * 64 + ((q ^ (lane >> 1 & 3)) << 4)) = v;   // 64-byte swizzle
+        }
+        warp_store_box(&tm_dqkv, stage, col + (kKeyMajor ? (which == 0 ? 2 * kD : kD) : 0), orow);
+      }
+      if (!ok) break;
+      tc_fence_before_sync();                    // the accumulators are read before the next P / dS is announced
+      __syncwarp();                              // every lane has read the response
+      if (lane == 0) mbar_arrive(clc_empty);
     }
+    if (lane == 0) bulk_wait_all<0>();
   }
   tc_fence_before_sync();
   __syncthreads();
@@ -1021,8 +1122,10 @@ cudaError_t attention_fwd(const void* qkv, void* out, float* lse, int batch, int
   const uint64_t width = (uint64_t)heads * 3 * kD;
   if (make_tensor_map_2d(&tm, qkv, width, (uint64_t)batch * seq, width * 2, 64, kBlk) != 0)
     return cudaErrorInvalidValue;
+  CUtensorMap to;
+  const uint64_t wout = (uint64_t)heads * kD;
+  if (make_tensor_map_2d(&to, out, wout, (uint64_t)batch * seq, wout * 2, 64, 32) != 0) return cudaErrorInvalidValue;
   AttnArgs a{};
-  a.out = out;
   a.lse = lse;
   a.batch = batch; a.seq = seq; a.heads = heads; a.causal = causal;
   a.scale = scale;
@@ -1034,7 +1137,7 @@ cudaError_t attention_fwd(const void* qkv, void* out, float* lse, int batch, int
   // K and V and overlap (batch 3 x 640, 5 heads, 75 tiles: 16.5 us either way; 16 heads x 8192: see the kernel).
   a.tiles_per_item = (int64_t)batch * heads * nblk <= sm_count() ? 1 : 2;
   dim3 grid(grp, (nblk + a.tiles_per_item - 1) / a.tiles_per_item, batch * heads / grp);
-  attn_fwd2_kernel<<<grid, kFwd2Threads, kFwd2Smem, stream>>>(tm, a);
+  attn_fwd2_kernel<<<grid, kFwd2Threads, kFwd2Smem, stream>>>(tm, to, a);
   return cudaGetLastError();
 }
 
@@ -1049,13 +1152,13 @@ cudaError_t attention_bwd(const void* qkv, const void* out, const void* dout, co
   }
   const int64_t tokens = (int64_t)batch * seq;
   {
-    // delta * scale into `delta`, lse * log2(e) into the head of the `dq_acc` scratch
-    const int64_t warps = tokens * heads;
-    const int threads = 256;
-    const int64_t blocks = (warps * 32 + threads - 1) / threads;
-    attn_delta_kernel<<<(unsigned)blocks, threads, 0, stream>>>(
-        reinterpret_cast<const __nv_bfloat16*>(out), reinterpret_cast<const __nv_bfloat16*>(dout), delta, batch, seq, heads,
-        lse, dq_acc, scale);
+    // -delta * scale into `delta`, -lse * log2(e) into the head of the `dq_acc` scratch
+    const int64_t groups = tokens / kDeltaRows * heads;   // below 2^32: a group is 2 KiB of activations
+    const int threads = 256, per_block = threads / 16;
+    const int64_t blocks = (groups + per_block - 1) / per_block;
+    auto kernel = (reinterpret_cast<uintptr_t>(out) & 15) == 0 ? attn_delta_kernel<true> : attn_delta_kernel<false>;
+    kernel<<<(unsigned)blocks, threads, 0, stream>>>(reinterpret_cast<const uint4*>(out), reinterpret_cast<const uint4*>(dout),
+                                                     delta, (uint32_t)groups, seq, heads, lse, dq_acc, scale);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   }
@@ -1063,21 +1166,22 @@ cudaError_t attention_bwd(const void* qkv, const void* out, const void* dout, co
   const uint64_t width = (uint64_t)heads * 3 * kD, wdo = (uint64_t)heads * kD;
   if (make_tensor_map_2d(&tq, qkv, width, (uint64_t)tokens, width * 2, 64, kBlk) != 0) return cudaErrorInvalidValue;
   if (make_tensor_map_2d(&td, dout, wdo, (uint64_t)tokens, wdo * 2, 64, kBlk) != 0) return cudaErrorInvalidValue;
+  CUtensorMap tg;
+  if (make_tensor_map_2d(&tg, dqkv, width, (uint64_t)tokens, width * 2, kBwdCols, 32, 64) != 0) return cudaErrorInvalidValue;
   // two deterministic kernels: dK / dV per key block, dQ per query block
   Bwd2Args g{};
-  g.dqkv = dqkv;
-  g.lse2 = dq_acc;     // lse * log2(e)
-  g.delta = delta;     // delta * scale
+  g.lse2 = dq_acc;     // -lse * log2(e)
+  g.delta = delta;     // -delta * scale
   g.batch = batch; g.seq = seq; g.heads = heads; g.causal = causal;
   g.scale = scale;
   g.status = status;
   g.timeout_ns = 2000000000ull;
   const int grp = bh_group(batch, heads);
   dim3 grid2(grp, seq / kBlk, batch * heads / grp);
-  attn_bwd2_kernel<true><<<grid2, kBwd2Threads, kBwd2Smem, stream>>>(tq, td, g);
+  attn_bwd2_kernel<true><<<grid2, kBwd2Threads, kBwd2Smem, stream>>>(tq, td, tg, g);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  attn_bwd2_kernel<false><<<grid2, kBwd2Threads, kBwd2Smem, stream>>>(tq, td, g);
+  attn_bwd2_kernel<false><<<grid2, kBwd2Threads, kBwd2Smem, stream>>>(tq, td, tg, g);
   return cudaGetLastError();
 }
 

@@ -44,24 +44,41 @@ def test_attention_fwd_bwd(shape, causal):
 
 @pytest.mark.parametrize("causal", [False, True])
 @pytest.mark.parametrize("shape", [(5, 384, 61), (2, 1280, 40), (37, 128, 4), (149, 128, 1)])
-def test_attention_forward_items(shape, causal):
+def test_attention_items(shape, causal):
     """More items than SMs (running CTAs take the rest over), an odd number of tiles (an item of one tile), and the
-    two sides of the rule that gives a CTA one or two tiles.  P and the result are rounded to bf16 (2^-9 each, of
-    values that are averages of |v| <= 5.5): 0.022, and 1e-3 for the fp32 sums and exponentials."""
+    two sides of the rule that gives a forward CTA one or two tiles.  P and the result are rounded to bf16 (2^-9 each,
+    of values that are averages of |v| <= 5.5): 0.022, and 1e-3 for the fp32 sums and exponentials.  Gradients: three
+    such roundings (P or dS, an operand, the result) of random sign, 2^-9 / sqrt(3) each, and four times that."""
     from meshslice_b200 import _native
     from meshslice_b200.ops import functional as F
     batch, seq, heads = shape
     g = torch.Generator(device="cuda").manual_seed(batch)
     qkv = torch.randn(batch * seq, heads * 3 * 128, device="cuda", generator=g).bfloat16()
+    dout = torch.randn(batch * seq, heads * 128, device="cuda", generator=g).bfloat16()
     out, lse = F.attention_fwd(qkv, batch, seq, heads, causal)
+    dqkv = F.attention_bwd(dout, qkv, out, lse, batch, seq, heads, causal)
     _native.check_status()
-    q, k, v = (qkv.view(batch, seq, heads, 3, 128)[:, :, :, i].transpose(1, 2).float() for i in range(3))
-    s = q @ k.transpose(-1, -2) / math.sqrt(128)
-    if causal:
-        s.masked_fill_(torch.ones(seq, seq, dtype=torch.bool, device="cuda").triu(1), float("-inf"))
-    ref = (torch.softmax(s, -1) @ v).transpose(1, 2).reshape(batch * seq, heads * 128)
+    ref, lse_ref, dref = _ref(qkv, batch, seq, heads, causal, dout)
     assert (out.float() - ref).abs().max().item() < 0.023
-    assert (lse - torch.logsumexp(s, -1)).abs().max().item() < 0.02
+    assert (lse - lse_ref).abs().max().item() < 0.02
+    assert ((dqkv.float() - dref).norm() / dref.norm()).item() < 4 * 2 ** -9
+
+
+def test_attention_backward_takes_out_on_an_8_byte_boundary():
+    """`out` is only read with plain loads: a tensor that starts 8 bytes off gives the same gradient."""
+    from meshslice_b200 import _native
+    from meshslice_b200.ops import functional as F
+    batch, seq, heads = 2, 256, 3
+    g = torch.Generator(device="cuda").manual_seed(11)
+    qkv = torch.randn(batch * seq, heads * 3 * 128, device="cuda", generator=g).bfloat16()
+    dout = torch.randn(batch * seq, heads * 128, device="cuda", generator=g).bfloat16()
+    out, lse = F.attention_fwd(qkv, batch, seq, heads, True)
+    moved = torch.empty(out.numel() + 4, dtype=out.dtype, device="cuda")[4:].view_as(out).copy_(out)
+    assert moved.data_ptr() % 16 == 8
+    a = F.attention_bwd(dout, qkv, out, lse, batch, seq, heads, True)
+    b = F.attention_bwd(dout, qkv, moved, lse, batch, seq, heads, True)
+    _native.check_status()
+    assert torch.equal(a, b)
 
 
 def test_attention_large_scores_exercise_rescaling():
