@@ -55,8 +55,12 @@ def available() -> bool:
 
 
 def stream_ptr() -> int:
+    """Current stream of the current device (asked for before every launch: without the stream object that
+    torch.cuda.current_stream() builds, 0.4 us instead of 8)."""
     import torch
-    return torch.cuda.current_stream().cuda_stream
+    if not torch.cuda.is_initialized():
+        torch.cuda.init()
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 class _Status:

@@ -4,6 +4,8 @@
 #include <pybind11/pybind11.h>
 #include <pybind11/stl.h>
 
+#include <algorithm>
+#include <cstdlib>
 #include <cstring>
 #include <stdexcept>
 #include <string>
@@ -263,6 +265,68 @@ void gemm_run(const py::dict& d) {
   check(launch_sm100_gemm(ta, tb, pm, a, grid, S(getp(d, "stream"))), "sm100_gemm launch");
 }
 
+// The plain local GEMM of `ops.gemm`: the few values it needs, positionally.  Filling the dict of gemm_run and reading
+// it back took longer than a small product takes on the GPU (a linear layer of 512 x 512 x 1536, forward and backward:
+// 108 us a pass, 59 us through this call).  MSB_TWO_CTA, MSB_G2_STAGES, MSB_G2_GROUP and MSB_G2_MAP3D are read per call, as they were.
+void gemm_local(int64_t M, int64_t N, int64_t K, uint64_t A, int64_t lda, int a_mn_major, uint64_t B, int64_t ldb,
+                int b_mn_major, uint64_t C, int64_t ldc, int c_fp32, int accumulate, uint64_t bias, int act,
+                uint64_t C_pre, int two_cta, int sms, uint64_t status, uint64_t stream) {
+  const auto env = [](const char* name, int otherwise) {
+    const char* v = std::getenv(name);
+    return v != nullptr ? std::atoi(v) : otherwise;
+  };
+  GemmArgs a;
+  std::memset(&a, 0, sizeof(a));
+  if (M <= 0 || N <= 0 || K <= 0) throw std::runtime_error("gemm: empty problem");
+  if ((lda % 8) || (ldb % 8) || (A & 15) || (B & 15))
+    throw std::runtime_error("gemm: operands need 16-byte aligned bases and pitches");
+  if (ldc % 8) throw std::runtime_error("gemm: ldc must be a multiple of 8");
+  if (status == 0) throw std::runtime_error("gemm: status pointer required");
+  a.M = (int)M;
+  a.N = (int)N;
+  a.K = (int)K;
+  a.a_mn_major = a_mn_major;
+  a.b_mn_major = b_mn_major;
+  a.C = P<void>(C);
+  a.ldc = ldc;
+  a.c_fp32 = c_fp32;
+  a.accumulate = accumulate;
+  a.bias = P<void>(bias);
+  a.act = act;
+  a.C_pre = P<void>(C_pre);
+  a.tiles_m = (a.M + 2 * kBM - 1) / (2 * kBM);
+  a.tiles_n = (a.N + kBN - 1) / kBN;
+  a.n_slices = a.cyc = a.push_extent = a.push_bufs = a.b_nchunk = a.a_kpanel = a.b_kpanel = 1;
+  a.group = std::max(1, env("MSB_G2_GROUP", 8));
+  a.stages = env("MSB_G2_STAGES", 7);
+  a.status = P<uint32_t>(status);
+  a.timeout_ns = 1000000000ull;
+
+  CUtensorMap ta, tb;
+  int r;
+  const bool try3d = env("MSB_G2_MAP3D", 1) != 0;
+  if (!a_mn_major) r = make_tensor_map_2d(&ta, P<void>(A), a.K, a.M, lda * 2, kBK, kBM);
+  else if (try3d && make_tensor_map_mn3d(&ta, P<void>(A), a.M, a.K, lda * 2, kBM / 64) == 0) { r = 0; a.a_map3d = 1; }
+  else r = make_tensor_map_2d(&ta, P<void>(A), a.M, a.K, lda * 2, 64, kBK);
+  if (r != 0) throw std::runtime_error("gemm: tensor map for A failed, code " + std::to_string(r));
+  if (!b_mn_major) r = make_tensor_map_2d(&tb, P<void>(B), a.K, a.N, ldb * 2, kBK, kBN / 2);
+  else if (try3d && make_tensor_map_mn3d(&tb, P<void>(B), a.N, a.K, ldb * 2, kBN / 128) == 0) { r = 0; a.b_map3d = 1; }
+  else r = make_tensor_map_2d(&tb, P<void>(B), a.N, a.K, ldb * 2, 64, kBK);
+  if (r != 0) throw std::runtime_error("gemm: tensor map for B failed, code " + std::to_string(r));
+
+  const int grid = std::max(2, std::min(sms & ~1, 2 * a.tiles_m * a.tiles_n));
+  if (two_cta < 0) {
+    const char* v = std::getenv("MSB_TWO_CTA");
+    two_cta = v == nullptr || std::strcmp(v, "0") != 0;
+  }
+  if (two_cta) {
+    check(launch_sm100_gemm2(ta, tb, a, grid, S(stream)), "sm100_gemm2 launch");
+  } else {
+    static const PushMaps no_push = {};
+    check(launch_sm100_gemm(ta, tb, no_push, a, grid, S(stream)), "sm100_gemm launch");
+  }
+}
+
 // ---------------------------------------------------------------------------------------
 // runtime: IPC-shared device memory, host-mapped status words
 // ---------------------------------------------------------------------------------------
@@ -320,6 +384,8 @@ PYBIND11_MODULE(_C, m) {
   m.attr("CHUNK_DESC_BYTES") = (int)sizeof(ChunkDesc);
 
   m.def("gemm_run", &gemm_run, "persistent tcgen05 GEMM with optional fused gather / push");
+  m.def("gemm_local", &gemm_local, "plain local GEMM: M, N, K, A, lda, a_mn_major, B, ldb, b_mn_major, C, ldc, c_fp32, "
+        "accumulate, bias, act, C_pre, two_cta (-1: MSB_TWO_CTA), sms, status, stream");
   m.def("symm_alloc", &symm_alloc);
   m.def("symm_open", &symm_open);
   m.def("symm_close", &symm_close);

@@ -170,6 +170,14 @@ def _split_qkv(qkv, batch, seq, heads):
     return t[:, :, :, 0], t[:, :, :, 1], t[:, :, :, 2], D  # each [b, s, h, D]
 
 
+def _head_dim(qkv, batch, seq, heads) -> int:
+    """Features per head of a [batch * seq, heads * 3 * D] tensor (what ``_split_qkv`` could view is accepted)."""
+    rows, width = qkv.shape
+    if rows != batch * seq or width % (3 * heads) or not qkv.is_contiguous():
+        return _split_qkv(qkv, batch, seq, heads)[3]
+    return width // (3 * heads)
+
+
 FALLBACKS = {"attention": 0}      # eager-PyTorch runs of an op on CUDA tensors (only with allow_fallback)
 
 
@@ -185,7 +193,7 @@ def _check_attention_shape(qkv, D: int, seq: int, allow_fallback: bool):
 
 def attention_fwd(qkv, batch: int, seq: int, heads: int, causal: bool = False, allow_fallback: bool = False):
     """softmax(Q K^T / sqrt(D)) V per (sequence, head).  Returns (out [b*s, heads*D], lse)."""
-    q, k, v, D = _split_qkv(qkv, batch, seq, heads)
+    D = _head_dim(qkv, batch, seq, heads)
     _check_attention_shape(qkv, D, seq, allow_fallback)
     if qkv.is_cuda and D == 128 and seq % 128 == 0:
         out = torch.empty(batch * seq, heads * D, dtype=qkv.dtype, device=qkv.device)
@@ -193,6 +201,7 @@ def attention_fwd(qkv, batch: int, seq: int, heads: int, causal: bool = False, a
         _C().attention_fwd(qkv.data_ptr(), out.data_ptr(), lse.data_ptr(), batch, seq, heads,
                            1 if causal else 0, 1.0 / math.sqrt(D), _native.status().dev, _st())
         return out, lse
+    q, k, v, D = _split_qkv(qkv, batch, seq, heads)
     qf, kf, vf = (t.permute(0, 2, 1, 3).float() for t in (q, k, v))  # [b, h, s, D]
     s = qf @ kf.transpose(-1, -2) / math.sqrt(D)
     if causal:
@@ -205,7 +214,7 @@ def attention_fwd(qkv, batch: int, seq: int, heads: int, causal: bool = False, a
 def attention_bwd(dout, qkv, out, lse, batch: int, seq: int, heads: int, causal: bool = False,
                   allow_fallback: bool = False):
     """Gradient w.r.t. qkv in the same interleaved layout."""
-    q, k, v, D = _split_qkv(qkv, batch, seq, heads)
+    D = _head_dim(qkv, batch, seq, heads)
     _check_attention_shape(qkv, D, seq, allow_fallback)
     if qkv.is_cuda and D == 128 and seq % 128 == 0:
         dqkv = torch.empty_like(qkv)
@@ -217,6 +226,7 @@ def attention_bwd(dout, qkv, out, lse, batch: int, seq: int, heads: int, causal:
                            1 if causal else 0,
                            1.0 / math.sqrt(D), _native.status().dev, _st())
         return dqkv
+    q, k, v, D = _split_qkv(qkv, batch, seq, heads)
     qf, kf, vf = (t.permute(0, 2, 1, 3).float() for t in (q, k, v))
     do = dout.view(batch, seq, heads, D).permute(0, 2, 1, 3).float()
     of = out.view(batch, seq, heads, D).permute(0, 2, 1, 3).float()
