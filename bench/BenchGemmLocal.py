@@ -5,8 +5,8 @@
 
 Every shape runs all arms round-robin inside each repetition, so that the clock drift of a power-capped GPU hits
 every arm alike; L2 is flushed (a 256 MiB write) before each timed call; times are CUDA-event medians.  With
-`--knobs` the kernel's stage count (6 / 7) and the 3-D tensor map of MN-major operands (off / on) are swept as
-separate arms through the environment variables that `meshslice_b200.ops.gemm.gemm` reads.
+`--knobs` the 3-D tensor map of MN-major operands (off / on) is swept as separate arms through the environment
+variable that `meshslice_b200.ops.gemm.gemm` reads.
 """
 import argparse
 import os
@@ -30,7 +30,7 @@ def main():
     args = ap.parse_args()
     arms = [("cublas", None)]
     if args.knobs:
-        arms += [(f"s{st}m{m3}", dict(MSB_G2_STAGES=str(st), MSB_G2_MAP3D=str(m3))) for st in (6, 7) for m3 in (0, 1)]
+        arms += [(f"m{m3}", dict(MSB_G2_MAP3D=str(m3))) for m3 in (0, 1)]
     else:
         arms += [("gemm", {})]
     flush = torch.empty(256 << 20, dtype=torch.uint8, device="cuda")

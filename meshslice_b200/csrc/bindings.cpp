@@ -138,7 +138,6 @@ void gemm_run(const py::dict& d) {
   if (a.n_slices < 1 || tiles_s % (a.n_slices * a.cyc) != 0)
     throw std::runtime_error("gemm: n_slices must divide the tile count of the sliced dimension");
   if (a.group < 1) a.group = 1;
-  a.stages = (int)geti(d, "stages", 7);
   a.rot = (int)geti(d, "rot", 0);
   if (a.rot < 0 || a.rot >= tiles_s / a.n_slices) a.rot = 0;
   if (geti(d, "no_tiles")) a.tiles_m = 0;  // reduce phase only
@@ -235,22 +234,20 @@ void gemm_run(const py::dict& d) {
   if (r != 0) throw std::runtime_error("gemm: tensor map for A failed, code " + std::to_string(r));
   const bool plain = a.n_chunks == 0 && a.n_ranks == 0 && a.red_n == 0 && a.push_n == 0 && a.tiles_m > 0;
   const bool pair = plain && geti(d, "two_cta", 1) != 0;
-  if (!a.b_mn_major) r = make_tensor_map_2d(&tb, P<void>(B), a.K, a.N, ldb * 2, kBK, kBN / 2);
-  else if (try3d && make_tensor_map_mn3d(&tb, P<void>(B), a.N, a.K, ldb * 2, kBN / 128) == 0) { r = 0; a.b_map3d = 1; }
+  const int sms = (int)geti(d, "grid", 148), tile_n = pair ? gemm2_tile_n(a.M, a.N, sms) : kBN;
+  if (!a.b_mn_major) r = make_tensor_map_2d(&tb, P<void>(B), a.K, a.N, ldb * 2, kBK, tile_n / 2);
+  else if (try3d && make_tensor_map_mn3d(&tb, P<void>(B), a.N, a.K, ldb * 2, tile_n / 128) == 0) { r = 0; a.b_map3d = 1; }
   else r = make_tensor_map_2d(&tb, P<void>(B), a.N, a.K, ldb * 2, 64, kBK);
   if (r != 0) throw std::runtime_error("gemm: tensor map for B failed, code " + std::to_string(r));
 
-  int grid = (int)geti(d, "grid", 148);
+  int grid = sms;
   const int ntiles = a.tiles_m * a.tiles_n;
   const bool needs_all = a.n_chunks > 0 || a.n_ranks > 0 || a.red_n > 0;
   if (!needs_all && grid > 2 * ntiles) grid = 2 * ntiles;
   grid &= ~1;
   if (grid < 2) grid = 2;
   if (pair) {
-    const int clusters = ((a.M + 2 * kBM - 1) / (2 * kBM)) * a.tiles_n;
-    int g2 = (int)geti(d, "grid", 148) & ~1;
-    if (g2 > 2 * clusters) g2 = 2 * clusters;
-    check(launch_sm100_gemm2(ta, tb, a, g2, S(getp(d, "stream"))), "sm100_gemm2 launch");
+    check(launch_sm100_gemm2(ta, tb, a, tile_n, sms, S(getp(d, "stream"))), "sm100_gemm2 launch");
     return;
   }
   static PushMaps pm;   // only the first push_n entries are read by the kernel
@@ -267,7 +264,7 @@ void gemm_run(const py::dict& d) {
 
 // The plain local GEMM of `ops.gemm`: the few values it needs, positionally.  Filling the dict of gemm_run and reading
 // it back took longer than a small product takes on the GPU (a linear layer of 512 x 512 x 1536, forward and backward:
-// 108 us a pass, 59 us through this call).  MSB_TWO_CTA, MSB_G2_STAGES, MSB_G2_GROUP and MSB_G2_MAP3D are read per call, as they were.
+// 108 us a pass, 59 us through this call).  MSB_TWO_CTA, MSB_G2_GROUP and MSB_G2_MAP3D are read per call, as they were.
 void gemm_local(int64_t M, int64_t N, int64_t K, uint64_t A, int64_t lda, int a_mn_major, uint64_t B, int64_t ldb,
                 int b_mn_major, uint64_t C, int64_t ldc, int c_fp32, int accumulate, uint64_t bias, int act,
                 uint64_t C_pre, int two_cta, int sms, uint64_t status, uint64_t stream) {
@@ -298,10 +295,13 @@ void gemm_local(int64_t M, int64_t N, int64_t K, uint64_t A, int64_t lda, int a_
   a.tiles_n = (a.N + kBN - 1) / kBN;
   a.n_slices = a.cyc = a.push_extent = a.push_bufs = a.b_nchunk = a.a_kpanel = a.b_kpanel = 1;
   a.group = std::max(1, env("MSB_G2_GROUP", 8));
-  a.stages = env("MSB_G2_STAGES", 7);
   a.status = P<uint32_t>(status);
   a.timeout_ns = 1000000000ull;
 
+  if (two_cta < 0) {
+    const char* v = std::getenv("MSB_TWO_CTA");
+    two_cta = v == nullptr || std::strcmp(v, "0") != 0;
+  }
   CUtensorMap ta, tb;
   int r;
   const bool try3d = env("MSB_G2_MAP3D", 1) != 0;
@@ -309,19 +309,16 @@ void gemm_local(int64_t M, int64_t N, int64_t K, uint64_t A, int64_t lda, int a_
   else if (try3d && make_tensor_map_mn3d(&ta, P<void>(A), a.M, a.K, lda * 2, kBM / 64) == 0) { r = 0; a.a_map3d = 1; }
   else r = make_tensor_map_2d(&ta, P<void>(A), a.M, a.K, lda * 2, 64, kBK);
   if (r != 0) throw std::runtime_error("gemm: tensor map for A failed, code " + std::to_string(r));
-  if (!b_mn_major) r = make_tensor_map_2d(&tb, P<void>(B), a.K, a.N, ldb * 2, kBK, kBN / 2);
-  else if (try3d && make_tensor_map_mn3d(&tb, P<void>(B), a.N, a.K, ldb * 2, kBN / 128) == 0) { r = 0; a.b_map3d = 1; }
+  const int tile_n = two_cta ? gemm2_tile_n(a.M, a.N, sms) : kBN;
+  if (!b_mn_major) r = make_tensor_map_2d(&tb, P<void>(B), a.K, a.N, ldb * 2, kBK, tile_n / 2);
+  else if (try3d && make_tensor_map_mn3d(&tb, P<void>(B), a.N, a.K, ldb * 2, tile_n / 128) == 0) { r = 0; a.b_map3d = 1; }
   else r = make_tensor_map_2d(&tb, P<void>(B), a.N, a.K, ldb * 2, 64, kBK);
   if (r != 0) throw std::runtime_error("gemm: tensor map for B failed, code " + std::to_string(r));
 
-  const int grid = std::max(2, std::min(sms & ~1, 2 * a.tiles_m * a.tiles_n));
-  if (two_cta < 0) {
-    const char* v = std::getenv("MSB_TWO_CTA");
-    two_cta = v == nullptr || std::strcmp(v, "0") != 0;
-  }
   if (two_cta) {
-    check(launch_sm100_gemm2(ta, tb, a, grid, S(stream)), "sm100_gemm2 launch");
+    check(launch_sm100_gemm2(ta, tb, a, tile_n, sms, S(stream)), "sm100_gemm2 launch");
   } else {
+    const int grid = std::max(2, std::min(sms & ~1, 2 * a.tiles_m * a.tiles_n));
     static const PushMaps no_push = {};
     check(launch_sm100_gemm(ta, tb, no_push, a, grid, S(stream)), "sm100_gemm launch");
   }

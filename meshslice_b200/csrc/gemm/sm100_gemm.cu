@@ -952,16 +952,20 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
                                   const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
-int make_tensor_map_2d(CUtensorMap* map, const void* base, uint64_t inner, uint64_t outer,
-                       uint64_t pitch_bytes, uint32_t box_inner, uint32_t box_outer, int swizzle_bytes) {
-  static EncodeTiledFn fn = nullptr;
-  if (fn == nullptr) {
+static EncodeTiledFn encode_tiled() {
+  static const EncodeTiledFn fn = [] {
     void* p = nullptr;
     cudaDriverEntryPointQueryResult qres;
     cudaError_t e = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &qres);
-    if (e != cudaSuccess || p == nullptr) return -1;
-    fn = reinterpret_cast<EncodeTiledFn>(p);
-  }
+    return e == cudaSuccess ? reinterpret_cast<EncodeTiledFn>(p) : nullptr;
+  }();
+  return fn;
+}
+
+int make_tensor_map_2d(CUtensorMap* map, const void* base, uint64_t inner, uint64_t outer,
+                       uint64_t pitch_bytes, uint32_t box_inner, uint32_t box_outer, int swizzle_bytes) {
+  const EncodeTiledFn fn = encode_tiled();
+  if (fn == nullptr) return -1;
   cuuint64_t dims[2] = {inner, outer};
   cuuint64_t strides[1] = {pitch_bytes};
   cuuint32_t box[2] = {box_inner, box_outer};
@@ -973,16 +977,25 @@ int make_tensor_map_2d(CUtensorMap* map, const void* base, uint64_t inner, uint6
   return r == CUDA_SUCCESS ? 0 : (int)r;
 }
 
+int make_tensor_map_out(CUtensorMap* map, const void* base, int64_t cols, int64_t rows, int64_t ld, bool fp32) {
+  const EncodeTiledFn fn = encode_tiled();
+  if (fn == nullptr) return -1;
+  const uint64_t pitch = (uint64_t)ld * (fp32 ? 4 : 2);
+  if ((reinterpret_cast<uintptr_t>(base) & 15) || (pitch & 15)) return -2;
+  cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+  cuuint64_t strides[1] = {pitch};
+  cuuint32_t box[2] = {fp32 ? 32u : 64u, 32};
+  cuuint32_t estr[2] = {1, 1};
+  CUresult r = fn(map, fp32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2,
+                  const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? 0 : (int)r;
+}
+
 int make_tensor_map_mn3d(CUtensorMap* map, const void* base, uint64_t mn_extent, uint64_t k_rows,
                          uint64_t pitch_bytes, uint32_t blocks_per_box) {
-  static EncodeTiledFn fn = nullptr;
-  if (fn == nullptr) {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult qres;
-    cudaError_t e = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &qres);
-    if (e != cudaSuccess || p == nullptr) return -1;
-    fn = reinterpret_cast<EncodeTiledFn>(p);
-  }
+  const EncodeTiledFn fn = encode_tiled();
+  if (fn == nullptr) return -1;
   if (mn_extent % 64 != 0) return -2;
   cuuint64_t dims[3] = {64, k_rows, mn_extent / 64};
   cuuint64_t strides[2] = {pitch_bytes, 128};

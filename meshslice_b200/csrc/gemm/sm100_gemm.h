@@ -159,8 +159,8 @@ struct GemmArgs {
   uint32_t* go_flag;           // local: set to epoch by CTA 0 once all peers have arrived
   uint32_t* done_counter;      // local: CTAs that finished their transfers (monotonic)
   uint32_t done_target;
-  // ---- tuning of the plain (two-CTA) kernel ----
-  int stages;                  // smem pipeline stages: 6 or 7
+  // ---- plain (two-CTA) kernel ----
+  int tma_c;                   // set by its launcher: C (and C_pre) leave through shared memory as TMA stores
   // ---- status ----
   uint32_t* status;            // [4]: code, blockIdx, detail, detail2
   uint64_t timeout_ns;
@@ -188,15 +188,21 @@ cudaError_t launch_sm100_gemm(const CUtensorMap& tma_a, const CUtensorMap& tma_b
                               const PushMaps& push_maps, const GemmArgs& args, int grid,
                               cudaStream_t stream);
 
-// Two-CTA (cta_group::2) variant for plain local GEMMs (no gather / push / reduce / barriers).
-// The tensor map of a K-major B must use a {64, kBN / 2} box.
-cudaError_t launch_sm100_gemm2(const CUtensorMap& tma_a, const CUtensorMap& tma_b,
-                               const GemmArgs& args, int grid, cudaStream_t stream);
+// Two-CTA (cta_group::2) variant for plain local GEMMs (no gather / push / reduce / barriers) on at most `sms` SMs.
+// `tile_n` columns per cluster tile (gemm2_tile_n); the tensor map of a K-major B must use a {64, tile_n / 2} box,
+// that of an MN-major B one box of tile_n / 128 blocks of 64 columns.
+int gemm2_tile_n(int M, int N, int sms);
+cudaError_t launch_sm100_gemm2(const CUtensorMap& tma_a, const CUtensorMap& tma_b, GemmArgs args, int tile_n, int sms,
+                               cudaStream_t stream);
 
 // Builds a 2-D bf16 tensor map with a swizzle of 128 (or 64) bytes.  `inner` is the contiguous extent,
 // `outer` the number of rows, `pitch_bytes` the row pitch.  Returns 0 on success.
 int make_tensor_map_2d(CUtensorMap* map, const void* base, uint64_t inner, uint64_t outer,
                        uint64_t pitch_bytes, uint32_t box_inner, uint32_t box_outer, int swizzle_bytes = 128);
+
+// Tensor map of an output matrix [rows, cols] with row pitch `ld` elements: boxes of 32 rows x 128 bytes, 128-byte
+// swizzle.  Returns non-zero where TMA cannot address it (base or pitch not a multiple of 16 bytes).
+int make_tensor_map_out(CUtensorMap* map, const void* base, int64_t cols, int64_t rows, int64_t ld, bool fp32);
 
 // Tensor map of an MN-major operand (stored [k_rows, mn_extent] row-major, mn_extent % 64 == 0) as
 // {64 elements, k_rows, mn_extent / 64 blocks}: one box of {64, kBK, blocks_per_box} fills the

@@ -21,8 +21,11 @@ namespace msb {
 namespace {
 
 constexpr uint32_t kAStage2 = kBM * kBK * 2;        // 16 KiB: this CTA's 128 rows of A
-constexpr uint32_t kBStage2 = (kBN / 2) * kBK * 2;  // 16 KiB: this CTA's 128 columns of B
-constexpr uint32_t smem_alloc2(int stages) { return stages * (kAStage2 + kBStage2) + 256 + 1024; }
+constexpr uint32_t b_stage2(int bn) { return (bn / 2) * kBK * 2; }   // this CTA's half of the tile's columns of B
+constexpr uint32_t kOutBox = 32 * 128;              // a staged box: 32 rows of 128 bytes
+constexpr uint32_t kOutStage = 4 * 2 * kOutBox;     // two per epilogue warp
+constexpr int stages2(int bn) { return bn == 256 ? 6 : 8; }
+constexpr uint32_t smem_alloc2(int bn) { return stages2(bn) * (kAStage2 + b_stage2(bn)) + kOutStage + 256 + 1024; }
 constexpr int kThreads2 = 224;   // warps: A producer, MMA, 4x epilogue, B producer
 
 __device__ __forceinline__ uint32_t cluster_ctarank() {
@@ -145,6 +148,55 @@ __device__ __forceinline__ void store32(void* base, int64_t ld, bool fp32, bool 
   }
 }
 
+// One box of a tensor map, shared -> global; the second form adds fp32 values to what is there.
+__device__ __forceinline__ void tma_store_box(const CUtensorMap* map, const void* src, int32_t x, int32_t y, bool add) {
+  if (add)
+    asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.bulk_group [%0, {%2, %3}], [%1];"
+                 ::"l"(map), "r"(smem_u32(src)), "r"(x), "r"(y) : "memory");
+  else
+    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];"
+                 ::"l"(map), "r"(smem_u32(src)), "r"(x), "r"(y) : "memory");
+}
+// Staging of one epilogue warp: two boxes in turn, each free again once the copy engine has read it: all but the last
+// `1 - taken` stores.  With taken = 1 (another box may be held unsent) none may be outstanding.
+struct OutStage {
+  uint8_t* base;
+  int next;
+  template <int taken = 0>
+  __device__ __forceinline__ uint8_t* take(int lane) {
+    if (lane == 0) bulk_wait_read<1 - taken>();
+    __syncwarp();
+    uint8_t* p = base + next * kOutBox;
+    next ^= 1;
+    return p;
+  }
+  __device__ __forceinline__ void send(const CUtensorMap* map, const uint8_t* box, int lane, int32_t x, int32_t y, bool add) {
+    fence_proxy_async_smem();
+    __syncwarp();
+    if (lane == 0) {
+      tma_store_box(map, box, x, y, add);
+      bulk_commit();
+    }
+  }
+};
+__device__ __forceinline__ void stage_bf16(uint8_t* box, int lane, int half, const float (&v)[32]) {
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    uint4 o;
+    o.x = pk2(v[q * 8 + 0], v[q * 8 + 1]);
+    o.y = pk2(v[q * 8 + 2], v[q * 8 + 3]);
+    o.z = pk2(v[q * 8 + 4], v[q * 8 + 5]);
+    o.w = pk2(v[q * 8 + 6], v[q * 8 + 7]);
+    *reinterpret_cast<uint4*>(box + lane * 128 + (((half * 4 + q) ^ (lane & 7)) << 4)) = o;   // 128-byte swizzle
+  }
+}
+__device__ __forceinline__ void stage_f32(uint8_t* box, int lane, const float (&v)[32]) {
+#pragma unroll
+  for (int q = 0; q < 8; ++q)
+    *reinterpret_cast<float4*>(box + lane * 128 + ((q ^ (lane & 7)) << 4)) =
+        make_float4(v[q * 4], v[q * 4 + 1], v[q * 4 + 2], v[q * 4 + 3]);
+}
+
 // cluster tile t -> (256-row block, 256-column block), grouped along M for L2 reuse
 __device__ __forceinline__ void tile2(int t, int tiles_m2, int tiles_n, int group, int& m2, int& nb) {
   const int span = group * tiles_n;
@@ -158,15 +210,20 @@ __device__ __forceinline__ void tile2(int t, int tiles_m2, int tiles_n, int grou
 
 }  // namespace
 
-template <int kStages2>
+// BN: columns of a cluster tile.  128 halves the tile where 256-column tiles would fill at most half of the SMs.
+template <int BN>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads2, 1)
 sm100_gemm2_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
+                   const __grid_constant__ CUtensorMap tma_c, const __grid_constant__ CUtensorMap tma_pre,
                    const __grid_constant__ GemmArgs a) {
+  constexpr int kStages2 = stages2(BN);
+  constexpr uint32_t kBStage2 = b_stage2(BN);
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
   constexpr uint32_t kSmemB2 = kStages2 * kAStage2;
-  constexpr uint32_t kSmemBar2 = kSmemB2 + kStages2 * kBStage2;
+  constexpr uint32_t kSmemOut2 = kSmemB2 + kStages2 * kBStage2;
+  constexpr uint32_t kSmemBar2 = kSmemOut2 + kOutStage;
   uint8_t* sA = smem;
   uint8_t* sB = smem + kSmemB2;
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kSmemBar2);
@@ -180,7 +237,7 @@ sm100_gemm2_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_const
   const uint32_t rank = cluster_ctarank();      // 0: leader
   const uint64_t tmo = a.timeout_ns;
   const int tiles_m2 = (a.M + 2 * kBM - 1) / (2 * kBM);
-  const int tiles_n = (a.N + kBN - 1) / kBN;
+  const int tiles_n = (a.N + BN - 1) / BN;
   const int num_tiles = tiles_m2 * tiles_n;
   const int kblocks = (a.K + kBK - 1) / kBK;
   const int cluster_id = blockIdx.x >> 1, n_clusters = gridDim.x >> 1;
@@ -195,13 +252,13 @@ sm100_gemm2_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_const
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(tfull_bar + i, 1);
-      mbar_init(tempty_bar + i, 256);
+      mbar_init(tempty_bar + i, 8);    // a lane of each epilogue warp of both CTAs
     }
     mbar_fence_init();
   }
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                 "r"(512u)
+                 "r"(2u * BN)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
@@ -223,7 +280,7 @@ sm100_gemm2_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_const
         int m2, nb;
         tile2(t, tiles_m2, tiles_n, group, m2, nb);
         const int row_a = (2 * m2 + (int)rank) * kBM;           // this CTA's 128 rows of A
-        const int col_b = nb * kBN + (int)rank * (kBN / 2);     // this CTA's 128 columns of B
+        const int col_b = nb * BN + (int)rank * (BN / 2);       // this CTA's half of the columns of B
         for (int kb = 0; kb < kblocks; ++kb) {
           if (!mbar_wait(empty_bar + stage, phase ^ 1, 5 * tmo)) {
             report2(a, kTimeoutEmpty, t, kb);
@@ -252,7 +309,7 @@ sm100_gemm2_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_const
               tma_load_3d_pair(db, &tma_b, fb, 0, kb * kBK, col_b >> 6);
             } else {
 #pragma unroll
-              for (int j = 0; j < kBN / 128; ++j)
+              for (int j = 0; j < BN / 128; ++j)
                 tma_load_2d_pair(db + j * (kBK * 128), &tma_b, fb, col_b + j * 64, kb * kBK);
             }
           }
@@ -263,7 +320,7 @@ sm100_gemm2_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_const
   } else if (warp == 1) {
     // ===================== MMA issuer (leader only) =====================
     if (lane == 0 && rank == 0) {
-      const uint32_t idesc = make_idesc_bf16(2 * kBM, kBN, a.a_mn_major, a.b_mn_major);
+      const uint32_t idesc = make_idesc_bf16(2 * kBM, BN, a.a_mn_major, a.b_mn_major);
       const uint32_t a_lbo = a.a_mn_major ? kBK * 128 : 16;
       const uint32_t b_lbo = a.b_mn_major ? kBK * 128 : 16;
       const uint32_t a_kstep = a.a_mn_major ? 16 * 128 : 32;
@@ -279,7 +336,7 @@ sm100_gemm2_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_const
           break;
         }
         tc_fence_after_sync();
-        const uint32_t tmem_d = tmem_base + acc * kBN;
+        const uint32_t tmem_d = tmem_base + acc * BN;
         for (int kb = 0; kb < kblocks; ++kb) {
           if (!mbar_wait(full_bar + stage, phase, 4 * tmo)) {
             report2(a, kTimeoutFull, t, kb);
@@ -311,6 +368,8 @@ sm100_gemm2_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_const
     // ===================== epilogue (both CTAs, own 128 rows) =====================
     const int q = warp & 3;
     const __nv_bfloat16* bias = reinterpret_cast<const __nv_bfloat16*>(a.bias);
+    const bool dual = a.act == 1 && a.C_pre != nullptr;   // two outputs: no store of one runs under the other's staging
+    OutStage out{smem + kSmemOut2 + q * 2 * kOutBox, 0};
     bool ok = true;
     int it = 0;
     for (int t = cluster_id; t < num_tiles && ok; t += n_clusters, ++it) {
@@ -327,40 +386,66 @@ sm100_gemm2_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_const
       }
       mbar_wait(tfull_bar + acc, acc_phase, tmo);
       tc_fence_after_sync();
-      const int64_t row = (int64_t)(2 * m2 + (int)rank) * kBM + q * 32 + lane;
-      const bool row_ok = row < a.M;
-      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * kBN;
+      const int row0 = (2 * m2 + (int)rank) * kBM + q * 32;
+      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * BN;
       const uint32_t te_leader = mapa_u32(smem_u32(tempty_bar + acc), 0);
+      uint8_t* box = nullptr;
+      uint8_t* box_pre = nullptr;
 #pragma unroll 1
-      for (int c = 0; c < kBN / 32; ++c) {
+      for (int c = 0; c < BN / 32; ++c) {
         uint32_t r[32];
         __syncwarp();
         tmem_ld_32x32(taddr + c * 32, r);
         tmem_ld_wait();
-        if (c == kBN / 32 - 1) {
+        if (c == BN / 32 - 1) {
           tc_fence_before_sync();
-          mbar_arrive_cluster(te_leader);     // accumulator drained: tell the leader's MMA warp
+          __syncwarp();
+          if (lane == 0) mbar_arrive_cluster(te_leader);     // accumulator drained: tell the leader's MMA warp
         }
-        const int col0 = nb * kBN + c * 32;
+        const int col0 = nb * BN + c * 32;
         const int nvalid = min(32, a.N - col0);
-        if (row_ok && nvalid > 0) {
-          float v[32];
+        if (row0 >= a.M || nb * BN + (c & ~1) * 32 >= a.N) continue;   // the two halves of a bf16 box go together
+        float v[32];
 #pragma unroll
-          for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
-          if (bias != nullptr) {
+        for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
+        if (bias != nullptr) {
 #pragma unroll
-            for (int i = 0; i < 32; ++i)
-              if (i < nvalid) v[i] += __bfloat162float(bias[col0 + i]);
-          }
+          for (int i = 0; i < 32; ++i)
+            if (i < nvalid) v[i] += __bfloat162float(bias[col0 + i]);
+        }
+        if (!a.tma_c) {
+          if (row0 + lane >= a.M || nvalid <= 0) continue;
           if (a.act == 1) {
-            if (a.C_pre != nullptr) store32(a.C_pre, a.ldc, false, false, row, col0, nvalid, v);
+            if (a.C_pre != nullptr) store32(a.C_pre, a.ldc, false, false, row0 + lane, col0, nvalid, v);
 #pragma unroll
             for (int i = 0; i < 32; ++i) v[i] = gelu_tanh2(v[i]);
           }
-          store32(a.C, a.ldc, a.c_fp32 != 0, a.accumulate != 0, row, col0, nvalid, v);
+          store32(a.C, a.ldc, a.c_fp32 != 0, a.accumulate != 0, row0 + lane, col0, nvalid, v);
+          continue;
+        }
+        // rows and columns beyond the matrix are clipped by the tensor map
+        if (a.act == 1) {
+          if (dual) {
+            if ((c & 1) == 0) box_pre = out.take(lane);
+            stage_bf16(box_pre, lane, c & 1, v);
+            if (c & 1) out.send(&tma_pre, box_pre, lane, col0 - 32, row0, false);
+          }
+#pragma unroll
+          for (int i = 0; i < 32; ++i) v[i] = gelu_tanh2(v[i]);
+        }
+        if (a.c_fp32) {
+          if (nvalid <= 0) continue;
+          box = dual ? out.take<1>(lane) : out.take(lane);
+          stage_f32(box, lane, v);
+          out.send(&tma_c, box, lane, col0, row0, a.accumulate != 0);
+        } else {
+          if ((c & 1) == 0) box = dual ? out.take<1>(lane) : out.take(lane);
+          stage_bf16(box, lane, c & 1, v);
+          if (c & 1) out.send(&tma_c, box, lane, col0 - 32, row0, false);
         }
       }
     }
+    if (lane == 0) bulk_wait_all<0>();
   }
 
   // both CTAs are done with shared memory, barriers and TMEM of the pair
@@ -368,33 +453,46 @@ sm100_gemm2_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_const
   cluster_sync_all();
   tc_fence_after_sync();
   if (warp == 1)
-    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(2u * BN) : "memory");
 }
 
-template <int kSt>
-static cudaError_t launch2(const CUtensorMap& tma_a, const CUtensorMap& tma_b, const GemmArgs& args, int grid,
-                           cudaStream_t stream) {
+template <int BN>
+static cudaError_t launch2(const CUtensorMap& tma_a, const CUtensorMap& tma_b, const CUtensorMap& tma_c,
+                           const CUtensorMap& tma_pre, const GemmArgs& args, int grid, cudaStream_t stream) {
   static bool configured[64] = {false};
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
-  constexpr int smem = (int)smem_alloc2(kSt);
+  constexpr int smem = (int)smem_alloc2(BN);
   if (dev < 64 && !configured[dev]) {
-    e = cudaFuncSetAttribute(sm100_gemm2_kernel<kSt>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    e = cudaFuncSetAttribute(sm100_gemm2_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
     configured[dev] = true;
   }
   // the cluster shape (2,1,1) is part of the kernel's definition
-  sm100_gemm2_kernel<kSt><<<grid, kThreads2, smem, stream>>>(tma_a, tma_b, args);
+  sm100_gemm2_kernel<BN><<<grid, kThreads2, smem, stream>>>(tma_a, tma_b, tma_c, tma_pre, args);
   return cudaGetLastError();
 }
 
-cudaError_t launch_sm100_gemm2(const CUtensorMap& tma_a, const CUtensorMap& tma_b, const GemmArgs& args,
-                               int grid, cudaStream_t stream) {
-  grid &= ~1;
+int gemm2_tile_n(int M, int N, int sms) {
+  const int64_t tiles = (int64_t)((M + 2 * kBM - 1) / (2 * kBM)) * ((N + 255) / 256);
+  return tiles * 4 <= sms ? 128 : 256;
+}
+
+cudaError_t launch_sm100_gemm2(const CUtensorMap& tma_a, const CUtensorMap& tma_b, GemmArgs args, int tile_n, int sms,
+                               cudaStream_t stream) {
+  // Output through shared memory and TMA where the tensor map allows it; bf16 accumulation adds before it rounds,
+  // which the copy engine cannot do.
+  CUtensorMap tc = tma_a, tp = tma_a;   // any valid map where it is not used
+  args.tma_c = !(args.accumulate && !args.c_fp32) &&
+               make_tensor_map_out(&tc, args.C, args.N, args.M, args.ldc, args.c_fp32 != 0) == 0 &&
+               (args.act == 0 || args.C_pre == nullptr ||
+                make_tensor_map_out(&tp, args.C_pre, args.N, args.M, args.ldc, false) == 0);
+  const int64_t tiles = (int64_t)((args.M + 2 * kBM - 1) / (2 * kBM)) * ((args.N + tile_n - 1) / tile_n);
+  int grid = (int)(2 * tiles < (sms & ~1) ? 2 * tiles : (sms & ~1));
   if (grid < 2) grid = 2;
-  if (args.stages == 6) return launch2<6>(tma_a, tma_b, args, grid, stream);
-  return launch2<7>(tma_a, tma_b, args, grid, stream);
+  if (tile_n == 128) return launch2<128>(tma_a, tma_b, tc, tp, args, grid, stream);
+  return launch2<256>(tma_a, tma_b, tc, tp, args, grid, stream);
 }
 
 }  // namespace msb

@@ -81,3 +81,43 @@ def test_gemm_many_tiles_persistent_schedule():
     out = gemm(a, b, "nt")
     _native.check_status()
     _check(out, _ref(a, b, "nt"), 512)
+
+
+@pytest.mark.parametrize("layout", ["nt", "nn", "tn"])
+@pytest.mark.parametrize("shape", [(8, 8, 8), (264, 136, 72), (1400, 1032, 200), (2344, 2056, 136), (2304, 4672, 64)])
+def test_gemm_output_boxes(layout, shape):
+    """Every way an output leaves the kernel, on both sides of the rule for the tile width (128 columns up to 37 tiles
+    of 256 x 256), with boxes of 32 rows x 64 or 32 columns cut at both edges and guard rows and columns around C:
+    bf16, fp32, fp32 added to, bf16 added to, and GeLU with its pre-activation.  Products of bf16 values are summed in
+    fp32 (K^0.5 * 2^-22 of the operands' scale at most), bf16 results are rounded once (2^-9)."""
+    from meshslice_b200 import _native
+    from meshslice_b200.ops.gemm import gemm
+    M, N, K = shape
+    a, b = _operands(M, N, K, layout, seed=M + N)
+    sa, sb = (a.double().t() if layout == "tn" else a.double()), (b.double().t() if layout == "nt" else b.double())
+    ref = sa @ sb
+
+    def guarded(dtype, fill):
+        full = torch.full((M + 2, N + 16), fill, device="cuda", dtype=dtype)
+        return full, full[1:-1, 8:-8]
+
+    def intact(full, fill):
+        return bool((full[0] == fill).all() and (full[-1] == fill).all() and (full[:, :8] == fill).all()
+                    and (full[:, -8:] == fill).all())
+
+    scale = ref.abs().max().item() + 3.0
+    for dtype, acc, tol in ((torch.bfloat16, False, 2 ** -8), (torch.float32, False, 1e-5), (torch.float32, True, 1e-5),
+                            (torch.bfloat16, True, 2 ** -8)):
+        full, out = guarded(dtype, 3.0)
+        gemm(a, b, layout, out=out, accumulate=acc)
+        _native.check_status()
+        assert intact(full, 3.0), (dtype, acc)
+        assert (out.double() - ref - (3.0 if acc else 0.0)).abs().max().item() <= tol * scale, (dtype, acc)
+    full, out = guarded(torch.bfloat16, 3.0)
+    fullp, pre = guarded(torch.bfloat16, 3.0)
+    gemm(a, b, layout, out=out, act="gelu", pre_act=pre)
+    _native.check_status()
+    assert intact(full, 3.0) and intact(fullp, 3.0)
+    assert (pre.double() - ref).abs().max().item() <= 2 ** -8 * scale
+    g = torch.nn.functional.gelu(ref, approximate="tanh")
+    assert ((out.double() - g).abs() <= 2 ** -8 * g.abs() + 2e-3 * ref.abs() + 1e-3).all()
