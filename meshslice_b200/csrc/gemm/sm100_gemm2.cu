@@ -2,14 +2,14 @@
 // neighbouring SMs computes one 256 x 256 tile with tcgen05.mma.cta_group::2.
 //
 // Each CTA loads 128 rows of A and 128 of the 256 B columns per k-block (32 KiB instead of 48 KiB
-// per stage, so seven stages fit) and owns the 128 accumulator rows that land in its own TMEM.  Only
+// per stage, so six stages and the output staging fit) and owns the 128 accumulator rows that land in its own TMEM.  Only
 // the leader CTA (even rank) issues MMAs; it reads both CTAs' shared memory.  Synchronisation:
 //   full[stage]    lives in the leader; both CTAs' TMA loads complete on it (the .cta_group::2
 //                  load form with the leader barrier's cluster address); two arrivals: the leader's
 //                  A producer and B producer each announce their operand's bytes
-//   empty[stage]   one per CTA; the leader commits to its own and to the peer's (mapa address)
+//   empty[stage]   one per CTA; one commit of the leader arrives on both
 //   tfull[acc]     one per CTA, committed by the leader to both
-//   tempty[acc]    lives in the leader, 256 arrivals: 128 local, 128 from the peer's epilogue
+//   tempty[acc]    lives in the leader, 8 arrivals: one per epilogue warp of both CTAs
 // No load uses cluster multicast.  Every wait is bounded as in the one-CTA kernel.
 #include <cuda_bf16.h>
 
@@ -70,9 +70,26 @@ __device__ __forceinline__ void umma_f16_pair(uint32_t tmem_d, uint64_t da, uint
       ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-__device__ __forceinline__ void umma_commit_pair(uint32_t bar_addr) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar_addr)
-               : "memory");
+// Arrives on the mbarrier at this offset of both CTAs' shared memory once all MMAs issued so far have finished.
+__device__ __forceinline__ void umma_commit_both(uint32_t bar_addr) {
+  asm volatile(
+      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+      ::"r"(bar_addr), "h"((uint16_t)3) : "memory");
+}
+// One look at a barrier, without the suspension of try_wait.
+__device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred P;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 P, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, P;\n\t}"
+      : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+  return ok != 0;
+}
+__device__ __forceinline__ uint64_t desc_at(uint32_t lo, uint32_t hi) {
+  uint64_t d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(lo), "r"(hi));
+  return d;
 }
 
 __device__ __forceinline__ void report2(const GemmArgs& a, uint32_t code, uint32_t d0, uint32_t d1) {
@@ -210,7 +227,7 @@ __device__ __forceinline__ void tile2(int t, int tiles_m2, int tiles_n, int grou
 
 }  // namespace
 
-// BN: columns of a cluster tile.  128 halves the tile where 256-column tiles would fill at most half of the SMs.
+// BN: columns of a cluster tile (gemm2_tile_n chooses).
 template <int BN>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads2, 1)
 sm100_gemm2_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
@@ -233,7 +250,7 @@ sm100_gemm2_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_const
   uint64_t* tempty_bar = tfull_bar + 2;         // [2], used in the leader
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty_bar + 2);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();      // 0: leader
   const uint64_t tmo = a.timeout_ns;
   const int tiles_m2 = (a.M + 2 * kBM - 1) / (2 * kBM);
@@ -272,22 +289,23 @@ sm100_gemm2_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_const
     // One thread issuing every load of a stage is what bounded the tensor pipe with MN-major
     // operands (two boxes per operand): the operands have a producer each, and an MN-major
     // operand is one 3-D box when its extent allows it.
-    if (lane == 0) {
+    if (elect_one()) {
       const bool is_a = warp == 0;
+      const uint32_t full0 = mapa_u32(smem_u32(full_bar), 0);     // the leader's barriers
       uint32_t stage = 0, phase = 0;
-      bool ok = true;
+      bool ok = true, free = true;                                // `free`: the next stage was seen empty
       for (int t = cluster_id; t < num_tiles && ok; t += n_clusters) {
         int m2, nb;
         tile2(t, tiles_m2, tiles_n, group, m2, nb);
         const int row_a = (2 * m2 + (int)rank) * kBM;           // this CTA's 128 rows of A
         const int col_b = nb * BN + (int)rank * (BN / 2);       // this CTA's half of the columns of B
         for (int kb = 0; kb < kblocks; ++kb) {
-          if (!mbar_wait(empty_bar + stage, phase ^ 1, 5 * tmo)) {
+          if (!free && !mbar_wait(empty_bar + stage, phase ^ 1, 5 * tmo)) {
             report2(a, kTimeoutEmpty, t, kb);
             ok = false;
             break;
           }
-          const uint32_t fb = mapa_u32(smem_u32(full_bar + stage), 0);   // the leader's barrier
+          const uint32_t fb = full0 + stage * 8;
           if (is_a) {
             if (rank == 0) mbar_expect_tx(full_bar + stage, 2 * kAStage2);
             uint8_t* da = sA + stage * kAStage2;
@@ -314,19 +332,25 @@ sm100_gemm2_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_const
             }
           }
           if (++stage == kStages2) { stage = 0; phase ^= 1; }
+          free = mbar_test(empty_bar + stage, phase ^ 1);
         }
       }
     }
   } else if (warp == 1) {
     // ===================== MMA issuer (leader only) =====================
-    if (lane == 0 && rank == 0) {
+    // What this thread does per k-block has to fit into the 512 (BN = 256) or 256 cycles that the four instructions
+    // take on the tensor pipe: with the descriptors rebuilt for every instruction, two commits and the wait on the
+    // critical path a k-block took 590 cycles whatever BN.  So only the low descriptor word changes, by additions; one
+    // commit reaches both CTAs; and the next stage is looked at before this one is issued.
+    if (rank == 0 && elect_one()) {
       const uint32_t idesc = make_idesc_bf16(2 * kBM, BN, a.a_mn_major, a.b_mn_major);
-      const uint32_t a_lbo = a.a_mn_major ? kBK * 128 : 16;
-      const uint32_t b_lbo = a.b_mn_major ? kBK * 128 : 16;
-      const uint32_t a_kstep = a.a_mn_major ? 16 * 128 : 32;
-      const uint32_t b_kstep = a.b_mn_major ? 16 * 128 : 32;
+      const uint64_t da0 = make_smem_desc(smem_u32(sA), a.a_mn_major ? kBK * 128 : 16, 1024);
+      const uint64_t db0 = make_smem_desc(smem_u32(sB), a.b_mn_major ? kBK * 128 : 16, 1024);
+      const uint32_t da_hi = (uint32_t)(da0 >> 32), db_hi = (uint32_t)(db0 >> 32);
+      const uint32_t a_kstep = (a.a_mn_major ? 16 * 128 : 32) >> 4;
+      const uint32_t b_kstep = (a.b_mn_major ? 16 * 128 : 32) >> 4;
       uint32_t stage = 0, phase = 0;
-      bool ok = true;
+      bool ok = true, full = false;                               // `full`: the next stage was seen complete
       int it = 0;
       for (int t = cluster_id; t < num_tiles && ok; t += n_clusters, ++it) {
         const uint32_t acc = it & 1, acc_phase = (it >> 1) & 1;
@@ -335,33 +359,26 @@ sm100_gemm2_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_const
           ok = false;
           break;
         }
-        tc_fence_after_sync();
         const uint32_t tmem_d = tmem_base + acc * BN;
         for (int kb = 0; kb < kblocks; ++kb) {
-          if (!mbar_wait(full_bar + stage, phase, 4 * tmo)) {
+          if (!full && !mbar_wait(full_bar + stage, phase, 4 * tmo)) {
             report2(a, kTimeoutFull, t, kb);
             ok = false;
             break;
           }
           tc_fence_after_sync();
-          const uint32_t sa = smem_u32(sA + stage * kAStage2);
-          const uint32_t sb = smem_u32(sB + stage * kBStage2);
-#pragma unroll
-          for (int k = 0; k < kBK / 16; ++k) {
-            const uint64_t da = make_smem_desc(sa + k * a_kstep, a_lbo, 1024);
-            const uint64_t db = make_smem_desc(sb + k * b_kstep, b_lbo, 1024);
-            umma_f16_pair(tmem_d, da, db, idesc, (kb | k) != 0 ? 1u : 0u);
-          }
+          const uint32_t da_lo = (uint32_t)da0 + stage * (kAStage2 >> 4);
+          const uint32_t db_lo = (uint32_t)db0 + stage * (kBStage2 >> 4);
           const uint32_t eb = smem_u32(empty_bar + stage);
-          umma_commit_pair(eb);                 // this CTA's stage is free
-          umma_commit_pair(mapa_u32(eb, 1));    // and the peer's
           if (++stage == kStages2) { stage = 0; phase ^= 1; }
+          full = mbar_test(full_bar + stage, phase);
+#pragma unroll
+          for (int k = 0; k < kBK / 16; ++k)
+            umma_f16_pair(tmem_d, desc_at(da_lo + k * a_kstep, da_hi), desc_at(db_lo + k * b_kstep, db_hi), idesc,
+                          (kb | k) != 0 ? 1u : 0u);
+          umma_commit_both(eb);                 // the stage is free in both CTAs
         }
-        if (ok) {
-          const uint32_t tb = smem_u32(tfull_bar + acc);
-          umma_commit_pair(tb);
-          umma_commit_pair(mapa_u32(tb, 1));
-        }
+        if (ok) umma_commit_both(smem_u32(tfull_bar + acc));
       }
     }
   } else {
@@ -474,9 +491,15 @@ static cudaError_t launch2(const CUtensorMap& tma_a, const CUtensorMap& tma_b, c
   return cudaGetLastError();
 }
 
+// The tile width with the shorter last wave.  A 64-deep k-block takes about 390 cycles on 128 columns (the loads: 24 KiB
+// a CTA) and 530 on 256 (the tensor pipe: 512), so a wave of narrow tiles counts three quarters of a wide one.
+// 2048 x 1024 x 4096 (32 wide tiles): 26.5 us wide, 19.6 narrow; 1024 x 2048 x 1024 11.9 and 8.7; 2048 x 2048 x 2048 (64
+// wide tiles, one wave against two): wide, 16.3 us.
 int gemm2_tile_n(int M, int N, int sms) {
-  const int64_t tiles = (int64_t)((M + 2 * kBM - 1) / (2 * kBM)) * ((N + 255) / 256);
-  return tiles * 4 <= sms ? 128 : 256;
+  const int64_t clusters = sms > 1 ? sms / 2 : 1, rows = (M + 2 * kBM - 1) / (2 * kBM);
+  const int64_t wide = (rows * ((N + 255) / 256) + clusters - 1) / clusters;
+  const int64_t narrow = (rows * ((N + 127) / 128) + clusters - 1) / clusters;
+  return 3 * narrow < 4 * wide ? 128 : 256;
 }
 
 cudaError_t launch_sm100_gemm2(const CUtensorMap& tma_a, const CUtensorMap& tma_b, GemmArgs args, int tile_n, int sms,

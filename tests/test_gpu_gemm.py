@@ -86,8 +86,7 @@ def test_gemm_many_tiles_persistent_schedule():
 @pytest.mark.parametrize("layout", ["nt", "nn", "tn"])
 @pytest.mark.parametrize("shape", [(8, 8, 8), (264, 136, 72), (1400, 1032, 200), (2344, 2056, 136), (2304, 4672, 64)])
 def test_gemm_output_boxes(layout, shape):
-    """Every way an output leaves the kernel, on both sides of the rule for the tile width (128 columns up to 37 tiles
-    of 256 x 256), with boxes of 32 rows x 64 or 32 columns cut at both edges and guard rows and columns around C:
+    """Every way an output leaves the kernel, on both sides of the rule for the tile width, with boxes of 32 rows x 64 or 32 columns cut at both edges and guard rows and columns around C:
     bf16, fp32, fp32 added to, bf16 added to, and GeLU with its pre-activation.  Products of bf16 values are summed in
     fp32 (K^0.5 * 2^-22 of the operands' scale at most), bf16 results are rounded once (2^-9)."""
     from meshslice_b200 import _native
