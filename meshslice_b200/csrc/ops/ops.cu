@@ -114,6 +114,21 @@ __device__ __forceinline__ void block_sum2(float& a, float& b, float* red) {
   a = warp_sum(a);
   b = warp_sum(b);
 }
+// The same for a loop over rows: `red` holds two such buffers that alternate, so that one barrier per row is enough (a
+// thread that writes buffer p again has passed the barrier of the other one, after every read of p).
+__device__ __forceinline__ void block_sum2_alt(float& a, float& b, float* red, int& parity) {
+  a = warp_sum(a);
+  b = warp_sum(b);
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nw = blockDim.x >> 5;
+  float* buf = red + parity * 64;
+  parity ^= 1;
+  if (l == 0) { buf[w] = a; buf[32 + w] = b; }
+  __syncthreads();
+  a = l < nw ? buf[l] : 0.f;
+  b = l < nw ? buf[32 + l] : 0.f;
+  a = warp_sum(a);
+  b = warp_sum(b);
+}
 __device__ __forceinline__ float block_max(float a, float* red) {
   a = warp_max(a);
   const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nw = blockDim.x >> 5;
@@ -137,17 +152,58 @@ __device__ __forceinline__ float gelu_grad_f(float x) {
 }
 
 // ------------------------------------------------------------------------------------------
-// LayerNorm forward.  One CTA per row (grid-stride), row cached in registers.
+// Row ring of the LayerNorm kernels: a thread copies the 16-byte vectors that it will read itself, two rows (one for the
+// widest backward rows) ahead, into shared memory (cp.async), so rows travel while earlier ones are reduced and written, at no registers and
+// without a barrier.  Layout [stage][input][vector of the thread][thread].
+// ------------------------------------------------------------------------------------------
+constexpr int ln_stages(bool backward, int maxv) { return backward && maxv > 3 ? 2 : 3; }
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;"
+               ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// ------------------------------------------------------------------------------------------
+// LayerNorm forward.  One CTA per row (grid-stride), row cached in registers.  Bound by HBM: it reads x (and res) and
+// writes h (with res) and y.  32768 x 4096 with residual: 240 us with loads of one row at a time, 172 us with the row ring
+// (copy bandwidth would give 161).
 // ------------------------------------------------------------------------------------------
 template <int MAXV>
-__global__ void __launch_bounds__(kLnThreads)
+__global__ void __launch_bounds__(kLnThreads, MAXV == 1 ? 5 : MAXV == 2 ? 4 : 1)
 ln_fwd_kernel(int mode, const uint4* __restrict__ x, const uint4* __restrict__ res,
               uint4* __restrict__ h_out, uint4* __restrict__ y, const uint4* __restrict__ gamma,
               const uint4* __restrict__ beta, float* __restrict__ stats,
               float* __restrict__ mean_rstd, int rows, int cols, int total_cols, float eps,
               const __grid_constant__ RowExchange ex) {
-  __shared__ float red[64];
-  const int nvec = cols >> 3;
+  extern __shared__ uint4 ring[];
+  constexpr int S = ln_stages(false, MAXV);
+  __shared__ float red[128];
+  int parity = 0;
+  const int nvec = cols >> 3, T = blockDim.x;
+  const bool add = mode != 2 && res != nullptr;
+  const int inputs = add ? 2 : 1;
+  auto slot = [&](int stage, int input, int k) {
+    return ring + ((stage * inputs + input) * MAXV + k) * T + threadIdx.x;
+  };
+  auto prefetch = [&](uint32_t row, int stage) {
+    if (row < (uint32_t)rows) {
+      const int64_t base = (int64_t)row * nvec;
+#pragma unroll
+      for (int k = 0; k < MAXV; ++k) {
+        const int v = threadIdx.x + k * T;
+        if (v < nvec) {
+          cp_async16(slot(stage, 0, k), x + base + v);
+          if (add) cp_async16(slot(stage, 1, k), res + base + v);
+        }
+      }
+    }
+    cp_async_commit();
+  };
+#pragma unroll
+  for (int i = 0; i < S - 1; ++i) prefetch(blockIdx.x + i * gridDim.x, i);
+  int stage = 0;
   // With an exchange (ex.n > 0) mode 1 writes the partial statistics of its rows to every GPU of
   // the mesh row and counts one arrival per CTA on every peer; mode 2 first waits (bounded) for
   // the arrivals of all peers' CTAs and then sums the sources' statistics in fixed order.
@@ -157,14 +213,16 @@ ln_fwd_kernel(int mode, const uint4* __restrict__ x, const uint4* __restrict__ r
     float vals[MAXV][8];
     float s = 0.f, ss = 0.f;
     const int64_t base = (int64_t)row * nvec;
+    prefetch((uint32_t)row + (S - 1) * gridDim.x, stage == 0 ? S - 1 : stage - 1);   // where the previous row was
+    cp_async_wait<S - 1>();
 #pragma unroll
     for (int k = 0; k < MAXV; ++k) {
-      const int v = threadIdx.x + k * blockDim.x;
+      const int v = threadIdx.x + k * T;
       if (v < nvec) {
-        unpack8(x[base + v], vals[k]);
-        if (mode != 2 && res != nullptr) {
+        unpack8(*slot(stage, 0, k), vals[k]);
+        if (add) {
           float r[8];
-          unpack8(res[base + v], r);
+          unpack8(*slot(stage, 1, k), r);
 #pragma unroll
           for (int i = 0; i < 8; ++i) vals[k][i] += r[i];
         }
@@ -177,6 +235,7 @@ ln_fwd_kernel(int mode, const uint4* __restrict__ x, const uint4* __restrict__ r
         for (int i = 0; i < 8; ++i) { s += vals[k][i]; ss += vals[k][i] * vals[k][i]; }
       }
     }
+    stage = stage + 1 == S ? 0 : stage + 1;
     float mean, rstd;
     if (mode == 2) {
       if (exchange) {
@@ -188,7 +247,7 @@ ln_fwd_kernel(int mode, const uint4* __restrict__ x, const uint4* __restrict__ r
         ss = stats[2 * row + 1];
       }
     } else {
-      block_sum2(s, ss, red);
+      block_sum2_alt(s, ss, red, parity);
       if (mode == 1) {
         if (threadIdx.x == 0) {
           if (exchange) {
@@ -210,7 +269,7 @@ ln_fwd_kernel(int mode, const uint4* __restrict__ x, const uint4* __restrict__ r
     }
 #pragma unroll
     for (int k = 0; k < MAXV; ++k) {
-      const int v = threadIdx.x + k * blockDim.x;
+      const int v = threadIdx.x + k * T;
       if (v < nvec) {
         float g[8], b[8], o[8];
         if (gamma != nullptr) unpack8(gamma[v], g);
@@ -233,23 +292,41 @@ ln_fwd_kernel(int mode, const uint4* __restrict__ x, const uint4* __restrict__ r
 // LayerNorm backward
 // ------------------------------------------------------------------------------------------
 // Sum of two values over the `gw` consecutive warps that share a row; every thread of the group gets the result.
-__device__ __forceinline__ void group_sum2(float& a, float& b, float* red, int gw) {
+// Alternating buffers as in block_sum2_alt.
+__device__ __forceinline__ void group_sum2(float& a, float& b, float* red, int& parity, int gw) {
   a = warp_sum(a);
   b = warp_sum(b);
   const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  __syncthreads();
-  if (l == 0) { red[w] = a; red[32 + w] = b; }
+  float* buf = red + parity * 64;
+  parity ^= 1;
+  if (l == 0) { buf[w] = a; buf[32 + w] = b; }
   __syncthreads();
   const int w0 = w / gw * gw;
   a = 0.f;
   b = 0.f;
-  for (int i = 0; i < gw; ++i) { a += red[w0 + i]; b += red[32 + w0 + i]; }
+  for (int i = 0; i < gw; ++i) { a += buf[w0 + i]; b += buf[32 + w0 + i]; }
+}
+// dst[0..4) += v: one 16-byte atomic where the address allows it.  Every CTA of the backward kernel ends with its sums
+// of dgamma and dbeta, to the same addresses: one by one they took 45 us for 4096 columns, of 102 for 8192 rows.
+__device__ __forceinline__ void add4(float* dst, float4 v) {
+  if ((reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
+    atomicAdd(reinterpret_cast<float4*>(dst), v);
+  } else {
+    atomicAdd(dst, v.x);
+    atomicAdd(dst + 1, v.y);
+    atomicAdd(dst + 2, v.z);
+    atomicAdd(dst + 3, v.w);
+  }
+}
+__device__ __forceinline__ void add8(float* dst, const float (&v)[8]) {
+  add4(dst, make_float4(v[0], v[1], v[2], v[3]));
+  add4(dst + 4, make_float4(v[4], v[5], v[6], v[7]));
 }
 
-// A CTA of up to kLnBwdThreads threads walks the rows grid-stride.  A 4096-wide row is one 16-byte vector per
-// thread: the per-thread dgamma / dbeta accumulators (16 registers per vector) are what limits occupancy, and all
-// three input vectors of a row (dy, h, dres) are requested before anything waits for them.  The rows stay packed
-// in registers between the two passes; gamma is loaded once per CTA.
+// A CTA of up to kLnBwdThreads threads walks the rows grid-stride.  A 4096-wide row is two 16-byte vectors per
+// thread: the per-thread dgamma / dbeta accumulators (16 registers per vector) are what limits occupancy, so the rows
+// ahead wait in the shared-memory ring and both passes over a row read it there; gamma is loaded once per CTA.  Bound by HBM (dy, h, dres read, dx written); 32768 x 4096 with dres: 254 us with loads of one row at a
+// time, 192 us now (copy bandwidth would give 161); 8192 x 12288: 290 and 146.
 // GROUPED (rows of at most 256 vectors, e.g. column shards): the CTA works on blockDim.x / tpr rows at a time,
 // `tpr` threads (whole warps) per row, and adds the row groups' dgamma / dbeta in shared memory before its one
 // atomic per column, so that narrow rows neither idle most of a CTA nor multiply the atomics.
@@ -261,8 +338,11 @@ ln_bwd_kernel(int mode, const uint4* __restrict__ dy, const uint4* __restrict__ 
               float* __restrict__ dgamma, float* __restrict__ dbeta, int rows, int cols,
               int total_cols, int tpr_arg, const __grid_constant__ RowExchange ex) {
   static_assert(!GROUPED || MAXV == 1, "grouped rows are one vector per thread");
-  __shared__ float red[64];
-  __shared__ float comb[GROUPED ? 2 * kLnGroupedMaxCols : 1];
+  extern __shared__ uint4 ring[];
+  constexpr int S = ln_stages(true, MAXV);
+  __shared__ float red[128];
+  int parity = 0;
+  __shared__ __align__(16) float comb[GROUPED ? 2 * kLnGroupedMaxCols : 1];
   const int nvec = cols >> 3;
   const int tpr = GROUPED ? tpr_arg : (int)blockDim.x;            // threads per row
   const int sub = GROUPED ? (int)threadIdx.x / tpr : 0;           // which of the CTA's rows
@@ -283,31 +363,49 @@ ln_bwd_kernel(int mode, const uint4* __restrict__ dy, const uint4* __restrict__ 
   const bool want_param_grads = mode != 2 && dgamma != nullptr;
   const bool want_dres = mode != 1 && dres != nullptr;
 
-  for (int r0 = blockIdx.x * rows_per_cta; r0 < rows; r0 += gridDim.x * rows_per_cta) {
-    const int row = r0 + sub;
-    const bool live = row < rows;          // the last rows of a grouped CTA may be missing; barriers stay uniform
-    const int64_t base = (int64_t)row * nvec;
-    uint4 pd[MAXV], ph[MAXV], pr[MAXV];
+  const int T = blockDim.x, inputs = want_dres ? 3 : 2;
+  auto slot = [&](int stage, int input, int k) {
+    return ring + ((stage * inputs + input) * MAXV + k) * T + threadIdx.x;
+  };
+  auto prefetch = [&](uint32_t row, int stage) {
+    if (row < (uint32_t)rows) {
+      const int64_t base = (int64_t)row * nvec;
 #pragma unroll
-    for (int k = 0; k < MAXV; ++k) {
-      const int v = tx + k * tpr;
-      pd[k] = make_uint4(0u, 0u, 0u, 0u);
-      ph[k] = make_uint4(0u, 0u, 0u, 0u);
-      if (live && v < nvec) {
-        pd[k] = __ldcs(dy + base + v);
-        ph[k] = __ldcs(h + base + v);
-        if (want_dres) pr[k] = __ldcs(dres + base + v);
+      for (int k = 0; k < MAXV; ++k) {
+        const int v = tx + k * tpr;
+        if (v < nvec) {
+          cp_async16(slot(stage, 0, k), dy + base + v);
+          cp_async16(slot(stage, 1, k), h + base + v);
+          if (want_dres) cp_async16(slot(stage, 2, k), dres + base + v);
+        }
       }
     }
-    const float mean = live ? mean_rstd[2 * row] : 0.f, rstd = live ? mean_rstd[2 * row + 1] : 0.f;
+    cp_async_commit();
+  };
+  const uint32_t n_rows = rows, step = gridDim.x * rows_per_cta, first = blockIdx.x * rows_per_cta + sub;
+#pragma unroll
+  for (int i = 0; i < S - 1; ++i) prefetch(first + i * step, i);
+  int stage = 0;
+  float2 stat_next = make_float2(0.f, 0.f);   // (mean, rstd) of the next row
+  if (first < n_rows) stat_next = make_float2(mean_rstd[2 * (int64_t)first], mean_rstd[2 * (int64_t)first + 1]);
+
+  for (uint32_t r0 = blockIdx.x * rows_per_cta; r0 < n_rows; r0 += step) {
+    const uint32_t row = r0 + sub;
+    const bool live = row < n_rows;        // the last rows of a grouped CTA may be missing; barriers stay uniform
+    const int64_t base = (int64_t)row * nvec;
+    prefetch(row + (S - 1) * step, stage == 0 ? S - 1 : stage - 1);
+    const float mean = stat_next.x, rstd = stat_next.y;
+    if (row + step < n_rows)
+      stat_next = make_float2(mean_rstd[2 * (int64_t)(row + step)], mean_rstd[2 * (int64_t)(row + step) + 1]);
+    cp_async_wait<S - 1>();
     float s1 = 0.f, s2 = 0.f;
 #pragma unroll
     for (int k = 0; k < MAXV; ++k) {
       const int v = tx + k * tpr;
       if (live && v < nvec) {
         float d[8], hv[8], gm[8];
-        unpack8(pd[k], d);
-        unpack8(ph[k], hv);
+        unpack8(*slot(stage, 0, k), d);
+        unpack8(*slot(stage, 1, k), hv);
         unpack8(pg[k], gm);
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
@@ -326,23 +424,24 @@ ln_bwd_kernel(int mode, const uint4* __restrict__ dy, const uint4* __restrict__ 
           s2 = 0.f;
           for (int q = 0; q < ex.n; ++q) { s1 += ex_get(ex, q, row, 2, 0); s2 += ex_get(ex, q, row, 2, 1); }
         } else {
-          s1 = stats[2 * row];
-          s2 = stats[2 * row + 1];
+          s1 = stats[2 * (int64_t)row];
+          s2 = stats[2 * (int64_t)row + 1];
         }
       }
     } else {
-      if (GROUPED) group_sum2(s1, s2, red, tpr >> 5);
-      else block_sum2(s1, s2, red);
+      if (GROUPED) group_sum2(s1, s2, red, parity, tpr >> 5);
+      else block_sum2_alt(s1, s2, red, parity);
       if (mode == 1) {
         if (tx == 0 && live) {
           if (exchange) {
             const float v2[2] = {s1, s2};
             ex_put<2>(ex, row, v2);
           } else {
-            stats[2 * row] = s1;
-            stats[2 * row + 1] = s2;
+            stats[2 * (int64_t)row] = s1;
+            stats[2 * (int64_t)row + 1] = s2;
           }
         }
+        stage = stage + 1 == S ? 0 : stage + 1;
         continue;
       }
     }
@@ -352,20 +451,21 @@ ln_bwd_kernel(int mode, const uint4* __restrict__ dy, const uint4* __restrict__ 
       const int v = tx + k * tpr;
       if (live && v < nvec) {
         float d[8], hv[8], gm[8], o[8];
-        unpack8(pd[k], d);
-        unpack8(ph[k], hv);
+        unpack8(*slot(stage, 0, k), d);
+        unpack8(*slot(stage, 1, k), hv);
         unpack8(pg[k], gm);
 #pragma unroll
         for (int i = 0; i < 8; ++i) o[i] = rstd * (d[i] * gm[i] - m1 - (hv[i] - mean) * rstd * m2);
         if (want_dres) {
           float r[8];
-          unpack8(pr[k], r);
+          unpack8(*slot(stage, 2, k), r);
 #pragma unroll
           for (int i = 0; i < 8; ++i) o[i] += r[i];
         }
         __stcs(dx + base + v, pack8(o));
       }
     }
+    stage = stage + 1 == S ? 0 : stage + 1;
   }
   if (exchange && mode == 1) ex_signal(ex);
   if (want_param_grads) {
@@ -380,20 +480,18 @@ ln_bwd_kernel(int mode, const uint4* __restrict__ dy, const uint4* __restrict__ 
         }
       }
       __syncthreads();
-      for (int i = threadIdx.x; i < cols; i += blockDim.x) {
-        atomicAdd(dgamma + i, comb[i]);
-        if (dbeta != nullptr) atomicAdd(dbeta + i, comb[cols + i]);
+      const float4* c4 = reinterpret_cast<const float4*>(comb);
+      for (int q = threadIdx.x; q < 2 * nvec; q += blockDim.x) {
+        add4(dgamma + q * 4, c4[q]);
+        if (dbeta != nullptr) add4(dbeta + q * 4, c4[2 * nvec + q]);
       }
     } else {
 #pragma unroll
       for (int k = 0; k < MAXV; ++k) {
         const int v = tx + k * tpr;
         if (v < nvec) {
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            atomicAdd(dgamma + v * 8 + i, accg[k][i]);
-            if (dbeta != nullptr) atomicAdd(dbeta + v * 8 + i, accb[k][i]);
-          }
+          add8(dgamma + v * 8, accg[k]);
+          if (dbeta != nullptr) add8(dbeta + v * 8, accb[k]);
         }
       }
     }
@@ -665,12 +763,12 @@ __global__ void embedding_bwd_pos_kernel(const uint4* __restrict__ dout, float* 
   }
 }
 
-// One CTA per row: as many threads as the row has 16-byte vectors (64..256), so that short
+// One CTA per row: as many threads as the row has 16-byte vectors (32..256), so that short
 // column-sharded rows do not leave half of the CTA idle.
 inline int ln_threads(int cols) {
   const int nvec = cols / 8;
   int t = (nvec + 31) / 32 * 32;
-  if (t < 64) t = 64;
+  if (t < 32) t = 32;
   if (t > kLnThreads) t = kLnThreads;
   return t;
 }
@@ -685,8 +783,28 @@ inline LnBwdShape ln_bwd_shape(int cols) {
     const int g = kLnBwdThreads / tpr;
     return {g * tpr, tpr, g, 1};
   }
+  // Two vectors per thread: the reductions and barriers of a row are shared by more of it than with one vector of twice
+  // the threads (32768 x 4096 with dres: 244 us with 512 threads of one vector, 192 us so).
+  tpr = ((nvec + 1) / 2 + 31) / 32 * 32;
   if (tpr > kLnBwdThreads) tpr = kLnBwdThreads;
   return {tpr, tpr, 1, (nvec + tpr - 1) / tpr};
+}
+
+// Shared memory of a row ring; CTAs of the forward kernel that an SM holds (by registers 1280 threads of one vector,
+// 1024 of two, 512 of four, 256 of eight; at most 24 CTAs), with a residual: that is the grid of one resident wave, whose rows follow one another.
+inline int ln_ring_bytes(bool backward, int inputs, int maxv, int threads) {
+  return ln_stages(backward, maxv) * inputs * maxv * threads * 16;
+}
+inline int ln_fwd_maxv(int cols) {
+  const int threads = ln_threads(cols), n = (cols / 8 + threads - 1) / threads;
+  return n <= 1 ? 1 : n <= 2 ? 2 : n <= 4 ? 4 : 8;
+}
+inline int ln_fwd_resident(int cols) {
+  const int threads = ln_threads(cols), maxv = ln_fwd_maxv(cols);
+  const int by_regs = (maxv == 1 ? 1280 : maxv == 2 ? 1024 : maxv == 4 ? 512 : 256) / threads;
+  const int by_smem = 224 * 1024 / (ln_ring_bytes(false, 2, maxv, threads) + 1280);
+  int n = by_regs < by_smem ? by_regs : by_smem;
+  return n < 1 ? 1 : n > 24 ? 24 : n;
 }
 
 inline int grid_for(int64_t n, int threads, int cap = 148 * 16) {
@@ -701,15 +819,25 @@ inline int grid_for(int64_t n, int threads, int cap = 148 * 16) {
 // ------------------------------------------------------------------------------------------
 // launchers
 // ------------------------------------------------------------------------------------------
+// Shared memory beyond 48 KiB, of which the kernels here use at most 17 statically, has to be allowed per kernel and
+// device.
+static cudaError_t allow_smem(const void* kernel, int bytes) {
+  return bytes <= 31 * 1024 ? cudaSuccess
+                            : cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+}
+
 int ce_grid(int rows) { return rows < 148 * 8 ? rows : 148 * 8; }
 
 int ln_grid(int backward, int rows, int cols) {
-  int cap = 148 * 16;
+  const int width = cols > 0 ? cols : 8 * kLnThreads;
+  // narrow rows: three waves, because few rows per CTA leave the last one uneven (32768 x 1024 with residual: 53 us with
+  // one wave, 48 with three, 65 without the ring)
+  int cap = 148 * ln_fwd_resident(width) * (ln_fwd_maxv(width) == 1 ? 3 : 1);
   if (backward) {
-    // one resident wave (1024 threads per SM at 64 registers): every CTA ends with one atomic per column for
+    // one resident wave (1024 threads per SM at 64 registers, 512 at 128): every CTA ends with its atomics for
     // dgamma / dbeta, so CTAs beyond what is resident only add atomics
     const LnBwdShape sh = ln_bwd_shape(cols > 0 ? cols : 8 * kLnBwdThreads);
-    cap = 148 * (1024 / sh.threads);
+    cap = 148 * ((sh.maxv == 1 ? 1024 : 512) / sh.threads);
     const int groups = (rows + sh.rows_per_cta - 1) / sh.rows_per_cta;
     return groups < cap ? groups : cap;
   }
@@ -721,6 +849,7 @@ cudaError_t ln_fwd(int mode, const void* x, const void* res, void* h_out, void* 
                    int cols, int total_cols, float eps, cudaStream_t stream, const RowExchange* exch) {
   if (cols % 8 != 0 || cols > 8 * kLnThreads * 8) return cudaErrorInvalidValue;
   if (exch != nullptr && mode != 1 && mode != 2) return cudaErrorInvalidValue;
+  if (rows <= 0) return cudaErrorInvalidValue;
   const int grid = ln_grid(0, rows, cols);
   RowExchange ex;
   if (exch != nullptr) ex = *exch; else memset(&ex, 0, sizeof(ex));
@@ -730,17 +859,18 @@ cudaError_t ln_fwd(int mode, const void* x, const void* res, void* h_out, void* 
   auto Y = reinterpret_cast<uint4*>(y);
   auto G = reinterpret_cast<const uint4*>(gamma);
   auto B = reinterpret_cast<const uint4*>(beta);
-  const int threads = ln_threads(cols);
-  const int nvec_per_thread = (cols / 8 + threads - 1) / threads;
-  if (nvec_per_thread <= 1)
-    ln_fwd_kernel<1><<<grid, threads, 0, stream>>>(mode, X, R, H, Y, G, B, stats, mean_rstd, rows, cols, total_cols, eps, ex);
-  else if (nvec_per_thread <= 2)
-    ln_fwd_kernel<2><<<grid, threads, 0, stream>>>(mode, X, R, H, Y, G, B, stats, mean_rstd, rows, cols, total_cols, eps, ex);
-  else if (nvec_per_thread <= 4)
-    ln_fwd_kernel<4><<<grid, threads, 0, stream>>>(mode, X, R, H, Y, G, B, stats, mean_rstd, rows, cols, total_cols, eps, ex);
-  else
-    ln_fwd_kernel<8><<<grid, threads, 0, stream>>>(mode, X, R, H, Y, G, B, stats, mean_rstd, rows, cols, total_cols, eps, ex);
-  return cudaGetLastError();
+  const int threads = ln_threads(cols), maxv = ln_fwd_maxv(cols);
+  const int smem = ln_ring_bytes(false, mode != 2 && res != nullptr ? 2 : 1, maxv, threads);
+  auto run = [&](auto kernel) {
+    const cudaError_t e = allow_smem(reinterpret_cast<const void*>(kernel), smem);
+    if (e != cudaSuccess) return e;
+    kernel<<<grid, threads, smem, stream>>>(mode, X, R, H, Y, G, B, stats, mean_rstd, rows, cols, total_cols, eps, ex);
+    return cudaGetLastError();
+  };
+  if (maxv == 1) return run(ln_fwd_kernel<1>);
+  if (maxv == 2) return run(ln_fwd_kernel<2>);
+  if (maxv == 4) return run(ln_fwd_kernel<4>);
+  return run(ln_fwd_kernel<8>);
 }
 
 cudaError_t ln_bwd(int mode, const void* dy, const void* h, const void* gamma,
@@ -758,15 +888,19 @@ cudaError_t ln_bwd(int mode, const void* dy, const void* h, const void* gamma,
   auto DR = reinterpret_cast<const uint4*>(dres);
   auto DX = reinterpret_cast<uint4*>(dx);
   const LnBwdShape sh = ln_bwd_shape(cols);
-  if (sh.rows_per_cta > 1 || cols <= kLnGroupedMaxCols)
-    ln_bwd_kernel<1, true><<<grid, sh.threads, 0, stream>>>(mode, DY, H, G, mean_rstd, DR, DX, stats, dgamma, dbeta, rows, cols, total_cols, sh.tpr, ex);
-  else if (sh.maxv <= 1)
-    ln_bwd_kernel<1, false><<<grid, sh.threads, 0, stream>>>(mode, DY, H, G, mean_rstd, DR, DX, stats, dgamma, dbeta, rows, cols, total_cols, sh.tpr, ex);
-  else if (sh.maxv <= 2)
-    ln_bwd_kernel<2, false><<<grid, sh.threads, 0, stream>>>(mode, DY, H, G, mean_rstd, DR, DX, stats, dgamma, dbeta, rows, cols, total_cols, sh.tpr, ex);
-  else
-    ln_bwd_kernel<4, false><<<grid, sh.threads, 0, stream>>>(mode, DY, H, G, mean_rstd, DR, DX, stats, dgamma, dbeta, rows, cols, total_cols, sh.tpr, ex);
-  return cudaGetLastError();
+  const int maxv = cols <= kLnGroupedMaxCols ? 1 : sh.maxv <= 2 ? 2 : sh.maxv;
+  const int smem = ln_ring_bytes(true, mode != 1 && dres != nullptr ? 3 : 2, maxv, sh.threads);
+  auto run = [&](auto kernel) {
+    const cudaError_t e = allow_smem(reinterpret_cast<const void*>(kernel), smem);
+    if (e != cudaSuccess) return e;
+    kernel<<<grid, sh.threads, smem, stream>>>(mode, DY, H, G, mean_rstd, DR, DX, stats, dgamma, dbeta, rows, cols,
+                                              total_cols, sh.tpr, ex);
+    return cudaGetLastError();
+  };
+  if (cols <= kLnGroupedMaxCols) return run(ln_bwd_kernel<1, true>);
+  if (maxv == 2) return run(ln_bwd_kernel<2, false>);
+  if (maxv == 3) return run(ln_bwd_kernel<3, false>);
+  return run(ln_bwd_kernel<4, false>);
 }
 
 cudaError_t gelu_fwd(const void* x, void* y, int64_t n, cudaStream_t stream) {

@@ -10,6 +10,36 @@ def _C():
     return _native.load(), _native.stream_ptr()
 
 
+@pytest.mark.parametrize("residual", [True, False])
+@pytest.mark.parametrize("cols,rows", [(8, 1), (264, 5000), (2048, 9001), (2056, 1300), (4096, 1187), (8192, 600), (8200, 333),
+                                       (12288, 450), (12296, 301), (16384, 300)])
+def test_layernorm_row_ring(cols, rows, residual):
+    """Every number of vectors per thread of both kernels, with fewer and with more rows than a CTA's ring holds, and
+    dgamma / dbeta on a 4-byte boundary (their 16-byte atomics need a check).  Row results are rounded to bf16 once (2^-8
+    of the value at most, with its fp32 statistics 2^-7 is safe); column sums are fp32 over ``rows`` values."""
+    from meshslice_b200.ops import functional as F
+    g = torch.Generator(device="cuda").manual_seed(cols + rows)
+    mk = lambda *s: torch.randn(*s, device="cuda", generator=g).bfloat16()
+    x, res, dy, dres = mk(rows, cols), mk(rows, cols), mk(rows, cols), mk(rows, cols)
+    gamma, beta = mk(cols), mk(cols)
+    h, y, mr = F.ln_full(x, res if residual else None, gamma, beta, 1e-5)
+    sums = torch.zeros(2 * cols + 2, device="cuda")
+    dg, db = sums[1:cols + 1], sums[cols + 1:2 * cols + 1]
+    dx = F.ln_bwd_full(dy, h, gamma, mr, dg, db, dres if residual else None)
+    torch.cuda.synchronize()
+    hh = (x.float() + res.float() if residual else x.float())
+    assert torch.equal(h, hh.bfloat16())
+    hd = h.double().requires_grad_(True)
+    gd, bd = gamma.double().requires_grad_(True), beta.double().requires_grad_(True)
+    ref = torch.nn.functional.layer_norm(hd, (cols,), gd, bd, 1e-5)
+    ref.backward(dy.double())
+    want = hd.grad + dres.double() if residual else hd.grad
+    close = lambda a, b: ((a.double() - b).abs() <= 2 ** -7 * b.abs() + 2 ** -7 * b.abs().mean()).all()
+    assert close(y, ref.detach()) and close(dx, want)
+    assert (dg.double() - gd.grad).abs().max() <= 1e-5 * rows ** 0.5 * 30 and (db.double() - bd.grad).abs().max() <= 1e-5 * rows ** 0.5 * 30
+    assert sums[0] == 0 and sums[-1] == 0
+
+
 @pytest.mark.parametrize("cols,rows", [(1024, 301), (768, 43), (64, 1000), (2048, 300), (4096, 300), (12288, 300)])
 def test_layernorm_fwd_bwd_single_pass(cols, rows):
     """Widths up to 2048 run several rows per CTA in the backward kernel (row counts that leave the last CTA
