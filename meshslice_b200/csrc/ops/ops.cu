@@ -614,6 +614,12 @@ __global__ void sumsq_kernel(const void* __restrict__ x, int is_fp32, int64_t nv
 // ------------------------------------------------------------------------------------------
 // vocab-parallel cross-entropy: one CTA per row
 // ------------------------------------------------------------------------------------------
+// Both kernels are bound by HBM and keep kCeVec vectors per thread in flight.  The partial pass reads a row once: every
+// thread keeps the maximum of its elements and the sum of exponentials relative to it, and rescales the sum when a group
+// of vectors raises the maximum (Milakov and Gimelshein, online softmax).  4096 rows x 50257: partial 124 us with two
+// passes over the row, 87 us so (now four fifths of the issue slots are taken); gradient 153 us with one vector in flight
+// and a test per element, 132 us so (copy bandwidth: 62 and 124).
+constexpr int kCeVec = 4;
 __global__ void __launch_bounds__(256)
 ce_partial_kernel(const __nv_bfloat16* __restrict__ logits, int64_t ld,
                   const int64_t* __restrict__ targets, int rows, int cols, int col_offset,
@@ -625,27 +631,55 @@ ce_partial_kernel(const __nv_bfloat16* __restrict__ logits, int64_t ld,
   for (int row = blockIdx.x; row < rows; row += gridDim.x) {
     const __nv_bfloat16* p = logits + (int64_t)row * ld;
     const uint4* pv = reinterpret_cast<const uint4*>(p);
-    float mx = -INFINITY;
-    for (int v = threadIdx.x; v < nvec; v += blockDim.x) {
-      float f[8];
-      unpack8(pv[v], f);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) mx = fmaxf(mx, f[i]);
-    }
-    for (int c = nvec * 8 + threadIdx.x; c < valid; c += blockDim.x)
-      mx = fmaxf(mx, __bfloat162float(p[c]));
-    mx = block_max(mx, red);
-    float s = 0.f, dummy = 0.f;
-    if (valid > 0) {
-      for (int v = threadIdx.x; v < nvec; v += blockDim.x) {
-        float f[8];
-        unpack8(pv[v], f);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) s += __expf(f[i] - mx);
+    float m = -INFINITY, s = 0.f;            // this thread's maximum, sum of exp(x - m)
+    auto raise = [&](float to) {
+      if (to > m) {
+        s *= __expf(m - to);                 // (0 while m is -inf: s is 0)
+        m = to;
       }
-      for (int c = nvec * 8 + threadIdx.x; c < valid; c += blockDim.x)
-        s += __expf(__bfloat162float(p[c]) - mx);
+    };
+    for (int v0 = threadIdx.x; v0 < nvec; v0 += blockDim.x * kCeVec) {
+      uint4 u[kCeVec];
+#pragma unroll
+      for (int j = 0; j < kCeVec; ++j) {
+        const int v = v0 + j * blockDim.x;
+        u[j] = v < nvec ? pv[v] : make_uint4(0xff80ff80u, 0xff80ff80u, 0xff80ff80u, 0xff80ff80u);   // -inf
+      }
+      float top = -INFINITY;
+#pragma unroll
+      for (int j = 0; j < kCeVec; ++j) {
+        float f[8];
+        unpack8(u[j], f);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) top = fmaxf(top, f[i]);
+      }
+      raise(top);
+      auto sum = [&](auto term) {
+        float part[kCeVec];
+#pragma unroll
+        for (int j = 0; j < kCeVec; ++j) {
+          float f[8];
+          unpack8(u[j], f);
+          part[j] = term(f[0]);
+#pragma unroll
+          for (int i = 1; i < 8; ++i) part[j] += term(f[i]);
+        }
+#pragma unroll
+        for (int j = 0; j < kCeVec; ++j) s += part[j];
+      };
+      // while everything seen is -inf nothing counts, except that a NaN has to show
+      if (m > -INFINITY) sum([&](float f) { return __expf(f - m); });
+      else sum([&](float f) { return f == f ? 0.f : f; });
     }
+    for (int c = nvec * 8 + threadIdx.x; c < valid; c += blockDim.x) {
+      const float f = __bfloat162float(p[c]);
+      raise(f);
+      if (f != -INFINITY) s += __expf(f - m);
+    }
+    const float mx = block_max(m, red);
+    float dummy = 0.f;
+    // a thread without elements adds nothing; a row of nothing but -inf has no sum (NaN), an empty one has 0
+    s = valid == 0 ? 0.f : m == -INFINITY && mx > -INFINITY ? s : s * __expf(m - mx);
     block_sum2(s, dummy, red);
     if (threadIdx.x == 0) {
       const int64_t t = targets[row] - col_offset;
@@ -693,17 +727,33 @@ ce_grad_kernel(__nv_bfloat16* __restrict__ logits, int64_t ld, const int64_t* __
     }
     const float inv = scale / se;
     const int64_t t = targets[row] - col_offset;
-    for (int v = threadIdx.x; v < nvec; v += blockDim.x) {
-      float f[8];
-      unpack8(pv[v], f);
+    for (int v0 = threadIdx.x; v0 < nvec; v0 += blockDim.x * kCeVec) {
+      uint4 u[kCeVec];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const int c = v * 8 + i;
-        float gsm = (c + col_offset < vocab) ? __expf(f[i] - mx) * inv : 0.f;
-        if (c == t) gsm -= scale;
-        f[i] = gsm;
+      for (int j = 0; j < kCeVec; ++j) {
+        const int v = v0 + j * blockDim.x;
+        if (v < nvec) u[j] = pv[v];
       }
-      pv[v] = pack8(f);
+#pragma unroll
+      for (int j = 0; j < kCeVec; ++j) {
+        const int v = v0 + j * blockDim.x;
+        if (v >= nvec) continue;
+        float f[8];
+        unpack8(u[j], f);
+        if (v * 8 + 8 + col_offset <= vocab && (t >> 3) != v) {   // neither padding nor the target: most vectors
+#pragma unroll
+          for (int i = 0; i < 8; ++i) f[i] = __expf(f[i] - mx) * inv;
+        } else {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const int c = v * 8 + i;
+            float gsm = (c + col_offset < vocab) ? __expf(f[i] - mx) * inv : 0.f;
+            if (c == t) gsm -= scale;
+            f[i] = gsm;
+          }
+        }
+        pv[v] = pack8(f);
+      }
     }
   }
 }
@@ -826,7 +876,9 @@ static cudaError_t allow_smem(const void* kernel, int bytes) {
                             : cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
 }
 
-int ce_grid(int rows) { return rows < 148 * 8 ? rows : 148 * 8; }
+// a row per CTA up to 32 per SM: blocks handed out as SMs get free leave no uneven last wave (4096 rows on 1184 CTAs: four
+// rows each, three for some)
+int ce_grid(int rows) { return rows < 148 * 32 ? rows : 148 * 32; }
 
 int ln_grid(int backward, int rows, int cols) {
   const int width = cols > 0 ? cols : 8 * kLnThreads;

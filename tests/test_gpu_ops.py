@@ -186,6 +186,47 @@ def test_adamw_matches_torch():
     assert (p.float() - ref.detach()).abs().max() < 0.02
 
 
+@pytest.mark.parametrize("cols,offset,vocab", [(8, 0, 5), (2048, 0, 2041), (8192, 0, 8192), (10240, 2048, 9999), (51200, 0, 50257),
+                                               (64, 128, 100)])
+def test_cross_entropy_row_statistics(cols, offset, vocab):
+    """One pass over a row: rows that raise the maximum late, masked columns (-inf), a lone finite value, nothing but -inf,
+    +inf, NaN and magnitudes of 1e4, against 64 bits.  The maximum is exact; the sum is fp32 over at most 51200 terms of
+    at most 1 whose exponentials carry 2^-21 of the argument's rounding each: 1e-4 relative."""
+    from meshslice_b200.ops import functional as F
+    g = torch.Generator(device="cuda").manual_seed(cols)
+    n = max(0, min(cols, vocab - offset))
+    x = torch.randn(12, cols, device="cuda", generator=g)
+    if n:
+        x[1] += torch.linspace(0, 30, cols, device="cuda")
+        x[2, ::2] = float("-inf")
+        x[3] = float("-inf"); x[3, n - 1] = -7.0
+        x[4] = float("-inf")
+        x[5, n // 2] = float("inf")
+        x[6, n // 3] = float("nan")
+        x[7] *= 1e4
+        x[8] = -1e4
+        x[9, : n - 1] = float("-inf")
+        x[10] = float("-inf"); x[10, 0] = float("nan")
+    x = x.bfloat16()
+    t = torch.full((12,), offset + max(0, n - 1), device="cuda")
+    mx, se, tl = F.ce_partial(x, t, offset, vocab)
+    torch.cuda.synchronize()
+    if n == 0:
+        assert (mx == float("-inf")).all() and (se == 0).all() and (tl == 0).all()
+        return
+    d = x[:, :n].double()
+    assert torch.equal(tl, x[:, n - 1].float())
+    for r in range(12):
+        row = d[r]
+        want_m = row[~row.isnan()].max() if (~row.isnan()).any() else torch.tensor(float("-inf"))
+        assert mx[r].item() == want_m.item(), r
+        want = torch.exp(row - want_m).sum().item()
+        if want != want:
+            assert se[r].item() != se[r].item(), r
+        else:
+            assert abs(se[r].item() - want) <= 1e-4 * want, (r, se[r].item(), want)
+
+
 def test_cross_entropy_vocab_parallel():
     C, st = _C()
     rows, vocab, parts = 96, 1000, 4
