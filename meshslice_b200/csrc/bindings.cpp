@@ -465,6 +465,9 @@ PYBIND11_MODULE(_C, m) {
   m.def("sumsq", [](uint64_t x, int is_fp32, int64_t n, uint64_t out, uint64_t stream) {
     check(sumsq(P<void>(x), is_fp32, n, P<float>(out), S(stream)), "sumsq");
   });
+  m.def("clip_scale", [](uint64_t sq, int n, float max_norm, uint64_t norm, uint64_t scale, uint64_t stream) {
+    check(clip_scale(P<float>(sq), n, max_norm, P<float>(norm), P<float>(scale), S(stream)), "clip_scale");
+  });
   m.def("ce_partial", [](uint64_t logits, int64_t ld, uint64_t targets, int rows, int cols,
                          int col_offset, int vocab, uint64_t row_max, uint64_t row_sumexp,
                          uint64_t tgt_logit, uint64_t stream, py::object exch) {
@@ -477,13 +480,14 @@ PYBIND11_MODULE(_C, m) {
      py::arg("stream"), py::arg("exch") = py::none());
   m.def("ce_grad", [](uint64_t logits, int64_t ld, uint64_t targets, int rows, int cols,
                       int col_offset, int vocab, uint64_t gmax, uint64_t gsum, float scale,
-                      uint64_t stream, uint64_t row_loss, py::object exch) {
+                      uint64_t stream, uint64_t row_loss, py::object exch, uint64_t tgt_logit) {
     const ParsedExchange e = parse_exchange(exch);
     check(ce_grad(P<void>(logits), ld, P<int64_t>(targets), rows, cols, col_offset, vocab,
-                  P<float>(gmax), P<float>(gsum), scale, S(stream), P<float>(row_loss), e.ptr()), "ce_grad");
+                  P<float>(gmax), P<float>(gsum), scale, S(stream), P<float>(row_loss), e.ptr(),
+                  P<float>(tgt_logit)), "ce_grad");
   }, py::arg("logits"), py::arg("ld"), py::arg("targets"), py::arg("rows"), py::arg("cols"),
      py::arg("col_offset"), py::arg("vocab"), py::arg("gmax"), py::arg("gsum"), py::arg("scale"),
-     py::arg("stream"), py::arg("row_loss") = 0, py::arg("exch") = py::none());
+     py::arg("stream"), py::arg("row_loss") = 0, py::arg("exch") = py::none(), py::arg("tgt_logit") = 0);
   m.def("embedding_fwd", [](uint64_t tokens, uint64_t tok, uint64_t pos, uint64_t out, int n_tokens,
                             int seq, int cols, uint64_t stream) {
     check(embedding_fwd(P<int64_t>(tokens), P<void>(tok), P<void>(pos), P<void>(out), n_tokens, seq,

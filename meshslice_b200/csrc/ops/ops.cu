@@ -592,6 +592,16 @@ __global__ void adamw_kernel(uint2* __restrict__ param, float4* __restrict__ mas
   }
 }
 
+// The clipping factor in one launch of one thread instead of seven of a scalar each (20 us of an optimizer step).
+__global__ void clip_scale_kernel(const float* __restrict__ sq, int n, float max_norm, float* __restrict__ norm,
+                                  float* __restrict__ scale) {
+  float s = 0.f;
+  for (int i = 0; i < n; ++i) s += sq[i];
+  const float len = sqrtf(s), f = max_norm / (len + 1e-6f);
+  *norm = len;
+  *scale = f > 1.0f ? 1.0f : f;    // NaN stays NaN
+}
+
 __global__ void sumsq_kernel(const void* __restrict__ x, int is_fp32, int64_t nvec,
                              float* __restrict__ out) {
   __shared__ float red[64];
@@ -701,7 +711,7 @@ __global__ void __launch_bounds__(256)
 ce_grad_kernel(__nv_bfloat16* __restrict__ logits, int64_t ld, const int64_t* __restrict__ targets,
                int rows, int cols, int col_offset, int vocab, const float* __restrict__ gmax,
                const float* __restrict__ gsumexp, float scale, float* __restrict__ row_loss,
-               const __grid_constant__ RowExchange ex) {
+               const float* __restrict__ tgt_logit, const __grid_constant__ RowExchange ex) {
   const int nvec = cols >> 3;
   if (ex.n > 0 && !ex_wait(ex, 2u)) return;
   for (int row = blockIdx.x; row < rows; row += gridDim.x) {
@@ -724,6 +734,7 @@ ce_grad_kernel(__nv_bfloat16* __restrict__ logits, int64_t ld, const int64_t* __
     } else {
       mx = gmax[row];
       se = gsumexp[row];
+      if (threadIdx.x == 0 && row_loss != nullptr) row_loss[row] = logf(se) + mx - tgt_logit[row];
     }
     const float inv = scale / se;
     const int64_t t = targets[row] - col_offset;
@@ -988,6 +999,12 @@ cudaError_t adamw_step(void* param, float* master, float* m, float* v, const voi
   return cudaGetLastError();
 }
 
+cudaError_t clip_scale(const float* sq, int n, float max_norm, float* norm, float* scale, cudaStream_t stream) {
+  if (n < 1) return cudaErrorInvalidValue;
+  clip_scale_kernel<<<1, 1, 0, stream>>>(sq, n, max_norm, norm, scale);
+  return cudaGetLastError();
+}
+
 cudaError_t sumsq(const void* x, int is_fp32, int64_t n, float* out, cudaStream_t stream) {
   if (n % 4) return cudaErrorInvalidValue;
   sumsq_kernel<<<grid_for(n / 4, 256, 148 * 8), 256, 0, stream>>>(x, is_fp32, n / 4, out);
@@ -1006,12 +1023,13 @@ cudaError_t ce_partial(const void* logits, int64_t ld, const int64_t* targets, i
 }
 cudaError_t ce_grad(void* logits, int64_t ld, const int64_t* targets, int rows, int cols,
                     int col_offset, int vocab, const float* gmax, const float* gsumexp, float scale,
-                    cudaStream_t stream, float* row_loss, const RowExchange* exch) {
+                    cudaStream_t stream, float* row_loss, const RowExchange* exch, const float* tgt_logit) {
+  if (row_loss != nullptr && exch == nullptr && tgt_logit == nullptr) return cudaErrorInvalidValue;
   RowExchange ex;
   if (exch != nullptr) ex = *exch; else memset(&ex, 0, sizeof(ex));
   if (ld % 8 || cols % 8) return cudaErrorInvalidValue;
   const int grid = ce_grid(rows);
-  ce_grad_kernel<<<grid, 256, 0, stream>>>(reinterpret_cast<__nv_bfloat16*>(logits), ld, targets, rows, cols, col_offset, vocab, gmax, gsumexp, scale, row_loss, ex);
+  ce_grad_kernel<<<grid, 256, 0, stream>>>(reinterpret_cast<__nv_bfloat16*>(logits), ld, targets, rows, cols, col_offset, vocab, gmax, gsumexp, scale, row_loss, tgt_logit, ex);
   return cudaGetLastError();
 }
 

@@ -76,6 +76,9 @@ cudaError_t adamw_step(void* param, float* master, float* m, float* v, const voi
                        float weight_decay, float bias_corr1, float bias_corr2,
                        const float* grad_scale, cudaStream_t stream);
 
+// norm[0] = sqrt(sq[0] + ... + sq[n - 1]); scale[0] = min(1, max_norm / (norm + 1e-6)), NaN if norm is.
+cudaError_t clip_scale(const float* sq, int n, float max_norm, float* norm, float* scale, cudaStream_t stream);
+
 // out[0] += sum of squares of x (bf16 or fp32), fp32 atomics.
 cudaError_t sumsq(const void* x, int is_fp32, int64_t n, float* out, cudaStream_t stream);
 
@@ -90,12 +93,13 @@ cudaError_t ce_partial(const void* logits, int64_t ld, const int64_t* targets, i
                        float* tgt_logit, cudaStream_t stream, const RowExchange* exch = nullptr);
 int ce_grid(int rows);   // CTAs of ce_partial (each counts one arrival in an exchange)
 // pass 2: logits <- (softmax - onehot) * scale, in place, using the global max / sumexp.
-// With `exch` the global max / sumexp are combined from the mesh row's published partials (gmax /
-// gsumexp unused) and row_loss[row] = log(sumexp) + max - target logit is written when non-null.
+// row_loss[row] = log(sumexp) + max - target logit is written when non-null: with `exch` the three values
+// are combined from the mesh row's published partials (gmax / gsumexp / tgt_logit unused), otherwise
+// they are the arrays given.
 cudaError_t ce_grad(void* logits, int64_t ld, const int64_t* targets, int rows, int cols,
                     int col_offset, int vocab, const float* gmax, const float* gsumexp,
                     float scale, cudaStream_t stream, float* row_loss = nullptr,
-                    const RowExchange* exch = nullptr);
+                    const RowExchange* exch = nullptr, const float* tgt_logit = nullptr);
 
 // ---- embedding ----------------------------------------------------------------------------
 // out[t, :] = tok_table[token[t], :] + pos_table[t % seq, :]   (tables bf16 [*, cols])

@@ -200,6 +200,11 @@ class GPTModel:
             F.ce_partial(l0, targets.shards[k0], k0[1] * vc, cfg.vocab, exch=prod)
             row_loss = F.ce_grad_exchanged_(l0, targets.shards[k0], k0[1] * vc, cfg.vocab, 1.0 / n_tokens_global, cons)
             loss = ShardedTensor(m, {k0: row_loss.sum() / n_tokens_global})
+        elif m.C == 1:
+            # whole rows on one device: nothing to combine between the two passes
+            row_loss = {k: F.ce_grad_loss_(l, targets.shards[k], 0, cfg.vocab, *F.ce_partial(l, targets.shards[k], 0, cfg.vocab),
+                                           1.0 / n_tokens_global) for k, l in logits.shards.items()}
+            loss = ShardedTensor(m, {k: v.sum() / n_tokens_global for k, v in row_loss.items()})
         else:
             parts = {k: F.ce_partial(logits.shards[k], targets.shards[k], k[1] * vc, cfg.vocab) for k in m.coords()}
             mx = ShardedTensor(m, {k: v[0] for k, v in parts.items()})

@@ -285,6 +285,18 @@ def ce_grad_exchanged_(logits, targets, col_offset: int, vocab: int, scale: floa
     return row_loss
 
 
+def ce_grad_loss_(logits, targets, col_offset: int, vocab: int, gmax, gsum, tgt_logit, scale: float):
+    """``ce_grad_`` that also returns the per-row loss log(gsum) + gmax - tgt_logit [rows] (one launch on a GPU)."""
+    if logits.is_cuda:
+        rows, cols = logits.shape
+        row_loss = torch.empty(rows, device=logits.device, dtype=torch.float32)
+        _C().ce_grad(logits.data_ptr(), logits.stride(0), targets.data_ptr(), rows, cols, col_offset, vocab,
+                     gmax.data_ptr(), gsum.data_ptr(), scale, _st(), row_loss.data_ptr(), None, tgt_logit.data_ptr())
+        return row_loss
+    ce_grad_(logits, targets, col_offset, vocab, gmax, gsum, scale)
+    return torch.log(gsum) + gmax - tgt_logit
+
+
 def ce_grad_(logits, targets, col_offset: int, vocab: int, gmax, gsum, scale: float):
     """In place: logits <- (softmax - onehot) * scale (padding columns get 0)."""
     rows, cols = logits.shape

@@ -50,17 +50,22 @@ class AdamW:
                                      g.grad.numel(), self._sq[idx:idx + 1].data_ptr(), _native.stream_ptr())
             else:
                 self._sq[idx] += g.grad.float().pow(2).sum()
-        sq = self._sq.clone()
+        sq = self._sq
         if self.mesh is not None and self.mesh.R * self.mesh.C > 1 and hasattr(self.mesh, "dist"):
             d = self.mesh.dist
+            sq = sq.clone()
             if self.mesh.R > 1:
                 # replicated parameters are identical along a mesh column: count them once
                 sq[1] = sq[1] / self.mesh.R
             d.all_reduce(sq, group=self.mesh.group)
-        norm = torch.sqrt(sq.sum())
-        self.last_grad_norm = norm
-        torch.clamp(self.max_grad_norm / (norm + 1e-6), max=1.0, out=self._scale[0:1]) if False else \
+        if sq.is_cuda:
+            norm = torch.empty((), dtype=torch.float32, device=sq.device)
+            _native.load().clip_scale(sq.data_ptr(), sq.numel(), self.max_grad_norm, norm.data_ptr(),
+                                      self._scale.data_ptr(), _native.stream_ptr())
+        else:
+            norm = torch.sqrt(sq.sum())
             self._scale.copy_(torch.clamp(self.max_grad_norm / (norm + 1e-6), max=1.0).reshape(1))
+        self.last_grad_norm = norm
         return self._scale
 
     def step(self):

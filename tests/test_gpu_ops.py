@@ -350,3 +350,29 @@ def test_layernorm_row_exchange_emulated_ranks(n, w, rows):
     # every rank's counter has seen exactly the other ranks' CTAs
     for q in range(n):
         assert int(keep2[1][q][0]) == (n - 1) * C.ln_grid(1, rows, w)
+
+
+@pytest.mark.parametrize("sq", [(0.0, 0.0), (9.0, 16.0), (0.09, 0.16), (float("inf"), 1.0), (float("nan"), 1.0)])
+def test_clip_scale(sq):
+    """Norm and clipping factor as the optimizer's CPU path computes them (three fp32 roundings: 2^-21)."""
+    C, st = _C()
+    t = torch.tensor(sq, device="cuda")
+    out = torch.zeros(2, device="cuda")
+    C.clip_scale(t.data_ptr(), 2, 1.0, out.data_ptr(), out.data_ptr() + 4, st)
+    norm = torch.sqrt(t.cpu().sum())
+    want = torch.stack([norm, torch.clamp(1.0 / (norm + 1e-6), max=1.0)])
+    assert torch.allclose(out.cpu(), want, rtol=2 ** -21, atol=0, equal_nan=True)
+
+
+def test_cross_entropy_gradient_returns_the_row_loss():
+    """One launch for gradient and loss: the gradient is that of ce_grad_ bit for bit, the loss log(sum) + max - target."""
+    from meshslice_b200.ops import functional as F
+    x = (3 * torch.randn(5, 4096, device="cuda")).bfloat16()
+    t = torch.tensor([0, 7, 8, 3990, 1234], device="cuda")
+    mx, se, tl = F.ce_partial(x, t, 0, 3991)
+    a, b = x.clone(), x.clone()
+    F.ce_grad_(a, t, 0, 3991, mx, se, 0.2)
+    loss = F.ce_grad_loss_(b, t, 0, 3991, mx, se, tl, 0.2)
+    ref = torch.nn.functional.cross_entropy(x[:, :3991].double(), t, reduction="none")
+    assert torch.equal(a, b)
+    assert (loss.double() - ref).abs().max() < 1e-4
