@@ -14,6 +14,7 @@
 #include <cuda_bf16.h>
 
 #include "../common/ptx.cuh"
+#include "out_turn.h"
 #include "sm100_gemm.h"
 
 namespace msb {
@@ -174,20 +175,20 @@ __device__ __forceinline__ void tma_store_box(const CUtensorMap* map, const void
     asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];"
                  ::"l"(map), "r"(smem_u32(src)), "r"(x), "r"(y) : "memory");
 }
-// Staging of one epilogue warp: two boxes in turn, each free again once the copy engine has read it: all but the last
-// `1 - taken` stores.  With taken = 1 (another box may be held unsent) none may be outstanding.
+// Staging of one epilogue warp: two boxes, each free again once the copy engine has read it.  take() waits for all but
+// the last `1 - taken` stores; OutTurn never names the box sent last.  With taken = 1 (the other box may be held unsent) no
+// store may be outstanding.
 struct OutStage {
   uint8_t* base;
-  int next;
+  OutTurn turn;
   template <int taken = 0>
   __device__ __forceinline__ uint8_t* take(int lane) {
     if (lane == 0) bulk_wait_read<1 - taken>();
     __syncwarp();
-    uint8_t* p = base + next * kOutBox;
-    next ^= 1;
-    return p;
+    return base + turn.take() * kOutBox;
   }
   __device__ __forceinline__ void send(const CUtensorMap* map, const uint8_t* box, int lane, int32_t x, int32_t y, bool add) {
+    turn.sent(box == base ? 0 : 1);
     fence_proxy_async_smem();
     __syncwarp();
     if (lane == 0) {
@@ -386,7 +387,7 @@ sm100_gemm2_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_const
     const int q = warp & 3;
     const __nv_bfloat16* bias = reinterpret_cast<const __nv_bfloat16*>(a.bias);
     const bool dual = a.act == 1 && a.C_pre != nullptr;   // two outputs: no store of one runs under the other's staging
-    OutStage out{smem + kSmemOut2 + q * 2 * kOutBox, 0};
+    OutStage out{smem + kSmemOut2 + q * 2 * kOutBox, {0}};
     bool ok = true;
     int it = 0;
     for (int t = cluster_id; t < num_tiles && ok; t += n_clusters, ++it) {

@@ -120,3 +120,22 @@ def test_gemm_output_boxes(layout, shape):
     assert (pre.double() - ref).abs().max().item() <= 2 ** -8 * scale
     g = torch.nn.functional.gelu(ref, approximate="tanh")
     assert ((out.double() - g).abs() <= 2 ** -8 * g.abs() + 2e-3 * ref.abs() + 1e-3).all()
+
+
+@pytest.mark.parametrize("shape", [(20000, 24, 72), (20000, 8, 64), (15300, 536, 136), (10200, 288, 64)])
+def test_gemm_gelu_fp32_output_with_half_a_box_left(shape):
+    """fp32 result and bf16 pre-activation with 1 to 32 columns in the last group of 64 (the second fp32 box is left out
+    there), several tiles per CTA: what one tile leaves in its staging must not meet the next one's.  Bounds as above."""
+    from meshslice_b200 import _native
+    from meshslice_b200.ops.gemm import gemm
+    M, N, K = shape
+    a, b = _operands(M, N, K, "nt", seed=N)
+    ref = a.double() @ b.double().t()
+    scale = ref.abs().max().item()
+    g = torch.nn.functional.gelu(ref, approximate="tanh")
+    for _ in range(3):
+        pre = torch.full((M, N), 3.0, device="cuda", dtype=torch.bfloat16)
+        out = gemm(a, b, "nt", out_dtype=torch.float32, act="gelu", pre_act=pre)
+        _native.check_status()
+        assert (pre.double() - ref).abs().max().item() <= 2 ** -8 * scale
+        assert ((out.double() - g).abs() <= 2e-3 * ref.abs() + 1e-3).all()
