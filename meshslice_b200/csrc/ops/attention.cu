@@ -588,7 +588,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_consta
 // Bound by HBM (it reads O and dO once): 16 lanes with a 16-byte vector each take one head of kDeltaRows consecutive
 // tokens, all loads requested before the first sum, and write neighbouring statistics.  33.5 M elements, cold: 52 us
 // with a warp per (token, head) and 8 bytes per lane, 26 us so.
-// kWide: `out` is 16-byte aligned (dout always is: the tensor map asks for it).
+// kWide: `out` is 16-byte aligned (dout always is: the host refuses other addresses).
 constexpr int kDeltaRows = 4;
 static_assert(kBlk % kDeltaRows == 0, "sequences are whole groups of rows");
 template <bool kWide>
@@ -1146,28 +1146,33 @@ cudaError_t attention_bwd(const void* qkv, const void* out, const void* dout, co
                           int causal, float scale, uint32_t* status, cudaStream_t stream) {
   if (seq % kBlk != 0 || batch <= 0 || heads <= 0 || (int64_t)batch * heads > 65535 || seq / kBlk > 65535)
     return cudaErrorInvalidValue;
+  // All that is refused is refused before the first launch: the row-sum kernel reads `dout` 16 and `out` at least 8 bytes
+  // at a time, bulk copies read the statistics.
+  const auto off = [](const void* p, uintptr_t align) { return (reinterpret_cast<uintptr_t>(p) & (align - 1)) != 0; };
+  if (off(qkv, 16) || off(dout, 16) || off(dqkv, 16) || off(out, 8) || off(dq_acc, 16) || off(delta, 16))
+    return cudaErrorInvalidValue;
   {
     cudaError_t e0 = configure_device();
     if (e0 != cudaSuccess) return e0;
   }
   const int64_t tokens = (int64_t)batch * seq;
-  {
-    // -delta * scale into `delta`, -lse * log2(e) into the head of the `dq_acc` scratch
-    const int64_t groups = tokens / kDeltaRows * heads;   // below 2^32: a group is 2 KiB of activations
-    const int threads = 256, per_block = threads / 16;
-    const int64_t blocks = (groups + per_block - 1) / per_block;
-    auto kernel = (reinterpret_cast<uintptr_t>(out) & 15) == 0 ? attn_delta_kernel<true> : attn_delta_kernel<false>;
-    kernel<<<(unsigned)blocks, threads, 0, stream>>>(reinterpret_cast<const uint4*>(out), reinterpret_cast<const uint4*>(dout),
-                                                     delta, (uint32_t)groups, seq, heads, lse, dq_acc, scale);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-  }
   CUtensorMap tq, td;
   const uint64_t width = (uint64_t)heads * 3 * kD, wdo = (uint64_t)heads * kD;
   if (make_tensor_map_2d(&tq, qkv, width, (uint64_t)tokens, width * 2, 64, kBlk) != 0) return cudaErrorInvalidValue;
   if (make_tensor_map_2d(&td, dout, wdo, (uint64_t)tokens, wdo * 2, 64, kBlk) != 0) return cudaErrorInvalidValue;
   CUtensorMap tg;
   if (make_tensor_map_2d(&tg, dqkv, width, (uint64_t)tokens, width * 2, kBwdCols, 32, 64) != 0) return cudaErrorInvalidValue;
+  {
+    // -delta * scale into `delta`, -lse * log2(e) into the head of the `dq_acc` scratch
+    const int64_t groups = tokens / kDeltaRows * heads;   // below 2^32: a group is 2 KiB of activations
+    const int threads = 256, per_block = threads / 16;
+    const int64_t blocks = (groups + per_block - 1) / per_block;
+    auto kernel = off(out, 16) ? attn_delta_kernel<false> : attn_delta_kernel<true>;
+    kernel<<<(unsigned)blocks, threads, 0, stream>>>(reinterpret_cast<const uint4*>(out), reinterpret_cast<const uint4*>(dout),
+                                                     delta, (uint32_t)groups, seq, heads, lse, dq_acc, scale);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+  }
   // two deterministic kernels: dK / dV per key block, dQ per query block
   Bwd2Args g{};
   g.lse2 = dq_acc;     // -lse * log2(e)

@@ -14,7 +14,8 @@ cudaError_t attention_fwd(const void* qkv, void* out, float* lse, int batch, int
 
 // dqkv (same layout as qkv) from dout.  `dq_acc` and `delta` are fp32 scratch of at least
 // batch * heads * seq elements each (they receive -lse * log2(e) and -rowsum(dO * O) * scale); both
-// are overwritten.  The gradients are accumulated in tensor memory by the CTA that owns them, so the
+// are overwritten.  qkv, dout, dqkv and the scratch start on 16-byte boundaries, out on 8 (cudaErrorInvalidValue
+// otherwise, before anything is launched).  The gradients are accumulated in tensor memory by the CTA that owns them, so the
 // result is bit-identical from run to run.
 cudaError_t attention_bwd(const void* qkv, const void* out, const void* dout, const float* lse,
                           void* dqkv, float* dq_acc, float* delta, int batch, int seq, int heads,

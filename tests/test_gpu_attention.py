@@ -81,6 +81,24 @@ def test_attention_backward_takes_out_on_an_8_byte_boundary():
     assert torch.equal(a, b)
 
 
+def test_attention_backward_refuses_dout_off_a_16_byte_boundary():
+    """The refusal comes from the host; the same call on an aligned copy works afterwards."""
+    from meshslice_b200 import _native
+    from meshslice_b200.ops import functional as F
+    batch, seq, heads = 1, 128, 2
+    qkv = torch.randn(batch * seq, heads * 3 * 128, device="cuda").bfloat16()
+    out, lse = F.attention_fwd(qkv, batch, seq, heads, True)
+    dout = torch.randn(out.numel() + 4, device="cuda").bfloat16()[4:].view_as(out)
+    assert dout.data_ptr() % 16 == 8
+    with pytest.raises(RuntimeError, match="invalid argument"):
+        F.attention_bwd(dout, qkv, out, lse, batch, seq, heads, True)
+    dqkv = F.attention_bwd(dout.clone(), qkv, out, lse, batch, seq, heads, True)
+    torch.cuda.synchronize()
+    _native.check_status()
+    _, _, dref = _ref(qkv, batch, seq, heads, True, dout)
+    assert ((dqkv.float() - dref).norm() / dref.norm()).item() < 4 * 2 ** -9
+
+
 def test_attention_large_scores_exercise_rescaling():
     """Scores that grow along the keys force the running maximum (and O) to be rescaled."""
     from meshslice_b200 import _native
