@@ -203,6 +203,7 @@ void gemm_run(const py::dict& d) {
     const int rt = a.red_slice_dim == 0 ? (a.red_rows + 2 * kBM - 1) / (2 * kBM) : (a.red_cols + kBN - 1) / kBN;
     if (rt % (a.n_slices * a.cyc) != 0 || a.red_cols % 8 != 0 || a.red_ld % 8 != 0)
       throw std::runtime_error("gemm: reduce phase shape not divisible by the slice count");
+    if (reinterpret_cast<uintptr_t>(a.C) & 15) throw std::runtime_error("gemm: the reduce phase needs a 16-byte aligned C");
   }
   // barriers
   BarrierArgs b = parse_barrier(d);

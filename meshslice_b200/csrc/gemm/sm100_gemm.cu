@@ -474,13 +474,16 @@ __device__ void aux_warp_main(const GemmArgs& a, int aux) {
 // ------------------------------------------------------------------------------------------
 // epilogue helpers
 // ------------------------------------------------------------------------------------------
+// Rows are a multiple of 16 bytes apart (ldc % 8 == 0 for both types), but the matrix may start anywhere.
+__device__ __forceinline__ bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+
 // Stores 32 consecutive columns of one row.  `v` holds fp32 accumulators.
 __device__ __forceinline__ void store_row32(const GemmArgs& a, void* base, int64_t ld, bool fp32,
                                             bool accumulate, int64_t row, int col0, int ncols_valid,
                                             float (&v)[32]) {
   if (fp32) {
     float* p = reinterpret_cast<float*>(base) + row * ld + col0;
-    if (ncols_valid == 32) {
+    if (ncols_valid == 32 && aligned16(p)) {
 #pragma unroll
       for (int i = 0; i < 32; i += 4) {
         float4 o = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
@@ -497,7 +500,7 @@ __device__ __forceinline__ void store_row32(const GemmArgs& a, void* base, int64
     }
   } else {
     __nv_bfloat16* p = reinterpret_cast<__nv_bfloat16*>(base) + row * ld + col0;
-    if (ncols_valid == 32) {
+    if (ncols_valid == 32 && aligned16(p)) {
 #pragma unroll
       for (int i = 0; i < 32; i += 8) {
         uint4 o;

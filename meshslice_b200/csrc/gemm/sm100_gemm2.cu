@@ -115,11 +115,14 @@ __device__ __forceinline__ uint32_t pk2(float lo, float hi) {
 __device__ __forceinline__ float blo(uint32_t v) { return __uint_as_float(v << 16); }
 __device__ __forceinline__ float bhi(uint32_t v) { return __uint_as_float(v & 0xffff0000u); }
 
+// Rows are a multiple of 16 bytes apart (ldc % 8 == 0 for both types), but the matrix may start anywhere.
+__device__ __forceinline__ bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+
 __device__ __forceinline__ void store32(void* base, int64_t ld, bool fp32, bool accumulate, int64_t row,
                                         int col0, int nvalid, float (&v)[32]) {
   if (fp32) {
     float* p = reinterpret_cast<float*>(base) + row * ld + col0;
-    if (nvalid == 32) {
+    if (nvalid == 32 && aligned16(p)) {
 #pragma unroll
       for (int i = 0; i < 32; i += 4) {
         float4 o = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
@@ -136,7 +139,7 @@ __device__ __forceinline__ void store32(void* base, int64_t ld, bool fp32, bool 
     }
   } else {
     __nv_bfloat16* p = reinterpret_cast<__nv_bfloat16*>(base) + row * ld + col0;
-    if (nvalid == 32) {
+    if (nvalid == 32 && aligned16(p)) {
 #pragma unroll
       for (int i = 0; i < 32; i += 8) {
         uint4 o;

@@ -68,3 +68,12 @@ def harness(tmp_path_factory):
 def test_no_box_is_written_while_its_store_is_unread(harness, dual, fp32, cols):
     out = subprocess.run([str(harness), str(dual), str(fp32), str(cols)], capture_output=True, text=True, check=True)
     assert out.stdout.strip() == "0"
+
+
+def test_reduce_phase_refuses_a_misaligned_result():
+    """The slot sums are written 16 bytes at a time; the refusal is the host's."""
+    from meshslice_b200 import _native
+    d = dict(M=256, N=256, K=64, A=1 << 20, B=1 << 20, lda=64, ldb=64, C=(1 << 20) + 8, ldc=256, red_n=2, red_work=1 << 20,
+             red_slots=1 << 20, red_rows=256, red_cols=256, red_ld=256, status=1 << 20)
+    with pytest.raises(RuntimeError, match="16-byte aligned C"):
+        _native.load().gemm_run(d)

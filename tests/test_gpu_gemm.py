@@ -139,3 +139,42 @@ def test_gemm_gelu_fp32_output_with_half_a_box_left(shape):
         _native.check_status()
         assert (pre.double() - ref).abs().max().item() <= 2 ** -8 * scale
         assert ((out.double() - g).abs() <= 2e-3 * ref.abs() + 1e-3).all()
+
+
+@pytest.mark.parametrize("two_cta", [True, False])
+@pytest.mark.parametrize("offset", [1, 2, 4, 6])
+def test_gemm_output_may_start_at_any_element(offset, two_cta):
+    """C and C_pre off a 16-byte boundary (TMA cannot address them): every kind of output, whole and cut groups of 32
+    columns, guard values before and behind.  Bounds as in test_gemm_output_boxes."""
+    from meshslice_b200 import _native
+    from meshslice_b200.ops.gemm import gemm
+    M, N, K = 264, 328, 72
+    a, b = _operands(M, N, K, "nt", seed=offset)
+    ref = a.double() @ b.double().t()
+    scale = ref.abs().max().item() + 3.0
+
+    def placed(dtype):
+        flat = torch.full((M * N + 32,), 3.0, device="cuda", dtype=dtype)
+        return flat, flat[8 + offset:8 + offset + M * N].view(M, N)
+
+    def intact(flat):
+        return bool((flat[:8 + offset] == 3.0).all() and (flat[8 + offset + M * N:] == 3.0).all())
+
+    for dtype, acc, tol in ((torch.bfloat16, False, 2 ** -8), (torch.float32, False, 1e-5), (torch.float32, True, 1e-5),
+                            (torch.bfloat16, True, 2 ** -8)):
+        flat, out = placed(dtype)
+        gemm(a, b, "nt", out=out, accumulate=acc, two_cta=two_cta)
+        _native.check_status()
+        assert intact(flat), (dtype, acc)
+        assert (out.double() - ref - (3.0 if acc else 0.0)).abs().max().item() <= tol * scale, (dtype, acc)
+    g = torch.nn.functional.gelu(ref, approximate="tanh")
+    for where in ("both", "pre"):
+        flat, out = placed(torch.bfloat16)
+        if where == "pre":
+            out = torch.empty(M, N, device="cuda", dtype=torch.bfloat16)
+        flatp, pre = placed(torch.bfloat16)
+        gemm(a, b, "nt", out=out, act="gelu", pre_act=pre, two_cta=two_cta)
+        _native.check_status()
+        assert intact(flat) and intact(flatp)
+        assert (pre.double() - ref).abs().max().item() <= 2 ** -8 * scale
+        assert ((out.double() - g).abs() <= 2 ** -8 * g.abs() + 2e-3 * ref.abs() + 1e-3).all()
