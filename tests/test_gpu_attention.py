@@ -99,6 +99,28 @@ def test_attention_backward_refuses_dout_off_a_16_byte_boundary():
     assert ((dqkv.float() - dref).norm() / dref.norm()).item() < 4 * 2 ** -9
 
 
+@pytest.mark.parametrize("causal", [False, True])
+def test_attention_on_strided_tensors(causal):
+    """qkv, out and dout as column slices of wider tensors and a transposed lse: the same bits as on contiguous copies."""
+    from meshslice_b200 import _native
+    from meshslice_b200.ops import functional as F
+    batch, seq, heads = 2, 256, 3
+    g = torch.Generator(device="cuda").manual_seed(5)
+    rand = lambda cols: torch.randn(batch * seq, cols, device="cuda", generator=g).bfloat16()
+    cut = lambda t, n: t[:, 24:24 + n]
+    qkv, dout = cut(rand(heads * 384 + 64), heads * 384), cut(rand(heads * 128 + 64), heads * 128)
+    assert not qkv.is_contiguous()
+    out, lse = F.attention_fwd(qkv, batch, seq, heads, causal)
+    want, want_lse = F.attention_fwd(qkv.contiguous(), batch, seq, heads, causal)
+    assert torch.equal(out, want) and torch.equal(lse, want_lse)
+    strided_out = cut(torch.zeros(batch * seq, heads * 128 + 64, device="cuda").bfloat16(), heads * 128).copy_(out)
+    strided_lse = lse.transpose(1, 2).contiguous().transpose(1, 2)
+    assert not strided_out.is_contiguous() and not strided_lse.is_contiguous()
+    got = F.attention_bwd(dout, qkv, strided_out, strided_lse, batch, seq, heads, causal)
+    assert torch.equal(got, F.attention_bwd(dout.contiguous(), qkv.contiguous(), want, want_lse, batch, seq, heads, causal))
+    _native.check_status()
+
+
 def test_attention_large_scores_exercise_rescaling():
     """Scores that grow along the keys force the running maximum (and O) to be rescaled."""
     from meshslice_b200 import _native
