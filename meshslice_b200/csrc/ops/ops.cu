@@ -887,11 +887,14 @@ static cudaError_t allow_smem(const void* kernel, int bytes) {
                             : cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
 }
 
-// a row per CTA up to 32 per SM: blocks handed out as SMs get free leave no uneven last wave (4096 rows on 1184 CTAs: four
-// rows each, three for some)
-int ce_grid(int rows) { return rows < 148 * 32 ? rows : 148 * 32; }
+// Launch shapes.  In a row exchange every CTA ends in a system-wide fence and an add to the same counter of every peer,
+// which takes longer than a row, and every CTA of the second pass polls its own: one resident wave with several rows a CTA
+// (ce_partial_kernel: five CTAs an SM by registers).  On one device a row per CTA up to 32 per SM: blocks handed out as SMs
+// get free leave no uneven last wave (4096 rows on 1184 CTAs: four rows each, three for some).
+int ce_grid(int rows) { return rows < 148 * 5 ? rows : 148 * 5; }
+static int ce_local_grid(int rows) { return rows < 148 * 32 ? rows : 148 * 32; }
 
-int ln_grid(int backward, int rows, int cols) {
+static int ln_local_grid(int backward, int rows, int cols) {
   const int width = cols > 0 ? cols : 8 * kLnThreads;
   // narrow rows: three waves, because few rows per CTA leave the last one uneven (32768 x 1024 with residual: 53 us with
   // one wave, 48 with three, 65 without the ring)
@@ -906,6 +909,11 @@ int ln_grid(int backward, int rows, int cols) {
   }
   return rows < cap ? rows : cap;
 }
+int ln_grid(int backward, int rows, int cols) {
+  if (backward) return ln_local_grid(backward, rows, cols);   // already one wave
+  const int resident = ln_fwd_resident(cols > 0 ? cols : 8 * kLnThreads), cap = 148 * (resident < 16 ? resident : 16);
+  return rows < cap ? rows : cap;
+}
 
 cudaError_t ln_fwd(int mode, const void* x, const void* res, void* h_out, void* y,
                    const void* gamma, const void* beta, float* stats, float* mean_rstd, int rows,
@@ -913,7 +921,7 @@ cudaError_t ln_fwd(int mode, const void* x, const void* res, void* h_out, void* 
   if (cols % 8 != 0 || cols > 8 * kLnThreads * 8) return cudaErrorInvalidValue;
   if (exch != nullptr && mode != 1 && mode != 2) return cudaErrorInvalidValue;
   if (rows <= 0) return cudaErrorInvalidValue;
-  const int grid = ln_grid(0, rows, cols);
+  const int grid = exch != nullptr ? ln_grid(0, rows, cols) : ln_local_grid(0, rows, cols);
   RowExchange ex;
   if (exch != nullptr) ex = *exch; else memset(&ex, 0, sizeof(ex));
   auto X = reinterpret_cast<const uint4*>(x);
@@ -942,7 +950,7 @@ cudaError_t ln_bwd(int mode, const void* dy, const void* h, const void* gamma,
                    const RowExchange* exch) {
   if (cols % 8 != 0 || cols > 8 * kLnBwdThreads * 4) return cudaErrorInvalidValue;
   if (exch != nullptr && mode != 1 && mode != 2) return cudaErrorInvalidValue;
-  const int grid = ln_grid(1, rows, cols);
+  const int grid = exch != nullptr ? ln_grid(1, rows, cols) : ln_local_grid(1, rows, cols);
   RowExchange ex;
   if (exch != nullptr) ex = *exch; else memset(&ex, 0, sizeof(ex));
   auto DY = reinterpret_cast<const uint4*>(dy);
@@ -1017,7 +1025,7 @@ cudaError_t ce_partial(const void* logits, int64_t ld, const int64_t* targets, i
   RowExchange ex;
   if (exch != nullptr) ex = *exch; else memset(&ex, 0, sizeof(ex));
   if (ld % 8) return cudaErrorInvalidValue;
-  const int grid = ce_grid(rows);
+  const int grid = exch != nullptr ? ce_grid(rows) : ce_local_grid(rows);
   ce_partial_kernel<<<grid, 256, 0, stream>>>(reinterpret_cast<const __nv_bfloat16*>(logits), ld, targets, rows, cols, col_offset, vocab, row_max, row_sumexp, tgt_logit, ex);
   return cudaGetLastError();
 }
@@ -1028,7 +1036,7 @@ cudaError_t ce_grad(void* logits, int64_t ld, const int64_t* targets, int rows, 
   RowExchange ex;
   if (exch != nullptr) ex = *exch; else memset(&ex, 0, sizeof(ex));
   if (ld % 8 || cols % 8) return cudaErrorInvalidValue;
-  const int grid = ce_grid(rows);
+  const int grid = exch != nullptr ? ce_grid(rows) : ce_local_grid(rows);
   ce_grad_kernel<<<grid, 256, 0, stream>>>(reinterpret_cast<__nv_bfloat16*>(logits), ld, targets, rows, cols, col_offset, vocab, gmax, gsumexp, scale, row_loss, tgt_logit, ex);
   return cudaGetLastError();
 }

@@ -30,8 +30,8 @@ struct RowExchange {
   uint64_t timeout_ns;
   uint32_t* status;                 // [4]: 20 (LayerNorm fwd) / 21 (bwd) / 22 (cross-entropy), CTA, seen, wanted
 };
-// CTAs the LayerNorm kernels launch for `rows` rows of `cols` local columns (0: widest case): with an exchange
-// every CTA of the producing pass counts one arrival, so the host needs this number for the consumers' targets.
+// CTAs that the LayerNorm kernels launch with an exchange for `rows` rows of `cols` local columns (0: widest case): every
+// CTA of the producing pass counts one arrival, so the host needs this number for the consumers' targets.
 int ln_grid(int backward, int rows, int cols = 0);
 
 // ---- LayerNorm over a feature dimension that may be split across the mesh columns --------
@@ -91,7 +91,7 @@ cudaError_t sumsq(const void* x, int is_fp32, int64_t n, float* out, cudaStream_
 cudaError_t ce_partial(const void* logits, int64_t ld, const int64_t* targets, int rows, int cols,
                        int col_offset, int vocab, float* row_max, float* row_sumexp,
                        float* tgt_logit, cudaStream_t stream, const RowExchange* exch = nullptr);
-int ce_grid(int rows);   // CTAs of ce_partial (each counts one arrival in an exchange)
+int ce_grid(int rows);   // CTAs of ce_partial with an exchange (each counts one arrival)
 // pass 2: logits <- (softmax - onehot) * scale, in place, using the global max / sumexp.
 // row_loss[row] = log(sumexp) + max - target logit is written when non-null: with `exch` the three values
 // are combined from the mesh row's published partials (gmax / gsumexp / tgt_logit unused), otherwise

@@ -352,6 +352,36 @@ def test_layernorm_row_exchange_emulated_ranks(n, w, rows):
         assert int(keep2[1][q][0]) == (n - 1) * C.ln_grid(1, rows, w)
 
 
+@pytest.mark.parametrize("rows", [1, 741, 5000])
+def test_cross_entropy_row_exchange_emulated_ranks(rows):
+    """Loss and gradient over a vocabulary split between two ranks, every producer before any consumer, with more rows than
+    the exchange has CTAs; the counters see exactly the CTAs that the host was told.  A relative error e of the sum (1e-4, see
+    the row-statistics test) is an absolute one of its logarithm, whatever the size of the loss; gradients are rounded to
+    bf16 once."""
+    from meshslice_b200 import _native
+    from meshslice_b200.ops import functional as F
+    C, st = _C()
+    n, w, vocab = 2, 512, 1000
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    logits = (3 * torch.randn(rows, n * w, device="cuda", generator=g)).bfloat16()
+    tgt = torch.randint(0, vocab, (rows,), device="cuda", generator=g)
+    parts = [logits[:, q * w:(q + 1) * w].clone(memory_format=torch.contiguous_format) for q in range(n)]   # updated in place
+    descs, keep = _emulated_exchange(n, rows, C.ce_grid(rows))
+    for q in range(n):
+        F.ce_partial(parts[q], tgt, q * w, vocab, exch=descs[q])
+    losses = [F.ce_grad_exchanged_(parts[q], tgt, q * w, vocab, 1.0, descs[q]) for q in range(n)]
+    _native.check_status()
+    x = logits[:, :vocab].double().requires_grad_(True)
+    ref = torch.nn.functional.cross_entropy(x, tgt, reduction="none")
+    ref.sum().backward()
+    got = torch.cat(parts, 1).double()
+    errors = [(l.double() - ref).abs().max().item() for l in losses]
+    assert max(errors) < 1e-4, (errors, ref.abs().max().item())
+    assert ((got[:, :vocab] - x.grad).abs() <= 2 ** -8 * x.grad.abs() + 1e-4).all() and (got[:, vocab:] == 0).all()
+    for q in range(n):
+        assert int(keep[1][q][0]) == (n - 1) * C.ce_grid(rows)
+
+
 @pytest.mark.parametrize("sq", [(0.0, 0.0), (9.0, 16.0), (0.09, 0.16), (float("inf"), 1.0), (float("nan"), 1.0)])
 def test_clip_scale(sq):
     """Norm and clipping factor as the optimizer's CPU path computes them (three fp32 roundings: 2^-21)."""
