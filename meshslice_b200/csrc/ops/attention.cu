@@ -727,6 +727,10 @@ attn_bwd2_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_consta
   // Streamed tiles, a ring each.  Q / K is read by the first and the last product of a block, dO (key-major) by the
   // second and third, V (query-major) by the second alone: four tiles are 2 + 2 stages or 3 + 1.
   constexpr uint32_t kRing0 = kKeyMajor ? 2 : 3, kRing1 = kKeyMajor ? 2 : 1;
+  // Key-major: a statistics slot travels with dO, whose stage is free after dV, while the warps still read delta for dS.
+  // What keeps the slot is the producer's wait for empty0 (after dK, hence after dS) of the block kRing0 before, which comes
+  // first: that block must not be older than the slot's last user, kRing1 before.
+  static_assert(!kKeyMajor || (kRing0 <= kRing1 && kRing1 == 2), "statistics would be overwritten before dS has read them");
   uint8_t* sS0 = smem + 2 * kTile;          // Q or K
   uint8_t* sS1 = sS0 + kRing0 * kTile;      // dO or V
   uint8_t* sO = smem + 6 * kTile;           // output staging
@@ -826,6 +830,7 @@ attn_bwd2_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_consta
         for (int it = 0; it < w.n_it && ok; ++it, ++g) {
           const uint32_t st0 = g % kRing0, st1 = g % kRing1;
           const int srow = (w.i0 + it) * kBlk;
+          // empty0 first: it also guards the statistics slot (see the static_assert)
           if (!(ok = mbar_wait(empty0 + st0, ((g / kRing0) & 1) ^ 1, 8 * tmo))) break;
           mbar_expect_tx(full0 + st0, kTile);
           load_tile(sS0 + st0 * kTile, &tm_qkv, full0 + st0, kKeyMajor ? colq : colq + kD, seq0 + srow);   // Q or K
