@@ -352,6 +352,25 @@ def test_layernorm_row_exchange_emulated_ranks(n, w, rows):
         assert int(keep2[1][q][0]) == (n - 1) * C.ln_grid(1, rows, w)
 
 
+def test_layernorm_exchange_gives_up_when_nothing_arrives():
+    """The consumers' waits run out (50 ms), with rows of theirs already on the way: a status, and the next call works."""
+    from meshslice_b200 import _native
+    from meshslice_b200.ops import functional as F
+    rows, w = 300, 1024
+    x = torch.randn(rows, w, device="cuda").bfloat16()
+    gamma, beta = torch.ones(w, device="cuda").bfloat16(), torch.zeros(w, device="cuda").bfloat16()
+    h, y, mr = F.ln_full(x, None, gamma, beta, 1e-5)
+    descs, keep = _emulated_exchange(2, rows, 300)
+    F.ln_apply(x, None, gamma, beta, 2 * w, 1e-5, exch=descs[0])
+    with pytest.raises(_native.KernelStatusError):
+        _native.check_status()
+    F.ln_bwd_apply(x, x, gamma, mr, None, 2 * w, None, exch=descs[1])
+    with pytest.raises(_native.KernelStatusError):
+        _native.check_status()
+    assert torch.equal(F.ln_full(x, None, gamma, beta, 1e-5)[1], y)
+    _native.check_status()
+
+
 @pytest.mark.parametrize("rows", [1, 741, 5000])
 def test_cross_entropy_row_exchange_emulated_ranks(rows):
     """Loss and gradient over a vocabulary split between two ranks, every producer before any consumer, with more rows than
