@@ -201,17 +201,14 @@ ln_fwd_kernel(int mode, const uint4* __restrict__ x, const uint4* __restrict__ r
     }
     cp_async_commit();
   };
-#pragma unroll
-  for (int i = 0; i < S - 1; ++i) prefetch(blockIdx.x + i * gridDim.x, i);
-  int stage = 0;
   // With an exchange (ex.n > 0) mode 1 writes the partial statistics of its rows to every GPU of
   // the mesh row and counts one arrival per CTA on every peer; mode 2 first waits (bounded) for
   // the arrivals of all peers' CTAs and then sums the sources' statistics in fixed order.
   const bool exchange = ex.n > 0;
-  if (exchange && mode == 2 && !ex_wait(ex, 0u)) {
-    cp_async_wait<0>();                    // rows that this thread asked for are still travelling
-    return;
-  }
+  if (exchange && mode == 2 && !ex_wait(ex, 0u)) return;   // nothing of this CTA is under way yet
+#pragma unroll
+  for (int i = 0; i < S - 1; ++i) prefetch(blockIdx.x + i * gridDim.x, i);
+  int stage = 0;
   for (int row = blockIdx.x; row < rows; row += gridDim.x) {
     float vals[MAXV][8];
     float s = 0.f, ss = 0.f;
@@ -362,10 +359,7 @@ ln_bwd_kernel(int mode, const uint4* __restrict__ dy, const uint4* __restrict__ 
   }
   // exchange of the partial sums with the GPUs of the mesh row: see ln_fwd_kernel
   const bool exchange = ex.n > 0;
-  if (exchange && mode == 2 && !ex_wait(ex, 1u)) {
-    cp_async_wait<0>();                    // rows that this thread asked for are still travelling
-    return;
-  }
+  if (exchange && mode == 2 && !ex_wait(ex, 1u)) return;   // nothing of this CTA is under way yet
   const bool want_param_grads = mode != 2 && dgamma != nullptr;
   const bool want_dres = mode != 1 && dres != nullptr;
 
