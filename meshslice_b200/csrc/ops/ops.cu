@@ -168,10 +168,11 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_gr
 // ------------------------------------------------------------------------------------------
 // LayerNorm forward.  One CTA per row (grid-stride), row cached in registers.  Bound by HBM: it reads x (and res) and
 // writes h (with res) and y.  32768 x 4096 with residual: 240 us with loads of one row at a time, 172 us with the row ring
-// (copy bandwidth would give 161).
+// (copy bandwidth would give 161).  RING = false loads the row when it is due: ln_fwd_direct says where that is faster.
+// (No minimum of blocks there: with one stated, of any number, the compiler takes 80 registers or spills instead of 40.)
 // ------------------------------------------------------------------------------------------
-template <int MAXV>
-__global__ void __launch_bounds__(kLnThreads, MAXV == 1 ? 5 : MAXV == 2 ? 4 : 1)
+template <int MAXV, bool RING>
+__global__ void __launch_bounds__(kLnThreads, !RING ? 0 : MAXV == 1 ? 5 : MAXV == 2 ? 4 : 1)
 ln_fwd_kernel(int mode, const uint4* __restrict__ x, const uint4* __restrict__ res,
               uint4* __restrict__ h_out, uint4* __restrict__ y, const uint4* __restrict__ gamma,
               const uint4* __restrict__ beta, float* __restrict__ stats,
@@ -206,23 +207,27 @@ ln_fwd_kernel(int mode, const uint4* __restrict__ x, const uint4* __restrict__ r
   // the arrivals of all peers' CTAs and then sums the sources' statistics in fixed order.
   const bool exchange = ex.n > 0;
   if (exchange && mode == 2 && !ex_wait(ex, 0u)) return;   // nothing of this CTA is under way yet
+  if (RING) {
 #pragma unroll
-  for (int i = 0; i < S - 1; ++i) prefetch(blockIdx.x + i * gridDim.x, i);
+    for (int i = 0; i < S - 1; ++i) prefetch(blockIdx.x + i * gridDim.x, i);
+  }
   int stage = 0;
   for (int row = blockIdx.x; row < rows; row += gridDim.x) {
     float vals[MAXV][8];
     float s = 0.f, ss = 0.f;
     const int64_t base = (int64_t)row * nvec;
-    prefetch((uint32_t)row + (S - 1) * gridDim.x, stage == 0 ? S - 1 : stage - 1);   // where the previous row was
-    cp_async_wait<S - 1>();
+    if (RING) {
+      prefetch((uint32_t)row + (S - 1) * gridDim.x, stage == 0 ? S - 1 : stage - 1);   // where the previous row was
+      cp_async_wait<S - 1>();
+    }
 #pragma unroll
     for (int k = 0; k < MAXV; ++k) {
       const int v = threadIdx.x + k * T;
       if (v < nvec) {
-        unpack8(*slot(stage, 0, k), vals[k]);
+        unpack8(RING ? *slot(stage, 0, k) : x[base + v], vals[k]);
         if (add) {
           float r[8];
-          unpack8(*slot(stage, 1, k), r);
+          unpack8(RING ? *slot(stage, 1, k) : res[base + v], r);
 #pragma unroll
           for (int i = 0; i < 8; ++i) vals[k][i] += r[i];
         }
@@ -868,6 +873,19 @@ inline int ln_fwd_resident(int cols) {
   return n < 1 ? 1 : n > 24 ? 24 : n;
 }
 
+// Rows of one vector per thread without the ring: while what a call moves stays in L2 there is no HBM latency to hide, and
+// the way through shared memory costs more than it gives.  Repeated calls, ring / direct, us: 4099 x 1544 with residual
+// (51 MB) 12.0 / 11.0, 8192 x 1024 with residual (67 MB) 12.8 / 11.5, 8192 x 2048 without (67 MB) 20.8 / 18.0; beyond L2 the
+// ring wins: 12000 x 1024 with residual (98 MB) 18.8 / 18.9, 16384 x 1024 (134 MB) 26.3 / 28.9; and below 8 MB, where a CTA
+// has one row, by 0.1 us (512 x 512 with residual 2.5 / 2.7).  With inputs from HBM the two differ by little up to the
+// line (8192 x 2048 26.6 / 26.6, 4099 x 1544 with residual 18.4 / 20.5).  Wider rows keep the ring: direct loads are faster
+// there only on inputs in L2, and slower from HBM (1024 x 12288: 21 / 17 and 27 / 33).
+constexpr int64_t kLnDirectMin = 8 << 20, kLnDirectMax = 80 << 20;
+inline bool ln_fwd_direct(int rows, int cols, int tensors) {
+  const int64_t bytes = 2 * (int64_t)rows * cols * tensors;
+  return ln_fwd_maxv(cols) == 1 && bytes >= kLnDirectMin && bytes <= kLnDirectMax;
+}
+
 inline int grid_for(int64_t n, int threads, int cap = 148 * 16) {
   int64_t g = (n + threads - 1) / threads;
   if (g > cap) g = cap;
@@ -931,17 +949,23 @@ cudaError_t ln_fwd(int mode, const void* x, const void* res, void* h_out, void* 
   auto G = reinterpret_cast<const uint4*>(gamma);
   auto B = reinterpret_cast<const uint4*>(beta);
   const int threads = ln_threads(cols), maxv = ln_fwd_maxv(cols);
-  const int smem = ln_ring_bytes(false, mode != 2 && res != nullptr ? 2 : 1, maxv, threads);
+  const int inputs = mode != 2 && res != nullptr ? 2 : 1;
+  const int tensors = inputs + (mode != 2 && h_out != nullptr ? 1 : 0) + (mode != 1 ? 1 : 0);
+  if (exch == nullptr && ln_fwd_direct(rows, cols, tensors)) {
+    ln_fwd_kernel<1, false><<<grid, threads, 0, stream>>>(mode, X, R, H, Y, G, B, stats, mean_rstd, rows, cols, total_cols, eps, ex);
+    return cudaGetLastError();
+  }
+  const int smem = ln_ring_bytes(false, inputs, maxv, threads);
   auto run = [&](auto kernel) {
     const cudaError_t e = allow_smem(reinterpret_cast<const void*>(kernel), smem);
     if (e != cudaSuccess) return e;
     kernel<<<grid, threads, smem, stream>>>(mode, X, R, H, Y, G, B, stats, mean_rstd, rows, cols, total_cols, eps, ex);
     return cudaGetLastError();
   };
-  if (maxv == 1) return run(ln_fwd_kernel<1>);
-  if (maxv == 2) return run(ln_fwd_kernel<2>);
-  if (maxv == 4) return run(ln_fwd_kernel<4>);
-  return run(ln_fwd_kernel<8>);
+  if (maxv == 1) return run(ln_fwd_kernel<1, true>);
+  if (maxv == 2) return run(ln_fwd_kernel<2, true>);
+  if (maxv == 4) return run(ln_fwd_kernel<4, true>);
+  return run(ln_fwd_kernel<8, true>);
 }
 
 cudaError_t ln_bwd(int mode, const void* dy, const void* h, const void* gamma,

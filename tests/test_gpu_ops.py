@@ -40,6 +40,32 @@ def test_layernorm_row_ring(cols, rows, residual):
     assert sums[0] == 0 and sums[-1] == 0
 
 
+@pytest.mark.parametrize("residual", [True, False])
+@pytest.mark.parametrize("cols", [264, 1024, 2048])
+def test_layernorm_forward_with_and_without_the_ring(cols, residual):
+    """A call that moves more than 80 MiB takes the row ring, one of a sixteenth of its rows (8 to 80 MiB) does not: the same
+    threads add the same vectors, so the results agree bit for bit, in one pass and in two (statistics, then rows)."""
+    from meshslice_b200.ops import functional as F
+    rows = 4 * (100 * 2 ** 20 // (2 * cols * 4))
+    if not residual:
+        rows *= 2
+    g = torch.Generator(device="cuda").manual_seed(cols)
+    x = torch.randn(rows, cols, device="cuda", generator=g).bfloat16()
+    res = torch.randn(rows, cols, device="cuda", generator=g).bfloat16() if residual else None
+    gamma, beta = (torch.randn(cols, device="cuda", generator=g).bfloat16() for _ in range(2))
+    whole = F.ln_full(x, res, gamma, beta, 1e-5)
+    h, stats = F.ln_stats(x, res)
+    two = F.ln_apply(h, stats, gamma, beta, cols, 1e-5)
+    q = rows // 16
+    for i in (0, 7 * q, rows - q):
+        cut = lambda t: None if t is None else t[i:i + q]
+        part = F.ln_full(cut(x), cut(res), gamma, beta, 1e-5)
+        assert all(torch.equal(p, cut(w)) for p, w in zip(part, whole))
+        hp, sp = F.ln_stats(cut(x), cut(res))
+        assert torch.equal(hp, cut(h)) and torch.equal(sp, cut(stats))
+        assert all(torch.equal(p, cut(w)) for p, w in zip(F.ln_apply(hp, sp, gamma, beta, cols, 1e-5), two))
+
+
 @pytest.mark.parametrize("cols,rows", [(1024, 301), (768, 43), (64, 1000), (2048, 300), (4096, 300), (12288, 300)])
 def test_layernorm_fwd_bwd_single_pass(cols, rows):
     """Widths up to 2048 run several rows per CTA in the backward kernel (row counts that leave the last CTA
