@@ -169,7 +169,8 @@ __device__ __forceinline__ void store32(void* base, int64_t ld, bool fp32, bool 
   }
 }
 
-// One box of a tensor map, shared -> global; the second form adds fp32 values to what is there.
+// One box of a tensor map, shared -> global; the second form adds fp32 values to what is there (the sum that a register add
+// would give, subnormal values included: test_gemm_fp32_accumulation_keeps_subnormals).
 __device__ __forceinline__ void tma_store_box(const CUtensorMap* map, const void* src, int32_t x, int32_t y, bool add) {
   if (add)
     asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.bulk_group [%0, {%2, %3}], [%1];"

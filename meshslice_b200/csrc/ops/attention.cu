@@ -26,11 +26,8 @@ constexpr int kD = 128;         // head dim
 constexpr int kBlk = 128;       // query / key rows per tile
 constexpr int kTile = kBlk * kD * 2;  // 32 KiB: one [128 x 128] bf16 tile = two swizzle halves
 constexpr int kHalf = kTile / 2;
-// Element-wise warps (softmax in the forward pass, P / dS and the dQ drain in the backward pass)
-// are a template parameter of the kernels.  Four warps give one thread per tile row; eight give
-// two threads per row, each owning 64 of the 128 columns: the exponentials and the TMEM traffic
-// of a block, which sit in series with the MMAs, take half as long.  A warp may touch the TMEM
-// lanes 32 * (warp % 4) ... + 31, so warps 2-5 and 6-9 both cover all four lane quarters.
+// A warp may touch the TMEM lanes 32 * (warp % 4) ... + 31: any four consecutive warps cover the 128 rows of a tile, whichever
+// warp the element-wise work starts at.
 constexpr uint32_t kErrAttn = 20;
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kLn2 = 0.6931471805599453f;
@@ -441,7 +438,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_consta
         const bool diag = a.causal && j == i_blk;
         uint32_t r[4][32];
         float mc[4];
-        // a quarter of the row is on its way while the maximum of the previous quarter is taken
+        // the whole row with one wait: four loads in flight
 #pragma unroll
         for (int c = 0; c < 4; ++c) tmem_ld_32x32(ts + c * 32, r[c]);
         tmem_ld_wait();
@@ -1139,7 +1136,9 @@ cudaError_t attention_fwd(const void* qkv, void* out, float* lse, int batch, int
   const int grp = bh_group(batch, heads);
   const int nblk = seq / kBlk;
   // With no more tiles than SMs a tile per CTA leaves none idle and runs without a neighbour; beyond that pairs share
-  // K and V and overlap (batch 3 x 640, 5 heads, 75 tiles: 16.5 us either way; 16 heads x 8192: see the kernel).
+  // K and V and overlap.  One tile / two, us: 1 head x 8192 (64 tiles) 104 / 114, 8 x 2048 (128) 29.8 / 32.7, batch 3 x 640
+  // with 5 heads (75) 12.4 / 14.2, batch 4 x 256 with 16 heads (128) 8.0 / 9.3; causal 104 / 114,
+  // 30.0 / 32.8, 13.1 / 14.2 and 8.7 / 8.7.
   a.tiles_per_item = (int64_t)batch * heads * nblk <= sm_count() ? 1 : 2;
   dim3 grid(grp, (nblk + a.tiles_per_item - 1) / a.tiles_per_item, batch * heads / grp);
   attn_fwd2_kernel<<<grid, kFwd2Threads, kFwd2Smem, stream>>>(tm, to, a);

@@ -153,8 +153,8 @@ __device__ __forceinline__ float gelu_grad_f(float x) {
 
 // ------------------------------------------------------------------------------------------
 // Row ring of the LayerNorm kernels: a thread copies the 16-byte vectors that it will read itself, two rows (one for the
-// widest backward rows) ahead, into shared memory (cp.async), so rows travel while earlier ones are reduced and written, at no registers and
-// without a barrier.  Layout [stage][input][vector of the thread][thread].
+// widest backward rows) ahead, into shared memory (cp.async), so rows travel while earlier ones are reduced and written, at
+// no registers and without a barrier.  Layout [stage][input][vector of the thread][thread].
 // ------------------------------------------------------------------------------------------
 constexpr int ln_stages(bool backward, int maxv) { return backward && maxv > 3 ? 2 : 3; }
 __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
@@ -330,8 +330,9 @@ __device__ __forceinline__ void add8(float* dst, const float (&v)[8]) {
 
 // A CTA of up to kLnBwdThreads threads walks the rows grid-stride.  A 4096-wide row is two 16-byte vectors per
 // thread: the per-thread dgamma / dbeta accumulators (16 registers per vector) are what limits occupancy, so the rows
-// ahead wait in the shared-memory ring and both passes over a row read it there; gamma is loaded once per CTA.  Bound by HBM (dy, h, dres read, dx written); 32768 x 4096 with dres: 254 us with loads of one row at a
-// time, 192 us now (copy bandwidth would give 161); 8192 x 12288: 290 and 146.
+// ahead wait in the shared-memory ring and both passes over a row read it there; gamma is loaded once per CTA.  Bound by
+// HBM (dy, h, dres read, dx written); 32768 x 4096 with dres: 254 us with loads of one row at a time, 192 us now (copy
+// bandwidth would give 161); 8192 x 12288: 290 and 146.
 // GROUPED (rows of at most 256 vectors, e.g. column shards): the CTA works on blockDim.x / tpr rows at a time,
 // `tpr` threads (whole warps) per row, and adds the row groups' dgamma / dbeta in shared memory before its one
 // atomic per column, so that narrow rows neither idle most of a CTA nor multiply the atomics.
@@ -857,7 +858,8 @@ inline LnBwdShape ln_bwd_shape(int cols) {
 }
 
 // Shared memory of a row ring; CTAs of the forward kernel that an SM holds (by registers 1280 threads of one vector,
-// 1024 of two, 512 of four, 256 of eight; at most 24 CTAs), with a residual: that is the grid of one resident wave, whose rows follow one another.
+// 1024 of two, 512 of four, 256 of eight; at most 24 CTAs), with a residual: that is the grid of one resident wave, whose
+// rows follow one another.
 inline int ln_ring_bytes(bool backward, int inputs, int maxv, int threads) {
   return ln_stages(backward, maxv) * inputs * maxv * threads * 16;
 }
@@ -907,8 +909,9 @@ static cudaError_t allow_smem(const void* kernel, int bytes) {
 
 // Launch shapes.  In a row exchange every CTA ends in a system-wide fence and an add to the same counter of every peer,
 // which takes longer than a row, and every CTA of the second pass polls its own: one resident wave with several rows a CTA
-// (ce_partial_kernel: five CTAs an SM by registers).  On one device a row per CTA up to 32 per SM: blocks handed out as SMs
-// get free leave no uneven last wave (4096 rows on 1184 CTAs: four rows each, three for some).
+// (ce_partial_kernel: five CTAs an SM by registers).  4096 rows of 6400 logits in a group of eight: 254 us with a row per
+// CTA, 83 with 740 CTAs (19 without an exchange).  On one device a row per CTA up to 32 per SM: blocks handed out as SMs get
+// free leave no uneven last wave (4096 rows on 1184 CTAs: four rows each, three for some).
 int ce_grid(int rows) { return rows < 148 * 5 ? rows : 148 * 5; }
 static int ce_local_grid(int rows) { return rows < 148 * 32 ? rows : 148 * 32; }
 

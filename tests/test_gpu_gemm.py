@@ -178,3 +178,22 @@ def test_gemm_output_may_start_at_any_element(offset, two_cta):
         assert intact(flat) and intact(flatp)
         assert (pre.double() - ref).abs().max().item() <= 2 ** -8 * scale
         assert ((out.double() - g).abs() <= 2 ** -8 * g.abs() + 2e-3 * ref.abs() + 1e-3).all()
+
+
+def test_gemm_fp32_accumulation_keeps_subnormals():
+    """The adds that the copy engine does are those of fp32 without flushing: exact for subnormal operands and results."""
+    from meshslice_b200 import _native
+    from meshslice_b200.ops.gemm import gemm
+    M, N, K = 256, 256, 64
+    before = torch.tensor([0.0, 1e-40, -1e-40, 2.0 ** -149, 2.0 ** -126, -(2.0 ** -126), 1.0, 2.0 ** -130])
+    before = before.repeat(M, N // 8)
+    for ea, eb in ((-70, -70), (-75, -70), (-66, -66), (-64, -60)):      # products 2^-134, 2^-139, 2^-126, 2^-118
+        a = torch.full((M, K), 2.0 ** ea, device="cuda").bfloat16()
+        b = torch.full((N, K), 2.0 ** eb, device="cuda").bfloat16()
+        b[::2] *= -1
+        alone = gemm(a, b, "nt", out_dtype=torch.float32).cpu()
+        out = before.cuda()
+        gemm(a, b, "nt", out=out, accumulate=True)
+        _native.check_status()
+        assert alone[0, 1].item() == 64 * 2.0 ** (ea + eb)
+        assert torch.equal(out.cpu(), (before.double() + alone.double()).float())
