@@ -172,10 +172,11 @@ def _split_qkv(qkv, batch, seq, heads):
 
 def _head_dim(qkv, batch, seq, heads) -> int:
     """Features per head of a [batch * seq, heads * 3 * D] tensor (what ``_split_qkv`` could view is accepted)."""
-    width = qkv.shape[1]
-    if qkv.dim() != 2 or qkv.shape[0] != batch * seq or width % (3 * heads) or not qkv.is_contiguous():
-        return _split_qkv(qkv, batch, seq, heads)[3]
-    return width // (3 * heads)
+    if qkv.dim() == 2 and qkv.is_contiguous():
+        rows, width = qkv.shape
+        if rows == batch * seq and width % (3 * heads) == 0:
+            return width // (3 * heads)
+    return _split_qkv(qkv, batch, seq, heads)[3]
 
 
 FALLBACKS = {"attention": 0}      # eager-PyTorch runs of an op on CUDA tensors (only with allow_fallback)
@@ -196,7 +197,8 @@ def attention_fwd(qkv, batch: int, seq: int, heads: int, causal: bool = False, a
     D = _head_dim(qkv, batch, seq, heads)
     _check_attention_shape(qkv, D, seq, allow_fallback)
     if qkv.is_cuda and D == 128 and seq % 128 == 0:
-        qkv = qkv.contiguous()       # the kernels address whole rows of heads * 3 * 128, without a row stride
+        if not qkv.is_contiguous():
+            qkv = qkv.contiguous()   # the kernels address whole rows of heads * 3 * 128, without a row stride
         out = torch.empty(batch * seq, heads * D, dtype=qkv.dtype, device=qkv.device)
         lse = torch.empty(batch, heads, seq, dtype=torch.float32, device=qkv.device)
         _C().attention_fwd(qkv.data_ptr(), out.data_ptr(), lse.data_ptr(), batch, seq, heads,
@@ -218,7 +220,9 @@ def attention_bwd(dout, qkv, out, lse, batch: int, seq: int, heads: int, causal:
     D = _head_dim(qkv, batch, seq, heads)
     _check_attention_shape(qkv, D, seq, allow_fallback)
     if qkv.is_cuda and D == 128 and seq % 128 == 0:
-        qkv, dout, out, lse = qkv.contiguous(), dout.contiguous(), out.contiguous(), lse.contiguous()
+        dout = dout.contiguous()
+        if not (qkv.is_contiguous() and out.is_contiguous() and lse.is_contiguous()):
+            qkv, out, lse = qkv.contiguous(), out.contiguous(), lse.contiguous()
         dqkv = torch.empty_like(qkv)
         delta = torch.empty(batch, heads, seq, dtype=torch.float32, device=qkv.device)
         dq_acc = torch.empty(batch, heads, seq, dtype=torch.float32, device=qkv.device)   # scratch: -lse * log2(e)
