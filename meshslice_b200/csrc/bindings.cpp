@@ -295,7 +295,7 @@ void gemm_local(int64_t M, int64_t N, int64_t K, uint64_t A, int64_t lda, int a_
   a.tiles_m = (a.M + 2 * kBM - 1) / (2 * kBM);
   a.tiles_n = (a.N + kBN - 1) / kBN;
   a.n_slices = a.cyc = a.push_extent = a.push_bufs = a.b_nchunk = a.a_kpanel = a.b_kpanel = 1;
-  a.group = std::max(1, env("MSB_G2_GROUP", 8));
+  a.group = env("MSB_G2_GROUP", 0);
   a.status = P<uint32_t>(status);
   a.timeout_ns = 1000000000ull;
 
@@ -320,6 +320,7 @@ void gemm_local(int64_t M, int64_t N, int64_t K, uint64_t A, int64_t lda, int a_
     check(launch_sm100_gemm2(ta, tb, a, tile_n, sms, S(stream)), "sm100_gemm2 launch");
   } else {
     const int grid = std::max(2, std::min(sms & ~1, 2 * a.tiles_m * a.tiles_n));
+    if (a.group <= 0) a.group = 8;
     static const PushMaps no_push = {};
     check(launch_sm100_gemm(ta, tb, no_push, a, grid, S(stream)), "sm100_gemm launch");
   }

@@ -160,6 +160,8 @@ struct GemmArgs {
   uint32_t* done_counter;      // local: CTAs that finished their transfers (monotonic)
   uint32_t done_target;
   // ---- plain (two-CTA) kernel ----
+  int along_n;                 // raster groups along N instead of M (with group <= 0 the launcher sets all three)
+  int k_turn;                  // every other tile of a CTA pair walks its k-blocks backwards
   int tma_c;                   // set by its launcher: C (and C_pre) leave through shared memory as TMA stores
   // ---- status ----
   uint32_t* status;            // [4]: code, blockIdx, detail, detail2
@@ -192,6 +194,8 @@ cudaError_t launch_sm100_gemm(const CUtensorMap& tma_a, const CUtensorMap& tma_b
 // `tile_n` columns per cluster tile (gemm2_tile_n); the tensor map of a K-major B must use a {64, tile_n / 2} box,
 // that of an MN-major B one box of tile_n / 128 blocks of 64 columns.
 int gemm2_tile_n(int M, int N, int sms);
+struct Gemm2Order { int group, along_n, k_turn; };
+Gemm2Order gemm2_order(int64_t M, int64_t N, int64_t K, int tile_n);
 cudaError_t launch_sm100_gemm2(const CUtensorMap& tma_a, const CUtensorMap& tma_b, GemmArgs args, int tile_n, int sms,
                                cudaStream_t stream);
 

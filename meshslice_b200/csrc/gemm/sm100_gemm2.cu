@@ -219,15 +219,18 @@ __device__ __forceinline__ void stage_f32(uint8_t* box, int lane, const float (&
         make_float4(v[q * 4], v[q * 4 + 1], v[q * 4 + 2], v[q * 4 + 3]);
 }
 
-// cluster tile t -> (256-row block, 256-column block), grouped along M for L2 reuse
-__device__ __forceinline__ void tile2(int t, int tiles_m2, int tiles_n, int group, int& m2, int& nb) {
-  const int span = group * tiles_n;
+// cluster tile t -> (256-row block, column block): panels of `group` blocks along M (or N, `along_n`), which the tiles of a
+// panel sweep along the other dimension
+__device__ __forceinline__ void tile2(int t, int tiles_m2, int tiles_n, int group, bool along_n, int& m2, int& nb) {
+  const int across = along_n ? tiles_m2 : tiles_n, along = along_n ? tiles_n : tiles_m2;
+  const int span = group * across;
   const int g = t / span;
   const int r = t - g * span;
   const int g0 = g * group;
-  const int geff = min(group, tiles_m2 - g0);
-  nb = r / geff;
-  m2 = g0 + (r - nb * geff);
+  const int geff = min(group, along - g0);
+  const int sweep = r / geff, in = g0 + (r - sweep * geff);
+  m2 = along_n ? sweep : in;
+  nb = along_n ? in : sweep;
 }
 
 }  // namespace
@@ -263,7 +266,7 @@ sm100_gemm2_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_const
   const int num_tiles = tiles_m2 * tiles_n;
   const int kblocks = (a.K + kBK - 1) / kBK;
   const int cluster_id = blockIdx.x >> 1, n_clusters = gridDim.x >> 1;
-  const int group = a.group > 0 ? a.group : 8;
+  const int group = a.group;
 
   if (warp == 0 && lane == 0) {
     tma_prefetch_desc(&tma_a);
@@ -299,9 +302,10 @@ sm100_gemm2_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_const
       const uint32_t full0 = mapa_u32(smem_u32(full_bar), 0);     // the leader's barriers
       uint32_t stage = 0, phase = 0;
       bool ok = true, free = true;                                // `free`: the next stage was seen empty
+      bool back = false;                                          // this tile's k-blocks run from the last to the first
       for (int t = cluster_id; t < num_tiles && ok; t += n_clusters) {
         int m2, nb;
-        tile2(t, tiles_m2, tiles_n, group, m2, nb);
+        tile2(t, tiles_m2, tiles_n, group, a.along_n != 0, m2, nb);
         const int row_a = (2 * m2 + (int)rank) * kBM;           // this CTA's 128 rows of A
         const int col_b = nb * BN + (int)rank * (BN / 2);       // this CTA's half of the columns of B
         for (int kb = 0; kb < kblocks; ++kb) {
@@ -311,34 +315,36 @@ sm100_gemm2_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_const
             break;
           }
           const uint32_t fb = full0 + stage * 8;
+          const int k0 = (back ? kblocks - 1 - kb : kb) * kBK;
           if (is_a) {
             if (rank == 0) mbar_expect_tx(full_bar + stage, 2 * kAStage2);
             uint8_t* da = sA + stage * kAStage2;
             if (!a.a_mn_major) {
-              tma_load_2d_pair(da, &tma_a, fb, kb * kBK, row_a);
+              tma_load_2d_pair(da, &tma_a, fb, k0, row_a);
             } else if (a.a_map3d) {
-              tma_load_3d_pair(da, &tma_a, fb, 0, kb * kBK, row_a >> 6);
+              tma_load_3d_pair(da, &tma_a, fb, 0, k0, row_a >> 6);
             } else {
 #pragma unroll
               for (int j = 0; j < kBM / 64; ++j)
-                tma_load_2d_pair(da + j * (kBK * 128), &tma_a, fb, row_a + j * 64, kb * kBK);
+                tma_load_2d_pair(da + j * (kBK * 128), &tma_a, fb, row_a + j * 64, k0);
             }
           } else {
             if (rank == 0) mbar_expect_tx(full_bar + stage, 2 * kBStage2);
             uint8_t* db = sB + stage * kBStage2;
             if (!a.b_mn_major) {
-              tma_load_2d_pair(db, &tma_b, fb, kb * kBK, col_b);
+              tma_load_2d_pair(db, &tma_b, fb, k0, col_b);
             } else if (a.b_map3d) {
-              tma_load_3d_pair(db, &tma_b, fb, 0, kb * kBK, col_b >> 6);
+              tma_load_3d_pair(db, &tma_b, fb, 0, k0, col_b >> 6);
             } else {
 #pragma unroll
               for (int j = 0; j < BN / 128; ++j)
-                tma_load_2d_pair(db + j * (kBK * 128), &tma_b, fb, col_b + j * 64, kb * kBK);
+                tma_load_2d_pair(db + j * (kBK * 128), &tma_b, fb, col_b + j * 64, k0);
             }
           }
           if (++stage == kStages2) { stage = 0; phase ^= 1; }
           free = mbar_test(empty_bar + stage, phase ^ 1);
         }
+        back = !back && a.k_turn;
       }
     }
   } else if (warp == 1) {
@@ -396,7 +402,7 @@ sm100_gemm2_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_const
     int it = 0;
     for (int t = cluster_id; t < num_tiles && ok; t += n_clusters, ++it) {
       int m2, nb;
-      tile2(t, tiles_m2, tiles_n, group, m2, nb);
+      tile2(t, tiles_m2, tiles_n, group, a.along_n != 0, m2, nb);
       const uint32_t acc = it & 1, acc_phase = (it >> 1) & 1;
       int okw = 1;
       if (lane == 0) okw = mbar_wait(tfull_bar + acc, acc_phase, 7 * tmo) ? 1 : 0;
@@ -507,6 +513,22 @@ int gemm2_tile_n(int M, int N, int sms) {
   return 3 * narrow < 4 * wide ? 128 : 256;
 }
 
+// The order of the tiles, by what they read from HBM: under the power cap that traffic costs clock.  A panel of sixteen
+// blocks along one dimension is kept in L2 (33 MB at K = 4096) while the tiles sweep the other, so the panels' operand is
+// read once and the other one once per panel: the dimension with the smaller sum.  Panels of eight / sixteen / thirty-two,
+// sustained: 8192 x 16384 x 4096 815 / 788 / 871 us (along N: 824 / 803 / 886), 4096 x 51200 x 1024 345 / 336 / 336.
+// Where a panel is more than L2 keeps, the wave before has left the end of the contraction there: every other tile walks it
+// backwards.  Panels of 8, of 16, of 16 with turns: 8192 x 4096 x 16384 833 / 840 / 822, 4096 x 16384 x 8192 added to fp32
+// 864 / 876 / 844, 4096 x 4096 x 8192 235 / 236 / 228; K = 4096 gains nothing (788 / 790 with turns).
+Gemm2Order gemm2_order(int64_t M, int64_t N, int64_t K, int tile_n) {
+  const int64_t panels_m = (M + 16 * 256 - 1) / (16 * 256), panels_n = (N + 16 * tile_n - 1) / (16 * tile_n);
+  Gemm2Order o;
+  o.group = 16;
+  o.along_n = N + panels_n * M < M + panels_m * N;
+  o.k_turn = K > 4096;
+  return o;
+}
+
 cudaError_t launch_sm100_gemm2(const CUtensorMap& tma_a, const CUtensorMap& tma_b, GemmArgs args, int tile_n, int sms,
                                cudaStream_t stream) {
   // Output through shared memory and TMA where the tensor map allows it; bf16 accumulation adds before it rounds,
@@ -516,6 +538,12 @@ cudaError_t launch_sm100_gemm2(const CUtensorMap& tma_a, const CUtensorMap& tma_
                make_tensor_map_out(&tc, args.C, args.N, args.M, args.ldc, args.c_fp32 != 0) == 0 &&
                (args.act == 0 || args.C_pre == nullptr ||
                 make_tensor_map_out(&tp, args.C_pre, args.N, args.M, args.ldc, false) == 0);
+  if (args.group <= 0) {
+    const Gemm2Order o = gemm2_order(args.M, args.N, args.K, tile_n);
+    args.group = o.group;
+    args.along_n = o.along_n;
+    args.k_turn = o.k_turn;
+  }
   const int64_t tiles = (int64_t)((args.M + 2 * kBM - 1) / (2 * kBM)) * ((args.N + tile_n - 1) / tile_n);
   int grid = (int)(2 * tiles < (sms & ~1) ? 2 * tiles : (sms & ~1));
   if (grid < 2) grid = 2;

@@ -73,6 +73,24 @@ def test_gemm_bias_gelu_epilogue():
     assert ((out.float() - ref).abs() <= 0.03 + 0.01 * ref.abs()).all()
 
 
+# Tile orders: panels of sixteen blocks along M (more than one, the last one short) and along N, contractions that are walked
+# backwards on every other tile, with an odd number of k-blocks whose last one is short.
+@pytest.mark.parametrize("layout", ["nt", "nn", "tn"])
+@pytest.mark.parametrize("shape", [(4360, 2056, 136), (2056, 8456, 136), (8456, 1288, 4168), (4360, 4616, 4104)])
+def test_gemm_tile_orders(layout, shape):
+    from meshslice_b200 import _native
+    from meshslice_b200.ops.gemm import gemm
+    M, N, K = shape
+    a, b = _operands(M, N, K, layout, seed=11)
+    out = gemm(a, b, layout)
+    acc = torch.ones(M, N, device="cuda", dtype=torch.float32)
+    gemm(a, b, layout, out=acc, accumulate=True)
+    _native.check_status()
+    ref = _ref(a, b, layout)
+    _check(out, ref, K)
+    _check(acc, ref + 1.0, K)
+
+
 def test_gemm_many_tiles_persistent_schedule():
     """More tiles than SMs, so every CTA walks several tiles and both TMEM accumulators."""
     from meshslice_b200 import _native
