@@ -63,6 +63,24 @@ __device__ __forceinline__ float fast_exp2(float x) {
   return y;
 }
 
+// The same on the FMA pipe, for the share of the exponentials that would queue for the special-function unit (16 results per
+// cycle and SM): x = n + f with n the nearest whole number, 2^f by the polynomial of degree 5 with the smallest largest
+// relative error on [-1/2, 1/2] (Remez exchange; 2^-23.7, with fp32 rounding 2^-22.2), times 2^n.  Below -125 the result is
+// 2^-125 and not zero; NaN stays NaN.  x stays below 127 wherever the result is used.
+__device__ __forceinline__ float exp2_fma(float x) {
+  float t;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(t) : "f"(x), "f"(-125.0f));
+  const float r = __fadd_rn(t, 12582912.0f);                 // 1.5 * 2^23: n in the low bits
+  const float f = __fsub_rn(t, __fsub_rn(r, 12582912.0f));
+  float p = 1.327647245e-03f;
+  p = fmaf(p, f, 9.675540961e-03f);
+  p = fmaf(p, f, 5.550713092e-02f);
+  p = fmaf(p, f, 2.402212024e-01f);
+  p = fmaf(p, f, 6.931469440e-01f);
+  p = fmaf(p, f, 1.000000119e+00f);
+  return p * __int_as_float((__float_as_int(r) << 23) + 0x3f800000);
+}
+
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<uint32_t*>(&v);
@@ -157,10 +175,26 @@ __device__ __forceinline__ void tmem_st_32x16(uint32_t taddr, const uint32_t (&r
       : "memory");
 }
 
-__device__ __forceinline__ void tmem_st_32x8(uint32_t taddr, const uint32_t (&r)[8]) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+// 16 lanes x 32 fp32 columns in the layout of a matrix fragment: thread t gets, of every group n of 8 columns, columns
+// 2 (t % 4) and + 1 of rows t / 4 (r[4n], r[4n + 1]) and t / 4 + 8 (r[4n + 2], r[4n + 3]).
+__device__ __forceinline__ void tmem_ld_16x32_frag(uint32_t taddr, uint32_t* r) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.16x256b.x4.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+}
+// The same elements as packed bf16: r[2n] / r[2n + 1] are the two columns of rows t / 4 / t / 4 + 8; groups of 8 columns: 4 or 2.
+__device__ __forceinline__ void tmem_st_16x32_frag(uint32_t taddr, const uint32_t* r) {
+  asm volatile("tcgen05.st.sync.aligned.16x128b.x4.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
                ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
                : "memory");
+}
+__device__ __forceinline__ void tmem_st_16x16_frag(uint32_t taddr, const uint32_t* r) {
+  asm volatile("tcgen05.st.sync.aligned.16x128b.x2.b32 [%0], {%1, %2, %3, %4};"
+               ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]) : "memory");
 }
 // shared -> global, one box of a tensor map; tracked by bulk groups
 __device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, const void* smem_src, int32_t x, int32_t y) {
@@ -648,34 +682,40 @@ attn_delta_kernel(const uint4* __restrict__ out, const uint4* __restrict__ dout,
 //
 // The products use full 128-wide blocks (eight instructions of 64 cycles each) and the kernels are organised
 // around keeping the tensor pipe fed: the element-wise work is split in two phases (P from S; dS from
-// dP and P) and the MMA warp issues the next block's S (and dP) between the gradient products of the
-// current block, so each phase runs under products that do not depend on it:
-//   key-major    S(i) dP(i) | P(i)? dV(i) S(i+1) | dS(i)? dK(i) dP(i+1) | P(i+1)? ...
-//   query-major  S(j) dP(j) S(j+1) | dS(j)? dQ(j) dP(j+1) S(j+2) | ...          (two S buffers)
+// dP and P) and the MMA warp issues the next block's S (and dP) where they do not depend on this block's phases:
+//   key-major    P(i)? dV(i) S(i+1) | dS(i)? dK(i) dP(i+1) | ...       P^T is written over S^T, so S(i+1) follows dV(i)
+//   query-major  S(j) read? S(j+1) dP(j+1) | dS(j)? dQ(j) | ...        P stays in registers: S is free once it is read
+// Blocks follow one another across items: the next item's first S is issued like the next block's.
 //
-//   warp 0      TMA: the two resident 128-row tiles, a two-stage ring of 128-row tile pairs and, key-major, the
-//               statistics of the streamed queries; asks for the next item (cluster launch control, as in forward)
+//   warp 0      TMA: the resident tile that S reads (K or Q), the three-stage ring of Q (with lse2) or K; asks for the next
+//               item (cluster launch control, as in forward)
+//   warp 18     TMA: the resident tile that dP reads (V or dO), the two-stage ring of dO (with delta) or V
 //   warp 1      MMA issuer
 //   warps 2-17  element-wise: four threads per TMEM lane, 32 of the 128 columns each
 //
-// What bounds it: the chain S -> P -> dV, S' and dP -> dS -> dK, dP'.  Per block pair the products take 2048
-// (key-major) and 1536 cycles, the exponentials 1024 of the SFU; measured 3350 and 2150, of which 350-450 cycles go
-// into every hand-over from the tensor pipe to the warps and back.  So sixteen warps share a phase, each thread reads its
-// 32 columns with one load and keeps P in fp32 registers for dS; P^T is handed over in two parts; the key-major
-// statistics come through shared memory (broadcast loads of them from global memory cost 7 L1 wavefronts each and a
-// miss per block); the rings are split by operand, because a shared stage of K and V was only free after dQ and the
-// products waited for the next one (query-major 3300 cycles a pair).  CTAs are persistent: the next item's tiles, S and
-// dP arrive while this item's accumulators leave as TMA stores (9000 cycles between items with 16-byte stores per
-// lane, 4000 staged through shared memory, as all SMs write at once).
-// Batch 4 x 2048, 32 heads, causal: key-major 424 -> 232 us, query-major 306 -> 179 us.
-constexpr int kStatBytes = 2 * kBlk * 4;   // lse2 and delta of 128 queries
+// What bounds it: the power cap first (1.4 to 1.65 GHz under these kernels: a block pair saved from waiting gives back half
+// of it in clock), then, key-major, the chain S -> P -> dV -> S' (2750 cycles a pair, 2048 of them products) and, query-major,
+// the 2000 cycles that a 32 KiB tile takes from L2 while every SM loads (1780 a pair, 1536 of products): K is held from the
+// load to dQ, two blocks later, so its ring is the deeper one, and either ring has a producer of its own, because a stage of
+// one is often free long before one of the other.  The place for that comes from the output: it is staged in the stage of
+// the item's last dO or V.  Sixteen warps share a phase, each thread reads its 32 columns with one load and keeps P in fp32
+// registers for dS; P^T is handed over in two parts.  Key-major, statistics vary along the columns: in the layout of a matrix
+// fragment a thread has 8 different columns and not 32, so 8 shared loads of 8 bytes replace 16 of 16 (1590 wavefronts a pair
+// became 490), and two exponentials of eight run on the FMA pipe (none of eight 363 -> 381 us, two 350, three 390 thousand
+// cycles for the first case below).
+// With one producer, rings of two stages each and a staging area: batch 4 x 2048, 32 heads, causal, 217 (key-major) and
+// 173 us (query-major), now 219 and 165 (429 -> 421 us with the row sums); full 737 -> 719, 16 heads x 8192 causal 709 -> 684.
+// P^T through shared memory, so that S(i+1) need not wait for dV(i): no faster (3500 cycles; Q's ring has two stages then).
+constexpr int kBwdPoly = 2;                 // key-major: exponentials of every eight that run on the FMA pipe
 constexpr int kBwdWarps = 16;               // element-wise warps
 constexpr int kBwdCols = kBlk * 4 / kBwdWarps;   // columns of a row per element-wise thread
 constexpr int kBwdStage = 32 * kBwdCols * 2;     // output staging per element-wise warp
-constexpr int kBwdAlignSlack = 512;
-constexpr size_t kBwd2Smem = 6 * kTile + kBwdWarps * kBwdStage + 2 * kStatBytes + 256 + kBwdAlignSlack;
+constexpr int kStatBytes = kBlk * 4;        // lse2 or delta of 128 queries
+constexpr int kBwdAlignSlack = 256;
+constexpr size_t kBwd2Smem = 7 * kTile + 5 * kStatBytes + 256 + kBwdAlignSlack;
+static_assert(kBwdWarps * kBwdStage == kTile, "an item's staged output takes the place of a tile");
 static_assert(kBwd2Smem <= 232448, "shared memory of a CTA");
-constexpr int kBwd2Threads = 64 + 32 * kBwdWarps;
+constexpr int kBwd2Threads = 96 + 32 * kBwdWarps;
 
 struct Bwd2Args {
   const float* lse2;    // -lse * log2(e)          (written by attn_delta_kernel)
@@ -722,32 +762,31 @@ attn_bwd2_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_consta
   uint8_t* sR0 = smem;                      // resident: K (key-major) or Q
   uint8_t* sR1 = smem + kTile;              // resident: V (key-major) or dO
   // Streamed tiles, a ring each.  Q / K is read by the first and the last product of a block, dO (key-major) by the
-  // second and third, V (query-major) by the second alone: four tiles are 2 + 2 stages or 3 + 1.
-  constexpr uint32_t kRing0 = kKeyMajor ? 2 : 3, kRing1 = kKeyMajor ? 2 : 1;
-  // Key-major: a statistics slot travels with dO, whose stage is free after dV, while the warps still read delta for dS.
-  // What keeps the slot is the producer's wait for empty0 (after dK, hence after dS) of the block kRing0 before, which comes
-  // first: that block must not be older than the slot's last user, kRing1 before.
-  static_assert(!kKeyMajor || (kRing0 <= kRing1 && kRing1 == 2), "statistics would be overwritten before dS has read them");
+  // second and third, V (query-major) by the second alone.
+  constexpr uint32_t kRing0 = 3, kRing1 = 2;
   uint8_t* sS0 = smem + 2 * kTile;          // Q or K
-  uint8_t* sS1 = sS0 + kRing0 * kTile;      // dO or V
-  uint8_t* sO = smem + 6 * kTile;           // output staging
-  float* sStat = reinterpret_cast<float*>(sO + kBwdWarps * kBwdStage);   // key-major: [2][lse2 | delta][128], with dO
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sO + kBwdWarps * kBwdStage + 2 * kStatBytes);
+  uint8_t* sS1 = smem + 5 * kTile;          // dO or V; between items the stage of an item's last block takes its output
+  // key-major: lse2 travels with Q, delta with dO.  delta(i+2) takes the slot of delta(i): its producer waits for dS(i).
+  float* sLse = reinterpret_cast<float*>(smem + 7 * kTile);   // [3][128]
+  float* sDelta = sLse + 3 * kBlk;                            // [2][128]
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + 7 * kTile + 5 * kStatBytes);
   uint8_t* clc_resp = reinterpret_cast<uint8_t*>(bars);   // 16 bytes
   uint64_t* clc_full = bars + 2;
   uint64_t* clc_empty = bars + 3;
-  uint64_t* res_full = bars + 4;
-  uint64_t* res_empty = bars + 5;
-  uint64_t* full0 = bars + 6;               // [3] rings
-  uint64_t* empty0 = bars + 9;              // [3]
-  uint64_t* full1 = bars + 12;              // [2]
-  uint64_t* empty1 = bars + 14;             // [2]
-  uint64_t* s_full = bars + 16;             // [2] (key-major uses [0] only)
-  uint64_t* dp_full = bars + 18;
-  uint64_t* p_ready = bars + 19;            // [2] key-major: the first / second 16 columns of every warp's P^T
-  uint64_t* ds_ready = bars + 21;           // dS is in TMEM
-  uint64_t* acc_done = bars + 22;           // [2] key-major: dV / dK; query-major: [1] dQ
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 24);
+  uint64_t* res_full = bars + 4;            // [2] resident tiles: the one that S reads, the one that dP reads
+  uint64_t* res_empty = bars + 6;           // [2]
+  uint64_t* full0 = bars + 8;               // [3] rings
+  uint64_t* empty0 = bars + 11;             // [3]
+  uint64_t* full1 = bars + 14;              // [2]
+  uint64_t* empty1 = bars + 16;             // [2]
+  uint64_t* s_full = bars + 18;
+  uint64_t* s_free = bars + 19;             // query-major: S is in registers
+  uint64_t* dp_full = bars + 20;            // [2] (key-major uses [0] only)
+  uint64_t* ds_ready = bars + 22;           // [2] dS is in TMEM, even and odd blocks
+  uint64_t* p_ready = bars + 24;            // [2] key-major: the first / second 16 columns of every warp's P^T
+  uint64_t* acc_done = bars + 26;           // [2] key-major: dV / dK; query-major: [1] dQ
+  uint64_t* out_read = bars + 28;           // [2] the copy engine has read the output staged in a stage of ring 1
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 30);
 
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const int group = gridDim.x;
@@ -757,25 +796,24 @@ attn_bwd2_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_consta
     tma_prefetch_desc(&tm_qkv);
     tma_prefetch_desc(&tm_do);
     mbar_init(clc_full, 1);
-    mbar_init(clc_empty, 2 + kBwdWarps);    // producer and MMA thread, element-wise warps
-    mbar_init(res_full, 1);
-    mbar_init(res_empty, 1);
+    mbar_init(clc_empty, 3 + kBwdWarps);    // producers and MMA thread, element-wise warps
     for (int i = 0; i < 3; ++i) {
       mbar_init(full0 + i, 1);
       mbar_init(empty0 + i, 1);
     }
+    mbar_init(s_full, 1);
+    mbar_init(s_free, kBwdWarps);
     for (int i = 0; i < 2; ++i) {
+      mbar_init(res_full + i, 1);
+      mbar_init(res_empty + i, 1);
       mbar_init(full1 + i, 1);
       mbar_init(empty1 + i, 1);
+      mbar_init(dp_full + i, 1);
+      mbar_init(ds_ready + i, kBwdWarps);
+      mbar_init(p_ready + i, kBwdWarps);
+      mbar_init(acc_done + i, 1);
+      mbar_init(out_read + i, kBwdWarps);
     }
-    mbar_init(s_full, 1);
-    mbar_init(s_full + 1, 1);
-    mbar_init(dp_full, 1);
-    mbar_init(p_ready, kBwdWarps);
-    mbar_init(p_ready + 1, kBwdWarps);
-    mbar_init(ds_ready, kBwdWarps);
-    mbar_init(acc_done, 1);
-    mbar_init(acc_done + 1, 1);
     mbar_fence_init();
   }
   if (warp == 1) {
@@ -787,8 +825,10 @@ attn_bwd2_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_consta
   tc_fence_after_sync();
   const uint32_t tmem = *tmem_slot;
   // key-major:   S^T [0,128)  dP^T [128,256)  dV [256,384)  dK [384,512)
-  // query-major: S buffers [0,128) [128,256)  dP [256,384)  dQ [384,512)
-  const uint32_t t_dp = tmem + (kKeyMajor ? 128 : 256);
+  // query-major: S [0,128)  dP buffers [128,256) [256,384)  dQ [384,512)
+  const uint32_t t_dp = tmem + 128;
+  const auto dp_buf = [](uint32_t q) -> uint32_t { return kKeyMajor ? 0 : q & 1; };         // of streamed block q
+  const auto dp_phase = [](uint32_t q) -> uint32_t { return (kKeyMajor ? q : q >> 1) & 1; };
   const uint32_t t_acc0 = tmem + (kKeyMajor ? 256 : 384), t_acc1 = tmem + 384;
 
   BwdItem w = bwd_item<kKeyMajor>(a, blockIdx.x, blockIdx.y, blockIdx.z, group);
@@ -809,37 +849,27 @@ attn_bwd2_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_consta
   uint32_t g = 0;                           // streamed blocks so far: stages and phases of the rings and the hand-overs
 
   if (warp == 0) {
+    // resident tile of S, ring of Q or K, next items
     if (elect_one()) {
       bool ok = true, more = true;
       while (ok && more) {
         const int colq = w.h * 3 * kD, seq0 = w.b * a.seq, rrow = seq0 + w.blk * kBlk;
         const int64_t stat0 = ((int64_t)w.b * a.heads + w.h) * a.seq;
-        if ((ok = mbar_wait(res_empty, (items & 1) ^ 1, 8 * tmo))) {
-          mbar_expect_tx(res_full, 2 * kTile);
-          if (kKeyMajor) {
-            load_tile(sR0, &tm_qkv, res_full, colq + kD, rrow);        // K
-            load_tile(sR1, &tm_qkv, res_full, colq + 2 * kD, rrow);    // V
-          } else {
-            load_tile(sR0, &tm_qkv, res_full, colq, rrow);             // Q
-            load_tile(sR1, &tm_do, res_full, w.h * kD, rrow);          // dO
+        // the resident tile of S first, then the item's first streamed tile: S needs no more
+        for (int it = -1; it < w.n_it && ok; ++it) {
+          if (it < 0) {
+            if (!(ok = mbar_wait(res_empty, (items & 1) ^ 1, 8 * tmo))) break;
+            mbar_expect_tx(res_full, kTile);
+            load_tile(sR0, &tm_qkv, res_full, kKeyMajor ? colq + kD : colq, rrow);           // K or Q
+            continue;
           }
-        }
-        for (int it = 0; it < w.n_it && ok; ++it, ++g) {
-          const uint32_t st0 = g % kRing0, st1 = g % kRing1;
+          const uint32_t st = g % kRing0;
           const int srow = (w.i0 + it) * kBlk;
-          // empty0 first: it also guards the statistics slot (see the static_assert)
-          if (!(ok = mbar_wait(empty0 + st0, ((g / kRing0) & 1) ^ 1, 8 * tmo))) break;
-          mbar_expect_tx(full0 + st0, kTile);
-          load_tile(sS0 + st0 * kTile, &tm_qkv, full0 + st0, kKeyMajor ? colq : colq + kD, seq0 + srow);   // Q or K
-          if (!(ok = mbar_wait(empty1 + st1, ((g / kRing1) & 1) ^ 1, 8 * tmo))) break;
-          mbar_expect_tx(full1 + st1, kTile + (kKeyMajor ? kStatBytes : 0));
-          if (kKeyMajor) {
-            load_tile(sS1 + st1 * kTile, &tm_do, full1 + st1, w.h * kD, seq0 + srow);                      // dO
-            bulk_g2s(sStat + st1 * 2 * kBlk, a.lse2 + stat0 + srow, kBlk * 4, full1 + st1);
-            bulk_g2s(sStat + st1 * 2 * kBlk + kBlk, a.delta + stat0 + srow, kBlk * 4, full1 + st1);
-          } else {
-            load_tile(sS1 + st1 * kTile, &tm_qkv, full1 + st1, colq + 2 * kD, seq0 + srow);                // V
-          }
+          if (!(ok = mbar_wait(empty0 + st, ((g / kRing0) & 1) ^ 1, 8 * tmo))) break;
+          mbar_expect_tx(full0 + st, kTile + (kKeyMajor ? kStatBytes : 0));
+          load_tile(sS0 + st * kTile, &tm_qkv, full0 + st, kKeyMajor ? colq : colq + kD, seq0 + srow);
+          if (kKeyMajor) bulk_g2s(sLse + st * kBlk, a.lse2 + stat0 + srow, kStatBytes, full0 + st);
+          ++g;
         }
         if (ok && (ok = mbar_wait(clc_empty, (items & 1) ^ 1, 8 * tmo))) {
           mbar_expect_tx(clc_full, 16);
@@ -848,6 +878,48 @@ attn_bwd2_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_consta
           mbar_arrive(clc_empty);
         }
         if (!ok) report(a.status, kErrAttn + 11, w.blk, g);
+      }
+    }
+  } else if (warp == 2 + kBwdWarps) {
+    // resident tile of dP, ring of dO or V: by a thread of its own, because a stage of one ring is often free long before one of the other
+    if (elect_one()) {
+      bool ok = true, more = true;
+      uint32_t outs[2] = {0, 0};              // outputs staged in either stage so far
+      bool staged[2] = {false, false};        // the last user of the stage was an item's output
+      while (ok && more) {
+        const int seq0 = w.b * a.seq, rrow = seq0 + w.blk * kBlk;
+        const int64_t stat0 = ((int64_t)w.b * a.heads + w.h) * a.seq;
+        if ((ok = mbar_wait(res_empty + 1, (items & 1) ^ 1, 8 * tmo))) {
+          mbar_expect_tx(res_full + 1, kTile);
+          if (kKeyMajor) load_tile(sR1, &tm_qkv, res_full + 1, w.h * 3 * kD + 2 * kD, rrow);     // V
+          else load_tile(sR1, &tm_do, res_full + 1, w.h * kD, rrow);                            // dO
+        }
+        for (int it = 0; it < w.n_it && ok; ++it, ++g) {
+          const uint32_t st = g % kRing1;
+          const int srow = (w.i0 + it) * kBlk;
+          if (!(ok = mbar_wait(empty1 + st, ((g / kRing1) & 1) ^ 1, 8 * tmo))) break;
+          if (staged[st] && !(ok = mbar_wait(out_read + st, (outs[st] - 1) & 1, 8 * tmo))) break;
+          staged[st] = false;
+          mbar_expect_tx(full1 + st, kTile + (kKeyMajor ? kStatBytes : 0));
+          if (kKeyMajor) {
+            load_tile(sS1 + st * kTile, &tm_do, full1 + st, w.h * kD, seq0 + srow);                                // dO
+            if (g > 1 && !(ok = mbar_wait(ds_ready + st, ((g - 2) >> 1) & 1, 8 * tmo))) break;
+            bulk_g2s(sDelta + st * kBlk, a.delta + stat0 + srow, kStatBytes, full1 + st);
+          } else {
+            load_tile(sS1 + st * kTile, &tm_qkv, full1 + st, w.h * 3 * kD + 2 * kD, seq0 + srow);                  // V
+          }
+        }
+        if (ok) {
+          const uint32_t st = (g - 1) % kRing1;
+          staged[st] = true;
+          ++outs[st];
+        }
+        if (ok) {
+          more = next_item();
+          mbar_arrive(clc_empty);
+        } else {
+          report(a.status, kErrAttn + 11, w.blk, g);
+        }
       }
     }
   } else if (warp == 1) {
@@ -868,18 +940,19 @@ attn_bwd2_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_consta
         report(a.status, kErrAttn + code, g, items);
         return false;
       };
-      // S (or S^T) / dP (or dP^T) of streamed block number q, once its tile is there
+      // S (or S^T) / dP (or dP^T) of streamed block number q, once its tile is there and the block before is out of S (key-major:
+      // the products that read its P^T were issued before)
       auto issue_s = [&](uint32_t q) -> bool {
         const uint32_t st = q % kRing0;
+        if (!kKeyMajor && q > 0 && !wait(s_free, (q - 1) & 1, 19)) return false;
         if (!wait(full0 + st, (q / kRing0) & 1, 13)) return false;
         const uint64_t tile = ds0k + st * kStageOff;
-        const int buf = kKeyMajor ? 0 : (q & 1);
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
           const uint64_t off = (uint64_t)(((k >> 2) * kHalf + (k & 3) * 32) >> 4);
-          umma_f16(tmem + buf * 128, dr0 + off, tile + off, id_s, k != 0);
+          umma_f16(tmem, dr0 + off, tile + off, id_s, k != 0);
         }
-        umma_commit(s_full + buf);
+        umma_commit(s_full);
         return true;
       };
       auto issue_dp = [&](uint32_t q) -> bool {
@@ -889,10 +962,21 @@ attn_bwd2_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_consta
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
           const uint64_t off = (uint64_t)(((k >> 2) * kHalf + (k & 3) * 32) >> 4);
-          umma_f16(t_dp, dr1 + off, tile + off, id_s, k != 0);
+          umma_f16(t_dp + dp_buf(q) * 128, dr1 + off, tile + off, id_s, k != 0);
         }
-        umma_commit(dp_full);
+        umma_commit(dp_full + dp_buf(q));
         if (!kKeyMajor) umma_commit(empty1 + st);         // V has no other reader
+        return true;
+      };
+      // The first blocks of an item also wait for its resident tiles.  An item's last products of either kind free them.
+      auto first_s = [&](uint32_t q) -> bool {
+        if (!(wait(res_full, items & 1, 12) && issue_s(q))) return false;
+        if (w.n_it == 1) umma_commit(res_empty);
+        return true;
+      };
+      auto first_dp = [&](uint32_t q) -> bool {
+        if (!(wait(res_full + 1, items & 1, 12) && issue_dp(q))) return false;
+        if (w.n_it == 1) umma_commit(res_empty + 1);
         return true;
       };
       // acc += (P or dS in TMEM at `src`: a warp's columns packed from its first column) * streamed tile; the k-steps
@@ -903,12 +987,13 @@ attn_bwd2_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_consta
           umma_f16_ts(acc, src + i * kBwdCols + part * 8, tile + (uint64_t)(((2 * i + part) * 2048) >> 4), id_g,
                       !(first && i == 0));
       };
+      // Blocks follow one another across items: the next item's first S is issued where the next block's would be, and its
+      // first dP behind this item's last product.
+      ok = first_s(g) && first_dp(g);
       while (ok && more) {
         const int n = w.n_it;
-        if (!(ok = wait(res_full, items & 1, 12) && issue_s(g) && issue_dp(g))) break;
-        if (n == 1) umma_commit(res_empty);
         for (int it = 0; it < n && ok; ++it, ++g) {
-          const bool next = it + 1 < n;
+          const bool last = it + 1 == n;
           const uint32_t st0 = g % kRing0, st1 = g % kRing1;
           if (kKeyMajor) {
             // dV += P^T dO (contraction over the queries)
@@ -917,21 +1002,32 @@ attn_bwd2_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_consta
             if (!(ok = wait(p_ready + 1, g & 1, 14))) break;
             issue_grad(t_acc0, tmem, ds1m + st1 * kStageOff, 1, false);
             umma_commit(empty1 + st1);
-            if (!next) umma_commit(acc_done);
+            if (last) umma_commit(acc_done);
           }
-          // key-major: P^T(it) is read by the products just issued; query-major: the other S buffer
-          if (next && !(ok = issue_s(g + 1))) break;
-          if (!(ok = wait(ds_ready, g & 1, 14))) break;
-          issue_grad(kKeyMajor ? t_acc1 : t_acc0, t_dp, ds0m + st0 * kStageOff, 0, it == 0);   // dK += dS^T Q / dQ += dS K
-          issue_grad(kKeyMajor ? t_acc1 : t_acc0, t_dp, ds0m + st0 * kStageOff, 1, false);
+          if (!last) {
+            if (!(ok = issue_s(g + 1))) break;
+            if (it + 2 == n) umma_commit(res_empty);
+            if (!kKeyMajor) {
+              if (!(ok = issue_dp(g + 1))) break;
+              if (it + 2 == n) umma_commit(res_empty + 1);
+            }
+          } else {
+            more = next_item();                           // w is the next item's from here on
+            mbar_arrive(clc_empty);
+            if (more && !(ok = first_s(g + 1))) break;
+          }
+          if (!(ok = wait(ds_ready + (g & 1), (g >> 1) & 1, 14))) break;
+          const uint32_t acc = kKeyMajor ? t_acc1 : t_acc0, ds = t_dp + dp_buf(g) * 128;
+          issue_grad(acc, ds, ds0m + st0 * kStageOff, 0, it == 0);     // dK += dS^T Q / dQ += dS K
+          issue_grad(acc, ds, ds0m + st0 * kStageOff, 1, false);
           umma_commit(empty0 + st0);
-          if (!next) umma_commit(acc_done + 1);
-          if (next && !(ok = issue_dp(g + 1))) break;
-          if (it + 2 == n) umma_commit(res_empty);
-        }
-        if (ok) {
-          more = next_item();
-          mbar_arrive(clc_empty);
+          if (last) umma_commit(acc_done + 1);
+          if (last) {
+            if (more && !(ok = first_dp(g + 1))) break;
+          } else if (kKeyMajor) {
+            if (!(ok = issue_dp(g + 1))) break;
+            if (it + 2 == n) umma_commit(res_empty + 1);
+          }
         }
       }
     }
@@ -940,12 +1036,11 @@ attn_bwd2_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_consta
     const int part = (warp - 2) >> 2;                     // which kBwdCols of the 128 columns
     const int row = q4 * 32 + lane;                       // TMEM lane: key (key-major) or query
     const uint32_t lane_off = static_cast<uint32_t>(q4 * 32) << 16;
-    const uint32_t tdp = t_dp + lane_off + part * kBwdCols;
     const uint64_t sl2 = f32x2(a.scale * kLog2e, a.scale * kLog2e), sc2 = f32x2(a.scale, a.scale);
-    uint8_t* stage = sO + (warp - 2) * kBwdStage;
     bool ok = true, more = true;
     while (more) {
-      const int me = w.blk * kBlk + row;                  // this lane's key (key-major) or query index
+      const int me = w.blk * kBlk + row;                  // query-major: this lane's query
+      const int me0 = w.blk * kBlk + q4 * 32 + (lane >> 2);   // key-major: the first of this thread's keys
       uint64_t my_lse2 = 0, my_delta = 0;
       if (!kKeyMajor) {
         const int64_t at = ((int64_t)w.b * a.heads + w.h) * a.seq + me;
@@ -953,17 +1048,18 @@ attn_bwd2_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_consta
         my_delta = f32x2(a.delta[at], a.delta[at]);
       }
       for (int it = 0; it < w.n_it; ++it, ++g) {
-        const int sb = kKeyMajor ? 0 : (g & 1);
-        const uint32_t ts = tmem + lane_off + sb * 128 + part * kBwdCols;
+        const uint32_t ts = tmem + lane_off + part * kBwdCols, tdp = ts + 128 + dp_buf(g) * 128;
         const int c0 = (w.i0 + it) * kBlk + part * kBwdCols;   // first streamed index of this thread's columns
-        const ulonglong2* stat = reinterpret_cast<const ulonglong2*>(sStat + (g & 1) * 2 * kBlk + part * kBwdCols);
+        const uint32_t st0 = g % kRing0;
+        // key-major: lse2 / delta of this thread's columns
+        const float* my_lse = sLse + st0 * kBlk + part * kBwdCols + (lane & 3) * 2;
+        const float* my_dlt = sDelta + (g & 1) * kBlk + part * kBwdCols + (lane & 3) * 2;
         // causal: a score survives when key <= query; only blocks that touch the diagonal pay for it
-        const bool masked = a.causal && (kKeyMajor ? (c0 < me) : (c0 + kBwdCols - 1 > me));
+        const bool masked = a.causal && (kKeyMajor ? (c0 < me0 + 24) : (c0 + kBwdCols - 1 > me));
         float e[kBwdCols];                                // P of this thread's columns
         // ---- phase 1: P = exp2(S * scale * log2(e) - lse2) ----
-        // (key-major: the statistics come with dO, whose barrier orders them for this thread)
-        if (!warp_wait(s_full + sb, kKeyMajor ? (g & 1) : ((g >> 1) & 1), 8 * tmo) ||
-            (kKeyMajor && !warp_wait(full1 + (g & 1), (g >> 1) & 1, 8 * tmo))) {
+        // (key-major: lse2 comes with Q and delta with dO, whose barriers order them for this thread)
+        if (!warp_wait(s_full, g & 1, 8 * tmo) || (kKeyMajor && !warp_wait(full0 + st0, (g / kRing0) & 1, 8 * tmo))) {
           if (lane == 0) report(a.status, kErrAttn + 15, it, 0);
           ok = false;
           break;
@@ -971,31 +1067,56 @@ attn_bwd2_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_consta
         tc_fence_after_sync();
         {
           uint32_t rs[kBwdCols];
-          tmem_ld_32x32(ts, rs);
+          if (kKeyMajor) {
+            tmem_ld_16x32_frag(ts, rs);
+            tmem_ld_16x32_frag(ts + (16u << 16), rs + 16);
+          } else {
+            tmem_ld_32x32(ts, rs);
+          }
           tmem_ld_wait();
+          if (!kKeyMajor) {
+            tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(s_free);           // the next block's S may be computed
+          }
+          uint64_t st[4] = {my_lse2, my_lse2, my_lse2, my_lse2};
+          if (kKeyMajor) {
+#pragma unroll
+            for (int n = 0; n < 4; ++n) st[n] = *reinterpret_cast<const uint64_t*>(my_lse + n * 8);
+          }
+          // key-major: columns of a fragment are in groups n of 8, elements 4 n + {0, 1} of this thread's first row of a
+          // lane half, + {2, 3} of its second; by halves of 16 columns, so that P^T can be handed over in two parts
 #pragma unroll
           for (int hp = 0; hp < 2; ++hp) {
 #pragma unroll
-            for (int k = hp * 16; k < hp * 16 + 16; k += 4) {
-              ulonglong2 st = make_ulonglong2(my_lse2, my_lse2);
-              if (kKeyMajor) st = stat[k >> 2];
-              split(fma2(f32x2(__uint_as_float(rs[k]), __uint_as_float(rs[k + 1])), sl2, st.x), e[k], e[k + 1]);
-              split(fma2(f32x2(__uint_as_float(rs[k + 2]), __uint_as_float(rs[k + 3])), sl2, st.y), e[k + 2], e[k + 3]);
-#pragma unroll
-              for (int u = 0; u < 4; ++u) e[k + u] = fast_exp2(e[k + u]);
+            for (int i = 0; i < kBwdCols / 2; i += 2) {
+              const int k = kKeyMajor ? (i >> 3) * 16 + hp * 8 + (i & 7) : hp * 16 + i;
+              split(fma2(f32x2(__uint_as_float(rs[k]), __uint_as_float(rs[k + 1])), sl2, st[(k >> 2) & 3]), e[k], e[k + 1]);
+              e[k] = kKeyMajor && i % 8 < kBwdPoly ? exp2_fma(e[k]) : fast_exp2(e[k]);
+              e[k + 1] = kKeyMajor && i % 8 + 1 < kBwdPoly ? exp2_fma(e[k + 1]) : fast_exp2(e[k + 1]);
             }
             if (masked) {
 #pragma unroll
-              for (int k = hp * 16; k < hp * 16 + 16; ++k)
-                if (!(kKeyMajor ? (me <= c0 + k) : (c0 + k <= me))) e[k] = 0.f;
+              for (int i = 0; i < kBwdCols / 2; ++i) {
+                const int k = kKeyMajor ? (i >> 3) * 16 + hp * 8 + (i & 7) : hp * 16 + i;
+                if (kKeyMajor) {
+                  const int key = me0 + (k >> 4) * 16 + (k >> 1 & 1) * 8, query = c0 + (k >> 2 & 3) * 8 + (lane & 3) * 2 + (k & 1);
+                  if (key > query) e[k] = 0.f;
+                } else if (c0 + k > me) {
+                  e[k] = 0.f;
+                }
+              }
             }
             if (kKeyMajor) {
-              // P^T over this thread's own S^T columns, packed from the first: the products that read the first 16
+              // P^T over this warp's own S^T columns, packed from the first: the products that read the first 16
               // run under the exponentials of the second
-              uint32_t pk[8];
 #pragma unroll
-              for (int i = 0; i < 8; ++i) pk[i] = pack_bf16(e[hp * 16 + 2 * i], e[hp * 16 + 2 * i + 1]);
-              tmem_st_32x8(ts + hp * 8, pk);
+              for (int h = 0; h < 2; ++h) {
+                uint32_t pk[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) pk[i] = pack_bf16(e[h * 16 + hp * 8 + 2 * i], e[h * 16 + hp * 8 + 2 * i + 1]);
+                tmem_st_16x16_frag(ts + hp * 8 + ((h * 16u) << 16), pk);
+              }
               tmem_st_wait();
               tc_fence_before_sync();
               __syncwarp();
@@ -1004,7 +1125,8 @@ attn_bwd2_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_consta
           }
         }
         // ---- phase 2: dS = P * (dP * scale - delta * scale) ----
-        if (!warp_wait(dp_full, g & 1, 8 * tmo)) {
+        if (!warp_wait(dp_full + dp_buf(g), dp_phase(g), 8 * tmo) ||
+            (kKeyMajor && !warp_wait(full1 + (g & 1), (g >> 1) & 1, 8 * tmo))) {
           if (lane == 0) report(a.status, kErrAttn + 16, it, 0);
           ok = false;
           break;
@@ -1012,25 +1134,34 @@ attn_bwd2_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_consta
         tc_fence_after_sync();
         {
           uint32_t rp[kBwdCols], dk[16];
-          tmem_ld_32x32(tdp, rp);
+          uint64_t st[4] = {my_delta, my_delta, my_delta, my_delta};
+          if (kKeyMajor) {
+            tmem_ld_16x32_frag(tdp, rp);
+            tmem_ld_16x32_frag(tdp + (16u << 16), rp + 16);
+#pragma unroll
+            for (int n = 0; n < 4; ++n) st[n] = *reinterpret_cast<const uint64_t*>(my_dlt + n * 8);
+          } else {
+            tmem_ld_32x32(tdp, rp);
+          }
           tmem_ld_wait();
 #pragma unroll
-          for (int k = 0; k < kBwdCols; k += 4) {
-            ulonglong2 st = make_ulonglong2(my_delta, my_delta);
-            if (kKeyMajor) st = stat[kBlk / 4 + (k >> 2)];
+          for (int k = 0; k < kBwdCols; k += 2) {
             float g0, g1;
             split(mul2(f32x2(e[k], e[k + 1]),
-                       fma2(f32x2(__uint_as_float(rp[k]), __uint_as_float(rp[k + 1])), sc2, st.x)), g0, g1);
+                       fma2(f32x2(__uint_as_float(rp[k]), __uint_as_float(rp[k + 1])), sc2, st[(k >> 2) & 3])), g0, g1);
             dk[k >> 1] = pack_bf16(g0, g1);
-            split(mul2(f32x2(e[k + 2], e[k + 3]),
-                       fma2(f32x2(__uint_as_float(rp[k + 2]), __uint_as_float(rp[k + 3])), sc2, st.y)), g0, g1);
-            dk[(k >> 1) + 1] = pack_bf16(g0, g1);
           }
-          tmem_st_32x16(tdp, dk);               // dS over this thread's own dP columns
+          // dS over this thread's own dP columns
+          if (kKeyMajor) {
+            tmem_st_16x32_frag(tdp, dk);
+            tmem_st_16x32_frag(tdp + (16u << 16), dk + 8);
+          } else {
+            tmem_st_32x16(tdp, dk);
+          }
           tmem_st_wait();
           tc_fence_before_sync();
           __syncwarp();
-          if (lane == 0) mbar_arrive(ds_ready);
+          if (lane == 0) mbar_arrive(ds_ready + (g & 1));
         }
       }
       if (!ok) break;
@@ -1038,6 +1169,8 @@ attn_bwd2_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_consta
       // (with plain stores the warps stall for 4000 cycles when all SMs write their items at the same time).
       const int col = w.h * 3 * kD + part * kBwdCols, orow = w.b * a.seq + w.blk * kBlk + q4 * 32;
       const uint32_t phase = items & 1;
+      const uint32_t out_st = (g - 1) & 1;
+      uint8_t* stage = sS1 + out_st * kTile + (warp - 2) * kBwdStage;   // where the item's last dO or V was
       more = next_item();                        // w is the next item's from here on
 #pragma unroll 1
       for (int which = kKeyMajor ? 0 : 1; which < 2; ++which) {
@@ -1064,6 +1197,10 @@ attn_bwd2_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_consta
         warp_store_box(&tm_dqkv, stage, col + (kKeyMajor ? (which == 0 ? 2 * kD : kD) : 0), orow);
       }
       if (!ok) break;
+      if (lane == 0) {
+        bulk_wait_read<0>();
+        mbar_arrive(out_read + out_st);          // the stage may take a tile again
+      }
       tc_fence_before_sync();                    // the accumulators are read before the next P / dS is announced
       __syncwarp();                              // every lane has read the response
       if (lane == 0) mbar_arrive(clc_empty);

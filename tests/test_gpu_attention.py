@@ -151,3 +151,35 @@ def test_attention_backward_is_bit_identical_from_run_to_run():
     b = F.attention_bwd(dout, qkv, out, lse, batch, seq, heads, True)
     _native.check_status()
     assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("causal", [False, True])
+def test_attention_backward_of_vanishing_probabilities_and_nan(causal):
+    """Scores up to 400 apart: most probabilities are below 2^-126 (the polynomial's exponent is clamped there), one per row
+    is not.  The oracle's are zero there, the kernel's at most 2^-125, which changes nothing in bf16.  A NaN in one head's
+    dout and one in the other's qkv show where the oracle has them, whatever pipe computes the exponential."""
+    from meshslice_b200 import _native
+    from meshslice_b200.ops import functional as F
+    batch, seq, heads = 1, 384, 3
+    g = torch.Generator(device="cuda").manual_seed(9)
+    qkv = torch.randn(batch * seq, heads * 3 * 128, device="cuda", generator=g).bfloat16()
+    for h in range(heads):
+        qkv[:, h * 384:h * 384 + 256] *= 4.0
+    dout = torch.randn(batch * seq, heads * 128, device="cuda", generator=g).bfloat16()
+    out, lse = F.attention_fwd(qkv, batch, seq, heads, causal)
+    dqkv = F.attention_bwd(dout, qkv, out, lse, batch, seq, heads, causal)
+    _native.check_status()
+    _, _, dref = _ref(qkv, batch, seq, heads, causal, dout)
+    assert ((dqkv.float() - dref).norm() / dref.norm()).item() < 8 * 2 ** -9   # probabilities near 0 or 1: P - delta cancels
+    dout[200, 5] = float("nan")                 # head 0
+    qkv[130, 384 + 128 + 7] = float("nan")      # a key of head 1
+    out, lse = F.attention_fwd(qkv, batch, seq, heads, causal)
+    dqkv = F.attention_bwd(dout, qkv, out, lse, batch, seq, heads, causal)
+    _native.check_status()
+    _, _, dref = _ref(qkv, batch, seq, heads, causal, dout)
+    rows = slice(200, 256) if causal else slice(0, seq)   # queries whose row holds a NaN
+    assert torch.isnan(dqkv[200, :128]).all() and torch.isnan(dref[200, :128]).all()
+    assert torch.isnan(dqkv[rows, 384:512]).all() and torch.isnan(dref[rows, 384:512]).all()
+    clean = slice(768, 1152)
+    assert torch.isfinite(dqkv[:, clean]).all()
+    assert ((dqkv[:, clean].float() - dref[:, clean]).norm() / dref[:, clean].norm()).item() < 8 * 2 ** -9
