@@ -196,6 +196,10 @@ __device__ __forceinline__ void tmem_st_16x16_frag(uint32_t taddr, const uint32_
   asm volatile("tcgen05.st.sync.aligned.16x128b.x2.b32 [%0], {%1, %2, %3, %4};"
                ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]) : "memory");
 }
+// Programmatic dependent launch: wait until the grids before this one in the stream are complete and their writes visible /
+// let the next grid start once every block of this one has come here.  Without the launch attribute both do nothing.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 // shared -> global, one box of a tensor map; tracked by bulk groups
 __device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, const void* smem_src, int32_t x, int32_t y) {
   asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];"
@@ -627,6 +631,7 @@ __global__ void __launch_bounds__(256)
 attn_delta_kernel(const uint4* __restrict__ out, const uint4* __restrict__ dout, float* __restrict__ delta,
                   uint32_t groups, uint32_t seq, uint32_t heads, const float* __restrict__ lse, float* __restrict__ lse2,
                   float scale) {
+  grid_trigger();                        // the key-major kernel may set up; it waits for this one before it reads a statistic
   const uint32_t sub = threadIdx.x & 15;
   const uint32_t w = blockIdx.x * (blockDim.x >> 4) + (threadIdx.x >> 4);   // (group of tokens, head)
   const bool live = w < groups;
@@ -868,7 +873,13 @@ attn_bwd2_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_consta
           if (!(ok = mbar_wait(empty0 + st, ((g / kRing0) & 1) ^ 1, 8 * tmo))) break;
           mbar_expect_tx(full0 + st, kTile + (kKeyMajor ? kStatBytes : 0));
           load_tile(sS0 + st * kTile, &tm_qkv, full0 + st, kKeyMajor ? colq : colq + kD, seq0 + srow);
-          if (kKeyMajor) bulk_g2s(sLse + st * kBlk, a.lse2 + stat0 + srow, kStatBytes, full0 + st);
+          if (kKeyMajor) {
+            if (g == 0) {
+              grid_wait();                    // the statistics are written (every read of them here comes after this or the
+              grid_trigger();                 // other producer's wait); then the query-major kernel may start on free SMs
+            }
+            bulk_g2s(sLse + st * kBlk, a.lse2 + stat0 + srow, kStatBytes, full0 + st);
+          }
           ++g;
         }
         if (ok && (ok = mbar_wait(clc_empty, (items & 1) ^ 1, 8 * tmo))) {
@@ -904,6 +915,7 @@ attn_bwd2_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_consta
           if (kKeyMajor) {
             load_tile(sS1 + st * kTile, &tm_do, full1 + st, w.h * kD, seq0 + srow);                                // dO
             if (g > 1 && !(ok = mbar_wait(ds_ready + st, ((g - 2) >> 1) & 1, 8 * tmo))) break;
+            if (g == 0) grid_wait();
             bulk_g2s(sDelta + st * kBlk, a.delta + stat0 + srow, kStatBytes, full1 + st);
           } else {
             load_tile(sS1 + st * kTile, &tm_qkv, full1 + st, w.h * 3 * kD + 2 * kD, seq0 + srow);                  // V
@@ -1211,6 +1223,8 @@ attn_bwd2_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_consta
   __syncthreads();
   tc_fence_after_sync();
   if (warp == 1) tmem_dealloc(tmem, 512);
+  // What follows in the stream waits for this grid alone: it ends after the key-major one, whose blocks all run or are done.
+  if (!kKeyMajor && threadIdx.x == 0) grid_wait();
 }
 
 // The shared-memory attribute is per device: set it once on every device that launches.
@@ -1323,12 +1337,21 @@ cudaError_t attention_bwd(const void* qkv, const void* out, const void* dout, co
   g.status = status;
   g.timeout_ns = 2000000000ull;
   const int grp = bh_group(batch, heads);
-  dim3 grid2(grp, seq / kBlk, batch * heads / grp);
-  attn_bwd2_kernel<true><<<grid2, kBwd2Threads, kBwd2Smem, stream>>>(tq, td, tg, g);
-  cudaError_t e = cudaGetLastError();
+  // Overlap of the three launches: the key-major kernel sets up and loads its first tiles while the row sums end, the
+  // query-major one, which reads nothing of it, takes SMs as they get free (batch 3 x 640, 5 heads: 75 items each).
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grp, seq / kBlk, batch * heads / grp);
+  cfg.blockDim = dim3(kBwd2Threads);
+  cfg.dynamicSmemBytes = kBwd2Smem;
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  cudaError_t e = cudaLaunchKernelEx(&cfg, attn_bwd2_kernel<true>, tq, td, tg, g);
   if (e != cudaSuccess) return e;
-  attn_bwd2_kernel<false><<<grid2, kBwd2Threads, kBwd2Smem, stream>>>(tq, td, tg, g);
-  return cudaGetLastError();
+  return cudaLaunchKernelEx(&cfg, attn_bwd2_kernel<false>, tq, td, tg, g);
 }
 
 }  // namespace msb

@@ -183,3 +183,34 @@ def test_attention_backward_of_vanishing_probabilities_and_nan(causal):
     clean = slice(768, 1152)
     assert torch.isfinite(dqkv[:, clean]).all()
     assert ((dqkv[:, clean].float() - dref[:, clean]).norm() / dref[:, clean].norm()).item() < 8 * 2 ** -9
+
+
+@pytest.mark.parametrize("shape", [(1, 128, 1), (3, 640, 5), (2, 1024, 24)])
+def test_attention_backward_launches_in_order(shape):
+    """The three launches of a call overlap; what comes before and after them in the stream does not.  Calls follow one
+    another on the same buffers, inputs are overwritten right behind a call and the result is copied right behind it: the
+    same bits as a call by itself.  Items: fewer than SMs in both kernels together, about as many, more."""
+    from meshslice_b200 import _native
+    from meshslice_b200.ops import functional as F
+    batch, seq, heads = shape
+    g = torch.Generator(device="cuda").manual_seed(3)
+    sets = []
+    for _ in range(3):
+        qkv = torch.randn(batch * seq, heads * 3 * 128, device="cuda", generator=g).bfloat16()
+        dout = torch.randn(batch * seq, heads * 128, device="cuda", generator=g).bfloat16()
+        out, lse = F.attention_fwd(qkv, batch, seq, heads, True)
+        torch.cuda.synchronize()
+        want = F.attention_bwd(dout, qkv, out, lse, batch, seq, heads, True)
+        torch.cuda.synchronize()
+        sets.append((qkv, dout, out, lse, want.clone()))
+    work = [torch.empty_like(t) for t in sets[0][:4]]
+    got = []
+    for i in range(24):
+        for w, t in zip(work, sets[i % 3]):
+            w.copy_(t)
+        got.append(F.attention_bwd(work[1], work[0], work[2], work[3], batch, seq, heads, True).clone())
+        for w in work:
+            w.fill_(float("nan"))
+    _native.check_status()
+    for i, t in enumerate(got):
+        assert torch.equal(t, sets[i % 3][4]), i
