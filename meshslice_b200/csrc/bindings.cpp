@@ -106,6 +106,17 @@ ParsedExchange parse_exchange(const py::object& o) {
 // ---------------------------------------------------------------------------------------
 // GEMM
 // ---------------------------------------------------------------------------------------
+void run_gemm2(const Gemm2Operands* o, int problems, int tile_n, int sms, uint32_t* status, uint64_t timeout_ns, uint64_t stream) {
+  Gemm2Args args;
+  for (int i = 0; i < problems; ++i) {
+    const int r = gemm2_problem(&args.p[i], o[i], tile_n);
+    if (r != 0) throw std::runtime_error("gemm: tensor map failed, code " + std::to_string(r));
+  }
+  args.status = status;
+  args.timeout_ns = timeout_ns;
+  check(launch_sm100_gemm2(args, problems, tile_n, sms, S(stream)), "sm100_gemm2 launch");
+}
+
 void gemm_run(const py::dict& d) {
   GemmArgs a;
   std::memset(&a, 0, sizeof(a));
@@ -226,18 +237,23 @@ void gemm_run(const py::dict& d) {
   if (a.trace != nullptr && (a.trace_cap <= 0 || (getp(d, "trace") & 15)))
     throw std::runtime_error("gemm: the timeline buffer needs trace_cap > 0 and 16-byte alignment");
 
+  const bool plain = a.n_chunks == 0 && a.n_ranks == 0 && a.red_n == 0 && a.push_n == 0 && a.tiles_m > 0;
+  const int sms = (int)geti(d, "grid", 148);
+  const bool try3d = geti(d, "map3d", 1) != 0;
+  if (plain && geti(d, "two_cta", 1) != 0) {
+    const Gemm2Operands o = {a.M, a.N, a.K, P<void>(A), lda, a.a_mn_major, P<void>(B), ldb, a.b_mn_major, a.C, a.ldc,
+                             a.c_fp32, a.accumulate, a.bias, a.act, a.C_pre, try3d, a.group};
+    run_gemm2(&o, 1, gemm2_tile_n(&o, 1, sms), sms, a.status, a.timeout_ns, getp(d, "stream"));
+    return;
+  }
   CUtensorMap ta, tb;
   int r;
-  const bool try3d = geti(d, "map3d", 1) != 0;
   if (!a.a_mn_major) r = make_tensor_map_2d(&ta, P<void>(A), a.K, a.M, lda * 2, kBK, kBM);
   else if (try3d && make_tensor_map_mn3d(&ta, P<void>(A), a.M, a.K, lda * 2, kBM / 64) == 0) { r = 0; a.a_map3d = 1; }
   else r = make_tensor_map_2d(&ta, P<void>(A), a.M, a.K, lda * 2, 64, kBK);
   if (r != 0) throw std::runtime_error("gemm: tensor map for A failed, code " + std::to_string(r));
-  const bool plain = a.n_chunks == 0 && a.n_ranks == 0 && a.red_n == 0 && a.push_n == 0 && a.tiles_m > 0;
-  const bool pair = plain && geti(d, "two_cta", 1) != 0;
-  const int sms = (int)geti(d, "grid", 148), tile_n = pair ? gemm2_tile_n(a.M, a.N, sms) : kBN;
-  if (!a.b_mn_major) r = make_tensor_map_2d(&tb, P<void>(B), a.K, a.N, ldb * 2, kBK, tile_n / 2);
-  else if (try3d && make_tensor_map_mn3d(&tb, P<void>(B), a.N, a.K, ldb * 2, tile_n / 128) == 0) { r = 0; a.b_map3d = 1; }
+  if (!a.b_mn_major) r = make_tensor_map_2d(&tb, P<void>(B), a.K, a.N, ldb * 2, kBK, kBN / 2);
+  else if (try3d && make_tensor_map_mn3d(&tb, P<void>(B), a.N, a.K, ldb * 2, kBN / 128) == 0) { r = 0; a.b_map3d = 1; }
   else r = make_tensor_map_2d(&tb, P<void>(B), a.N, a.K, ldb * 2, 64, kBK);
   if (r != 0) throw std::runtime_error("gemm: tensor map for B failed, code " + std::to_string(r));
 
@@ -247,10 +263,6 @@ void gemm_run(const py::dict& d) {
   if (!needs_all && grid > 2 * ntiles) grid = 2 * ntiles;
   grid &= ~1;
   if (grid < 2) grid = 2;
-  if (pair) {
-    check(launch_sm100_gemm2(ta, tb, a, tile_n, sms, S(getp(d, "stream"))), "sm100_gemm2 launch");
-    return;
-  }
   static PushMaps pm;   // only the first push_n entries are read by the kernel
   if (a.push_n > 0) {
     const uint64_t rows = (uint64_t)geti(d, "push_rows");
@@ -266,64 +278,92 @@ void gemm_run(const py::dict& d) {
 // The plain local GEMM of `ops.gemm`: the few values it needs, positionally.  Filling the dict of gemm_run and reading
 // it back took longer than a small product takes on the GPU (a linear layer of 512 x 512 x 1536, forward and backward:
 // 108 us a pass, 59 us through this call).  MSB_TWO_CTA, MSB_G2_GROUP and MSB_G2_MAP3D are read per call, as they were.
-void gemm_local(int64_t M, int64_t N, int64_t K, uint64_t A, int64_t lda, int a_mn_major, uint64_t B, int64_t ldb,
-                int b_mn_major, uint64_t C, int64_t ldc, int c_fp32, int accumulate, uint64_t bias, int act,
-                uint64_t C_pre, int two_cta, int sms, uint64_t status, uint64_t stream) {
-  const auto env = [](const char* name, int otherwise) {
-    const char* v = std::getenv(name);
-    return v != nullptr ? std::atoi(v) : otherwise;
-  };
-  GemmArgs a;
-  std::memset(&a, 0, sizeof(a));
+int env_int(const char* name, int otherwise) {
+  const char* v = std::getenv(name);
+  return v != nullptr ? std::atoi(v) : otherwise;
+}
+bool two_cta_default() {
+  const char* v = std::getenv("MSB_TWO_CTA");
+  return v == nullptr || std::strcmp(v, "0") != 0;
+}
+Gemm2Operands local_operands(int64_t M, int64_t N, int64_t K, uint64_t A, int64_t lda, int a_mn_major, uint64_t B, int64_t ldb,
+                             int b_mn_major, uint64_t C, int64_t ldc, int c_fp32, int accumulate, uint64_t status) {
   if (M <= 0 || N <= 0 || K <= 0) throw std::runtime_error("gemm: empty problem");
   if ((lda % 8) || (ldb % 8) || (A & 15) || (B & 15))
     throw std::runtime_error("gemm: operands need 16-byte aligned bases and pitches");
   if (ldc % 8) throw std::runtime_error("gemm: ldc must be a multiple of 8");
   if (status == 0) throw std::runtime_error("gemm: status pointer required");
-  a.M = (int)M;
-  a.N = (int)N;
-  a.K = (int)K;
-  a.a_mn_major = a_mn_major;
-  a.b_mn_major = b_mn_major;
-  a.C = P<void>(C);
-  a.ldc = ldc;
-  a.c_fp32 = c_fp32;
-  a.accumulate = accumulate;
-  a.bias = P<void>(bias);
-  a.act = act;
-  a.C_pre = P<void>(C_pre);
+  return {M, N, K, P<void>(A), lda, a_mn_major, P<void>(B), ldb, b_mn_major, P<void>(C), ldc, c_fp32, accumulate,
+          nullptr, 0, nullptr, env_int("MSB_G2_MAP3D", 1) != 0, std::max(0, env_int("MSB_G2_GROUP", 0))};
+}
+constexpr uint64_t kLocalTimeoutNs = 1000000000ull;
+
+// The one-CTA kernel on a plain product (MSB_TWO_CTA=0).
+void run_gemm1(const Gemm2Operands& o, int sms, uint64_t status, uint64_t stream) {
+  GemmArgs a;
+  std::memset(&a, 0, sizeof(a));
+  a.M = (int)o.M;
+  a.N = (int)o.N;
+  a.K = (int)o.K;
+  a.a_mn_major = o.a_mn_major;
+  a.b_mn_major = o.b_mn_major;
+  a.C = o.C;
+  a.ldc = o.ldc;
+  a.c_fp32 = o.c_fp32;
+  a.accumulate = o.accumulate;
+  a.bias = o.bias;
+  a.act = o.act;
+  a.C_pre = o.C_pre;
   a.tiles_m = (a.M + 2 * kBM - 1) / (2 * kBM);
   a.tiles_n = (a.N + kBN - 1) / kBN;
   a.n_slices = a.cyc = a.push_extent = a.push_bufs = a.b_nchunk = a.a_kpanel = a.b_kpanel = 1;
-  a.group = env("MSB_G2_GROUP", 0);
+  a.group = o.group > 0 ? o.group : 8;
   a.status = P<uint32_t>(status);
-  a.timeout_ns = 1000000000ull;
-
-  if (two_cta < 0) {
-    const char* v = std::getenv("MSB_TWO_CTA");
-    two_cta = v == nullptr || std::strcmp(v, "0") != 0;
-  }
+  a.timeout_ns = kLocalTimeoutNs;
   CUtensorMap ta, tb;
   int r;
-  const bool try3d = env("MSB_G2_MAP3D", 1) != 0;
-  if (!a_mn_major) r = make_tensor_map_2d(&ta, P<void>(A), a.K, a.M, lda * 2, kBK, kBM);
-  else if (try3d && make_tensor_map_mn3d(&ta, P<void>(A), a.M, a.K, lda * 2, kBM / 64) == 0) { r = 0; a.a_map3d = 1; }
-  else r = make_tensor_map_2d(&ta, P<void>(A), a.M, a.K, lda * 2, 64, kBK);
+  if (!o.a_mn_major) r = make_tensor_map_2d(&ta, o.A, a.K, a.M, o.lda * 2, kBK, kBM);
+  else if (o.map3d && make_tensor_map_mn3d(&ta, o.A, a.M, a.K, o.lda * 2, kBM / 64) == 0) { r = 0; a.a_map3d = 1; }
+  else r = make_tensor_map_2d(&ta, o.A, a.M, a.K, o.lda * 2, 64, kBK);
   if (r != 0) throw std::runtime_error("gemm: tensor map for A failed, code " + std::to_string(r));
-  const int tile_n = two_cta ? gemm2_tile_n(a.M, a.N, sms) : kBN;
-  if (!b_mn_major) r = make_tensor_map_2d(&tb, P<void>(B), a.K, a.N, ldb * 2, kBK, tile_n / 2);
-  else if (try3d && make_tensor_map_mn3d(&tb, P<void>(B), a.N, a.K, ldb * 2, tile_n / 128) == 0) { r = 0; a.b_map3d = 1; }
-  else r = make_tensor_map_2d(&tb, P<void>(B), a.N, a.K, ldb * 2, 64, kBK);
+  if (!o.b_mn_major) r = make_tensor_map_2d(&tb, o.B, a.K, a.N, o.ldb * 2, kBK, kBN / 2);
+  else if (o.map3d && make_tensor_map_mn3d(&tb, o.B, a.N, a.K, o.ldb * 2, kBN / 128) == 0) { r = 0; a.b_map3d = 1; }
+  else r = make_tensor_map_2d(&tb, o.B, a.N, a.K, o.ldb * 2, 64, kBK);
   if (r != 0) throw std::runtime_error("gemm: tensor map for B failed, code " + std::to_string(r));
+  const int grid = std::max(2, std::min(sms & ~1, 2 * a.tiles_m * a.tiles_n));
+  static const PushMaps no_push = {};
+  check(launch_sm100_gemm(ta, tb, no_push, a, grid, S(stream)), "sm100_gemm launch");
+}
 
-  if (two_cta) {
-    check(launch_sm100_gemm2(ta, tb, a, tile_n, sms, S(stream)), "sm100_gemm2 launch");
-  } else {
-    const int grid = std::max(2, std::min(sms & ~1, 2 * a.tiles_m * a.tiles_n));
-    if (a.group <= 0) a.group = 8;
-    static const PushMaps no_push = {};
-    check(launch_sm100_gemm(ta, tb, no_push, a, grid, S(stream)), "sm100_gemm launch");
+void gemm_local(int64_t M, int64_t N, int64_t K, uint64_t A, int64_t lda, int a_mn_major, uint64_t B, int64_t ldb,
+                int b_mn_major, uint64_t C, int64_t ldc, int c_fp32, int accumulate, uint64_t bias, int act,
+                uint64_t C_pre, int two_cta, int sms, uint64_t status, uint64_t stream) {
+  Gemm2Operands o = local_operands(M, N, K, A, lda, a_mn_major, B, ldb, b_mn_major, C, ldc, c_fp32, accumulate, status);
+  o.bias = P<void>(bias);
+  o.act = act;
+  o.C_pre = P<void>(C_pre);
+  if (two_cta < 0) two_cta = two_cta_default();
+  if (two_cta) run_gemm2(&o, 1, gemm2_tile_n(&o, 1, sms), sms, P<uint32_t>(status), kLocalTimeoutNs, stream);
+  else run_gemm1(o, sms, status, stream);
+}
+
+// Two independent products in one launch, the longer contraction first (thirteen values each, as in gemm_local).
+void gemm_pair(const py::args& v, int sms, uint64_t status, uint64_t stream) {
+  if (v.size() != 26) throw std::runtime_error("gemm_pair: thirteen values per product");
+  const auto i = [&](int k) { return v[k].cast<int64_t>(); };
+  const auto u = [&](int k) { return v[k].cast<uint64_t>(); };
+  Gemm2Operands o[2];
+  for (int k = 0; k < 2; ++k) {
+    const int b = 13 * k;
+    o[k] = local_operands(i(b), i(b + 1), i(b + 2), u(b + 3), i(b + 4), (int)i(b + 5), u(b + 6), i(b + 7), (int)i(b + 8), u(b + 9),
+                          i(b + 10), (int)i(b + 11), (int)i(b + 12), status);
   }
+  if (!two_cta_default()) {
+    for (const Gemm2Operands& p : o) run_gemm1(p, sms, status, stream);
+    return;
+  }
+  if (o[1].K > o[0].K) std::swap(o[0], o[1]);
+  run_gemm2(o, 2, gemm2_tile_n(o, 2, sms), sms, P<uint32_t>(status), kLocalTimeoutNs, stream);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -385,6 +425,9 @@ PYBIND11_MODULE(_C, m) {
   m.def("gemm_run", &gemm_run, "persistent tcgen05 GEMM with optional fused gather / push");
   m.def("gemm_local", &gemm_local, "plain local GEMM: M, N, K, A, lda, a_mn_major, B, ldb, b_mn_major, C, ldc, c_fp32, "
         "accumulate, bias, act, C_pre, two_cta (-1: MSB_TWO_CTA), sms, status, stream");
+  m.def("gemm_pair", &gemm_pair, py::kw_only(), py::arg("sms"), py::arg("status"), py::arg("stream"),
+        "two independent plain GEMMs in one launch: M, N, K, A, lda, a_mn_major, B, ldb, b_mn_major, C, ldc, c_fp32, accumulate "
+        "of either");
   m.def("symm_alloc", &symm_alloc);
   m.def("symm_open", &symm_open);
   m.def("symm_close", &symm_close);

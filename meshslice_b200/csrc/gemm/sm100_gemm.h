@@ -159,10 +159,6 @@ struct GemmArgs {
   uint32_t* go_flag;           // local: set to epoch by CTA 0 once all peers have arrived
   uint32_t* done_counter;      // local: CTAs that finished their transfers (monotonic)
   uint32_t done_target;
-  // ---- plain (two-CTA) kernel ----
-  int along_n;                 // raster groups along N instead of M (with group <= 0 the launcher sets all three)
-  int k_turn;                  // every other tile of a CTA pair walks its k-blocks backwards
-  int tma_c;                   // set by its launcher: C (and C_pre) leave through shared memory as TMA stores
   // ---- status ----
   uint32_t* status;            // [4]: code, blockIdx, detail, detail2
   uint64_t timeout_ns;
@@ -190,14 +186,54 @@ cudaError_t launch_sm100_gemm(const CUtensorMap& tma_a, const CUtensorMap& tma_b
                               const PushMaps& push_maps, const GemmArgs& args, int grid,
                               cudaStream_t stream);
 
-// Two-CTA (cta_group::2) variant for plain local GEMMs (no gather / push / reduce / barriers) on at most `sms` SMs.
-// `tile_n` columns per cluster tile (gemm2_tile_n); the tensor map of a K-major B must use a {64, tile_n / 2} box,
-// that of an MN-major B one box of tile_n / 128 blocks of 64 columns.
-int gemm2_tile_n(int M, int N, int sms);
+// Two-CTA (cta_group::2) kernel for plain local GEMMs (no gather / push / reduce / barriers): C (+)= op(A) op(B).
+struct Gemm2Operands {
+  int64_t M, N, K;
+  const void* A;
+  int64_t lda;
+  int a_mn_major;      // 0: A stored [M,K] row-major; 1: A stored [K,M] row-major
+  const void* B;
+  int64_t ldb;
+  int b_mn_major;      // 0: B stored [N,K] row-major; 1: B stored [K,N] row-major
+  void* C;
+  int64_t ldc;
+  int c_fp32;          // 1: C is float, 0: C is bf16
+  int accumulate;      // 1: C += result
+  const void* bias;    // bf16 [N] or null
+  int act;             // 0: none, 1: tanh-GeLU
+  void* C_pre;         // bf16, same layout as C: pre-activation copy (act != 0), may be null
+  int map3d;           // MN-major operands through the 3-D map where their extent allows it
+  int group;           // raster group along M, 0: gemm2_order chooses
+};
+// The same as the kernel reads it.
+struct Gemm2Problem {
+  CUtensorMap a, b, c, pre;    // c, pre: used when tma_c
+  void* C;
+  int64_t ldc;
+  const void* bias;
+  void* C_pre;
+  int M, N, K;
+  int a_mn_major, b_mn_major;
+  int a_map3d, b_map3d;        // the tensor map of an MN-major operand is the 3-D form of make_tensor_map_mn3d
+  int c_fp32, accumulate, act;
+  int tma_c;                   // C (and C_pre) leave through shared memory as TMA stores
+  int group, along_n, k_turn;  // tile order: panels of `group` blocks along M or N; every other tile of a CTA pair walks its
+                               // k-blocks backwards
+};
+struct Gemm2Args {
+  Gemm2Problem p[2];
+  int tiles[2];                // tiles of the first problem, of both (set by the launcher)
+  uint32_t* status;            // [4]: code, blockIdx, detail, detail2
+  uint64_t timeout_ns;
+};
+// Columns of a cluster tile for a launch of one or two problems, the order of a problem's tiles, and its maps for that width
+// (0, or an error code).
+int gemm2_tile_n(const Gemm2Operands* o, int problems, int sms);
 struct Gemm2Order { int group, along_n, k_turn; };
 Gemm2Order gemm2_order(int64_t M, int64_t N, int64_t K, int tile_n);
-cudaError_t launch_sm100_gemm2(const CUtensorMap& tma_a, const CUtensorMap& tma_b, GemmArgs args, int tile_n, int sms,
-                               cudaStream_t stream);
+int gemm2_problem(Gemm2Problem* p, const Gemm2Operands& o, int tile_n);
+// One or two problems of the same tile width in a launch on at most `sms` SMs.
+cudaError_t launch_sm100_gemm2(Gemm2Args& args, int problems, int tile_n, int sms, cudaStream_t stream);
 
 // Builds a 2-D bf16 tensor map with a swizzle of 128 (or 64) bytes.  `inner` is the contiguous extent,
 // `outer` the number of rows, `pitch_bytes` the row pitch.  Returns 0 on success.

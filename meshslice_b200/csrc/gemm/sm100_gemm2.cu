@@ -12,6 +12,7 @@
 //   tempty[acc]    lives in the leader, 8 arrivals: one per epilogue warp of both CTAs
 // No load uses cluster multicast.  Every wait is bounded as in the one-CTA kernel.
 #include <cuda_bf16.h>
+#include <string.h>
 
 #include "../common/ptx.cuh"
 #include "out_turn.h"
@@ -83,7 +84,7 @@ __device__ __forceinline__ uint64_t desc_at(uint32_t lo, uint32_t hi) {
   return d;
 }
 
-__device__ __forceinline__ void report2(const GemmArgs& a, uint32_t code, uint32_t d0, uint32_t d1) {
+__device__ __forceinline__ void report2(const Gemm2Args& a, uint32_t code, uint32_t d0, uint32_t d1) {
   if (atomicCAS(a.status, 0u, code) == 0u) {
     a.status[1] = blockIdx.x;
     a.status[2] = d0;
@@ -225,12 +226,14 @@ __device__ __forceinline__ void tile2(int t, int tiles_m2, int tiles_n, int grou
 
 }  // namespace
 
-// BN: columns of a cluster tile (gemm2_tile_n chooses).
+// BN: columns of a cluster tile (gemm2_tile_n chooses).  A launch works on one problem or on two independent ones: the tiles
+// of the second follow those of the first, so that CTA pairs without a tile in the first one's last wave begin with the
+// second.  The two gradients of a linear layer that way, in one launch and in two: 1992 x 4104 x 1032 (85 tiles of 32
+// k-blocks and 136 of 17 on 74 pairs) 92.9 -> 81.9 us for the whole layer, 512 x 512 x 1536 38 -> 34, 4096 x 1024 x 51200 with
+// its loss 1309 -> 1296; 8192 x 4096 x 16384 is under the power cap either way (2541 and 2537).
 template <int BN>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads2, 1)
-sm100_gemm2_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
-                   const __grid_constant__ CUtensorMap tma_c, const __grid_constant__ CUtensorMap tma_pre,
-                   const __grid_constant__ GemmArgs a) {
+sm100_gemm2_kernel(const __grid_constant__ Gemm2Args a) {
   constexpr int kStages2 = stages2(BN);
   constexpr uint32_t kBStage2 = b_stage2(BN);
   extern __shared__ uint8_t smem_raw[];
@@ -251,16 +254,21 @@ sm100_gemm2_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_const
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();      // 0: leader
   const uint64_t tmo = a.timeout_ns;
-  const int tiles_m2 = (a.M + 2 * kBM - 1) / (2 * kBM);
-  const int tiles_n = (a.N + BN - 1) / BN;
-  const int num_tiles = tiles_m2 * tiles_n;
-  const int kblocks = (a.K + kBK - 1) / kBK;
+  const int num_tiles = a.tiles[1];
   const int cluster_id = blockIdx.x >> 1, n_clusters = gridDim.x >> 1;
-  const int group = a.group;
+  // Tile t: its problem and its place in it.
+  const auto place = [&](int t, bool& second, int& m2, int& nb) {
+    second = t >= a.tiles[0];
+    const Gemm2Problem& p0 = a.p[0];
+    const Gemm2Problem& p1 = a.p[1];
+    const int M = second ? p1.M : p0.M, N = second ? p1.N : p0.N;
+    tile2(second ? t - a.tiles[0] : t, (M + 2 * kBM - 1) / (2 * kBM), (N + BN - 1) / BN, second ? p1.group : p0.group,
+          (second ? p1.along_n : p0.along_n) != 0, m2, nb);
+  };
 
   if (warp == 0 && lane == 0) {
-    tma_prefetch_desc(&tma_a);
-    tma_prefetch_desc(&tma_b);
+    tma_prefetch_desc(&a.p[0].a);
+    tma_prefetch_desc(&a.p[0].b);
     for (int i = 0; i < kStages2; ++i) {
       mbar_init(full_bar + i, 2);    // the leader's two producers announce their operand's bytes
       mbar_init(empty_bar + i, 1);
@@ -294,10 +302,19 @@ sm100_gemm2_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_const
       bool ok = true, free = true;                                // `free`: the next stage was seen empty
       bool back = false;                                          // this tile's k-blocks run from the last to the first
       for (int t = cluster_id; t < num_tiles && ok; t += n_clusters) {
+        bool second;
         int m2, nb;
-        tile2(t, tiles_m2, tiles_n, group, a.along_n != 0, m2, nb);
-        const int row_a = (2 * m2 + (int)rank) * kBM;           // this CTA's 128 rows of A
-        const int col_b = nb * BN + (int)rank * (BN / 2);       // this CTA's half of the columns of B
+        place(t, second, m2, nb);
+        const Gemm2Problem* p = second ? &a.p[1] : &a.p[0];
+        const CUtensorMap* map = is_a ? &p->a : &p->b;
+        const bool mn_major = (is_a ? p->a_mn_major : p->b_mn_major) != 0, map3d = (is_a ? p->a_map3d : p->b_map3d) != 0;
+        const int kblocks = (p->K + kBK - 1) / kBK;
+        const bool turn = p->k_turn != 0;
+        // this CTA's 128 rows of A / its half of the columns of B
+        const int row = is_a ? (2 * m2 + (int)rank) * kBM : nb * BN + (int)rank * (BN / 2);
+        const uint32_t bytes = is_a ? kAStage2 : kBStage2;
+        uint8_t* ring = is_a ? sA : sB;
+        const int boxes = is_a ? kBM / 64 : BN / 128;
         for (int kb = 0; kb < kblocks; ++kb) {
           if (!free && !mbar_wait(empty_bar + stage, phase ^ 1, 5 * tmo)) {
             report2(a, kTimeoutEmpty, t, kb);
@@ -306,35 +323,19 @@ sm100_gemm2_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_const
           }
           const uint32_t fb = full0 + stage * 8;
           const int k0 = (back ? kblocks - 1 - kb : kb) * kBK;
-          if (is_a) {
-            if (rank == 0) mbar_expect_tx(full_bar + stage, 2 * kAStage2);
-            uint8_t* da = sA + stage * kAStage2;
-            if (!a.a_mn_major) {
-              tma_load_2d_pair(da, &tma_a, fb, k0, row_a);
-            } else if (a.a_map3d) {
-              tma_load_3d_pair(da, &tma_a, fb, 0, k0, row_a >> 6);
-            } else {
-#pragma unroll
-              for (int j = 0; j < kBM / 64; ++j)
-                tma_load_2d_pair(da + j * (kBK * 128), &tma_a, fb, row_a + j * 64, k0);
-            }
+          if (rank == 0) mbar_expect_tx(full_bar + stage, 2 * bytes);
+          uint8_t* dst = ring + stage * bytes;
+          if (!mn_major) {
+            tma_load_2d_pair(dst, map, fb, k0, row);
+          } else if (map3d) {
+            tma_load_3d_pair(dst, map, fb, 0, k0, row >> 6);
           } else {
-            if (rank == 0) mbar_expect_tx(full_bar + stage, 2 * kBStage2);
-            uint8_t* db = sB + stage * kBStage2;
-            if (!a.b_mn_major) {
-              tma_load_2d_pair(db, &tma_b, fb, k0, col_b);
-            } else if (a.b_map3d) {
-              tma_load_3d_pair(db, &tma_b, fb, 0, k0, col_b >> 6);
-            } else {
-#pragma unroll
-              for (int j = 0; j < BN / 128; ++j)
-                tma_load_2d_pair(db + j * (kBK * 128), &tma_b, fb, col_b + j * 64, k0);
-            }
+            for (int j = 0; j < boxes; ++j) tma_load_2d_pair(dst + j * (kBK * 128), map, fb, row + j * 64, k0);
           }
           if (++stage == kStages2) { stage = 0; phase ^= 1; }
           free = mbar_test(empty_bar + stage, phase ^ 1);
         }
-        back = !back && a.k_turn;
+        back = !back && turn;
       }
     }
   } else if (warp == 1) {
@@ -344,12 +345,6 @@ sm100_gemm2_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_const
     // critical path a k-block took 590 cycles whatever BN.  So only the low descriptor word changes, by additions; one
     // commit reaches both CTAs; and the next stage is looked at before this one is issued.
     if (rank == 0 && elect_one()) {
-      const uint32_t idesc = make_idesc_bf16(2 * kBM, BN, a.a_mn_major, a.b_mn_major);
-      const uint64_t da0 = make_smem_desc(smem_u32(sA), a.a_mn_major ? kBK * 128 : 16, 1024);
-      const uint64_t db0 = make_smem_desc(smem_u32(sB), a.b_mn_major ? kBK * 128 : 16, 1024);
-      const uint32_t da_hi = (uint32_t)(da0 >> 32), db_hi = (uint32_t)(db0 >> 32);
-      const uint32_t a_kstep = (a.a_mn_major ? 16 * 128 : 32) >> 4;
-      const uint32_t b_kstep = (a.b_mn_major ? 16 * 128 : 32) >> 4;
       uint32_t stage = 0, phase = 0;
       bool ok = true, full = false;                               // `full`: the next stage was seen complete
       int it = 0;
@@ -361,6 +356,15 @@ sm100_gemm2_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_const
           break;
         }
         const uint32_t tmem_d = tmem_base + acc * BN;
+        const Gemm2Problem* p = t >= a.tiles[0] ? &a.p[1] : &a.p[0];
+        const int kblocks = (p->K + kBK - 1) / kBK;
+        const bool a_mn = p->a_mn_major != 0, b_mn = p->b_mn_major != 0;
+        const uint32_t idesc = make_idesc_bf16(2 * kBM, BN, a_mn, b_mn);
+        const uint64_t da0 = make_smem_desc(smem_u32(sA), a_mn ? kBK * 128 : 16, 1024);
+        const uint64_t db0 = make_smem_desc(smem_u32(sB), b_mn ? kBK * 128 : 16, 1024);
+        const uint32_t da_hi = (uint32_t)(da0 >> 32), db_hi = (uint32_t)(db0 >> 32);
+        const uint32_t a_kstep = (a_mn ? 16 * 128 : 32) >> 4;
+        const uint32_t b_kstep = (b_mn ? 16 * 128 : 32) >> 4;
         for (int kb = 0; kb < kblocks; ++kb) {
           if (!full && !mbar_wait(full_bar + stage, phase, 4 * tmo)) {
             report2(a, kTimeoutFull, t, kb);
@@ -385,14 +389,21 @@ sm100_gemm2_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_const
   } else {
     // ===================== epilogue (both CTAs, own 128 rows) =====================
     const int q = warp & 3;
-    const __nv_bfloat16* bias = reinterpret_cast<const __nv_bfloat16*>(a.bias);
-    const bool dual = a.act == 1 && a.C_pre != nullptr;   // two outputs: no store of one runs under the other's staging
     OutStage out{smem + kSmemOut2 + q * 2 * kOutBox, {0}};
     bool ok = true;
     int it = 0;
     for (int t = cluster_id; t < num_tiles && ok; t += n_clusters, ++it) {
+      bool second;
       int m2, nb;
-      tile2(t, tiles_m2, tiles_n, group, a.along_n != 0, m2, nb);
+      place(t, second, m2, nb);
+      const Gemm2Problem& p = second ? a.p[1] : a.p[0];
+      const __nv_bfloat16* bias = reinterpret_cast<const __nv_bfloat16*>(p.bias);
+      void* const C = p.C;
+      void* const C_pre = p.C_pre;
+      const int64_t ldc = p.ldc;
+      const int M = p.M, N = p.N, act = p.act;
+      const bool fp32 = p.c_fp32 != 0, add = p.accumulate != 0, tma_c = p.tma_c != 0;
+      const bool dual = act == 1 && C_pre != nullptr;       // two outputs: no store of one runs under the other's staging
       const uint32_t acc = it & 1, acc_phase = (it >> 1) & 1;
       int okw = 1;
       if (lane == 0) okw = mbar_wait(tfull_bar + acc, acc_phase, 7 * tmo) ? 1 : 0;
@@ -421,8 +432,8 @@ sm100_gemm2_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_const
           if (lane == 0) mbar_arrive_cluster(te_leader);     // accumulator drained: tell the leader's MMA warp
         }
         const int col0 = nb * BN + c * 32;
-        const int nvalid = min(32, a.N - col0);
-        if (row0 >= a.M || nb * BN + (c & ~1) * 32 >= a.N) continue;   // the two halves of a bf16 box go together
+        const int nvalid = min(32, N - col0);
+        if (row0 >= M || nb * BN + (c & ~1) * 32 >= N) continue;   // the two halves of a bf16 box go together
         float v[32];
 #pragma unroll
         for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
@@ -431,35 +442,35 @@ sm100_gemm2_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_const
           for (int i = 0; i < 32; ++i)
             if (i < nvalid) v[i] += __bfloat162float(bias[col0 + i]);
         }
-        if (!a.tma_c) {
-          if (row0 + lane >= a.M || nvalid <= 0) continue;
-          if (a.act == 1) {
-            if (a.C_pre != nullptr) store32(a.C_pre, a.ldc, false, false, row0 + lane, col0, nvalid, v);
+        if (!tma_c) {
+          if (row0 + lane >= M || nvalid <= 0) continue;
+          if (act == 1) {
+            if (C_pre != nullptr) store32(C_pre, ldc, false, false, row0 + lane, col0, nvalid, v);
 #pragma unroll
             for (int i = 0; i < 32; ++i) v[i] = gelu_tanh2(v[i]);
           }
-          store32(a.C, a.ldc, a.c_fp32 != 0, a.accumulate != 0, row0 + lane, col0, nvalid, v);
+          store32(C, ldc, fp32, add, row0 + lane, col0, nvalid, v);
           continue;
         }
         // rows and columns beyond the matrix are clipped by the tensor map
-        if (a.act == 1) {
+        if (act == 1) {
           if (dual) {
             if ((c & 1) == 0) box_pre = out.take(lane);
             stage_bf16(box_pre, lane, c & 1, v);
-            if (c & 1) out.send(&tma_pre, box_pre, lane, col0 - 32, row0, false);
+            if (c & 1) out.send(&p.pre, box_pre, lane, col0 - 32, row0, false);
           }
 #pragma unroll
           for (int i = 0; i < 32; ++i) v[i] = gelu_tanh2(v[i]);
         }
-        if (a.c_fp32) {
+        if (fp32) {
           if (nvalid <= 0) continue;
           box = dual ? out.take<1>(lane) : out.take(lane);
           stage_f32(box, lane, v);
-          out.send(&tma_c, box, lane, col0, row0, a.accumulate != 0);
+          out.send(&p.c, box, lane, col0, row0, add);
         } else {
           if ((c & 1) == 0) box = dual ? out.take<1>(lane) : out.take(lane);
           stage_bf16(box, lane, c & 1, v);
-          if (c & 1) out.send(&tma_c, box, lane, col0 - 32, row0, false);
+          if (c & 1) out.send(&p.c, box, lane, col0 - 32, row0, false);
         }
       }
     }
@@ -475,8 +486,7 @@ sm100_gemm2_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_const
 }
 
 template <int BN>
-static cudaError_t launch2(const CUtensorMap& tma_a, const CUtensorMap& tma_b, const CUtensorMap& tma_c,
-                           const CUtensorMap& tma_pre, const GemmArgs& args, int grid, cudaStream_t stream) {
+static cudaError_t launch2(const Gemm2Args& args, int grid, cudaStream_t stream) {
   static bool configured[64] = {false};
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
@@ -488,19 +498,33 @@ static cudaError_t launch2(const CUtensorMap& tma_a, const CUtensorMap& tma_b, c
     configured[dev] = true;
   }
   // the cluster shape (2,1,1) is part of the kernel's definition
-  sm100_gemm2_kernel<BN><<<grid, kThreads2, smem, stream>>>(tma_a, tma_b, tma_c, tma_pre, args);
+  sm100_gemm2_kernel<BN><<<grid, kThreads2, smem, stream>>>(args);
   return cudaGetLastError();
 }
 
-// The tile width with the shorter last wave.  A 64-deep k-block takes about 390 cycles on 128 columns (the loads: 24 KiB
-// a CTA) and 530 on 256 (the tensor pipe: 512), so a wave of narrow tiles counts three quarters of a wide one.
+// The tile width that ends sooner.  A 64-deep k-block takes about 390 cycles on 128 columns (the loads: 24 KiB
+// a CTA) and 530 on 256 (the tensor pipe: 512), so a narrow tile counts three quarters of a wide one.  A CTA pair takes every
+// n-th tile: the last pair to end is the one with one tile more of either problem (pair 0) or the first without.
 // 2048 x 1024 x 4096 (32 wide tiles): 26.5 us wide, 19.6 narrow; 1024 x 2048 x 1024 11.9 and 8.7; 2048 x 2048 x 2048 (64
 // wide tiles, one wave against two): wide, 16.3 us.
-int gemm2_tile_n(int M, int N, int sms) {
-  const int64_t clusters = sms > 1 ? sms / 2 : 1, rows = (M + 2 * kBM - 1) / (2 * kBM);
-  const int64_t wide = (rows * ((N + 255) / 256) + clusters - 1) / clusters;
-  const int64_t narrow = (rows * ((N + 127) / 128) + clusters - 1) / clusters;
-  return 3 * narrow < 4 * wide ? 128 : 256;
+static int64_t last_end(const Gemm2Operands* o, int problems, int tile_n, int64_t pairs) {
+  int64_t tiles[2] = {0, 0}, kb[2] = {0, 0};
+  for (int i = 0; i < problems; ++i) {
+    tiles[i] = ((o[i].M + 2 * kBM - 1) / (2 * kBM)) * ((o[i].N + tile_n - 1) / tile_n);
+    kb[i] = (o[i].K + kBK - 1) / kBK;
+  }
+  const int64_t all = tiles[0] + tiles[1], at[3] = {0, tiles[0] % pairs, all % pairs};
+  int64_t last = 0;
+  for (int64_t i : at) {
+    const int64_t n0 = (tiles[0] - i + pairs - 1) / pairs, n = (all - i + pairs - 1) / pairs;
+    const int64_t end = n0 * kb[0] + (n - n0) * kb[1];
+    last = end > last ? end : last;
+  }
+  return last;
+}
+int gemm2_tile_n(const Gemm2Operands* o, int problems, int sms) {
+  const int64_t pairs = sms > 1 ? sms / 2 : 1;
+  return 3 * last_end(o, problems, 128, pairs) < 4 * last_end(o, problems, 256, pairs) ? 128 : 256;
 }
 
 // The order of the tiles, by what they read from HBM: under the power cap that traffic costs clock.  A panel of sixteen
@@ -519,26 +543,52 @@ Gemm2Order gemm2_order(int64_t M, int64_t N, int64_t K, int tile_n) {
   return o;
 }
 
-cudaError_t launch_sm100_gemm2(const CUtensorMap& tma_a, const CUtensorMap& tma_b, GemmArgs args, int tile_n, int sms,
-                               cudaStream_t stream) {
+int gemm2_problem(Gemm2Problem* p, const Gemm2Operands& o, int tile_n) {
+  memset(static_cast<void*>(p), 0, sizeof(*p));
+  p->M = (int)o.M;
+  p->N = (int)o.N;
+  p->K = (int)o.K;
+  p->a_mn_major = o.a_mn_major;
+  p->b_mn_major = o.b_mn_major;
+  p->C = o.C;
+  p->ldc = o.ldc;
+  p->c_fp32 = o.c_fp32;
+  p->accumulate = o.accumulate;
+  p->bias = o.bias;
+  p->act = o.act;
+  p->C_pre = o.C_pre;
+  int r;
+  if (!o.a_mn_major) r = make_tensor_map_2d(&p->a, o.A, o.K, o.M, o.lda * 2, kBK, kBM);
+  else if (o.map3d && make_tensor_map_mn3d(&p->a, o.A, o.M, o.K, o.lda * 2, kBM / 64) == 0) { r = 0; p->a_map3d = 1; }
+  else r = make_tensor_map_2d(&p->a, o.A, o.M, o.K, o.lda * 2, 64, kBK);
+  if (r != 0) return r;
+  if (!o.b_mn_major) r = make_tensor_map_2d(&p->b, o.B, o.K, o.N, o.ldb * 2, kBK, tile_n / 2);
+  else if (o.map3d && make_tensor_map_mn3d(&p->b, o.B, o.N, o.K, o.ldb * 2, tile_n / 128) == 0) { r = 0; p->b_map3d = 1; }
+  else r = make_tensor_map_2d(&p->b, o.B, o.N, o.K, o.ldb * 2, 64, kBK);
+  if (r != 0) return r;
   // Output through shared memory and TMA where the tensor map allows it; bf16 accumulation adds before it rounds,
   // which the copy engine cannot do.
-  CUtensorMap tc = tma_a, tp = tma_a;   // any valid map where it is not used
-  args.tma_c = !(args.accumulate && !args.c_fp32) &&
-               make_tensor_map_out(&tc, args.C, args.N, args.M, args.ldc, args.c_fp32 != 0) == 0 &&
-               (args.act == 0 || args.C_pre == nullptr ||
-                make_tensor_map_out(&tp, args.C_pre, args.N, args.M, args.ldc, false) == 0);
-  if (args.group <= 0) {
-    const Gemm2Order o = gemm2_order(args.M, args.N, args.K, tile_n);
-    args.group = o.group;
-    args.along_n = o.along_n;
-    args.k_turn = o.k_turn;
+  p->tma_c = !(o.accumulate && !o.c_fp32) && make_tensor_map_out(&p->c, o.C, o.N, o.M, o.ldc, o.c_fp32 != 0) == 0 &&
+             (o.act == 0 || o.C_pre == nullptr || make_tensor_map_out(&p->pre, o.C_pre, o.N, o.M, o.ldc, false) == 0);
+  const Gemm2Order order = o.group > 0 ? Gemm2Order{o.group, 0, 0} : gemm2_order(o.M, o.N, o.K, tile_n);
+  p->group = order.group;
+  p->along_n = order.along_n;
+  p->k_turn = order.k_turn;
+  return 0;
+}
+
+cudaError_t launch_sm100_gemm2(Gemm2Args& args, int problems, int tile_n, int sms, cudaStream_t stream) {
+  int64_t tiles = 0;
+  for (int i = 0; i < 2; ++i) {
+    if (i < problems) {
+      const Gemm2Problem& p = args.p[i];
+      tiles += (int64_t)((p.M + 2 * kBM - 1) / (2 * kBM)) * ((p.N + tile_n - 1) / tile_n);
+    }
+    args.tiles[i] = (int)tiles;
   }
-  const int64_t tiles = (int64_t)((args.M + 2 * kBM - 1) / (2 * kBM)) * ((args.N + tile_n - 1) / tile_n);
   int grid = (int)(2 * tiles < (sms & ~1) ? 2 * tiles : (sms & ~1));
   if (grid < 2) grid = 2;
-  if (tile_n == 128) return launch2<128>(tma_a, tma_b, tc, tp, args, grid, stream);
-  return launch2<256>(tma_a, tma_b, tc, tp, args, grid, stream);
+  return tile_n == 128 ? launch2<128>(args, grid, stream) : launch2<256>(args, grid, stream);
 }
 
 }  // namespace msb

@@ -63,6 +63,7 @@ class ShardedFFLayer:
         b = SPMD(mesh, algorithm, blocksize, backend=backend)
         self._OS, self._LS, self._RS = b.OS(ksplit), b.LS(ksplit), b.RS(ksplit)
         self._fused = b._fused() is not None
+        self._dw_dx = getattr(b._fused(), "dw_dx", None)      # both gradients in one launch (1 x 1 mesh)
         self._x = None
 
     # dW accumulates across micro-batches: the fused kernels add into the gradient buffer in
@@ -100,6 +101,9 @@ class ShardedFFLayer:
     def backward(self, dy: ShardedTensor, need_dx: bool = True) -> Optional[ShardedTensor]:
         x, w = self._x, self.weight
         self._x = None
+        if need_dx and self._dw_dx is not None:
+            (key, g), = self.grad.shards.items()
+            return ShardedTensor(self.mesh, {key: self._dw_dx(self.dataflow, x, dy, w, g)})
         if self.dataflow == "os":
             self._dw(self._RS, x, dy)
             return self._LS(dy, w) if need_dx else None

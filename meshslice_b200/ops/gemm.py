@@ -61,3 +61,28 @@ def gemm(a, b, layout="nn", *, out=None, out_dtype=torch.bfloat16, accumulate=Fa
         0 if act is None or pre_act is None else pre_act.data_ptr(), -1 if two_cta is None else int(bool(two_cta)),
         _SM_COUNT.get(a.device.index) or sm_count(a.device), _native.status().dev, _native.stream_ptr())
     return out
+
+
+def _operands(a, b, layout, out, accumulate):
+    M, N, K = _dims(a, b, layout)
+    if out is None:
+        if accumulate:
+            raise ValueError("accumulate=True needs an output tensor")
+        out = a.new_empty((M, N))
+    (lda, sa), (ldb, sb), (ldc, sc) = a.stride(), b.stride(), out.stride()
+    if a.dtype != torch.bfloat16 or b.dtype != torch.bfloat16 or sa != 1 or sb != 1:
+        raise ValueError("GEMM operands must be bf16 with a contiguous last dimension")
+    if out.shape != (M, N) or sc != 1:
+        raise ValueError("bad output shape")
+    return out, (M, N, K, a.data_ptr(), lda, 1 if layout == "tn" else 0, b.data_ptr(), ldb, 0 if layout == "nt" else 1,
+                 out.data_ptr(), ldc, 1 if out.dtype == torch.float32 else 0, 1 if accumulate else 0)
+
+
+def gemm_pair(a0, b0, layout0, out0, accumulate0, a1, b1, layout1, out1=None, accumulate1=False):
+    """Two independent products as ``gemm`` computes them, in one launch (the two gradients of a linear layer): returns
+    both outputs.  Neither output may overlap an operand or the output of the other product."""
+    out0, v0 = _operands(a0, b0, layout0, out0, accumulate0)
+    out1, v1 = _operands(a1, b1, layout1, out1, accumulate1)
+    _native.load().gemm_pair(*v0, *v1, sms=_SM_COUNT.get(a0.device.index) or sm_count(a0.device),
+                             status=_native.status().dev, stream=_native.stream_ptr())
+    return out0, out1

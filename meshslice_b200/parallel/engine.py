@@ -14,7 +14,7 @@ from typing import Optional
 import torch
 
 from .. import _native
-from ..ops.gemm import gemm, sm_count
+from ..ops.gemm import gemm, gemm_pair, sm_count
 from . import runtime as rt
 from .fused import FusedGemm, FusedPlanError, MeshCoord
 from .mesh import DistMesh, ShardedTensor
@@ -185,6 +185,16 @@ class LocalGemmEngine:
 
     def rs(self, X, W, n_slices=1, out=None, accumulate=False, rot_index=None):
         return self._run(X, W, "tn", out, accumulate)
+
+    def dw_dx(self, dataflow, x, dy, w, grad):
+        """Both gradients of a linear layer, which do not depend on each other, in one launch: the weight's is added to
+        ``grad``, the input's is returned."""
+        x, dy, w = _local(x), _local(dy), _local(w)
+        if dataflow == "os":
+            return gemm_pair(x, dy, "tn", grad, True, dy, w, "nt")[1]
+        if dataflow == "ls":
+            return gemm_pair(dy, x, "tn", grad, True, dy, w, "nn")[1]
+        return gemm_pair(x, dy, "nn", grad, True, w, dy, "nt")[1]
 
     def check(self):
         _native.check_status()

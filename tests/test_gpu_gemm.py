@@ -215,3 +215,46 @@ def test_gemm_fp32_accumulation_keeps_subnormals():
         _native.check_status()
         assert alone[0, 1].item() == 64 * 2.0 ** (ea + eb)
         assert torch.equal(out.cpu(), (before.double() + alone.double()).float())
+
+
+# Shapes (tokens, d_in, d_out) of the two gradients in one launch: fewer tiles than CTA pairs in both (narrow tiles), ragged
+# edges and rows whose pitch is no multiple of 128 bytes, one problem longer than a wave, one with a single short k-block,
+# contractions walked backwards in one of the two.
+@pytest.mark.parametrize("dataflow", ["os", "ls", "rs"])
+@pytest.mark.parametrize("shape", [(512, 512, 1536), (1992, 1032, 4104), (264, 5128, 72), (8, 264, 520), (4360, 2048, 3080)])
+def test_gemm_pair_is_both_products(shape, dataflow):
+    """Against the fp32 reference of each product, and bit for bit from run to run."""
+    from meshslice_b200 import _native
+    from meshslice_b200.ops.gemm import gemm_pair
+    t, i, o = shape
+    g = torch.Generator(device="cuda").manual_seed(t)
+    rand = lambda *s: torch.randn(s, device="cuda", generator=g).bfloat16()
+    x, dy, w = rand(t, i), rand(t, o), rand(o, i) if dataflow == "ls" else rand(i, o)
+    if dataflow == "rs":
+        x = rand(i, t)              # transposed input: y = x^T w, dw = x dy, dx = w dy^T
+    first = {"os": (x, dy, "tn"), "ls": (dy, x, "tn"), "rs": (x, dy, "nn")}[dataflow]
+    second = {"os": (dy, w, "nt"), "ls": (dy, w, "nn"), "rs": (w, dy, "nt")}[dataflow]
+    got = []
+    for _ in range(2):
+        grad = torch.ones(w.shape, device="cuda", dtype=torch.float32)
+        dw, dx = gemm_pair(*first, grad, True, *second)
+        assert dw is grad
+        got.append((dw, dx))
+    _native.check_status()
+    _check(got[0][0], _ref(*first) + 1.0, first[0].shape[0] if first[2] == "tn" else first[0].shape[1])
+    _check(got[0][1], _ref(*second), second[0].shape[1])
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+
+
+def test_gemm_pair_refuses_what_gemm_refuses():
+    from meshslice_b200.ops.gemm import gemm_pair
+    a, b = _operands(128, 256, 64, "nn")
+    out = torch.zeros(128, 256, device="cuda")
+    with pytest.raises(ValueError):
+        gemm_pair(a, b, "nn", None, True, a, b, "nn")
+    with pytest.raises(ValueError):
+        gemm_pair(a, b, "nn", out, True, a, b, "nt")
+    with pytest.raises(ValueError):
+        gemm_pair(a, b.float(), "nn", out, True, a, b, "nn")
+    with pytest.raises(RuntimeError):
+        gemm_pair(a[:, :60], b[:60, 4:252], "nn", None, False, a, b, "nn")   # 8 bytes off the alignment
