@@ -347,8 +347,9 @@ void gemm_local(int64_t M, int64_t N, int64_t K, uint64_t A, int64_t lda, int a_
   else run_gemm1(o, sms, status, stream);
 }
 
-// Two independent products in one launch, the longer contraction first (thirteen values each, as in gemm_local).
-void gemm_pair(const py::args& v, int sms, uint64_t status, uint64_t stream) {
+// Two independent products in one launch, the longer contraction first (thirteen values each, as in gemm_local).  With
+// `gelu_pre`, which has the layout of the second product's result, that one is multiplied by the derivative of GeLU there.
+void gemm_pair(const py::args& v, int sms, uint64_t status, uint64_t stream, uint64_t gelu_pre) {
   if (v.size() != 26) throw std::runtime_error("gemm_pair: thirteen values per product");
   const auto i = [&](int k) { return v[k].cast<int64_t>(); };
   const auto u = [&](int k) { return v[k].cast<uint64_t>(); };
@@ -358,9 +359,16 @@ void gemm_pair(const py::args& v, int sms, uint64_t status, uint64_t stream) {
     o[k] = local_operands(i(b), i(b + 1), i(b + 2), u(b + 3), i(b + 4), (int)i(b + 5), u(b + 6), i(b + 7), (int)i(b + 8), u(b + 9),
                           i(b + 10), (int)i(b + 11), (int)i(b + 12), status);
   }
+  if (gelu_pre != 0 && (o[1].c_fp32 || o[1].accumulate)) throw std::runtime_error("gemm_pair: gelu_pre needs a plain bf16 result");
   if (!two_cta_default()) {
+    if (gelu_pre != 0 && o[1].ldc != o[1].N) throw std::runtime_error("gemm_pair: gelu_pre needs a contiguous result");
     for (const Gemm2Operands& p : o) run_gemm1(p, sms, status, stream);
+    if (gelu_pre != 0) check(gelu_bwd(o[1].C, P<void>(gelu_pre), o[1].C, o[1].M * o[1].N, S(stream)), "gelu_bwd");
     return;
+  }
+  if (gelu_pre != 0) {
+    o[1].act = 2;
+    o[1].C_pre = P<void>(gelu_pre);
   }
   if (o[1].K > o[0].K) std::swap(o[0], o[1]);
   run_gemm2(o, 2, gemm2_tile_n(o, 2, sms), sms, P<uint32_t>(status), kLocalTimeoutNs, stream);
@@ -426,7 +434,7 @@ PYBIND11_MODULE(_C, m) {
   m.def("gemm_local", &gemm_local, "plain local GEMM: M, N, K, A, lda, a_mn_major, B, ldb, b_mn_major, C, ldc, c_fp32, "
         "accumulate, bias, act, C_pre, two_cta (-1: MSB_TWO_CTA), sms, status, stream");
   m.def("gemm_pair", &gemm_pair, py::kw_only(), py::arg("sms"), py::arg("status"), py::arg("stream"),
-        "two independent plain GEMMs in one launch: M, N, K, A, lda, a_mn_major, B, ldb, b_mn_major, C, ldc, c_fp32, accumulate "
+        py::arg("gelu_pre") = 0, "two independent plain GEMMs in one launch: M, N, K, A, lda, a_mn_major, B, ldb, b_mn_major, C, ldc, c_fp32, accumulate "
         "of either");
   m.def("symm_alloc", &symm_alloc);
   m.def("symm_open", &symm_open);

@@ -200,8 +200,8 @@ struct Gemm2Operands {
   int c_fp32;          // 1: C is float, 0: C is bf16
   int accumulate;      // 1: C += result
   const void* bias;    // bf16 [N] or null
-  int act;             // 0: none, 1: tanh-GeLU
-  void* C_pre;         // bf16, same layout as C: pre-activation copy (act != 0), may be null
+  int act;             // 0: none, 1: tanh-GeLU, 2: times its derivative at C_pre
+  void* C_pre;         // bf16, same layout as C; act 1: pre-activation copy, may be null; act 2: read
   int map3d;           // MN-major operands through the 3-D map where their extent allows it
   int group;           // raster group along M, 0: gemm2_order chooses
 };

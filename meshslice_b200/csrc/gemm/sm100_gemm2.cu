@@ -14,6 +14,7 @@
 #include <cuda_bf16.h>
 #include <string.h>
 
+#include "../common/gelu.cuh"
 #include "../common/ptx.cuh"
 #include "out_turn.h"
 #include "sm100_gemm.h"
@@ -160,6 +161,23 @@ __device__ __forceinline__ void store32(void* base, int64_t ld, bool fp32, bool 
   }
 }
 
+// 32 bf16 of a row as packed pairs; columns beyond `nvalid` are not read.
+__device__ __forceinline__ void load32(const void* base, int64_t ld, int64_t row, int col0, int nvalid, uint32_t (&v)[16]) {
+  const __nv_bfloat16* p = reinterpret_cast<const __nv_bfloat16*>(base) + row * ld + col0;
+  if (nvalid == 32 && aligned16(p)) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const uint4 u = __ldcs(reinterpret_cast<const uint4*>(p) + i);
+      v[4 * i] = u.x; v[4 * i + 1] = u.y; v[4 * i + 2] = u.z; v[4 * i + 3] = u.w;
+    }
+  } else {
+    const unsigned short* q = reinterpret_cast<const unsigned short*>(p);
+#pragma unroll
+    for (int i = 0; i < 16; ++i)
+      v[i] = (2 * i < nvalid ? q[2 * i] : 0u) | (2 * i + 1 < nvalid ? (uint32_t)q[2 * i + 1] << 16 : 0u);
+  }
+}
+
 // One box of a tensor map, shared -> global; the second form adds fp32 values to what is there (the sum that a register add
 // would give, subnormal values included: test_gemm_fp32_accumulation_keeps_subnormals).
 __device__ __forceinline__ void tma_store_box(const CUtensorMap* map, const void* src, int32_t x, int32_t y, bool add) {
@@ -231,7 +249,10 @@ __device__ __forceinline__ void tile2(int t, int tiles_m2, int tiles_n, int grou
 // second.  The two gradients of a linear layer that way, in one launch and in two: 1992 x 4104 x 1032 (85 tiles of 32
 // k-blocks and 136 of 17 on 74 pairs) 92.9 -> 81.9 us for the whole layer, 512 x 512 x 1536 38 -> 34, 4096 x 1024 x 51200 with
 // its loss 1309 -> 1296; 8192 x 4096 x 16384 is under the power cap either way (2541 and 2537).
-template <int BN>
+// kDGelu: a problem may have act 2.  An instance of its own: with it the kernel takes 230 registers instead of 94, and the
+// layer of 1992 x 4104 x 1032, which has no GeLU, 81.9 us instead of 81.2.  The derivative here instead of a pass over the
+// gradient (268 MB read twice and written in 160 us): decoder block of width 4096, 8192 tokens, 8817 -> 8643 us.
+template <int BN, bool kDGelu>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads2, 1)
 sm100_gemm2_kernel(const __grid_constant__ Gemm2Args a) {
   constexpr int kStages2 = stages2(BN);
@@ -420,6 +441,10 @@ sm100_gemm2_kernel(const __grid_constant__ Gemm2Args a) {
       const uint32_t te_leader = mapa_u32(smem_u32(tempty_bar + acc), 0);
       uint8_t* box = nullptr;
       uint8_t* box_pre = nullptr;
+      // act 2: the result times the derivative of GeLU at C_pre, whose elements are asked for one step ahead
+      const bool live = kDGelu && act == 2 && row0 + lane < M;
+      uint32_t x_next[16];
+      if (live) load32(C_pre, ldc, row0 + lane, nb * BN, min(32, N - nb * BN), x_next);
 #pragma unroll 1
       for (int c = 0; c < BN / 32; ++c) {
         uint32_t r[32];
@@ -441,6 +466,17 @@ sm100_gemm2_kernel(const __grid_constant__ Gemm2Args a) {
 #pragma unroll
           for (int i = 0; i < 32; ++i)
             if (i < nvalid) v[i] += __bfloat162float(bias[col0 + i]);
+        }
+        if (live) {
+          uint32_t x[16];
+#pragma unroll
+          for (int i = 0; i < 16; ++i) x[i] = x_next[i];
+          if (c + 1 < BN / 32 && col0 + 32 < N) load32(C_pre, ldc, row0 + lane, col0 + 32, min(32, N - col0 - 32), x_next);
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            v[2 * i] *= gelu_grad_f(blo(x[i]));
+            v[2 * i + 1] *= gelu_grad_f(bhi(x[i]));
+          }
         }
         if (!tma_c) {
           if (row0 + lane >= M || nvalid <= 0) continue;
@@ -485,7 +521,7 @@ sm100_gemm2_kernel(const __grid_constant__ Gemm2Args a) {
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(2u * BN) : "memory");
 }
 
-template <int BN>
+template <int BN, bool kDGelu>
 static cudaError_t launch2(const Gemm2Args& args, int grid, cudaStream_t stream) {
   static bool configured[64] = {false};
   int dev = 0;
@@ -493,12 +529,12 @@ static cudaError_t launch2(const Gemm2Args& args, int grid, cudaStream_t stream)
   if (e != cudaSuccess) return e;
   constexpr int smem = (int)smem_alloc2(BN);
   if (dev < 64 && !configured[dev]) {
-    e = cudaFuncSetAttribute(sm100_gemm2_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    e = cudaFuncSetAttribute(sm100_gemm2_kernel<BN, kDGelu>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
     configured[dev] = true;
   }
   // the cluster shape (2,1,1) is part of the kernel's definition
-  sm100_gemm2_kernel<BN><<<grid, kThreads2, smem, stream>>>(args);
+  sm100_gemm2_kernel<BN, kDGelu><<<grid, kThreads2, smem, stream>>>(args);
   return cudaGetLastError();
 }
 
@@ -569,7 +605,7 @@ int gemm2_problem(Gemm2Problem* p, const Gemm2Operands& o, int tile_n) {
   // Output through shared memory and TMA where the tensor map allows it; bf16 accumulation adds before it rounds,
   // which the copy engine cannot do.
   p->tma_c = !(o.accumulate && !o.c_fp32) && make_tensor_map_out(&p->c, o.C, o.N, o.M, o.ldc, o.c_fp32 != 0) == 0 &&
-             (o.act == 0 || o.C_pre == nullptr || make_tensor_map_out(&p->pre, o.C_pre, o.N, o.M, o.ldc, false) == 0);
+             (o.act != 1 || o.C_pre == nullptr || make_tensor_map_out(&p->pre, o.C_pre, o.N, o.M, o.ldc, false) == 0);
   const Gemm2Order order = o.group > 0 ? Gemm2Order{o.group, 0, 0} : gemm2_order(o.M, o.N, o.K, tile_n);
   p->group = order.group;
   p->along_n = order.along_n;
@@ -579,16 +615,19 @@ int gemm2_problem(Gemm2Problem* p, const Gemm2Operands& o, int tile_n) {
 
 cudaError_t launch_sm100_gemm2(Gemm2Args& args, int problems, int tile_n, int sms, cudaStream_t stream) {
   int64_t tiles = 0;
+  bool dgelu = false;
   for (int i = 0; i < 2; ++i) {
     if (i < problems) {
       const Gemm2Problem& p = args.p[i];
+      dgelu = dgelu || p.act == 2;
       tiles += (int64_t)((p.M + 2 * kBM - 1) / (2 * kBM)) * ((p.N + tile_n - 1) / tile_n);
     }
     args.tiles[i] = (int)tiles;
   }
   int grid = (int)(2 * tiles < (sms & ~1) ? 2 * tiles : (sms & ~1));
   if (grid < 2) grid = 2;
-  return tile_n == 128 ? launch2<128>(args, grid, stream) : launch2<256>(args, grid, stream);
+  if (dgelu) return tile_n == 128 ? launch2<128, true>(args, grid, stream) : launch2<256, true>(args, grid, stream);
+  return tile_n == 128 ? launch2<128, false>(args, grid, stream) : launch2<256, false>(args, grid, stream);
 }
 
 }  // namespace msb

@@ -6,6 +6,8 @@
 #include <cuda_bf16.h>
 #include <string.h>
 
+#include "../common/gelu.cuh"
+
 namespace msb {
 
 namespace {
@@ -137,18 +139,6 @@ __device__ __forceinline__ float block_max(float a, float* red) {
   __syncthreads();
   a = l < nw ? red[l] : -INFINITY;
   return warp_max(a);
-}
-
-__device__ __forceinline__ float gelu_f(float x) {
-  const float k0 = 0.7978845608028654f, k1 = 0.044715f;
-  return 0.5f * x * (1.0f + tanhf(k0 * (x + k1 * x * x * x)));
-}
-__device__ __forceinline__ float gelu_grad_f(float x) {
-  const float k0 = 0.7978845608028654f, k1 = 0.044715f;
-  const float u = k0 * (x + k1 * x * x * x);
-  const float t = tanhf(u);
-  const float du = k0 * (1.0f + 3.0f * k1 * x * x);
-  return 0.5f * (1.0f + t) + 0.5f * x * (1.0f - t * t) * du;
 }
 
 // ------------------------------------------------------------------------------------------

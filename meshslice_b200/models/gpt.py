@@ -115,7 +115,11 @@ class GPTBlock:
     def backward(self, dh: ShardedTensor, dm: ShardedTensor):
         """dh: gradient of the residual stream after this block, dm: gradient of the MLP output.
         Returns (dx, ddelta) for the block below."""
-        d = self._lin_bwd(self.ff1, self.gelu.backward(self._lin_bwd(self.ff2, dm)))
+        if _FUSE_GELU and self.ff2.dataflow != "rs":
+            d = self.ff2.backward_gelu(dm, self.gelu)     # GeLU's derivative in the GEMM epilogue
+        else:
+            d = self.gelu.backward(self._lin_bwd(self.ff2, dm))
+        d = self._lin_bwd(self.ff1, d)
         dh2 = self.ln2.backward(d, dh)            # gradient of h = x + a
         d = self._lin_bwd(self.in_proj, self.attn.backward(self._lin_bwd(self.out_proj, dh2)))
         dx = self.ln1.backward(d, dh2)            # gradient of x + delta

@@ -102,8 +102,7 @@ class ShardedFFLayer:
         x, w = self._x, self.weight
         self._x = None
         if need_dx and self._dw_dx is not None:
-            (key, g), = self.grad.shards.items()
-            return ShardedTensor(self.mesh, {key: self._dw_dx(self.dataflow, x, dy, w, g)})
+            return self._both(x, dy)
         if self.dataflow == "os":
             self._dw(self._RS, x, dy)
             return self._LS(dy, w) if need_dx else None
@@ -112,6 +111,18 @@ class ShardedFFLayer:
             return self._OS(dy, w) if need_dx else None
         self._dw(self._OS, x, dy)
         return self._LS(w, dy) if need_dx else None
+
+    def _both(self, x, dy, gelu_pre=None) -> ShardedTensor:
+        (key, g), = self.grad.shards.items()
+        return ShardedTensor(self.mesh, {key: self._dw_dx(self.dataflow, x, dy, self.weight, g, gelu_pre)})
+
+    def backward_gelu(self, dy: ShardedTensor, gelu: "GeLU") -> Optional[ShardedTensor]:
+        """``gelu.backward(self.backward(dy))`` for a layer whose input is the output of ``gelu``: on a 1 x 1 mesh in the
+        epilogue of the input's gradient, without a pass of its own."""
+        if self._dw_dx is None or self.dataflow == "rs" or not gelu.fits(self._x):
+            return gelu.backward(self.backward(dy))
+        x, self._x = self._x, None
+        return self._both(x, dy, gelu.take())
 
     def zero_grad(self):
         for g in self.grad.shards.values():
@@ -270,6 +281,18 @@ class GeLU:
         """Used when the forward pass was fused into the producing GEMM's epilogue."""
         self._x = pre_activation
 
+    def take(self) -> ShardedTensor:
+        """The remembered pre-activation, for a backward pass that is fused into a product's epilogue."""
+        x, self._x = self._x, None
+        return x
+
+    def fits(self, y: Optional[ShardedTensor]) -> bool:
+        """The remembered pre-activation has the shape and type of ``y``."""
+        if self._x is None or y is None or len(y.shards) != 1 or len(self._x.shards) != 1:
+            return False
+        a, b = self._x.local(), y.local()
+        return a.is_cuda and a.shape == b.shape and a.dtype == b.dtype == torch.bfloat16
+
     def forward(self, x: ShardedTensor) -> ShardedTensor:
         self._x = x
         return x.map(F.gelu)
@@ -318,8 +341,7 @@ class TransformerBlock:
 
     def backward(self, dy: ShardedTensor) -> ShardedTensor:
         d3 = self.norm3.backward(dy)              # grad of (ff2_out + res)
-        d = self.ff2.backward(d3)
-        d = self.gelu.backward(d)
+        d = self.ff2.backward_gelu(d3, self.gelu)
         d = self.ff1.backward(d)
         dres = _add(d, d3)                        # res feeds ff1 and the norm3 residual
         d2 = self.norm2.backward(dres)            # grad of (out_proj_out + x)

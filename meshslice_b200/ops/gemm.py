@@ -78,11 +78,21 @@ def _operands(a, b, layout, out, accumulate):
                  out.data_ptr(), ldc, 1 if out.dtype == torch.float32 else 0, 1 if accumulate else 0)
 
 
-def gemm_pair(a0, b0, layout0, out0, accumulate0, a1, b1, layout1, out1=None, accumulate1=False):
+def gemm_pair(a0, b0, layout0, out0, accumulate0, a1, b1, layout1, out1=None, accumulate1=False, gelu_pre=None):
     """Two independent products as ``gemm`` computes them, in one launch (the two gradients of a linear layer): returns
-    both outputs.  Neither output may overlap an operand or the output of the other product."""
+    both outputs.  Neither output may overlap an operand or the output of the other product.  ``gelu_pre`` (bf16, the shape
+    of the second product): the second result is multiplied by the derivative of GeLU at it before it is rounded."""
     out0, v0 = _operands(a0, b0, layout0, out0, accumulate0)
     out1, v1 = _operands(a1, b1, layout1, out1, accumulate1)
-    _native.load().gemm_pair(*v0, *v1, sms=_SM_COUNT.get(a0.device.index) or sm_count(a0.device),
+    pre = 0
+    if gelu_pre is not None:
+        if gelu_pre.shape != out1.shape or gelu_pre.dtype != torch.bfloat16 or out1.dtype != torch.bfloat16:
+            raise ValueError("gelu_pre must be bf16 and of the shape of the second product")
+        if gelu_pre.stride() != out1.stride():
+            if not out1.is_contiguous():
+                raise ValueError("gelu_pre needs a contiguous output")
+            gelu_pre = gelu_pre.contiguous()
+        pre = gelu_pre.data_ptr()
+    _native.load().gemm_pair(*v0, *v1, gelu_pre=pre, sms=_SM_COUNT.get(a0.device.index) or sm_count(a0.device),
                              status=_native.status().dev, stream=_native.stream_ptr())
     return out0, out1

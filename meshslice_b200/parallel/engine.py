@@ -186,15 +186,15 @@ class LocalGemmEngine:
     def rs(self, X, W, n_slices=1, out=None, accumulate=False, rot_index=None):
         return self._run(X, W, "tn", out, accumulate)
 
-    def dw_dx(self, dataflow, x, dy, w, grad):
+    def dw_dx(self, dataflow, x, dy, w, grad, gelu_pre=None):
         """Both gradients of a linear layer, which do not depend on each other, in one launch: the weight's is added to
-        ``grad``, the input's is returned."""
-        x, dy, w = _local(x), _local(dy), _local(w)
+        ``grad``, the input's is returned (with ``gelu_pre``: the one of the GeLU's input, when x is the GeLU of that)."""
+        x, dy, w, gelu_pre = _local(x), _local(dy), _local(w), _local(gelu_pre)
         if dataflow == "os":
-            return gemm_pair(x, dy, "tn", grad, True, dy, w, "nt")[1]
+            return gemm_pair(x, dy, "tn", grad, True, dy, w, "nt", gelu_pre=gelu_pre)[1]
         if dataflow == "ls":
-            return gemm_pair(dy, x, "tn", grad, True, dy, w, "nn")[1]
-        return gemm_pair(x, dy, "nn", grad, True, w, dy, "nt")[1]
+            return gemm_pair(dy, x, "tn", grad, True, dy, w, "nn", gelu_pre=gelu_pre)[1]
+        return gemm_pair(x, dy, "nn", grad, True, w, dy, "nt", gelu_pre=gelu_pre)[1]
 
     def check(self):
         _native.check_status()

@@ -258,3 +258,38 @@ def test_gemm_pair_refuses_what_gemm_refuses():
         gemm_pair(a, b.float(), "nn", out, True, a, b, "nn")
     with pytest.raises(RuntimeError):
         gemm_pair(a[:, :60], b[:60, 4:252], "nn", None, False, a, b, "nn")   # 8 bytes off the alignment
+
+
+# (tokens, width, ffn): narrow and wide tiles, edges inside a group of 32 columns and of 32 rows, more tiles than CTA pairs
+@pytest.mark.parametrize("dataflow", ["os", "ls"])
+@pytest.mark.parametrize("shape", [(256, 128, 512), (1000, 264, 1048), (2056, 512, 8200)])
+@pytest.mark.parametrize("offset", [0, 3])
+def test_gemm_pair_times_gelu_derivative(shape, dataflow, offset):
+    """dx * GeLU'(pre) in the epilogue against fp32: one bf16 rounding of the result (2^-9 of it) and the sum's fp32 error.
+    `offset`: the pre-activation starts so many elements off a 16-byte boundary.  Infinite and NaN pre-activations give what
+    the stand-alone kernel gives."""
+    from meshslice_b200 import _native
+    from meshslice_b200.ops import functional as F
+    from meshslice_b200.ops.gemm import gemm_pair
+    t, d, f = shape
+    g = torch.Generator(device="cuda").manual_seed(f)
+    rand = lambda *s: torch.randn(s, device="cuda", generator=g).bfloat16()
+    x, dy, w = rand(t, f), rand(t, d), rand(*((d, f) if dataflow == "ls" else (f, d)))
+    pre = (rand(t * f + offset) * 2)[offset:].view(t, f)
+    assert pre.data_ptr() % 16 == 2 * offset
+    first, layout = ((dy, x, "tn"), "nn") if dataflow == "ls" else ((x, dy, "tn"), "nt")
+    both = lambda p: gemm_pair(*first, torch.zeros(w.shape, device="cuda"), True, dy, w, layout, gelu_pre=p)
+    dw, got = both(pre)
+    plain = _ref(dy, w, layout)
+    xr = pre.float().requires_grad_(True)
+    torch.nn.functional.gelu(xr, approximate="tanh").backward(plain)
+    _native.check_status()
+    assert ((got.float() - xr.grad).norm() / xr.grad.norm()).item() < 2 ** -9
+    _check(dw, _ref(*first), t)
+    odd = pre.clone()                # starts on a 16-byte boundary, which the stand-alone kernel needs
+    odd[5, :40:8] = torch.tensor([float("inf"), -float("inf"), float("nan"), 1e20, -1e20], device="cuda").bfloat16()
+    got, want = both(odd)[1], F.gelu_bwd(both(None)[1], odd)
+    _native.check_status()
+    assert torch.equal(torch.isnan(got), torch.isnan(want)) and torch.isnan(want[5]).any()
+    ok = ~torch.isnan(want)
+    assert ((got[ok].float() - want[ok].float()).norm() / want[ok].float().norm()).item() < 2 ** -8
