@@ -12,6 +12,7 @@ import threading
 _lock = threading.Lock()
 _mod = None
 _status = None
+_cuda = None          # torch._C once CUDA is initialised
 
 STATUS_NAMES = {
     0: "ok", 1: "timeout: producer waiting for a free stage", 2: "timeout: MMA waiting for TMA data",
@@ -56,11 +57,26 @@ def available() -> bool:
 
 def stream_ptr() -> int:
     """Current stream of the current device (asked for before every launch: without the stream object that
-    torch.cuda.current_stream() builds, 0.4 us instead of 8)."""
+    torch.cuda.current_stream() builds, 0.2 us instead of 8)."""
+    if _cuda is None:
+        _init_cuda()
+    return _cuda._cuda_getCurrentRawStream(_cuda._cuda_getDevice())
+
+
+def _init_cuda():
+    global _cuda
     import torch
     if not torch.cuda.is_initialized():
         torch.cuda.init()
-    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+    _cuda = torch._C
+
+
+def zero_(t) -> None:
+    """``t.zero_()`` without the tensor library's dispatch where the memory is one block on a GPU."""
+    if t.is_cuda and t.is_contiguous():
+        load().memset_zero(t.data_ptr(), t.numel() * t.element_size(), stream_ptr())
+    else:
+        t.zero_()
 
 
 class _Status:

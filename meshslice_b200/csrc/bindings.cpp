@@ -5,10 +5,14 @@
 #include <pybind11/stl.h>
 
 #include <algorithm>
+#include <array>
 #include <cstdlib>
 #include <cstring>
 #include <stdexcept>
 #include <string>
+#include <tuple>
+#include <type_traits>
+#include <utility>
 #include <vector>
 
 #include "comm/p2p.h"
@@ -276,8 +280,7 @@ void gemm_run(const py::dict& d) {
 }
 
 // The plain local GEMM of `ops.gemm`: the few values it needs, positionally.  Filling the dict of gemm_run and reading
-// it back took longer than a small product takes on the GPU (a linear layer of 512 x 512 x 1536, forward and backward:
-// 108 us a pass, 59 us through this call).  MSB_TWO_CTA, MSB_G2_GROUP and MSB_G2_MAP3D are read per call, as they were.
+// it back took longer than a small product takes on the GPU.  MSB_TWO_CTA, MSB_G2_GROUP and MSB_G2_MAP3D are read per call.
 int env_int(const char* name, int otherwise) {
   const char* v = std::getenv(name);
   return v != nullptr ? std::atoi(v) : otherwise;
@@ -347,17 +350,17 @@ void gemm_local(int64_t M, int64_t N, int64_t K, uint64_t A, int64_t lda, int a_
   else run_gemm1(o, sms, status, stream);
 }
 
-// Two independent products in one launch, the longer contraction first (thirteen values each, as in gemm_local).  With
-// `gelu_pre`, which has the layout of the second product's result, that one is multiplied by the derivative of GeLU there.
-void gemm_pair(const py::args& v, int sms, uint64_t status, uint64_t stream, uint64_t gelu_pre) {
-  if (v.size() != 26) throw std::runtime_error("gemm_pair: thirteen values per product");
-  const auto i = [&](int k) { return v[k].cast<int64_t>(); };
-  const auto u = [&](int k) { return v[k].cast<uint64_t>(); };
+// Two independent products in one launch, the longer contraction first: thirteen values each, as in gemm_local, then sms, status,
+// stream and gelu_pre.  With `gelu_pre`, which has the layout of the second product's result, that one is multiplied by the
+// derivative of GeLU there.
+void gemm_pair(const std::array<int64_t, 30>& v) {
+  const int sms = (int)v[26];
+  const uint64_t status = (uint64_t)v[27], stream = (uint64_t)v[28], gelu_pre = (uint64_t)v[29];
   Gemm2Operands o[2];
   for (int k = 0; k < 2; ++k) {
-    const int b = 13 * k;
-    o[k] = local_operands(i(b), i(b + 1), i(b + 2), u(b + 3), i(b + 4), (int)i(b + 5), u(b + 6), i(b + 7), (int)i(b + 8), u(b + 9),
-                          i(b + 10), (int)i(b + 11), (int)i(b + 12), status);
+    const int64_t* p = v.data() + 13 * k;
+    o[k] = local_operands(p[0], p[1], p[2], (uint64_t)p[3], p[4], (int)p[5], (uint64_t)p[6], p[7], (int)p[8], (uint64_t)p[9], p[10],
+                          (int)p[11], (int)p[12], status);
   }
   if (gelu_pre != 0 && (o[1].c_fp32 || o[1].accumulate)) throw std::runtime_error("gemm_pair: gelu_pre needs a plain bf16 result");
   if (!two_cta_default()) {
@@ -411,6 +414,113 @@ py::tuple status_read(uint64_t host_ptr) {
 }
 void status_clear(uint64_t host_ptr) { std::memset(P<void>(host_ptr), 0, 64); }
 
+// ---------------------------------------------------------------------------------------
+// Direct calls: what every layer of a step goes through takes its numbers straight from the interpreter's argument vector
+// (positional, one conversion each).  pybind11's dispatch of a call with 15 to 20 numbers takes 1 us, of 2.4 for the launch.
+// With that, gradients cleared by the copy engine's memset, one scratch tensor for the attention's backward pass and fewer
+// wrappers around a product: linear layer of 512 x 512 x 1536, forward and backward, 34.1 -> 26.4 us; two-layer model of width
+// 512 566 -> 477.
+// ---------------------------------------------------------------------------------------
+template <class T>
+bool from_py(PyObject* o, T& v) {
+  if constexpr (std::is_floating_point_v<T>) {
+    const double d = PyFloat_AsDouble(o);
+    v = (T)d;
+    return d != -1.0 || !PyErr_Occurred();
+  } else if constexpr (std::is_signed_v<T>) {
+    const long long l = PyLong_AsLongLong(o);
+    v = (T)l;
+    if (l == -1 && PyErr_Occurred()) return false;
+    if ((long long)v == l) return true;
+    PyErr_SetString(PyExc_OverflowError, "argument does not fit its 32 bits");
+    return false;
+  } else {
+    static_assert(sizeof(T) == 8);
+    v = (T)PyLong_AsUnsignedLongLong(o);
+    return v != (T)-1 || !PyErr_Occurred();
+  }
+}
+template <class F>
+PyObject* guarded(F&& f) {
+  try {
+    f();
+  } catch (const std::exception& e) {
+    PyErr_SetString(PyExc_RuntimeError, e.what());
+    return nullptr;
+  }
+  Py_RETURN_NONE;
+}
+PyObject* wrong_count(Py_ssize_t want, Py_ssize_t got) {
+  PyErr_Format(PyExc_TypeError, "expected %zd arguments, got %zd", want, got);
+  return nullptr;
+}
+template <auto F, class... A, size_t... I>
+PyObject* call_with(void (*)(A...), std::index_sequence<I...>, PyObject* const* args) {
+  std::tuple<A...> v;
+  if (!(from_py(args[I], std::get<I>(v)) && ...)) return nullptr;
+  return guarded([&] { F(std::get<I>(v)...); });
+}
+template <class... A>
+constexpr size_t count_of(void (*)(A...)) { return sizeof...(A); }
+template <auto F>
+PyObject* direct(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  constexpr size_t want = count_of(F);
+  if (n != (Py_ssize_t)want) return wrong_count(want, n);
+  return call_with<F>(F, std::make_index_sequence<want>{}, args);
+}
+template <auto F, size_t N>
+PyObject* direct_values(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  if (n != (Py_ssize_t)N) return wrong_count(N, n);
+  std::array<int64_t, N> v;
+  for (size_t i = 0; i < N; ++i)
+    if (!from_py(args[i], v[i])) return nullptr;
+  return guarded([&] { F(v); });
+}
+
+void ln_fwd_local(uint64_t x, uint64_t res, uint64_t h_out, uint64_t y, uint64_t gamma, uint64_t beta, uint64_t mean_rstd, int rows,
+                  int cols, float eps, uint64_t stream) {
+  check(ln_fwd(0, P<void>(x), P<void>(res), P<void>(h_out), P<void>(y), P<void>(gamma), P<void>(beta), nullptr, P<float>(mean_rstd),
+               rows, cols, cols, eps, S(stream), nullptr), "ln_fwd");
+}
+void ln_bwd_local(uint64_t dy, uint64_t h, uint64_t gamma, uint64_t mean_rstd, uint64_t dres, uint64_t dx, uint64_t dgamma,
+                  uint64_t dbeta, int rows, int cols, uint64_t stream) {
+  check(ln_bwd(0, P<void>(dy), P<void>(h), P<void>(gamma), P<float>(mean_rstd), P<void>(dres), P<void>(dx), nullptr,
+               P<float>(dgamma), P<float>(dbeta), rows, cols, cols, S(stream), nullptr), "ln_bwd");
+}
+void py_gelu_fwd(uint64_t x, uint64_t y, int64_t n, uint64_t stream) { check(gelu_fwd(P<void>(x), P<void>(y), n, S(stream)), "gelu_fwd"); }
+void py_gelu_bwd(uint64_t dy, uint64_t x, uint64_t dx, int64_t n, uint64_t stream) {
+  check(gelu_bwd(P<void>(dy), P<void>(x), P<void>(dx), n, S(stream)), "gelu_bwd");
+}
+void py_add_bf16(uint64_t a, uint64_t b, uint64_t o, int64_t n, uint64_t stream) {
+  check(add_bf16(P<void>(a), P<void>(b), P<void>(o), n, S(stream)), "add_bf16");
+}
+void ce_partial_local(uint64_t logits, int64_t ld, uint64_t targets, int rows, int cols, int col_offset, int vocab, uint64_t row_max,
+                      uint64_t row_sumexp, uint64_t tgt_logit, uint64_t stream) {
+  check(ce_partial(P<void>(logits), ld, P<int64_t>(targets), rows, cols, col_offset, vocab, P<float>(row_max), P<float>(row_sumexp),
+                   P<float>(tgt_logit), S(stream), nullptr), "ce_partial");
+}
+void ce_grad_local(uint64_t logits, int64_t ld, uint64_t targets, int rows, int cols, int col_offset, int vocab, uint64_t gmax,
+                   uint64_t gsum, float scale, uint64_t stream, uint64_t row_loss, uint64_t tgt_logit) {
+  check(ce_grad(P<void>(logits), ld, P<int64_t>(targets), rows, cols, col_offset, vocab, P<float>(gmax), P<float>(gsum), scale,
+                S(stream), P<float>(row_loss), nullptr, P<float>(tgt_logit)), "ce_grad");
+}
+void py_embedding_fwd(uint64_t tokens, uint64_t tok, uint64_t pos, uint64_t out, int n_tokens, int seq, int cols, uint64_t stream) {
+  check(embedding_fwd(P<int64_t>(tokens), P<void>(tok), P<void>(pos), P<void>(out), n_tokens, seq, cols, S(stream)), "embedding_fwd");
+}
+void py_embedding_bwd(uint64_t tokens, uint64_t dout, uint64_t dtok, uint64_t dpos, int n_tokens, int seq, int cols, uint64_t stream) {
+  check(embedding_bwd(P<int64_t>(tokens), P<void>(dout), P<float>(dtok), P<float>(dpos), n_tokens, seq, cols, S(stream)), "embedding_bwd");
+}
+void py_attention_fwd(uint64_t qkv, uint64_t out, uint64_t lse, int batch, int seq, int heads, int causal, float scale, uint64_t status,
+                      uint64_t stream) {
+  check(attention_fwd(P<void>(qkv), P<void>(out), P<float>(lse), batch, seq, heads, causal, scale, P<uint32_t>(status), S(stream)),
+        "attention_fwd");
+}
+void py_attention_bwd(uint64_t qkv, uint64_t out, uint64_t dout, uint64_t lse, uint64_t dqkv, uint64_t dq_acc, uint64_t delta, int batch,
+                      int seq, int heads, int causal, float scale, uint64_t status, uint64_t stream) {
+  check(attention_bwd(P<void>(qkv), P<void>(out), P<void>(dout), P<float>(lse), P<void>(dqkv), P<float>(dq_acc), P<float>(delta), batch,
+                      seq, heads, causal, scale, P<uint32_t>(status), S(stream)), "attention_bwd");
+}
+
 void memset_zero(uint64_t ptr, size_t bytes, uint64_t stream) {
   check(cudaMemsetAsync(P<void>(ptr), 0, bytes,
                         reinterpret_cast<cudaStream_t>(static_cast<uintptr_t>(stream))),
@@ -431,11 +541,6 @@ PYBIND11_MODULE(_C, m) {
   m.attr("CHUNK_DESC_BYTES") = (int)sizeof(ChunkDesc);
 
   m.def("gemm_run", &gemm_run, "persistent tcgen05 GEMM with optional fused gather / push");
-  m.def("gemm_local", &gemm_local, "plain local GEMM: M, N, K, A, lda, a_mn_major, B, ldb, b_mn_major, C, ldc, c_fp32, "
-        "accumulate, bias, act, C_pre, two_cta (-1: MSB_TWO_CTA), sms, status, stream");
-  m.def("gemm_pair", &gemm_pair, py::kw_only(), py::arg("sms"), py::arg("status"), py::arg("stream"),
-        py::arg("gelu_pre") = 0, "two independent plain GEMMs in one launch: M, N, K, A, lda, a_mn_major, B, ldb, b_mn_major, C, ldc, c_fp32, accumulate "
-        "of either");
   m.def("symm_alloc", &symm_alloc);
   m.def("symm_open", &symm_open);
   m.def("symm_close", &symm_close);
@@ -443,7 +548,6 @@ PYBIND11_MODULE(_C, m) {
   m.def("status_alloc", &status_alloc);
   m.def("status_read", &status_read);
   m.def("status_clear", &status_clear);
-  m.def("memset_zero", &memset_zero);
   m.def("launch_count", []() { return g_launches; }, "kernel launches issued by this module so far");
 
   m.def("p2p_copy", [](uint64_t jobs, int n_jobs, const py::dict& bar, int grid, uint64_t stream) {
@@ -496,15 +600,6 @@ PYBIND11_MODULE(_C, m) {
   m.def("ln_grid", &ln_grid, py::arg("backward"), py::arg("rows"), py::arg("cols") = 0,
         "CTAs of the LayerNorm kernels in a row exchange for a row count and local width (0: forward, 1: backward)");
   m.def("ce_grid", &ce_grid, "CTAs of the cross-entropy kernels in a row exchange for a row count");
-  m.def("gelu_fwd", [](uint64_t x, uint64_t y, int64_t n, uint64_t stream) {
-    check(gelu_fwd(P<void>(x), P<void>(y), n, S(stream)), "gelu_fwd");
-  });
-  m.def("gelu_bwd", [](uint64_t dy, uint64_t x, uint64_t dx, int64_t n, uint64_t stream) {
-    check(gelu_bwd(P<void>(dy), P<void>(x), P<void>(dx), n, S(stream)), "gelu_bwd");
-  });
-  m.def("add_bf16", [](uint64_t a, uint64_t b, uint64_t o, int64_t n, uint64_t stream) {
-    check(add_bf16(P<void>(a), P<void>(b), P<void>(o), n, S(stream)), "add_bf16");
-  });
   m.def("cast_f32_to_bf16", [](uint64_t in, uint64_t out, int64_t n, int accumulate, uint64_t stream) {
     check(cast_f32_to_bf16(P<float>(in), P<void>(out), n, accumulate, S(stream)), "cast_f32_to_bf16");
   });
@@ -541,26 +636,31 @@ PYBIND11_MODULE(_C, m) {
   }, py::arg("logits"), py::arg("ld"), py::arg("targets"), py::arg("rows"), py::arg("cols"),
      py::arg("col_offset"), py::arg("vocab"), py::arg("gmax"), py::arg("gsum"), py::arg("scale"),
      py::arg("stream"), py::arg("row_loss") = 0, py::arg("exch") = py::none(), py::arg("tgt_logit") = 0);
-  m.def("embedding_fwd", [](uint64_t tokens, uint64_t tok, uint64_t pos, uint64_t out, int n_tokens,
-                            int seq, int cols, uint64_t stream) {
-    check(embedding_fwd(P<int64_t>(tokens), P<void>(tok), P<void>(pos), P<void>(out), n_tokens, seq,
-                        cols, S(stream)), "embedding_fwd");
-  });
-  m.def("embedding_bwd", [](uint64_t tokens, uint64_t dout, uint64_t dtok, uint64_t dpos,
-                            int n_tokens, int seq, int cols, uint64_t stream) {
-    check(embedding_bwd(P<int64_t>(tokens), P<void>(dout), P<float>(dtok), P<float>(dpos), n_tokens,
-                        seq, cols, S(stream)), "embedding_bwd");
-  });
-  m.def("attention_fwd", [](uint64_t qkv, uint64_t out, uint64_t lse, int batch, int seq, int heads,
-                            int causal, float scale, uint64_t status, uint64_t stream) {
-    check(attention_fwd(P<void>(qkv), P<void>(out), P<float>(lse), batch, seq, heads, causal, scale,
-                        P<uint32_t>(status), S(stream)), "attention_fwd");
-  });
-  m.def("attention_bwd", [](uint64_t qkv, uint64_t out, uint64_t dout, uint64_t lse, uint64_t dqkv,
-                            uint64_t dq_acc, uint64_t delta, int batch, int seq, int heads, int causal,
-                            float scale, uint64_t status, uint64_t stream) {
-    check(attention_bwd(P<void>(qkv), P<void>(out), P<void>(dout), P<float>(lse), P<void>(dqkv),
-                        P<float>(dq_acc), P<float>(delta), batch, seq, heads, causal, scale,
-                        P<uint32_t>(status), S(stream)), "attention_bwd");
-  });
+
+  static PyMethodDef direct_calls[] = {
+#define MSB_DIRECT(name, fn, doc) \
+  {name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(&direct<&fn>)), METH_FASTCALL, doc}
+      MSB_DIRECT("gemm_local", gemm_local, "plain local GEMM: M, N, K, A, lda, a_mn_major, B, ldb, b_mn_major, C, ldc, c_fp32, "
+                 "accumulate, bias, act, C_pre, two_cta (-1: MSB_TWO_CTA), sms, status, stream"),
+      {"gemm_pair", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(&direct_values<&gemm_pair, 30>)), METH_FASTCALL,
+       "two independent plain GEMMs in one launch: M, N, K, A, lda, a_mn_major, B, ldb, b_mn_major, C, ldc, c_fp32, accumulate "
+       "of either, sms, status, stream, gelu_pre"},
+      MSB_DIRECT("memset_zero", memset_zero, "ptr, bytes, stream"),
+      MSB_DIRECT("ln_fwd_local", ln_fwd_local, "x, res, h_out, y, gamma, beta, mean_rstd, rows, cols, eps, stream"),
+      MSB_DIRECT("ln_bwd_local", ln_bwd_local, "dy, h, gamma, mean_rstd, dres, dx, dgamma, dbeta, rows, cols, stream"),
+      MSB_DIRECT("gelu_fwd", py_gelu_fwd, "x, y, n, stream"),
+      MSB_DIRECT("gelu_bwd", py_gelu_bwd, "dy, x, dx, n, stream"),
+      MSB_DIRECT("add_bf16", py_add_bf16, "a, b, out, n, stream"),
+      MSB_DIRECT("ce_partial_local", ce_partial_local, "logits, ld, targets, rows, cols, col_offset, vocab, row_max, row_sumexp, "
+                 "tgt_logit, stream"),
+      MSB_DIRECT("ce_grad_local", ce_grad_local, "logits, ld, targets, rows, cols, col_offset, vocab, gmax, gsum, scale, stream, "
+                 "row_loss, tgt_logit"),
+      MSB_DIRECT("embedding_fwd", py_embedding_fwd, "tokens, tok, pos, out, n_tokens, seq, cols, stream"),
+      MSB_DIRECT("embedding_bwd", py_embedding_bwd, "tokens, dout, dtok, dpos, n_tokens, seq, cols, stream"),
+      MSB_DIRECT("attention_fwd", py_attention_fwd, "qkv, out, lse, batch, seq, heads, causal, scale, status, stream"),
+      MSB_DIRECT("attention_bwd", py_attention_bwd, "qkv, out, dout, lse, dqkv, dq_acc, delta, batch, seq, heads, causal, scale, "
+                 "status, stream"),
+      {nullptr, nullptr, 0, nullptr}};
+#undef MSB_DIRECT
+  if (PyModule_AddFunctions(m.ptr(), direct_calls) != 0) throw py::error_already_set();
 }

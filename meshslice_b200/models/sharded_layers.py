@@ -23,6 +23,7 @@ from typing import Callable, List, Optional
 
 import torch
 
+from .._native import zero_
 from ..ops import functional as F
 from ..parallel.mesh import Mesh, ShardedTensor
 from ..parallel.tensor_parallel import SPMD, createMultihostMatrix
@@ -126,7 +127,7 @@ class ShardedFFLayer:
 
     def zero_grad(self):
         for g in self.grad.shards.values():
-            g.zero_()
+            zero_(g)
 
     def parameters(self):
         return [("weight", self.weight, self.grad, "sharded")]
@@ -153,17 +154,14 @@ class ShardedLayerNorm:
     def forward(self, x: ShardedTensor, res: Optional[ShardedTensor] = None):
         """Returns y; ``self.h`` holds x + res (the new residual stream)."""
         m = self.mesh
+        if m.C == 1:
+            return self._forward_rows(x, res)
         g = self.gamma if self.affine else None
         b = self.bias if self.affine else None
         G = lambda k: g.shards[k] if g is not None else None
         Bt = lambda k: b.shards[k] if b is not None else None
         R = lambda k: res.shards[k] if res is not None else None
-        if m.C == 1:
-            outs = {k: F.ln_full(x.shards[k], R(k), G(k), Bt(k), self.eps) for k in m.coords()}
-            h = ShardedTensor(m, {k: v[0] for k, v in outs.items()})
-            y = ShardedTensor(m, {k: v[1] for k, v in outs.items()})
-            mr = ShardedTensor(m, {k: v[2] for k, v in outs.items()})
-        elif self._exchanger(x) is not None:
+        if self._exchanger(x) is not None:
             # statistics travel inside the two kernels (peer stores + arrival counters): no collective
             (k, xl), = x.shards.items()
             prod, cons = self._exchange(xl.shape[0], xl.shape[1], backward=False)
@@ -184,6 +182,16 @@ class ShardedLayerNorm:
         self._saved = (h, mr)
         return y
 
+    def _forward_rows(self, x: ShardedTensor, res: Optional[ShardedTensor]) -> ShardedTensor:
+        """Whole rows on every device: one kernel per shard."""
+        h, y, mr = {}, {}, {}
+        for k in self.mesh.coords():
+            g, b = (self.gamma.shards[k], self.bias.shards[k]) if self.affine else (None, None)
+            h[k], y[k], mr[k] = F.ln_full(x.shards[k], None if res is None else res.shards[k], g, b, self.eps)
+        self.h = ShardedTensor(self.mesh, h)
+        self._saved = (self.h, ShardedTensor(self.mesh, mr))
+        return ShardedTensor(self.mesh, y)
+
     def _exchanger(self, t: ShardedTensor):
         """The mesh's in-kernel row exchange, when it has one and the shard lives on its GPU."""
         ex = getattr(getattr(self.mesh, "engine", None), "row_exchange", None)
@@ -201,13 +209,18 @@ class ShardedLayerNorm:
         m = self.mesh
         h, mr = self._saved
         self._saved = None
+        if m.C == 1:
+            out = {}
+            for k in m.coords():
+                g, dg, db = ((self.gamma.shards[k], self.dgamma.shards[k], self.dbias.shards[k]) if self.affine
+                             else (None, None, None))
+                out[k] = F.ln_bwd_full(dy.shards[k], h.shards[k], g, mr.shards[k], dg, db,
+                                       None if dres is None else dres.shards[k])
+            return ShardedTensor(m, out)
         G = lambda k: self.gamma.shards[k] if self.affine else None
         DG = lambda k: self.dgamma.shards[k] if self.affine else None
         DB = lambda k: self.dbias.shards[k] if self.affine else None
         DR = lambda k: dres.shards[k] if dres is not None else None
-        if m.C == 1:
-            return ShardedTensor(m, {k: F.ln_bwd_full(dy.shards[k], h.shards[k], G(k), mr.shards[k], DG(k),
-                                                      DB(k), DR(k)) for k in m.coords()})
         if self._exchanger(dy) is not None:
             (k, dyl), = dy.shards.items()
             prod, cons = self._exchange(dyl.shape[0], dyl.shape[1], backward=True)
@@ -221,8 +234,10 @@ class ShardedLayerNorm:
                                                    stats.shards[k], self.in_dim, DR(k)) for k in m.coords()})
 
     def zero_grad(self):
-        for t in list(self.dgamma.shards.values()) + list(self.dbias.shards.values()):
-            t.zero_()
+        for t in self.dgamma.shards.values():
+            zero_(t)
+        for t in self.dbias.shards.values():
+            zero_(t)
 
     def parameters(self):
         if not self.affine:

@@ -15,12 +15,8 @@ GELU_K0 = 0.7978845608028654
 GELU_K1 = 0.044715
 
 
-def _C():
-    return _native.load()
-
-
-def _st():
-    return _native.stream_ptr()
+_C = _native.load
+_st = _native.stream_ptr
 
 
 def _p(t: Optional[torch.Tensor]) -> int:
@@ -74,8 +70,8 @@ def ln_full(x, res, gamma, beta, eps: float):
         h = torch.empty_like(x) if res is not None else x
         y = torch.empty_like(x)
         mr = torch.empty(rows, 2, device=x.device, dtype=torch.float32)
-        _C().ln_fwd(0, x.data_ptr(), _p(res), h.data_ptr() if res is not None else 0, y.data_ptr(),
-                    _p(gamma), _p(beta), 0, mr.data_ptr(), rows, cols, cols, eps, _st())
+        _C().ln_fwd_local(x.data_ptr(), _p(res), h.data_ptr() if res is not None else 0, y.data_ptr(),
+                          _p(gamma), _p(beta), mr.data_ptr(), rows, cols, eps, _st())
         return h, y, mr
     h, stats = ln_stats(x, res)
     y, mr = ln_apply(h, stats, gamma, beta, cols, eps)
@@ -122,8 +118,8 @@ def ln_bwd_full(dy, h, gamma, mean_rstd, dgamma, dbeta, dres=None):
     rows, cols = dy.shape
     if dy.is_cuda:
         dx = torch.empty_like(dy)
-        _C().ln_bwd(0, dy.data_ptr(), h.data_ptr(), _p(gamma), mean_rstd.data_ptr(), _p(dres),
-                    dx.data_ptr(), 0, _p(dgamma), _p(dbeta), rows, cols, cols, _st())
+        _C().ln_bwd_local(dy.data_ptr(), h.data_ptr(), _p(gamma), mean_rstd.data_ptr(), _p(dres),
+                          dx.data_ptr(), _p(dgamma), _p(dbeta), rows, cols, _st())
         return dx
     stats = ln_bwd_stats(dy, h, gamma, mean_rstd, dgamma, dbeta)
     return ln_bwd_apply(dy, h, gamma, mean_rstd, stats, cols, dres)
@@ -224,10 +220,11 @@ def attention_bwd(dout, qkv, out, lse, batch: int, seq: int, heads: int, causal:
         if not (qkv.is_contiguous() and out.is_contiguous() and lse.is_contiguous()):
             qkv, out, lse = qkv.contiguous(), out.contiguous(), lse.contiguous()
         dqkv = torch.empty_like(qkv)
-        delta = torch.empty(batch, heads, seq, dtype=torch.float32, device=qkv.device)
-        dq_acc = torch.empty(batch, heads, seq, dtype=torch.float32, device=qkv.device)   # scratch: -lse * log2(e)
+        n = batch * heads * seq
+        scratch = torch.empty(2 * n, dtype=torch.float32, device=qkv.device)   # -lse * log2(e), scaled row sums
+        at = scratch.data_ptr()
         _C().attention_bwd(qkv.data_ptr(), out.data_ptr(), dout.data_ptr(), lse.data_ptr(),
-                           dqkv.data_ptr(), dq_acc.data_ptr(), delta.data_ptr(), batch, seq, heads,
+                           dqkv.data_ptr(), at, at + 4 * n, batch, seq, heads,
                            1 if causal else 0,
                            1.0 / math.sqrt(D), _native.status().dev, _st())
         return dqkv
@@ -263,8 +260,8 @@ def ce_partial(logits, targets, col_offset: int, vocab: int, exch=None):
                             vocab, 0, 0, 0, _st(), exch)
             return None
         mx, se, tl = (torch.empty(rows, device=logits.device, dtype=torch.float32) for _ in range(3))
-        _C().ce_partial(logits.data_ptr(), logits.stride(0), targets.data_ptr(), rows, cols, col_offset,
-                        vocab, mx.data_ptr(), se.data_ptr(), tl.data_ptr(), _st())
+        _C().ce_partial_local(logits.data_ptr(), logits.stride(0), targets.data_ptr(), rows, cols, col_offset,
+                              vocab, mx.data_ptr(), se.data_ptr(), tl.data_ptr(), _st())
         return mx, se, tl
     valid = max(0, min(cols, vocab - col_offset))
     lf = logits.float()[:, :valid]
@@ -295,8 +292,8 @@ def ce_grad_loss_(logits, targets, col_offset: int, vocab: int, gmax, gsum, tgt_
     if logits.is_cuda:
         rows, cols = logits.shape
         row_loss = torch.empty(rows, device=logits.device, dtype=torch.float32)
-        _C().ce_grad(logits.data_ptr(), logits.stride(0), targets.data_ptr(), rows, cols, col_offset, vocab,
-                     gmax.data_ptr(), gsum.data_ptr(), scale, _st(), row_loss.data_ptr(), None, tgt_logit.data_ptr())
+        _C().ce_grad_local(logits.data_ptr(), logits.stride(0), targets.data_ptr(), rows, cols, col_offset, vocab,
+                           gmax.data_ptr(), gsum.data_ptr(), scale, _st(), row_loss.data_ptr(), tgt_logit.data_ptr())
         return row_loss
     ce_grad_(logits, targets, col_offset, vocab, gmax, gsum, scale)
     return torch.log(gsum) + gmax - tgt_logit
@@ -306,8 +303,8 @@ def ce_grad_(logits, targets, col_offset: int, vocab: int, gmax, gsum, scale: fl
     """In place: logits <- (softmax - onehot) * scale (padding columns get 0)."""
     rows, cols = logits.shape
     if logits.is_cuda:
-        _C().ce_grad(logits.data_ptr(), logits.stride(0), targets.data_ptr(), rows, cols, col_offset,
-                     vocab, gmax.data_ptr(), gsum.data_ptr(), scale, _st())
+        _C().ce_grad_local(logits.data_ptr(), logits.stride(0), targets.data_ptr(), rows, cols, col_offset,
+                           vocab, gmax.data_ptr(), gsum.data_ptr(), scale, _st(), 0, 0)
         return logits
     col = torch.arange(cols) + col_offset
     p = torch.exp(logits.float() - gmax[:, None]) / gsum[:, None] * scale

@@ -38,37 +38,13 @@ def _dims(a, b, layout):
     return M, N, K
 
 
-def gemm(a, b, layout="nn", *, out=None, out_dtype=torch.bfloat16, accumulate=False, bias=None,
-         act=None, pre_act=None, two_cta=None):
-    """C = op(A) @ op(B) on the tensor cores of the current GPU.  ``two_cta`` selects the
-    cta_group::2 kernel (default: on, MSB_TWO_CTA=0 turns it off)."""
+def _operands(a, b, layout, out, accumulate, out_dtype=torch.bfloat16):
+    """Checks one product; returns its output and the thirteen values that the native calls take."""
     M, N, K = _dims(a, b, layout)
     if out is None:
         if accumulate:
             raise ValueError("accumulate=True needs an output tensor")
-        out = torch.empty((M, N), dtype=out_dtype, device=a.device)
-    (lda, sa), (ldb, sb), (ldc, sc) = a.stride(), b.stride(), out.stride()
-    if a.dtype != torch.bfloat16 or b.dtype != torch.bfloat16 or sa != 1 or sb != 1:
-        raise ValueError("GEMM operands must be bf16 with a contiguous last dimension")
-    if out.shape != (M, N) or sc != 1:
-        raise ValueError("bad output shape")
-    if act is not None and act != "gelu":
-        raise ValueError("only act='gelu' is fused")
-    _native.load().gemm_local(
-        M, N, K, a.data_ptr(), lda, 1 if layout == "tn" else 0, b.data_ptr(), ldb, 0 if layout == "nt" else 1,
-        out.data_ptr(), ldc, 1 if out.dtype == torch.float32 else 0, 1 if accumulate else 0,
-        0 if bias is None else bias.data_ptr(), 0 if act is None else 1,
-        0 if act is None or pre_act is None else pre_act.data_ptr(), -1 if two_cta is None else int(bool(two_cta)),
-        _SM_COUNT.get(a.device.index) or sm_count(a.device), _native.status().dev, _native.stream_ptr())
-    return out
-
-
-def _operands(a, b, layout, out, accumulate):
-    M, N, K = _dims(a, b, layout)
-    if out is None:
-        if accumulate:
-            raise ValueError("accumulate=True needs an output tensor")
-        out = a.new_empty((M, N))
+        out = torch.empty(M, N, dtype=out_dtype, device=a.device)
     (lda, sa), (ldb, sb), (ldc, sc) = a.stride(), b.stride(), out.stride()
     if a.dtype != torch.bfloat16 or b.dtype != torch.bfloat16 or sa != 1 or sb != 1:
         raise ValueError("GEMM operands must be bf16 with a contiguous last dimension")
@@ -76,6 +52,20 @@ def _operands(a, b, layout, out, accumulate):
         raise ValueError("bad output shape")
     return out, (M, N, K, a.data_ptr(), lda, 1 if layout == "tn" else 0, b.data_ptr(), ldb, 0 if layout == "nt" else 1,
                  out.data_ptr(), ldc, 1 if out.dtype == torch.float32 else 0, 1 if accumulate else 0)
+
+
+def gemm(a, b, layout="nn", *, out=None, out_dtype=torch.bfloat16, accumulate=False, bias=None,
+         act=None, pre_act=None, two_cta=None):
+    """C = op(A) @ op(B) on the tensor cores of the current GPU.  ``two_cta`` selects the
+    cta_group::2 kernel (default: on, MSB_TWO_CTA=0 turns it off)."""
+    out, v = _operands(a, b, layout, out, accumulate, out_dtype)
+    if act is not None and act != "gelu":
+        raise ValueError("only act='gelu' is fused")
+    _native.load().gemm_local(
+        *v, 0 if bias is None else bias.data_ptr(), 0 if act is None else 1,
+        0 if act is None or pre_act is None else pre_act.data_ptr(), -1 if two_cta is None else int(bool(two_cta)),
+        _SM_COUNT.get(a.device.index) or sm_count(a.device), _native.status().dev, _native.stream_ptr())
+    return out
 
 
 def gemm_pair(a0, b0, layout0, out0, accumulate0, a1, b1, layout1, out1=None, accumulate1=False, gelu_pre=None):
@@ -93,6 +83,6 @@ def gemm_pair(a0, b0, layout0, out0, accumulate0, a1, b1, layout1, out1=None, ac
                 raise ValueError("gelu_pre needs a contiguous output")
             gelu_pre = gelu_pre.contiguous()
         pre = gelu_pre.data_ptr()
-    _native.load().gemm_pair(*v0, *v1, gelu_pre=pre, sms=_SM_COUNT.get(a0.device.index) or sm_count(a0.device),
-                             status=_native.status().dev, stream=_native.stream_ptr())
+    _native.load().gemm_pair(*v0, *v1, _SM_COUNT.get(a0.device.index) or sm_count(a0.device), _native.status().dev,
+                             _native.stream_ptr(), pre)
     return out0, out1

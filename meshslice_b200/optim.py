@@ -42,7 +42,7 @@ class AdamW:
         """Device scalar that rescales the gradients so that their global norm is <= max."""
         if self.max_grad_norm is None:
             return None
-        self._sq.zero_()
+        _native.zero_(self._sq)
         for g in self.groups:
             idx = 0 if g.kind == "sharded" else 1
             if g.grad.is_cuda:
@@ -89,7 +89,7 @@ class AdamW:
 
     def zero_grad(self):
         for g in self.groups:
-            g.grad.zero_()
+            _native.zero_(g.grad)
 
     def resync_from_params(self, step: int = 0):
         """Rebuild the optimizer state from the current bf16 parameters: the fp32 master copies

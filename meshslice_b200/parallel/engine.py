@@ -169,22 +169,17 @@ class LocalGemmEngine:
         self.mesh = mesh
         mesh.engine = self
 
-    @staticmethod
-    def _run(X, W, layout, out, accumulate, **kw):
-        X, W = _local(X), _local(W)
-        return gemm(X, W, layout, out=out, accumulate=accumulate, **kw)
-
     def os(self, X, W, n_slices=1, out=None, accumulate=False, bias=None, act=None, pre_act=None):
-        return self._run(X, W, "nn", out, accumulate, bias=bias, act=act, pre_act=pre_act)
+        return gemm(_local(X), _local(W), "nn", out=out, accumulate=accumulate, bias=bias, act=act, pre_act=pre_act)
 
     def os_kpanel(self, X, W, order="summa", sub=1, out=None, accumulate=False):
-        return self._run(X, W, "nn", out, accumulate)
+        return gemm(_local(X), _local(W), "nn", out=out, accumulate=accumulate)
 
     def ls(self, X, W, n_slices=1, out=None, accumulate=False, rot_index=None):
-        return self._run(X, W, "nt", out, accumulate)
+        return gemm(_local(X), _local(W), "nt", out=out, accumulate=accumulate)
 
     def rs(self, X, W, n_slices=1, out=None, accumulate=False, rot_index=None):
-        return self._run(X, W, "tn", out, accumulate)
+        return gemm(_local(X), _local(W), "tn", out=out, accumulate=accumulate)
 
     def dw_dx(self, dataflow, x, dy, w, grad, gelu_pre=None):
         """Both gradients of a linear layer, which do not depend on each other, in one launch: the weight's is added to
