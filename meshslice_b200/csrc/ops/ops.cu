@@ -6,6 +6,8 @@
 #include <cuda_bf16.h>
 #include <string.h>
 
+#include <type_traits>
+
 #include "../common/gelu.cuh"
 
 namespace msb {
@@ -156,9 +158,10 @@ template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 // ------------------------------------------------------------------------------------------
-// LayerNorm forward.  One CTA per row (grid-stride), row cached in registers.  Bound by HBM: it reads x (and res) and
-// writes h (with res) and y.  32768 x 4096 with residual: 240 us with loads of one row at a time, 172 us with the row ring
-// (copy bandwidth would give 161).  RING = false loads the row when it is due: ln_fwd_direct says where that is faster.
+// LayerNorm forward in two passes (column-sharded rows: mode 1 statistics, mode 2 the rest; a row on one device is
+// ln_fwd_row_kernel's, below).  One CTA per row (grid-stride), row cached in registers.  Bound by HBM: it reads x (and res) and
+// writes h (with res) and y.  Both passes in one, 32768 x 4096 with residual: 240 us with loads of one row at a time, 172 us with
+// the row ring.  RING = false loads the row when it is due: ln_fwd_direct says where that is faster.
 // (No minimum of blocks there: with one stated, of any number, the compiler takes 80 registers or spills instead of 40.)
 // ------------------------------------------------------------------------------------------
 template <int MAXV, bool RING>
@@ -490,6 +493,176 @@ ln_bwd_kernel(int mode, const uint4* __restrict__ dy, const uint4* __restrict__ 
           if (dbeta != nullptr) add8(dbeta + v * 8, accb[k]);
         }
       }
+    }
+  }
+}
+
+// ------------------------------------------------------------------------------------------
+// LayerNorm of whole rows: W warps per row
+// ------------------------------------------------------------------------------------------
+// Bound by HBM or, while a call's tensors stay in L2, by latency.  A row is read once, into registers, by one warp (no barrier
+// at all, four rows per CTA), four or eight warps (one barrier); every CTA has one set of rows, so what hides the latency is the
+// number of CTAs, and no row waits for another one.  ln_fwd_row_shape / ln_bwd_row_shape choose W.  The kernels above walk
+// their rows in persistent CTAs with a barrier per row; the same sizes there / here, us: forward 4099 x 1544 9.0 / 5.7, with
+// residual 11.2 / 9.4, 32768 x 4096 119 / 81 (6.6 TB/s), with residual 172 / 158 (6.8 TB/s), 8192 x 12288 with residual
+// 196 / 122, 512 x 512 2.5 / 2.1; backward without parameter gradients 4099 x 1544 15.0 / 6.8, with dres 16.4 / 8.2, 32768 x
+// 2048 111 / 61 (6.6 TB/s), with dres 120 / 88.
+constexpr int ln_row_warps(int w) { return w < 4 ? 4 : w; }     // warps of a CTA; rows of a CTA: ln_row_warps(w) / w
+
+// Sum of two values over the W warps that share a row; every thread gets the result.  `red` is used once.
+template <int W>
+__device__ __forceinline__ void row_sum2(float& a, float& b, float2* red) {
+  static_assert(W == 1 || W == ln_row_warps(W), "the barrier is the CTA's");
+  a = warp_sum(a);
+  b = warp_sum(b);
+  if (W == 1) return;
+  const int w = threadIdx.x >> 5;
+  if ((threadIdx.x & 31) == 0) red[w] = make_float2(a, b);
+  __syncthreads();
+  a = 0.f;
+  b = 0.f;
+#pragma unroll
+  for (int i = 0; i < W; ++i) {
+    const float2 v = red[i];
+    a += v.x;
+    b += v.y;
+  }
+}
+
+template <int V, int W, bool RES>
+__global__ void __launch_bounds__(32 * ln_row_warps(W))
+ln_fwd_row_kernel(const uint4* __restrict__ x, const uint4* __restrict__ res, uint4* __restrict__ h_out, uint4* __restrict__ y,
+                  const uint4* __restrict__ gamma, const uint4* __restrict__ beta, float* __restrict__ mean_rstd, int rows,
+                  int cols, float eps) {
+  __shared__ float2 red[ln_row_warps(W)];
+  const int warp = threadIdx.x >> 5, row = blockIdx.x * (ln_row_warps(W) / W) + warp / W;
+  const int t = (warp % W) * 32 + (threadIdx.x & 31);            // this row's thread
+  if (W < 4 && row >= rows) return;                              // (W >= 4: a CTA is one row, and there is one for each)
+  const int nvec = cols >> 3;
+  const int64_t base = (int64_t)row * nvec;
+  uint4 u[V], r[RES ? V : 1];
+#pragma unroll
+  for (int k = 0; k < V; ++k) {
+    const int v = t + k * 32 * W;
+    if (v < nvec) {
+      u[k] = x[base + v];
+      if (RES) r[k] = res[base + v];
+    }
+  }
+  float s = 0.f, ss = 0.f;
+#pragma unroll
+  for (int k = 0; k < V; ++k) {
+    const int v = t + k * 32 * W;
+    if (v < nvec) {
+      float f[8];
+      unpack8(u[k], f);
+      if (RES) {
+        float g[8];
+        unpack8(r[k], g);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) f[i] += g[i];
+      }
+      if (h_out != nullptr) {
+        if (RES) u[k] = pack8(f);
+        h_out[base + v] = u[k];
+        unpack8(u[k], f);   // statistics of the rounded values the backward pass sees
+      }
+#pragma unroll
+      for (int i = 0; i < 8; ++i) { s += f[i]; ss += f[i] * f[i]; }
+    }
+  }
+  row_sum2<W>(s, ss, red);
+  const float mean = s / (float)cols, rstd = rsqrtf(fmaxf(ss / (float)cols - mean * mean, 0.f) + eps);
+  if (t == 0 && mean_rstd != nullptr) {
+    mean_rstd[2 * (int64_t)row] = mean;
+    mean_rstd[2 * (int64_t)row + 1] = rstd;
+  }
+#pragma unroll
+  for (int k = 0; k < V; ++k) {
+    const int v = t + k * 32 * W;
+    if (v < nvec) {
+      float f[8], g[8], b[8];
+      unpack8(u[k], f);
+      if (RES && h_out == nullptr) {          // the sum was not kept
+        unpack8(r[k], g);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) f[i] += g[i];
+      }
+      if (gamma != nullptr) unpack8(gamma[v], g);
+      if (beta != nullptr) unpack8(beta[v], b);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        float o = (f[i] - mean) * rstd;
+        if (gamma != nullptr) o *= g[i];
+        if (beta != nullptr) o += b[i];
+        f[i] = o;
+      }
+      y[base + v] = pack8(f);
+    }
+  }
+}
+
+// Without gradients of gamma and beta, whose sums over the rows the persistent kernel above keeps in registers.
+template <int V, int W, bool DRES>
+__global__ void __launch_bounds__(32 * ln_row_warps(W))
+ln_bwd_row_kernel(const uint4* __restrict__ dy, const uint4* __restrict__ h, const uint4* __restrict__ gamma,
+                  const float* __restrict__ mean_rstd, const uint4* __restrict__ dres, uint4* __restrict__ dx, int rows, int cols) {
+  __shared__ float2 red[ln_row_warps(W)];
+  const int warp = threadIdx.x >> 5, row = blockIdx.x * (ln_row_warps(W) / W) + warp / W;
+  const int t = (warp % W) * 32 + (threadIdx.x & 31);
+  if (W < 4 && row >= rows) return;
+  const int nvec = cols >> 3;
+  const int64_t base = (int64_t)row * nvec;
+  uint4 d[V], hv[V], r[DRES ? V : 1];
+#pragma unroll
+  for (int k = 0; k < V; ++k) {
+    const int v = t + k * 32 * W;
+    if (v < nvec) {
+      d[k] = dy[base + v];
+      hv[k] = h[base + v];
+    }
+  }
+  const float mean = mean_rstd[2 * (int64_t)row], rstd = mean_rstd[2 * (int64_t)row + 1];
+  float s1 = 0.f, s2 = 0.f;
+#pragma unroll
+  for (int k = 0; k < V; ++k) {
+    const int v = t + k * 32 * W;
+    if (v < nvec) {
+      float df[8], hf[8], gm[8];
+      unpack8(d[k], df);
+      unpack8(hv[k], hf);
+      if (gamma != nullptr) unpack8(gamma[v], gm);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const float g = gamma != nullptr ? df[i] * gm[i] : df[i];
+        s1 += g;
+        s2 += g * ((hf[i] - mean) * rstd);
+      }
+      if (DRES) r[k] = dres[base + v];
+    }
+  }
+  row_sum2<W>(s1, s2, red);
+  const float m1 = s1 / (float)cols, m2 = s2 / (float)cols;
+#pragma unroll
+  for (int k = 0; k < V; ++k) {
+    const int v = t + k * 32 * W;
+    if (v < nvec) {
+      float df[8], hf[8], gm[8], o[8];
+      unpack8(d[k], df);
+      unpack8(hv[k], hf);
+      if (gamma != nullptr) unpack8(gamma[v], gm);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const float g = gamma != nullptr ? df[i] * gm[i] : df[i];
+        o[i] = rstd * (g - m1 - (hf[i] - mean) * rstd * m2);
+      }
+      if (DRES) {
+        float rf[8];
+        unpack8(r[k], rf);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) o[i] += rf[i];
+      }
+      dx[base + v] = pack8(o);
     }
   }
 }
@@ -866,7 +1039,7 @@ inline int ln_fwd_resident(int cols) {
 }
 
 // Rows of one vector per thread without the ring: while what a call moves stays in L2 there is no HBM latency to hide, and
-// the way through shared memory costs more than it gives.  Repeated calls, ring / direct, us: 4099 x 1544 with residual
+// the way through shared memory costs more than it gives.  Repeated calls of both passes in one, ring / direct, us: 4099 x 1544 with residual
 // (51 MB) 12.0 / 11.0, 8192 x 1024 with residual (67 MB) 12.8 / 11.5, 8192 x 2048 without (67 MB) 20.8 / 18.0; beyond L2 the
 // ring wins: 12000 x 1024 with residual (98 MB) 18.8 / 18.9, 16384 x 1024 (134 MB) 26.3 / 28.9; and below 8 MB, where a CTA
 // has one row, by 0.1 us (512 x 512 with residual 2.5 / 2.7).  With inputs from HBM the two differ by little up to the
@@ -876,6 +1049,41 @@ constexpr int64_t kLnDirectMin = 8 << 20, kLnDirectMax = 80 << 20;
 inline bool ln_fwd_direct(int rows, int cols, int tensors) {
   const int64_t bytes = 2 * (int64_t)rows * cols * tensors;
   return ln_fwd_maxv(cols) == 1 && bytes >= kLnDirectMin && bytes <= kLnDirectMax;
+}
+
+// Warps per row and 16-byte vectors per thread of the row kernels (w = 0: the persistent kernel).  One warp as long as its
+// vectors fit the registers that still leave enough warps per SM, four or eight beyond; with few rows more warps, down to a
+// vector each, because a row's latency is all there is.  us for W = 1 / 4 / 8:
+//   forward            32768 x 2048 42 / 51 / 71, x 4096 - / 81 / 106; 33 x 2048 2.9 / 2.2 / 2.0
+//   with residual      65536 x 1024 82 / 89 / 133, 32768 x 1544 64 / 68 / 85, x 2048 85 / 81 / 94; 8192 x 6000 - / 63 / 62, x 8192 - /
+//                      85 / 83
+//   backward           32768 x 2048 61 / 63 / 77, x 4096 - / 117 / 129
+//   with dres          65536 x 512 46 / 53 / 92, 32768 x 1024 52 / 41 / 56, x 3072 - / 132 / 145, x 4096 - / 192 / 172 (persistent 183),
+//                      8192 x 8192 - / 125 / 110 (persistent 96): three tensors in registers beyond three vectors each are too many
+struct LnRowShape { int v, w; };
+inline LnRowShape ln_row_shape(int rows, int cols, int max1, int max4, int max8) {
+  const int nvec = cols / 8;
+  const auto vectors = [&](int w) { return (nvec + 32 * w - 1) / (32 * w); };
+  int w = vectors(1) <= max1 ? 1 : vectors(4) <= max4 ? 4 : vectors(8) <= max8 ? 8 : 0;
+  if (w == 0) return {0, 0};
+  while (w < 8 && vectors(w) > 1 && (int64_t)rows * w < 1024) w = w == 1 ? 4 : 8;
+  return {vectors(w), w};
+}
+inline LnRowShape ln_fwd_row_shape(int rows, int cols, bool res) {
+  return res ? ln_row_shape(rows, cols, 7, 5, 8) : ln_row_shape(rows, cols, 8, 8, 8);
+}
+inline LnRowShape ln_bwd_row_shape(int rows, int cols, bool dres) {
+  return dres ? ln_row_shape(rows, cols, 2, 3, 3) : ln_row_shape(rows, cols, 8, 8, 8);
+}
+// f(vectors, warps) as integral constants
+template <class F>
+cudaError_t with_row_shape(LnRowShape s, F&& f) {
+#define MSB_ROW(V, W) if (s.v == V && s.w == W) return f(std::integral_constant<int, V>{}, std::integral_constant<int, W>{});
+#define MSB_ROWS(W) MSB_ROW(1, W) MSB_ROW(2, W) MSB_ROW(3, W) MSB_ROW(4, W) MSB_ROW(5, W) MSB_ROW(6, W) MSB_ROW(7, W) MSB_ROW(8, W)
+  MSB_ROWS(1) MSB_ROWS(4) MSB_ROWS(8)
+#undef MSB_ROWS
+#undef MSB_ROW
+  return cudaErrorInvalidValue;
 }
 
 inline int grid_for(int64_t n, int threads, int cap = 148 * 16) {
@@ -944,6 +1152,14 @@ cudaError_t ln_fwd(int mode, const void* x, const void* res, void* h_out, void* 
   const int threads = ln_threads(cols), maxv = ln_fwd_maxv(cols);
   const int inputs = mode != 2 && res != nullptr ? 2 : 1;
   const int tensors = inputs + (mode != 2 && h_out != nullptr ? 1 : 0) + (mode != 1 ? 1 : 0);
+  if (exch == nullptr && mode == 0 && total_cols == cols) {
+    return with_row_shape(ln_fwd_row_shape(rows, cols, R != nullptr), [&](auto v, auto w) {
+      constexpr int per = ln_row_warps(w.value) / w.value;
+      auto kernel = R != nullptr ? ln_fwd_row_kernel<v.value, w.value, true> : ln_fwd_row_kernel<v.value, w.value, false>;
+      kernel<<<(rows + per - 1) / per, 32 * ln_row_warps(w.value), 0, stream>>>(X, R, H, Y, G, B, mean_rstd, rows, cols, eps);
+      return cudaGetLastError();
+    });
+  }
   if (exch == nullptr && ln_fwd_direct(rows, cols, tensors)) {
     ln_fwd_kernel<1, false><<<grid, threads, 0, stream>>>(mode, X, R, H, Y, G, B, stats, mean_rstd, rows, cols, total_cols, eps, ex);
     return cudaGetLastError();
@@ -975,6 +1191,15 @@ cudaError_t ln_bwd(int mode, const void* dy, const void* h, const void* gamma,
   auto G = reinterpret_cast<const uint4*>(gamma);
   auto DR = reinterpret_cast<const uint4*>(dres);
   auto DX = reinterpret_cast<uint4*>(dx);
+  const LnRowShape rs = ln_bwd_row_shape(rows, cols, DR != nullptr);
+  if (exch == nullptr && mode == 0 && total_cols == cols && dgamma == nullptr && dbeta == nullptr && rs.w > 0 && rows > 0) {
+    return with_row_shape(rs, [&](auto v, auto w) {
+      constexpr int per = ln_row_warps(w.value) / w.value;
+      auto kernel = DR != nullptr ? ln_bwd_row_kernel<v.value, w.value, true> : ln_bwd_row_kernel<v.value, w.value, false>;
+      kernel<<<(rows + per - 1) / per, 32 * ln_row_warps(w.value), 0, stream>>>(DY, H, G, mean_rstd, DR, DX, rows, cols);
+      return cudaGetLastError();
+    });
+  }
   const LnBwdShape sh = ln_bwd_shape(cols);
   const int maxv = cols <= kLnGroupedMaxCols ? 1 : sh.maxv <= 2 ? 2 : sh.maxv;
   const int smem = ln_ring_bytes(true, mode != 1 && dres != nullptr ? 3 : 2, maxv, sh.threads);

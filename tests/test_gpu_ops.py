@@ -41,6 +41,41 @@ def test_layernorm_row_ring(cols, rows, residual):
 
 
 @pytest.mark.parametrize("residual", [True, False])
+@pytest.mark.parametrize("cols,rows", [(8, 1), (256, 1025), (264, 1027), (1544, 1), (1544, 257), (1800, 1500), (2048, 256), (2048, 1030),
+                                       (2056, 1025), (3080, 130), (4096, 300), (5128, 1024), (6152, 130), (8192, 128), (8200, 40),
+                                       (16384, 33)])
+def test_layernorm_of_whole_rows(cols, rows, residual):
+    """One, four and eight warps per row at the edges of the rule (a vector more than a warp's registers take, few rows, the last
+    CTA partly empty, the last vector in one lane), without affine parameters, and the backward pass without their gradients
+    where the persistent kernel would otherwise run.  One bf16 rounding (2^-8 of the value, 2^-7 with the statistics)."""
+    from meshslice_b200.ops import functional as F
+    g = torch.Generator(device="cuda").manual_seed(cols * 7 + rows)
+    mk = lambda *s: torch.randn(*s, device="cuda", generator=g).bfloat16()
+    x, res, dy, dres = mk(rows, cols) + 1, mk(rows, cols), mk(rows, cols), mk(rows, cols)
+    h, y, mr = F.ln_full(x, res if residual else None, None, None, 1e-5)
+    dx = F.ln_bwd_full(dy, h, None, mr, None, None, dres if residual else None)
+    gamma = mk(cols)
+    dxg = F.ln_bwd_full(dy, h, gamma, mr, None, None, dres if residual else None)
+    torch.cuda.synchronize()
+    assert torch.equal(h, (x.float() + res.float()).bfloat16() if residual else x)
+    close = lambda a, b: ((a.double() - b).abs() <= 2 ** -7 * b.abs() + 2 ** -7 * b.abs().mean()).all()
+    for got, scale in ((dx, None), (dxg, gamma.double())):
+        hd = h.double().requires_grad_(True)
+        ref = torch.nn.functional.layer_norm(hd, (cols,), scale, None, 1e-5)
+        ref.backward(dy.double())
+        assert close(got, hd.grad + dres.double() if residual else hd.grad)
+        if scale is None:
+            assert close(y, ref.detach())
+    # rows with an infinity or a NaN are NaN, the others are not touched
+    bad = x.clone()
+    bad[0, 0], bad[rows // 2, cols - 1] = float("inf"), float("nan")
+    hb, yb, mb = F.ln_full(bad, res if residual else None, None, None, 1e-5)
+    keep = torch.ones(rows, dtype=torch.bool, device="cuda")
+    keep[0] = keep[rows // 2] = False
+    assert torch.isnan(yb[~keep]).any(1).all() and torch.equal(yb[keep], y[keep]) and torch.equal(mb[keep], mr[keep])
+
+
+@pytest.mark.parametrize("residual", [True, False])
 @pytest.mark.parametrize("cols", [264, 1024, 2048])
 def test_layernorm_forward_with_and_without_the_ring(cols, residual):
     """A call that moves more than 80 MiB takes the row ring, one of a sixteenth of its rows (8 to 80 MiB) does not: the same
