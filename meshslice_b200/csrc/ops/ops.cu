@@ -8,6 +8,7 @@
 
 #include <type_traits>
 
+#include "../common/f32x2.cuh"
 #include "../common/gelu.cuh"
 
 namespace msb {
@@ -88,6 +89,13 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
 __device__ __forceinline__ void unpack8(const uint4& u, float (&f)[8]) {
   f[0] = bf_lo(u.x); f[1] = bf_hi(u.x); f[2] = bf_lo(u.y); f[3] = bf_hi(u.y);
   f[4] = bf_lo(u.z); f[5] = bf_hi(u.z); f[6] = bf_lo(u.w); f[7] = bf_hi(u.w);
+}
+// Word i of a vector; its two bf16 as packed fp32 lanes; four such pairs as floats.
+__device__ __forceinline__ uint32_t word(const uint4& u, int i) { return i == 0 ? u.x : i == 1 ? u.y : i == 2 ? u.z : u.w; }
+__device__ __forceinline__ uint64_t unpack2(uint32_t u) { return f32x2(bf_lo(u), bf_hi(u)); }
+__device__ __forceinline__ void split4(const uint64_t (&v)[4], float (&f)[8]) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) split(v[i], f[2 * i], f[2 * i + 1]);
 }
 __device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
   uint4 u;
@@ -324,8 +332,9 @@ __device__ __forceinline__ void add8(float* dst, const float (&v)[8]) {
 // A CTA of up to kLnBwdThreads threads walks the rows grid-stride.  A 4096-wide row is two 16-byte vectors per
 // thread: the per-thread dgamma / dbeta accumulators (16 registers per vector) are what limits occupancy, so the rows
 // ahead wait in the shared-memory ring and both passes over a row read it there; gamma is loaded once per CTA.  Bound by
-// HBM (dy, h, dres read, dx written); 32768 x 4096 with dres: 254 us with loads of one row at a time, 192 us now (copy
-// bandwidth would give 161); 8192 x 12288: 290 and 146.
+// HBM (dy, h, dres read, dx written); 32768 x 4096 with dres: 254 us with loads of one row at a time, 192 us with the ring,
+// 181 us with packed arithmetic and the normalised row kept between the two passes (65 % of the issue slots were taken; copy
+// bandwidth would give 161); 8192 x 12288: 290, 146 and 136.
 // GROUPED (rows of at most 256 vectors, e.g. column shards): the CTA works on blockDim.x / tpr rows at a time,
 // `tpr` threads (whole warps) per row, and adds the row groups' dgamma / dbeta in shared memory before its one
 // atomic per column, so that narrow rows neither idle most of a CTA nor multiply the atomics.
@@ -337,6 +346,7 @@ ln_bwd_kernel(int mode, const uint4* __restrict__ dy, const uint4* __restrict__ 
               float* __restrict__ dgamma, float* __restrict__ dbeta, int rows, int cols,
               int total_cols, int tpr_arg, const __grid_constant__ RowExchange ex) {
   static_assert(!GROUPED || MAXV == 1, "grouped rows are one vector per thread");
+  constexpr bool kKeep = MAXV == 2;      // what both passes over a row need stays in registers where there is room for it
   extern __shared__ uint4 ring[];
   constexpr int S = ln_stages(true, MAXV);
   __shared__ float red[128];
@@ -347,12 +357,12 @@ ln_bwd_kernel(int mode, const uint4* __restrict__ dy, const uint4* __restrict__ 
   const int sub = GROUPED ? (int)threadIdx.x / tpr : 0;           // which of the CTA's rows
   const int tx = GROUPED ? (int)threadIdx.x - sub * tpr : (int)threadIdx.x;
   const int rows_per_cta = GROUPED ? (int)blockDim.x / tpr : 1;
-  float accg[MAXV][8], accb[MAXV][8];
+  uint64_t accg[MAXV][4], accb[MAXV][4];
   uint4 pg[MAXV];
 #pragma unroll
   for (int k = 0; k < MAXV; ++k) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) { accg[k][i] = 0.f; accb[k][i] = 0.f; }
+    for (int i = 0; i < 4; ++i) { accg[k][i] = 0; accb[k][i] = 0; }
     const int v = tx + k * tpr;
     pg[k] = (gamma != nullptr && v < nvec) ? gamma[v] : make_uint4(0x3f803f80u, 0x3f803f80u, 0x3f803f80u, 0x3f803f80u);
   }
@@ -397,25 +407,35 @@ ln_bwd_kernel(int mode, const uint4* __restrict__ dy, const uint4* __restrict__ 
     if (row + step < n_rows)
       stat_next = make_float2(mean_rstd[2 * (int64_t)(row + step)], mean_rstd[2 * (int64_t)(row + step) + 1]);
     cp_async_wait<S - 1>();
-    float s1 = 0.f, s2 = 0.f;
+    const uint64_t neg_mean = f32x2(-mean, -mean), rstd2 = f32x2(rstd, rstd);
+    uint64_t sum1 = 0, sum2 = 0;
+    uint64_t xs[kKeep ? MAXV : 1][4], gs[kKeep ? MAXV : 1][4];   // normalised row and dy * gamma
+    const auto both = [&](int k, int i, const uint4& du, const uint4& hu, uint64_t& d, uint64_t& xh, uint64_t& g) {
+      d = unpack2(word(du, i));
+      xh = mul2(add2(unpack2(word(hu, i)), neg_mean), rstd2);
+      g = mul2(d, unpack2(word(pg[k], i)));
+    };
 #pragma unroll
     for (int k = 0; k < MAXV; ++k) {
       const int v = tx + k * tpr;
       if (live && v < nvec) {
-        float d[8], hv[8], gm[8];
-        unpack8(*slot(stage, 0, k), d);
-        unpack8(*slot(stage, 1, k), hv);
-        unpack8(pg[k], gm);
+        const uint4 du = *slot(stage, 0, k), hu = *slot(stage, 1, k);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const float xh = (hv[i] - mean) * rstd;
-          const float g = d[i] * gm[i];
-          s1 += g;
-          s2 += g * xh;
-          if (want_param_grads) { accg[k][i] += d[i] * xh; accb[k][i] += d[i]; }
+        for (int i = 0; i < 4; ++i) {
+          uint64_t d, xh, g;
+          both(k, i, du, hu, d, xh, g);
+          sum1 = add2(sum1, g);
+          sum2 = fma2(g, xh, sum2);
+          if (want_param_grads) { accg[k][i] = fma2(d, xh, accg[k][i]); accb[k][i] = add2(accb[k][i], d); }
+          if (kKeep) { xs[k][i] = xh; gs[k][i] = g; }
         }
       }
     }
+    float s1, s2, hi;
+    split(sum1, s1, hi);
+    s1 += hi;
+    split(sum2, s2, hi);
+    s2 += hi;
     if (mode == 2) {
       if (live) {
         if (exchange) {
@@ -445,23 +465,29 @@ ln_bwd_kernel(int mode, const uint4* __restrict__ dy, const uint4* __restrict__ 
       }
     }
     const float m1 = s1 / (float)total_cols, m2 = s2 / (float)total_cols;
+    const uint64_t neg_m1 = f32x2(-m1, -m1), neg_m2 = f32x2(-m2, -m2);
 #pragma unroll
     for (int k = 0; k < MAXV; ++k) {
       const int v = tx + k * tpr;
       if (live && v < nvec) {
-        float d[8], hv[8], gm[8], o[8];
-        unpack8(*slot(stage, 0, k), d);
-        unpack8(*slot(stage, 1, k), hv);
-        unpack8(pg[k], gm);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) o[i] = rstd * (d[i] * gm[i] - m1 - (hv[i] - mean) * rstd * m2);
-        if (want_dres) {
-          float r[8];
-          unpack8(*slot(stage, 2, k), r);
-#pragma unroll
-          for (int i = 0; i < 8; ++i) o[i] += r[i];
+        uint4 du = make_uint4(0u, 0u, 0u, 0u), hu = du, ru = du, o;
+        if (!kKeep) {
+          du = *slot(stage, 0, k);
+          hu = *slot(stage, 1, k);
         }
-        __stcs(dx + base + v, pack8(o));
+        if (want_dres) ru = *slot(stage, 2, k);
+        uint32_t* ow = &o.x;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          uint64_t d, xh, g;
+          if (kKeep) { xh = xs[k][i]; g = gs[k][i]; }
+          else both(k, i, du, hu, d, xh, g);
+          const uint64_t t = fma2(xh, neg_m2, add2(g, neg_m1));
+          float lo, hi;
+          split(want_dres ? fma2(t, rstd2, unpack2(word(ru, i))) : mul2(t, rstd2), lo, hi);
+          ow[i] = pack2(lo, hi);
+        }
+        __stcs(dx + base + v, o);
       }
     }
     stage = stage + 1 == S ? 0 : stage + 1;
@@ -472,10 +498,13 @@ ln_bwd_kernel(int mode, const uint4* __restrict__ dy, const uint4* __restrict__ 
       for (int i = threadIdx.x; i < 2 * cols; i += blockDim.x) comb[i] = 0.f;
       __syncthreads();
       if (tx < nvec) {
+        float fg[8], fb[8];
+        split4(accg[0], fg);
+        split4(accb[0], fb);
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-          atomicAdd(comb + tx * 8 + i, accg[0][i]);
-          atomicAdd(comb + cols + tx * 8 + i, accb[0][i]);
+          atomicAdd(comb + tx * 8 + i, fg[i]);
+          atomicAdd(comb + cols + tx * 8 + i, fb[i]);
         }
       }
       __syncthreads();
@@ -489,8 +518,11 @@ ln_bwd_kernel(int mode, const uint4* __restrict__ dy, const uint4* __restrict__ 
       for (int k = 0; k < MAXV; ++k) {
         const int v = tx + k * tpr;
         if (v < nvec) {
-          add8(dgamma + v * 8, accg[k]);
-          if (dbeta != nullptr) add8(dbeta + v * 8, accb[k]);
+          float f[8];
+          split4(accg[k], f);
+          add8(dgamma + v * 8, f);
+          split4(accb[k], f);
+          if (dbeta != nullptr) add8(dbeta + v * 8, f);
         }
       }
     }
@@ -602,13 +634,83 @@ ln_fwd_row_kernel(const uint4* __restrict__ x, const uint4* __restrict__ res, ui
   }
 }
 
-// Without gradients of gamma and beta, whose sums over the rows the persistent kernel above keeps in registers.
-template <int V, int W, bool DRES>
+// dgamma += sum over the rows of dy * xhat, dbeta += sum of dy, for 32 columns and one of `slices` interleaved parts of the rows:
+// four threads with a vector each per row, T / 4 rows at a time.
+template <int T>
+__device__ __forceinline__ void ln_column_sums(const uint4* __restrict__ dy, const uint4* __restrict__ h,
+                                               const float* __restrict__ mean_rstd, int rows, int cols, float* __restrict__ dgamma,
+                                               float* __restrict__ dbeta, int block, int slice, int slices) {
+  __shared__ float part[T / 32][2][32];
+  const int nvec = cols >> 3, sub = threadIdx.x & 3, v = block * 4 + sub;
+  uint64_t g[4] = {0, 0, 0, 0}, b[4] = {0, 0, 0, 0};
+  constexpr int kStep = T / 4, kAhead = 4;
+  if (v < nvec) {
+    for (int r0 = slice * kStep + (threadIdx.x >> 2); r0 < rows; r0 += slices * kStep * kAhead) {
+      uint4 du[kAhead], hu[kAhead];
+      float mean[kAhead], rstd[kAhead];
+#pragma unroll
+      for (int j = 0; j < kAhead; ++j) {
+        const int64_t row = r0 + (int64_t)j * slices * kStep;
+        const bool live = row < rows;
+        du[j] = live ? dy[row * nvec + v] : make_uint4(0u, 0u, 0u, 0u);
+        hu[j] = live ? h[row * nvec + v] : make_uint4(0u, 0u, 0u, 0u);
+        mean[j] = live ? mean_rstd[2 * row] : 0.f;
+        rstd[j] = live ? mean_rstd[2 * row + 1] : 0.f;
+      }
+#pragma unroll
+      for (int j = 0; j < kAhead; ++j) {
+        const uint64_t neg_mean = f32x2(-mean[j], -mean[j]), rstd2 = f32x2(rstd[j], rstd[j]);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const uint64_t d = unpack2(word(du[j], i));
+          g[i] = fma2(d, mul2(add2(unpack2(word(hu[j], i)), neg_mean), rstd2), g[i]);
+          b[i] = add2(b[i], d);
+        }
+      }
+    }
+  }
+  float fg[8], fb[8];
+  split4(g, fg);
+  split4(b, fb);
+#pragma unroll
+  for (int o = 4; o < 32; o <<= 1)
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      fg[i] += __shfl_xor_sync(0xffffffffu, fg[i], o);
+      fb[i] += __shfl_xor_sync(0xffffffffu, fb[i], o);
+    }
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (lane < 4) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      part[warp][0][lane * 8 + i] = fg[i];
+      part[warp][1][lane * 8 + i] = fb[i];
+    }
+  }
+  __syncthreads();
+  const int c = block * 32 + lane;
+  if (warp < 2 && c < cols) {
+    float* dst = warp == 0 ? dgamma : dbeta;
+    float sum = 0.f;
+#pragma unroll
+    for (int i = 0; i < T / 32; ++i) sum += part[i][warp][lane];
+    if (dst != nullptr) atomicAdd(dst + c, sum);
+  }
+}
+
+// SUMS: the first `sum_ctas` CTAs add up dgamma and dbeta, from a second look at dy and h: `slices` of the rows for every 32 columns.
+template <int V, int W, bool DRES, bool SUMS>
 __global__ void __launch_bounds__(32 * ln_row_warps(W))
 ln_bwd_row_kernel(const uint4* __restrict__ dy, const uint4* __restrict__ h, const uint4* __restrict__ gamma,
-                  const float* __restrict__ mean_rstd, const uint4* __restrict__ dres, uint4* __restrict__ dx, int rows, int cols) {
+                  const float* __restrict__ mean_rstd, const uint4* __restrict__ dres, uint4* __restrict__ dx, int rows, int cols,
+                  float* __restrict__ dgamma, float* __restrict__ dbeta, int sum_ctas, int slices) {
+  if (SUMS && (int)blockIdx.x < sum_ctas) {
+    ln_column_sums<32 * ln_row_warps(W)>(dy, h, mean_rstd, rows, cols, dgamma, dbeta, blockIdx.x / slices, blockIdx.x % slices, slices);
+    return;
+  }
+  const int cta = SUMS ? (int)blockIdx.x - sum_ctas : (int)blockIdx.x;
   __shared__ float2 red[ln_row_warps(W)];
-  const int warp = threadIdx.x >> 5, row = blockIdx.x * (ln_row_warps(W) / W) + warp / W;
+  const int warp = threadIdx.x >> 5, row = cta * (ln_row_warps(W) / W) + warp / W;
   const int t = (warp % W) * 32 + (threadIdx.x & 31);
   if (W < 4 && row >= rows) return;
   const int nvec = cols >> 3;
@@ -1075,6 +1177,17 @@ inline LnRowShape ln_fwd_row_shape(int rows, int cols, bool res) {
 inline LnRowShape ln_bwd_row_shape(int rows, int cols, bool dres) {
   return dres ? ln_row_shape(rows, cols, 2, 3, 3) : ln_row_shape(rows, cols, 8, 8, 8);
 }
+// dgamma and dbeta from a second look at dy and h, in CTAs of the same launch, instead of the persistent kernel's registers: that
+// kernel ends with atomics of every CTA to the same addresses (5 us and more), and rows of up to 2048 columns wait there at a
+// barrier each.  The second look is from L2 as long as the tensors stay there.  Persistent / here, us, with dres: 512 x 512
+// 8.2 / 3.0, 4099 x 1544 22.1 / 11.2, 8192 x 2048 (34 MB a tensor) 40.8 / 30.0, 16384 x 2048 (67 MB) 70.4 / 66.0, 32768 x 1024 (67 MB)
+// 67.0 / 76.6, 4099 x 3072 (25 MB) 27.1 / 24.4, 4099 x 4096 (34 MB) 33.3 / 33.0, 8192 x 4096 57.2 / 72.2; without dres 32768 x 2048
+// (134 MB) 124 / 106, 4099 x 4096 26.4 / 24.9, 8192 x 4096 50.7 / 58.0.
+inline bool ln_sums_from_second_look(int rows, int cols, bool dres) {
+  const int64_t mb = 2 * (int64_t)rows * cols / 1000000;
+  if (cols <= kLnGroupedMaxCols) return !dres || mb <= 64;
+  return mb <= (dres ? 25 : 34);
+}
 // f(vectors, warps) as integral constants
 template <class F>
 cudaError_t with_row_shape(LnRowShape s, F&& f) {
@@ -1192,12 +1305,20 @@ cudaError_t ln_bwd(int mode, const void* dy, const void* h, const void* gamma,
   auto DR = reinterpret_cast<const uint4*>(dres);
   auto DX = reinterpret_cast<uint4*>(dx);
   const LnRowShape rs = ln_bwd_row_shape(rows, cols, DR != nullptr);
-  if (exch == nullptr && mode == 0 && total_cols == cols && dgamma == nullptr && dbeta == nullptr && rs.w > 0 && rows > 0) {
+  const bool sums = dgamma != nullptr;
+  if (exch == nullptr && mode == 0 && total_cols == cols && (sums || dbeta == nullptr) && rs.w > 0 && rows > 0 &&
+      (!sums || ln_sums_from_second_look(rows, cols, DR != nullptr))) {
     return with_row_shape(rs, [&](auto v, auto w) {
-      constexpr int per = ln_row_warps(w.value) / w.value;
-      auto kernel = DR != nullptr ? ln_bwd_row_kernel<v.value, w.value, true> : ln_bwd_row_kernel<v.value, w.value, false>;
-      kernel<<<(rows + per - 1) / per, 32 * ln_row_warps(w.value), 0, stream>>>(DY, H, G, mean_rstd, DR, DX, rows, cols);
-      return cudaGetLastError();
+      constexpr int T = 32 * ln_row_warps(w.value), per = ln_row_warps(w.value) / w.value;
+      // column sums: at least 128 CTAs, and no more than eight steps of T rows for one
+      const int blocks = (cols + 31) / 32, most = (rows + T - 1) / T, few = (128 + blocks - 1) / blocks, deep = rows / (8 * T);
+      const int want = few > deep ? few : deep, slices = !sums ? 1 : want < most ? want : most, sum_ctas = sums ? blocks * slices : 0;
+      auto run = [&](auto kernel) {
+        kernel<<<sum_ctas + (rows + per - 1) / per, T, 0, stream>>>(DY, H, G, mean_rstd, DR, DX, rows, cols, dgamma, dbeta, sum_ctas, slices);
+        return cudaGetLastError();
+      };
+      if (sums) return DR != nullptr ? run(ln_bwd_row_kernel<v.value, w.value, true, true>) : run(ln_bwd_row_kernel<v.value, w.value, false, true>);
+      return DR != nullptr ? run(ln_bwd_row_kernel<v.value, w.value, true, false>) : run(ln_bwd_row_kernel<v.value, w.value, false, false>);
     });
   }
   const LnBwdShape sh = ln_bwd_shape(cols);

@@ -76,6 +76,34 @@ def test_layernorm_of_whole_rows(cols, rows, residual):
 
 
 @pytest.mark.parametrize("residual", [True, False])
+@pytest.mark.parametrize("cols,rows", [(8, 1), (40, 3000), (264, 129), (1544, 127), (1800, 4099), (2048, 513), (2056, 1025), (3080, 4100),
+                                       (6152, 33), (16384, 20), (1024, 31500), (4096, 3052)])
+def test_layernorm_parameter_gradients(cols, rows, residual):
+    """Column sums from a second look at the rows (last block of 32 columns partly empty, fewer rows than a step, several slices)
+    and, in the last sizes with a residual, either side of the rule.  They are added to what is there; fp32 sums of ``rows``
+    products of normal values: 1e-5 sqrt(rows) times thirty."""
+    from meshslice_b200.ops import functional as F
+    g = torch.Generator(device="cuda").manual_seed(cols * 3 + rows)
+    mk = lambda *s: torch.randn(*s, device="cuda", generator=g).bfloat16()
+    h, dy, dres, gamma = mk(rows, cols) + 1, mk(rows, cols), mk(rows, cols), mk(cols)
+    _, _, mr = F.ln_full(h, None, None, None, 1e-5)
+    sums = torch.ones(2 * cols + 2, device="cuda")
+    dg, db = sums[1:cols + 1], sums[cols + 1:2 * cols + 1]
+    dx = F.ln_bwd_full(dy, h, gamma, mr, dg, db, dres if residual else None)
+    only = torch.zeros(cols, device="cuda")
+    assert torch.equal(F.ln_bwd_full(dy, h, gamma, mr, only, None, dres if residual else None), dx)
+    torch.cuda.synchronize()
+    hd, gd, bd = h.double().requires_grad_(True), gamma.double().requires_grad_(True), torch.zeros(cols, device="cuda", dtype=torch.double).requires_grad_(True)
+    torch.nn.functional.layer_norm(hd, (cols,), gd, bd, 1e-5).backward(dy.double())
+    want = hd.grad + dres.double() if residual else hd.grad
+    assert ((dx.double() - want).abs() <= 2 ** -7 * want.abs() + 2 ** -7 * want.abs().mean()).all()
+    tol = 3e-4 * rows ** 0.5
+    assert (dg.double() - 1 - gd.grad).abs().max() <= tol and (db.double() - 1 - bd.grad).abs().max() <= tol
+    assert (only.double() - gd.grad).abs().max() <= tol
+    assert sums[0] == 1 and sums[-1] == 1
+
+
+@pytest.mark.parametrize("residual", [True, False])
 @pytest.mark.parametrize("cols", [264, 1024, 2048])
 def test_layernorm_forward_with_and_without_the_ring(cols, residual):
     """A call that moves more than 80 MiB takes the row ring, one of a sixteenth of its rows (8 to 80 MiB) does not: the same
