@@ -825,6 +825,9 @@ __global__ void cast_kernel(const float4* __restrict__ in, uint2* __restrict__ o
 // ------------------------------------------------------------------------------------------
 // AdamW: 4 elements per thread
 // ------------------------------------------------------------------------------------------
+// Bound by HBM: 30 bytes an element.  One step per thread in as many CTAs as that takes: 188 M elements with their norm 1040 us
+// with 2368 CTAs that walk the arrays, 995 with 9472, 957 so (6.7 TB/s); streaming hints or the order from the last element, whose
+// gradient the norm has left in L2, to the first give nothing.
 __global__ void adamw_kernel(uint2* __restrict__ param, float4* __restrict__ master,
                              float4* __restrict__ m, float4* __restrict__ v,
                              const void* __restrict__ grad, int grad_fp32, int64_t nvec, float lr,
@@ -873,20 +876,35 @@ __global__ void clip_scale_kernel(const float* __restrict__ sq, int n, float max
   *scale = f > 1.0f ? 1.0f : f;    // NaN stays NaN
 }
 
-__global__ void sumsq_kernel(const void* __restrict__ x, int is_fp32, int64_t nvec,
-                             float* __restrict__ out) {
+// Bound by HBM (with the write-back of what the step before left in L2).  Four vectors per thread in flight and 32 CTAs an SM, each
+// with one atomic: the optimizer step of 188 M elements 957 -> 948 us (eight CTAs an SM 953, 128 951).
+constexpr int kSumVec = 4;
+__global__ void __launch_bounds__(256)
+sumsq_kernel(const void* __restrict__ x, int is_fp32, int64_t nvec, float* __restrict__ out) {
   __shared__ float red[64];
   float s = 0.f, dummy = 0.f;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nvec;
-       i += (int64_t)gridDim.x * blockDim.x) {
+  const int64_t step = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t i0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i0 < nvec; i0 += step * kSumVec) {
+    float part[kSumVec];
     if (is_fp32) {
-      const float4 g = reinterpret_cast<const float4*>(x)[i];
-      s += g.x * g.x + g.y * g.y + g.z * g.z + g.w * g.w;
+      float4 g[kSumVec];
+#pragma unroll
+      for (int j = 0; j < kSumVec; ++j)
+        g[j] = i0 + j * step < nvec ? reinterpret_cast<const float4*>(x)[i0 + j * step] : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int j = 0; j < kSumVec; ++j) part[j] = g[j].x * g[j].x + g[j].y * g[j].y + g[j].z * g[j].z + g[j].w * g[j].w;
     } else {
-      const uint2 g = reinterpret_cast<const uint2*>(x)[i];
-      const float a = bf_lo(g.x), b = bf_hi(g.x), c = bf_lo(g.y), d = bf_hi(g.y);
-      s += a * a + b * b + c * c + d * d;
+      uint2 g[kSumVec];
+#pragma unroll
+      for (int j = 0; j < kSumVec; ++j)
+        g[j] = i0 + j * step < nvec ? reinterpret_cast<const uint2*>(x)[i0 + j * step] : make_uint2(0u, 0u);
+#pragma unroll
+      for (int j = 0; j < kSumVec; ++j) {
+        const float a = bf_lo(g[j].x), b = bf_hi(g[j].x), c = bf_lo(g[j].y), d = bf_hi(g[j].y);
+        part[j] = a * a + b * b + c * c + d * d;
+      }
     }
+    s += (part[0] + part[1]) + (part[2] + part[3]);
   }
   block_sum2(s, dummy, red);
   if (threadIdx.x == 0) atomicAdd(out, s);
@@ -1349,7 +1367,9 @@ cudaError_t gelu_bwd(const void* dy, const void* x, void* dx, int64_t n, cudaStr
 }
 cudaError_t add_bf16(const void* a, const void* b, void* out, int64_t n, cudaStream_t stream) {
   if (n % 8) return cudaErrorInvalidValue;
-  add_kernel<<<grid_for(n / 8, 256), 256, 0, stream>>>(reinterpret_cast<const uint4*>(a), reinterpret_cast<const uint4*>(b), reinterpret_cast<uint4*>(out), n / 8);
+  // a step per thread: 134 M elements 124 us with CTAs that walk the arrays, 113 so (the GeLU kernels, bound by issue slots, the
+  // other way round: 113 and 131)
+  add_kernel<<<grid_for(n / 8, 256, 1 << 22), 256, 0, stream>>>(reinterpret_cast<const uint4*>(a), reinterpret_cast<const uint4*>(b), reinterpret_cast<uint4*>(out), n / 8);
   return cudaGetLastError();
 }
 cudaError_t cast_f32_to_bf16(const float* in, void* out, int64_t n, int accumulate, cudaStream_t stream) {
@@ -1363,7 +1383,7 @@ cudaError_t adamw_step(void* param, float* master, float* m, float* v, const voi
                        float weight_decay, float bias_corr1, float bias_corr2,
                        const float* grad_scale, cudaStream_t stream) {
   if (n % 4) return cudaErrorInvalidValue;
-  adamw_kernel<<<grid_for(n / 4, 256), 256, 0, stream>>>(
+  adamw_kernel<<<grid_for(n / 4, 256, 1 << 22), 256, 0, stream>>>(
       reinterpret_cast<uint2*>(param), reinterpret_cast<float4*>(master), reinterpret_cast<float4*>(m),
       reinterpret_cast<float4*>(v), grad, grad_fp32, n / 4, lr, beta1, beta2, eps, weight_decay,
       bias_corr1, bias_corr2, grad_scale);
@@ -1378,7 +1398,7 @@ cudaError_t clip_scale(const float* sq, int n, float max_norm, float* norm, floa
 
 cudaError_t sumsq(const void* x, int is_fp32, int64_t n, float* out, cudaStream_t stream) {
   if (n % 4) return cudaErrorInvalidValue;
-  sumsq_kernel<<<grid_for(n / 4, 256, 148 * 8), 256, 0, stream>>>(x, is_fp32, n / 4, out);
+  sumsq_kernel<<<grid_for(n / 4, 256, 148 * 32), 256, 0, stream>>>(x, is_fp32, n / 4, out);
   return cudaGetLastError();
 }
 

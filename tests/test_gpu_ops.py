@@ -514,3 +514,19 @@ def test_cross_entropy_gradient_returns_the_row_loss():
     ref = torch.nn.functional.cross_entropy(x[:, :3991].double(), t, reduction="none")
     assert torch.equal(a, b)
     assert (loss.double() - ref).abs().max() < 1e-4
+
+
+@pytest.mark.parametrize("fp32", [True, False])
+@pytest.mark.parametrize("n", [4, 148 * 32 * 256 * 4, 148 * 32 * 256 * 16 + 12, 30000004])
+def test_sumsq_steps(n, fp32):
+    """One vector, less than a step of four vectors per thread, a whole one and a remainder: fp32 sums over at most a few hundred
+    values per thread, then over threads (1e-5 relative)."""
+    C, st = _C()
+    g = torch.Generator(device="cuda").manual_seed(n)
+    x = torch.randn(n, device="cuda", generator=g)
+    x = x if fp32 else x.bfloat16()
+    out = torch.zeros(1, device="cuda")
+    C.sumsq(x.data_ptr(), 1 if fp32 else 0, n, out.data_ptr(), st)
+    torch.cuda.synchronize()
+    want = x.double().square().sum().item()
+    assert abs(out.item() - want) <= 1e-5 * want
