@@ -916,9 +916,23 @@ sumsq_kernel(const void* __restrict__ x, int is_fp32, int64_t nvec, float* __res
 // Both kernels are bound by HBM and keep kCeVec vectors per thread in flight.  The partial pass reads a row once: every
 // thread keeps the maximum of its elements and the sum of exponentials relative to it, and rescales the sum when a group
 // of vectors raises the maximum (Milakov and Gimelshein, online softmax).  4096 rows x 50257: partial 124 us with two
-// passes over the row, 87 us so (now four fifths of the issue slots are taken); gradient 153 us with one vector in flight
+// passes over the row, 82 us with one (four fifths of the issue slots taken), 67 us with maxima of packed bf16, packed
+// differences and products and one-instruction exponentials; gradient 153 us with one vector in flight
 // and a test per element, 132 us so (copy bandwidth: 62 and 124).
 constexpr int kCeVec = 4;
+static_assert(kCeVec == 4, "the sums below are written out");
+// Larger of two bf16, twice (a NaN only where both are NaN: the sum shows the others).
+__device__ __forceinline__ uint32_t max_bf16x2(uint32_t a, uint32_t b) {
+  uint32_t d;
+  asm("max.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+  return d;
+}
+// 2^x in one instruction, results below 2^-126 zero: in a sum whose largest term is 1 they are nothing.
+__device__ __forceinline__ float exp2_ftz(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
 __global__ void __launch_bounds__(256)
 ce_partial_kernel(const __nv_bfloat16* __restrict__ logits, int64_t ld,
                   const int64_t* __restrict__ targets, int rows, int cols, int col_offset,
@@ -944,31 +958,36 @@ ce_partial_kernel(const __nv_bfloat16* __restrict__ logits, int64_t ld,
         const int v = v0 + j * blockDim.x;
         u[j] = v < nvec ? pv[v] : make_uint4(0xff80ff80u, 0xff80ff80u, 0xff80ff80u, 0xff80ff80u);   // -inf
       }
-      float top = -INFINITY;
+      uint32_t top = 0xff80ff80u;
 #pragma unroll
-      for (int j = 0; j < kCeVec; ++j) {
-        float f[8];
-        unpack8(u[j], f);
+      for (int j = 0; j < kCeVec; ++j)
 #pragma unroll
-        for (int i = 0; i < 8; ++i) top = fmaxf(top, f[i]);
-      }
-      raise(top);
-      auto sum = [&](auto term) {
-        float part[kCeVec];
+        for (int i = 0; i < 4; ++i) top = max_bf16x2(top, word(u[j], i));
+      raise(fmaxf(bf_lo(top), bf_hi(top)));
+      if (m > -INFINITY) {
+        const uint64_t neg_m = f32x2(-m, -m), log2e = f32x2(1.4426950408889634f, 1.4426950408889634f);
+        uint64_t part[kCeVec] = {};
+#pragma unroll
+        for (int j = 0; j < kCeVec; ++j)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            float lo, hi;
+            split(mul2(add2(unpack2(word(u[j], i)), neg_m), log2e), lo, hi);
+            part[j] = add2(part[j], f32x2(exp2_ftz(lo), exp2_ftz(hi)));
+          }
+        float lo, hi;
+        split(add2(add2(part[0], part[1]), add2(part[2], part[3])), lo, hi);
+        s += lo + hi;
+      } else {
+        // while everything seen is -inf nothing counts, except that a NaN has to show
 #pragma unroll
         for (int j = 0; j < kCeVec; ++j) {
           float f[8];
           unpack8(u[j], f);
-          part[j] = term(f[0]);
 #pragma unroll
-          for (int i = 1; i < 8; ++i) part[j] += term(f[i]);
+          for (int i = 0; i < 8; ++i) s += f[i] == f[i] ? 0.f : f[i];
         }
-#pragma unroll
-        for (int j = 0; j < kCeVec; ++j) s += part[j];
-      };
-      // while everything seen is -inf nothing counts, except that a NaN has to show
-      if (m > -INFINITY) sum([&](float f) { return __expf(f - m); });
-      else sum([&](float f) { return f == f ? 0.f : f; });
+      }
     }
     for (int c = nvec * 8 + threadIdx.x; c < valid; c += blockDim.x) {
       const float f = __bfloat162float(p[c]);
