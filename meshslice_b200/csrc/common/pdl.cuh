@@ -1,0 +1,32 @@
+// Programmatic dependent launch: a kernel's blocks may become resident, and set up, while the kernel before it in the stream ends.
+// Between two kernels of a few us that is 1 to 1.5 us, and the launch itself takes the host 2.2 us instead of 2.6: attention forward
+// and backward of batch 3 x 640 with 5 heads 35.3 -> 31.0 us, the linear layer of 1992 x 4104 x 1032 81.7 -> 78.5, of 512 x 512 x
+// 1536 26.4 -> 24.8, a two-layer model of width 512 481 -> 453; calls of several hundred us stay as they are.  Kernels of a row
+// exchange, which wait for other GPUs, are launched plainly.
+#pragma once
+#include <cuda_runtime.h>
+
+namespace msb {
+
+// Wait until the grids before this one in the stream are complete and their writes visible / let the next grid start once every
+// block of this one has come here or left.  Without the launch attribute both do nothing.  Every block of a grid launched with
+// launch_dependent() waits, before it touches memory that an earlier grid may use: then what follows this grid follows those too.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <class... P, class... A>
+cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args) {
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
+}  // namespace msb

@@ -15,6 +15,7 @@
 #include <string.h>
 
 #include "../common/gelu.cuh"
+#include "../common/pdl.cuh"
 #include "../common/ptx.cuh"
 #include "out_turn.h"
 #include "sm100_gemm.h"
@@ -310,6 +311,8 @@ sm100_gemm2_kernel(const __grid_constant__ Gemm2Args a) {
   cluster_sync_all();      // barriers of both CTAs are initialised before any remote arrival
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  grid_trigger();
+  grid_wait();
 
   if (warp == 0 || warp == 6) {
     // ===================== TMA producers (both CTAs): warp 0 loads A, warp 6 loads B ==========
@@ -534,8 +537,7 @@ static cudaError_t launch2(const Gemm2Args& args, int grid, cudaStream_t stream)
     configured[dev] = true;
   }
   // the cluster shape (2,1,1) is part of the kernel's definition
-  sm100_gemm2_kernel<BN, kDGelu><<<grid, kThreads2, smem, stream>>>(args);
-  return cudaGetLastError();
+  return launch_dependent(sm100_gemm2_kernel<BN, kDGelu>, grid, kThreads2, smem, stream, args);
 }
 
 // The tile width that ends sooner.  A 64-deep k-block takes about 390 cycles on 128 columns (the loads: 24 KiB

@@ -16,6 +16,7 @@
 #include <type_traits>
 
 #include "../common/f32x2.cuh"
+#include "../common/pdl.cuh"
 #include "../common/ptx.cuh"
 #include "../gemm/sm100_gemm.h"  // make_tensor_map_2d
 
@@ -197,10 +198,6 @@ __device__ __forceinline__ void tmem_st_16x16_frag(uint32_t taddr, const uint32_
   asm volatile("tcgen05.st.sync.aligned.16x128b.x2.b32 [%0], {%1, %2, %3, %4};"
                ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]) : "memory");
 }
-// Programmatic dependent launch: wait until the grids before this one in the stream are complete and their writes visible /
-// let the next grid start once every block of this one has come here.  Without the launch attribute both do nothing.
-__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void grid_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 // shared -> global, one box of a tensor map; tracked by bulk groups
 __device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, const void* smem_src, int32_t x, int32_t y) {
   asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];"
@@ -297,6 +294,8 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_consta
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem = *tmem_slot;
+  grid_trigger();
+  grid_wait();
 
   // The next item as the producer got it: false when there is none (or on a timeout).
   uint32_t clc_phase = 0;
@@ -608,7 +607,8 @@ __global__ void __launch_bounds__(256)
 attn_delta_kernel(const uint4* __restrict__ out, const uint4* __restrict__ dout, float* __restrict__ delta,
                   uint32_t groups, uint32_t seq, uint32_t heads, const float* __restrict__ lse, float* __restrict__ lse2,
                   float scale) {
-  grid_trigger();                        // the key-major kernel may set up; it waits for this one before it reads a statistic
+  grid_wait();
+  grid_trigger();                        // the key-major kernel may start: what it reads before its own wait is complete
   const uint32_t sub = threadIdx.x & 15;
   const uint32_t w = blockIdx.x * (blockDim.x >> 4) + (threadIdx.x >> 4);   // (group of tokens, head)
   const bool live = w < groups;
@@ -1269,8 +1269,7 @@ cudaError_t attention_fwd(const void* qkv, void* out, float* lse, int batch, int
   // 30.0 / 32.8, 13.1 / 14.2 and 8.7 / 8.7.
   a.tiles_per_item = (int64_t)batch * heads * nblk <= sm_count() ? 1 : 2;
   dim3 grid(grp, (nblk + a.tiles_per_item - 1) / a.tiles_per_item, batch * heads / grp);
-  attn_fwd2_kernel<<<grid, kFwd2Threads, kFwd2Smem, stream>>>(tm, to, a);
-  return cudaGetLastError();
+  return launch_dependent(attn_fwd2_kernel, grid, kFwd2Threads, kFwd2Smem, stream, tm, to, a);
 }
 
 cudaError_t attention_bwd(const void* qkv, const void* out, const void* dout, const float* lse,
@@ -1300,9 +1299,9 @@ cudaError_t attention_bwd(const void* qkv, const void* out, const void* dout, co
     const int threads = 256, per_block = threads / 16;
     const int64_t blocks = (groups + per_block - 1) / per_block;
     auto kernel = off(out, 16) ? attn_delta_kernel<false> : attn_delta_kernel<true>;
-    kernel<<<(unsigned)blocks, threads, 0, stream>>>(reinterpret_cast<const uint4*>(out), reinterpret_cast<const uint4*>(dout),
-                                                     delta, (uint32_t)groups, seq, heads, lse, dq_acc, scale);
-    cudaError_t e = cudaGetLastError();
+    const cudaError_t e = launch_dependent(kernel, (unsigned)blocks, threads, 0, stream, reinterpret_cast<const uint4*>(out),
+                                           reinterpret_cast<const uint4*>(dout), delta, (uint32_t)groups, (uint32_t)seq,
+                                           (uint32_t)heads, lse, dq_acc, scale);
     if (e != cudaSuccess) return e;
   }
   // two deterministic kernels: dK / dV per key block, dQ per query block
@@ -1316,19 +1315,10 @@ cudaError_t attention_bwd(const void* qkv, const void* out, const void* dout, co
   const int grp = bh_group(batch, heads);
   // Overlap of the three launches: the key-major kernel sets up and loads its first tiles while the row sums end, the
   // query-major one, which reads nothing of it, takes SMs as they get free (batch 3 x 640, 5 heads: 75 items each).
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(grp, seq / kBlk, batch * heads / grp);
-  cfg.blockDim = dim3(kBwd2Threads);
-  cfg.dynamicSmemBytes = kBwd2Smem;
-  cfg.stream = stream;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, attn_bwd2_kernel<true>, tq, td, tg, g);
+  const dim3 grid2(grp, seq / kBlk, batch * heads / grp);
+  cudaError_t e = launch_dependent(attn_bwd2_kernel<true>, grid2, kBwd2Threads, kBwd2Smem, stream, tq, td, tg, g);
   if (e != cudaSuccess) return e;
-  return cudaLaunchKernelEx(&cfg, attn_bwd2_kernel<false>, tq, td, tg, g);
+  return launch_dependent(attn_bwd2_kernel<false>, grid2, kBwd2Threads, kBwd2Smem, stream, tq, td, tg, g);
 }
 
 }  // namespace msb

@@ -10,6 +10,7 @@
 
 #include "../common/f32x2.cuh"
 #include "../common/gelu.cuh"
+#include "../common/pdl.cuh"
 
 namespace msb {
 
@@ -345,6 +346,8 @@ ln_bwd_kernel(int mode, const uint4* __restrict__ dy, const uint4* __restrict__ 
               const uint4* __restrict__ dres, uint4* __restrict__ dx, float* __restrict__ stats,
               float* __restrict__ dgamma, float* __restrict__ dbeta, int rows, int cols,
               int total_cols, int tpr_arg, const __grid_constant__ RowExchange ex) {
+  grid_trigger();
+  grid_wait();
   static_assert(!GROUPED || MAXV == 1, "grouped rows are one vector per thread");
   constexpr bool kKeep = MAXV == 2;      // what both passes over a row need stays in registers where there is room for it
   extern __shared__ uint4 ring[];
@@ -566,6 +569,8 @@ __global__ void __launch_bounds__(32 * ln_row_warps(W))
 ln_fwd_row_kernel(const uint4* __restrict__ x, const uint4* __restrict__ res, uint4* __restrict__ h_out, uint4* __restrict__ y,
                   const uint4* __restrict__ gamma, const uint4* __restrict__ beta, float* __restrict__ mean_rstd, int rows,
                   int cols, float eps) {
+  grid_trigger();
+  grid_wait();
   __shared__ float2 red[ln_row_warps(W)];
   const int warp = threadIdx.x >> 5, row = blockIdx.x * (ln_row_warps(W) / W) + warp / W;
   const int t = (warp % W) * 32 + (threadIdx.x & 31);            // this row's thread
@@ -704,6 +709,8 @@ __global__ void __launch_bounds__(32 * ln_row_warps(W))
 ln_bwd_row_kernel(const uint4* __restrict__ dy, const uint4* __restrict__ h, const uint4* __restrict__ gamma,
                   const float* __restrict__ mean_rstd, const uint4* __restrict__ dres, uint4* __restrict__ dx, int rows, int cols,
                   float* __restrict__ dgamma, float* __restrict__ dbeta, int sum_ctas, int slices) {
+  grid_trigger();
+  grid_wait();
   if (SUMS && (int)blockIdx.x < sum_ctas) {
     ln_column_sums<32 * ln_row_warps(W)>(dy, h, mean_rstd, rows, cols, dgamma, dbeta, blockIdx.x / slices, blockIdx.x % slices, slices);
     return;
@@ -773,6 +780,8 @@ ln_bwd_row_kernel(const uint4* __restrict__ dy, const uint4* __restrict__ h, con
 // elementwise
 // ------------------------------------------------------------------------------------------
 __global__ void gelu_fwd_kernel(const uint4* __restrict__ x, uint4* __restrict__ y, int64_t nvec) {
+  grid_trigger();
+  grid_wait();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nvec;
        i += (int64_t)gridDim.x * blockDim.x) {
     float f[8];
@@ -784,6 +793,8 @@ __global__ void gelu_fwd_kernel(const uint4* __restrict__ x, uint4* __restrict__
 }
 __global__ void gelu_bwd_kernel(const uint4* __restrict__ dy, const uint4* __restrict__ x,
                                 uint4* __restrict__ dx, int64_t nvec) {
+  grid_trigger();
+  grid_wait();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nvec;
        i += (int64_t)gridDim.x * blockDim.x) {
     float f[8], d[8];
@@ -796,6 +807,8 @@ __global__ void gelu_bwd_kernel(const uint4* __restrict__ dy, const uint4* __res
 }
 __global__ void add_kernel(const uint4* __restrict__ a, const uint4* __restrict__ b,
                            uint4* __restrict__ o, int64_t nvec) {
+  grid_trigger();
+  grid_wait();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nvec;
        i += (int64_t)gridDim.x * blockDim.x) {
     float f[8], g[8];
@@ -808,6 +821,8 @@ __global__ void add_kernel(const uint4* __restrict__ a, const uint4* __restrict_
 }
 __global__ void cast_kernel(const float4* __restrict__ in, uint2* __restrict__ out, int64_t nvec,
                             int accumulate) {
+  grid_trigger();
+  grid_wait();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nvec;
        i += (int64_t)gridDim.x * blockDim.x) {
     float4 f = in[i];
@@ -833,6 +848,8 @@ __global__ void adamw_kernel(uint2* __restrict__ param, float4* __restrict__ mas
                              const void* __restrict__ grad, int grad_fp32, int64_t nvec, float lr,
                              float beta1, float beta2, float eps, float wd, float bc1, float bc2,
                              const float* __restrict__ grad_scale) {
+  grid_trigger();
+  grid_wait();
   const float gs = grad_scale != nullptr ? *grad_scale : 1.0f;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nvec;
        i += (int64_t)gridDim.x * blockDim.x) {
@@ -869,6 +886,8 @@ __global__ void adamw_kernel(uint2* __restrict__ param, float4* __restrict__ mas
 // The clipping factor in one launch of one thread instead of seven of a scalar each (20 us of an optimizer step).
 __global__ void clip_scale_kernel(const float* __restrict__ sq, int n, float max_norm, float* __restrict__ norm,
                                   float* __restrict__ scale) {
+  grid_trigger();
+  grid_wait();
   float s = 0.f;
   for (int i = 0; i < n; ++i) s += sq[i];
   const float len = sqrtf(s), f = max_norm / (len + 1e-6f);
@@ -881,6 +900,8 @@ __global__ void clip_scale_kernel(const float* __restrict__ sq, int n, float max
 constexpr int kSumVec = 4;
 __global__ void __launch_bounds__(256)
 sumsq_kernel(const void* __restrict__ x, int is_fp32, int64_t nvec, float* __restrict__ out) {
+  grid_trigger();
+  grid_wait();
   __shared__ float red[64];
   float s = 0.f, dummy = 0.f;
   const int64_t step = (int64_t)gridDim.x * blockDim.x;
@@ -938,6 +959,8 @@ ce_partial_kernel(const __nv_bfloat16* __restrict__ logits, int64_t ld,
                   const int64_t* __restrict__ targets, int rows, int cols, int col_offset,
                   int vocab, float* __restrict__ row_max, float* __restrict__ row_sumexp,
                   float* __restrict__ tgt_logit, const __grid_constant__ RowExchange ex) {
+  grid_trigger();
+  grid_wait();
   __shared__ float red[64];
   const int valid = max(0, min(cols, vocab - col_offset));
   const int nvec = valid >> 3;
@@ -1020,6 +1043,8 @@ ce_grad_kernel(__nv_bfloat16* __restrict__ logits, int64_t ld, const int64_t* __
                int rows, int cols, int col_offset, int vocab, const float* __restrict__ gmax,
                const float* __restrict__ gsumexp, float scale, float* __restrict__ row_loss,
                const float* __restrict__ tgt_logit, const __grid_constant__ RowExchange ex) {
+  grid_trigger();
+  grid_wait();
   const int nvec = cols >> 3;
   if (ex.n > 0 && !ex_wait(ex, 2u)) return;
   for (int row = blockIdx.x; row < rows; row += gridDim.x) {
@@ -1084,6 +1109,8 @@ __global__ void embedding_fwd_kernel(const int64_t* __restrict__ tokens,
                                      const uint4* __restrict__ tok_table,
                                      const uint4* __restrict__ pos_table, uint4* __restrict__ out,
                                      int n_tokens, int seq, int nvec) {
+  grid_trigger();
+  grid_wait();
   for (int t = blockIdx.x; t < n_tokens; t += gridDim.x) {
     const int64_t tok = tokens[t];
     const int pos = t % seq;
@@ -1101,6 +1128,8 @@ __global__ void embedding_fwd_kernel(const int64_t* __restrict__ tokens,
 __global__ void embedding_bwd_tok_kernel(const int64_t* __restrict__ tokens,
                                          const uint4* __restrict__ dout, float* __restrict__ dtok,
                                          int n_tokens, int nvec) {
+  grid_trigger();
+  grid_wait();
   for (int t = blockIdx.x; t < n_tokens; t += gridDim.x) {
     const int64_t tok = tokens[t];
     for (int v = threadIdx.x; v < nvec; v += blockDim.x) {
@@ -1114,6 +1143,8 @@ __global__ void embedding_bwd_tok_kernel(const int64_t* __restrict__ tokens,
 }
 __global__ void embedding_bwd_pos_kernel(const uint4* __restrict__ dout, float* __restrict__ dpos,
                                          int n_tokens, int seq, int nvec) {
+  grid_trigger();
+  grid_wait();
   const int64_t total = (int64_t)seq * nvec;
   const int nb = n_tokens / seq;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total;
@@ -1306,8 +1337,8 @@ cudaError_t ln_fwd(int mode, const void* x, const void* res, void* h_out, void* 
     return with_row_shape(ln_fwd_row_shape(rows, cols, R != nullptr), [&](auto v, auto w) {
       constexpr int per = ln_row_warps(w.value) / w.value;
       auto kernel = R != nullptr ? ln_fwd_row_kernel<v.value, w.value, true> : ln_fwd_row_kernel<v.value, w.value, false>;
-      kernel<<<(rows + per - 1) / per, 32 * ln_row_warps(w.value), 0, stream>>>(X, R, H, Y, G, B, mean_rstd, rows, cols, eps);
-      return cudaGetLastError();
+      return launch_dependent(kernel, (rows + per - 1) / per, 32 * ln_row_warps(w.value), 0, stream, X, R, H, Y, G, B, mean_rstd, rows,
+                              cols, eps);
     });
   }
   if (exch == nullptr && ln_fwd_direct(rows, cols, tensors)) {
@@ -1351,8 +1382,8 @@ cudaError_t ln_bwd(int mode, const void* dy, const void* h, const void* gamma,
       const int blocks = (cols + 31) / 32, most = (rows + T - 1) / T, few = (128 + blocks - 1) / blocks, deep = rows / (8 * T);
       const int want = few > deep ? few : deep, slices = !sums ? 1 : want < most ? want : most, sum_ctas = sums ? blocks * slices : 0;
       auto run = [&](auto kernel) {
-        kernel<<<sum_ctas + (rows + per - 1) / per, T, 0, stream>>>(DY, H, G, mean_rstd, DR, DX, rows, cols, dgamma, dbeta, sum_ctas, slices);
-        return cudaGetLastError();
+        return launch_dependent(kernel, sum_ctas + (rows + per - 1) / per, T, 0, stream, DY, H, G, mean_rstd, DR, DX, rows, cols, dgamma,
+                                dbeta, sum_ctas, slices);
       };
       if (sums) return DR != nullptr ? run(ln_bwd_row_kernel<v.value, w.value, true, true>) : run(ln_bwd_row_kernel<v.value, w.value, false, true>);
       return DR != nullptr ? run(ln_bwd_row_kernel<v.value, w.value, true, false>) : run(ln_bwd_row_kernel<v.value, w.value, false, false>);
@@ -1364,6 +1395,9 @@ cudaError_t ln_bwd(int mode, const void* dy, const void* h, const void* gamma,
   auto run = [&](auto kernel) {
     const cudaError_t e = allow_smem(reinterpret_cast<const void*>(kernel), smem);
     if (e != cudaSuccess) return e;
+    if (exch == nullptr)
+      return launch_dependent(kernel, grid, sh.threads, smem, stream, mode, DY, H, G, mean_rstd, DR, DX, stats, dgamma, dbeta, rows,
+                              cols, total_cols, sh.tpr, ex);
     kernel<<<grid, sh.threads, smem, stream>>>(mode, DY, H, G, mean_rstd, DR, DX, stats, dgamma, dbeta, rows, cols,
                                               total_cols, sh.tpr, ex);
     return cudaGetLastError();
@@ -1376,25 +1410,21 @@ cudaError_t ln_bwd(int mode, const void* dy, const void* h, const void* gamma,
 
 cudaError_t gelu_fwd(const void* x, void* y, int64_t n, cudaStream_t stream) {
   if (n % 8) return cudaErrorInvalidValue;
-  gelu_fwd_kernel<<<grid_for(n / 8, 256), 256, 0, stream>>>(reinterpret_cast<const uint4*>(x), reinterpret_cast<uint4*>(y), n / 8);
-  return cudaGetLastError();
+  return launch_dependent(gelu_fwd_kernel, grid_for(n / 8, 256), 256, 0, stream, reinterpret_cast<const uint4*>(x), reinterpret_cast<uint4*>(y), n / 8);
 }
 cudaError_t gelu_bwd(const void* dy, const void* x, void* dx, int64_t n, cudaStream_t stream) {
   if (n % 8) return cudaErrorInvalidValue;
-  gelu_bwd_kernel<<<grid_for(n / 8, 256), 256, 0, stream>>>(reinterpret_cast<const uint4*>(dy), reinterpret_cast<const uint4*>(x), reinterpret_cast<uint4*>(dx), n / 8);
-  return cudaGetLastError();
+  return launch_dependent(gelu_bwd_kernel, grid_for(n / 8, 256), 256, 0, stream, reinterpret_cast<const uint4*>(dy), reinterpret_cast<const uint4*>(x), reinterpret_cast<uint4*>(dx), n / 8);
 }
 cudaError_t add_bf16(const void* a, const void* b, void* out, int64_t n, cudaStream_t stream) {
   if (n % 8) return cudaErrorInvalidValue;
   // a step per thread: 134 M elements 124 us with CTAs that walk the arrays, 113 so (the GeLU kernels, bound by issue slots, the
   // other way round: 113 and 131)
-  add_kernel<<<grid_for(n / 8, 256, 1 << 22), 256, 0, stream>>>(reinterpret_cast<const uint4*>(a), reinterpret_cast<const uint4*>(b), reinterpret_cast<uint4*>(out), n / 8);
-  return cudaGetLastError();
+  return launch_dependent(add_kernel, grid_for(n / 8, 256, 1 << 22), 256, 0, stream, reinterpret_cast<const uint4*>(a), reinterpret_cast<const uint4*>(b), reinterpret_cast<uint4*>(out), n / 8);
 }
 cudaError_t cast_f32_to_bf16(const float* in, void* out, int64_t n, int accumulate, cudaStream_t stream) {
   if (n % 4) return cudaErrorInvalidValue;
-  cast_kernel<<<grid_for(n / 4, 256), 256, 0, stream>>>(reinterpret_cast<const float4*>(in), reinterpret_cast<uint2*>(out), n / 4, accumulate);
-  return cudaGetLastError();
+  return launch_dependent(cast_kernel, grid_for(n / 4, 256), 256, 0, stream, reinterpret_cast<const float4*>(in), reinterpret_cast<uint2*>(out), n / 4, accumulate);
 }
 
 cudaError_t adamw_step(void* param, float* master, float* m, float* v, const void* grad,
@@ -1402,23 +1432,17 @@ cudaError_t adamw_step(void* param, float* master, float* m, float* v, const voi
                        float weight_decay, float bias_corr1, float bias_corr2,
                        const float* grad_scale, cudaStream_t stream) {
   if (n % 4) return cudaErrorInvalidValue;
-  adamw_kernel<<<grid_for(n / 4, 256, 1 << 22), 256, 0, stream>>>(
-      reinterpret_cast<uint2*>(param), reinterpret_cast<float4*>(master), reinterpret_cast<float4*>(m),
-      reinterpret_cast<float4*>(v), grad, grad_fp32, n / 4, lr, beta1, beta2, eps, weight_decay,
-      bias_corr1, bias_corr2, grad_scale);
-  return cudaGetLastError();
+  return launch_dependent(adamw_kernel, grid_for(n / 4, 256, 1 << 22), 256, 0, stream, reinterpret_cast<uint2*>(param), reinterpret_cast<float4*>(master), reinterpret_cast<float4*>(m), reinterpret_cast<float4*>(v), grad, grad_fp32, n / 4, lr, beta1, beta2, eps, weight_decay, bias_corr1, bias_corr2, grad_scale);
 }
 
 cudaError_t clip_scale(const float* sq, int n, float max_norm, float* norm, float* scale, cudaStream_t stream) {
   if (n < 1) return cudaErrorInvalidValue;
-  clip_scale_kernel<<<1, 1, 0, stream>>>(sq, n, max_norm, norm, scale);
-  return cudaGetLastError();
+  return launch_dependent(clip_scale_kernel, 1, 1, 0, stream, sq, n, max_norm, norm, scale);
 }
 
 cudaError_t sumsq(const void* x, int is_fp32, int64_t n, float* out, cudaStream_t stream) {
   if (n % 4) return cudaErrorInvalidValue;
-  sumsq_kernel<<<grid_for(n / 4, 256, 148 * 32), 256, 0, stream>>>(x, is_fp32, n / 4, out);
-  return cudaGetLastError();
+  return launch_dependent(sumsq_kernel, grid_for(n / 4, 256, 148 * 32), 256, 0, stream, x, is_fp32, n / 4, out);
 }
 
 cudaError_t ce_partial(const void* logits, int64_t ld, const int64_t* targets, int rows, int cols,
@@ -1428,6 +1452,8 @@ cudaError_t ce_partial(const void* logits, int64_t ld, const int64_t* targets, i
   if (exch != nullptr) ex = *exch; else memset(&ex, 0, sizeof(ex));
   if (ld % 8) return cudaErrorInvalidValue;
   const int grid = exch != nullptr ? ce_grid(rows) : ce_local_grid(rows);
+  if (exch == nullptr)
+    return launch_dependent(ce_partial_kernel, grid, 256, 0, stream, reinterpret_cast<const __nv_bfloat16*>(logits), ld, targets, rows, cols, col_offset, vocab, row_max, row_sumexp, tgt_logit, ex);
   ce_partial_kernel<<<grid, 256, 0, stream>>>(reinterpret_cast<const __nv_bfloat16*>(logits), ld, targets, rows, cols, col_offset, vocab, row_max, row_sumexp, tgt_logit, ex);
   return cudaGetLastError();
 }
@@ -1439,6 +1465,8 @@ cudaError_t ce_grad(void* logits, int64_t ld, const int64_t* targets, int rows, 
   if (exch != nullptr) ex = *exch; else memset(&ex, 0, sizeof(ex));
   if (ld % 8 || cols % 8) return cudaErrorInvalidValue;
   const int grid = exch != nullptr ? ce_grid(rows) : ce_local_grid(rows);
+  if (exch == nullptr)
+    return launch_dependent(ce_grad_kernel, grid, 256, 0, stream, reinterpret_cast<__nv_bfloat16*>(logits), ld, targets, rows, cols, col_offset, vocab, gmax, gsumexp, scale, row_loss, tgt_logit, ex);
   ce_grad_kernel<<<grid, 256, 0, stream>>>(reinterpret_cast<__nv_bfloat16*>(logits), ld, targets, rows, cols, col_offset, vocab, gmax, gsumexp, scale, row_loss, tgt_logit, ex);
   return cudaGetLastError();
 }
@@ -1447,18 +1475,15 @@ cudaError_t embedding_fwd(const int64_t* tokens, const void* tok_table, const vo
                           void* out, int n_tokens, int seq, int cols, cudaStream_t stream) {
   if (cols % 8) return cudaErrorInvalidValue;
   const int grid = n_tokens < 148 * 16 ? n_tokens : 148 * 16;
-  embedding_fwd_kernel<<<grid, 128, 0, stream>>>(tokens, reinterpret_cast<const uint4*>(tok_table), reinterpret_cast<const uint4*>(pos_table), reinterpret_cast<uint4*>(out), n_tokens, seq, cols / 8);
-  return cudaGetLastError();
+  return launch_dependent(embedding_fwd_kernel, grid, 128, 0, stream, tokens, reinterpret_cast<const uint4*>(tok_table), reinterpret_cast<const uint4*>(pos_table), reinterpret_cast<uint4*>(out), n_tokens, seq, cols / 8);
 }
 cudaError_t embedding_bwd(const int64_t* tokens, const void* dout, float* dtok, float* dpos,
                           int n_tokens, int seq, int cols, cudaStream_t stream) {
   if (cols % 8 || n_tokens % seq) return cudaErrorInvalidValue;
   const int grid = n_tokens < 148 * 16 ? n_tokens : 148 * 16;
-  embedding_bwd_tok_kernel<<<grid, 128, 0, stream>>>(tokens, reinterpret_cast<const uint4*>(dout), dtok, n_tokens, cols / 8);
-  cudaError_t e = cudaGetLastError();
+  const cudaError_t e = launch_dependent(embedding_bwd_tok_kernel, grid, 128, 0, stream, tokens, reinterpret_cast<const uint4*>(dout), dtok, n_tokens, cols / 8);
   if (e != cudaSuccess) return e;
-  embedding_bwd_pos_kernel<<<grid_for((int64_t)seq * (cols / 8), 256), 256, 0, stream>>>(reinterpret_cast<const uint4*>(dout), dpos, n_tokens, seq, cols / 8);
-  return cudaGetLastError();
+  return launch_dependent(embedding_bwd_pos_kernel, grid_for((int64_t)seq * (cols / 8), 256), 256, 0, stream, reinterpret_cast<const uint4*>(dout), dpos, n_tokens, seq, cols / 8);
 }
 
 }  // namespace msb

@@ -530,3 +530,40 @@ def test_sumsq_steps(n, fp32):
     torch.cuda.synchronize()
     want = x.double().square().sum().item()
     assert abs(out.item() - want) <= 1e-5 * want
+
+
+@pytest.mark.parametrize("rows,d", [(64, 128), (512, 512), (2056, 1032)])
+def test_dependent_launches_stay_in_order(rows, d):
+    """A chain of kernels that set up while the one before ends, on buffers that the next turn overwrites: the bits of the same
+    chain with a synchronisation after every call (fewer blocks than SMs, about as many, more)."""
+    from meshslice_b200 import _native
+    from meshslice_b200.ops import functional as F
+    from meshslice_b200.ops.gemm import gemm, gemm_pair
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    mk = lambda *s: torch.randn(*s, device="cuda", generator=g).bfloat16()
+    inputs = [(mk(rows, d), mk(rows, d)) for _ in range(3)]
+    w, gamma, beta = mk(d, d) * 0.1, mk(d), mk(d)
+    targets = torch.randint(0, d, (rows,), device="cuda", generator=g)
+    x, r, buf = torch.empty_like(inputs[0][0]), torch.empty_like(inputs[0][0]), torch.empty(rows, d, device="cuda").bfloat16()
+
+    def turn(i, sync):
+        done = torch.cuda.synchronize if sync else (lambda: None)
+        x.copy_(inputs[i][0]); r.copy_(inputs[i][1]); done()
+        h, y, mr = F.ln_full(x, r, gamma, beta, 1e-5); done()
+        gemm(y, w, "nn", out=buf); done()
+        z = F.add(F.gelu(buf), h); done()
+        mx, se, tl = F.ce_partial(z, targets, 0, d); done()
+        loss = F.ce_grad_loss_(z, targets, 0, d, mx, se, tl, 1.0 / rows); done()
+        dw = torch.zeros(d, d, device="cuda"); done()
+        _, dx = gemm_pair(y, z, "tn", dw, True, z, w, "nt", gelu_pre=buf); done()
+        dx = F.ln_bwd_full(dx, h, gamma, mr, None, None, z); done()
+        out = [t.clone() for t in (loss, dw, dx, buf)]
+        buf.fill_(float("nan")); x.fill_(float("nan")); r.fill_(float("nan")); done()
+        return out
+
+    want = [turn(i, True) for i in range(3)]
+    got = [turn(i % 3, False) for i in range(18)]
+    torch.cuda.synchronize()
+    _native.check_status()
+    for i, out in enumerate(got):
+        assert all(torch.equal(a, b) for a, b in zip(out, want[i % 3])), i
