@@ -79,6 +79,17 @@ def zero_(t) -> None:
         t.zero_()
 
 
+def zero_both_(a, b) -> None:
+    """``zero_`` of two tensors, in one launch where ``b`` follows ``a`` without a gap in the same GPU memory block."""
+    n = a.numel() * a.element_size()
+    if (a.is_cuda and b.is_cuda and a.is_contiguous() and b.is_contiguous() and b.data_ptr() == a.data_ptr() + n
+            and a.untyped_storage().data_ptr() == b.untyped_storage().data_ptr()):
+        load().memset_zero(a.data_ptr(), n + b.numel() * b.element_size(), stream_ptr())
+    else:
+        zero_(a)
+        zero_(b)
+
+
 class _Status:
     def __init__(self):
         C = load()

@@ -23,7 +23,7 @@ from typing import Callable, List, Optional
 
 import torch
 
-from .._native import zero_
+from .._native import zero_, zero_both_
 from ..ops import functional as F
 from ..parallel.mesh import Mesh, ShardedTensor
 from ..parallel.tensor_parallel import SPMD, createMultihostMatrix
@@ -146,9 +146,12 @@ class ShardedLayerNorm:
         a = alloc or _default_alloc
         mk = lambda fill: ShardedTensor(mesh, {k: a((local,), dtype, device).fill_(fill) for k in mesh.coords()})
         self.gamma, self.bias = mk(1.0), mk(0.0)
-        ga = grad_alloc or _default_alloc
-        z = lambda: ShardedTensor(mesh, {k: ga((local,), torch.float32, device).zero_() for k in mesh.coords()})
-        self.dgamma, self.dbias = z(), z()
+        if grad_alloc is None:      # one block per coordinate, so that one launch clears both
+            both = {k: torch.zeros(2, local, dtype=torch.float32, device=device) for k in mesh.coords()}
+            self.dgamma, self.dbias = (ShardedTensor(mesh, {k: t[i] for k, t in both.items()}) for i in (0, 1))
+        else:
+            z = lambda: ShardedTensor(mesh, {k: grad_alloc((local,), torch.float32, device).zero_() for k in mesh.coords()})
+            self.dgamma, self.dbias = z(), z()
         self._saved = None
 
     def forward(self, x: ShardedTensor, res: Optional[ShardedTensor] = None):
@@ -234,10 +237,8 @@ class ShardedLayerNorm:
                                                    stats.shards[k], self.in_dim, DR(k)) for k in m.coords()})
 
     def zero_grad(self):
-        for t in self.dgamma.shards.values():
-            zero_(t)
-        for t in self.dbias.shards.values():
-            zero_(t)
+        for k, t in self.dgamma.shards.items():
+            zero_both_(t, self.dbias.shards[k])
 
     def parameters(self):
         if not self.affine:
