@@ -504,6 +504,13 @@ void ce_grad_local(uint64_t logits, int64_t ld, uint64_t targets, int rows, int 
   check(ce_grad(P<void>(logits), ld, P<int64_t>(targets), rows, cols, col_offset, vocab, P<float>(gmax), P<float>(gsum), scale,
                 S(stream), P<float>(row_loss), nullptr, P<float>(tgt_logit)), "ce_grad");
 }
+void ce_row_local(uint64_t logits, int64_t ld, uint64_t targets, int rows, int cols, int vocab, float scale, uint64_t row_loss,
+                  uint64_t stream) {
+  check(ce_row(P<void>(logits), ld, P<int64_t>(targets), rows, cols, vocab, scale, P<float>(row_loss), S(stream)), "ce_row");
+}
+void py_sum_over(uint64_t x, int n, float divisor, uint64_t out, uint64_t stream) {
+  check(sum_over(P<float>(x), n, divisor, P<float>(out), S(stream)), "sum_over");
+}
 void py_embedding_fwd(uint64_t tokens, uint64_t tok, uint64_t pos, uint64_t out, int n_tokens, int seq, int cols, uint64_t stream) {
   check(embedding_fwd(P<int64_t>(tokens), P<void>(tok), P<void>(pos), P<void>(out), n_tokens, seq, cols, S(stream)), "embedding_fwd");
 }
@@ -599,6 +606,7 @@ PYBIND11_MODULE(_C, m) {
      py::arg("total_cols"), py::arg("stream"), py::arg("exch") = py::none());
   m.def("ln_grid", &ln_grid, py::arg("backward"), py::arg("rows"), py::arg("cols") = 0,
         "CTAs of the LayerNorm kernels in a row exchange for a row count and local width (0: forward, 1: backward)");
+  m.attr("CE_ROW_COLS") = ce_row_cols();
   m.def("ce_grid", &ce_grid, "CTAs of the cross-entropy kernels in a row exchange for a row count");
   m.def("cast_f32_to_bf16", [](uint64_t in, uint64_t out, int64_t n, int accumulate, uint64_t stream) {
     check(cast_f32_to_bf16(P<float>(in), P<void>(out), n, accumulate, S(stream)), "cast_f32_to_bf16");
@@ -655,6 +663,8 @@ PYBIND11_MODULE(_C, m) {
                  "tgt_logit, stream"),
       MSB_DIRECT("ce_grad_local", ce_grad_local, "logits, ld, targets, rows, cols, col_offset, vocab, gmax, gsum, scale, stream, "
                  "row_loss, tgt_logit"),
+      MSB_DIRECT("ce_row_local", ce_row_local, "logits, ld, targets, rows, cols, vocab, scale, row_loss, stream"),
+      MSB_DIRECT("sum_over", py_sum_over, "x, n, divisor, out, stream"),
       MSB_DIRECT("embedding_fwd", py_embedding_fwd, "tokens, tok, pos, out, n_tokens, seq, cols, stream"),
       MSB_DIRECT("embedding_bwd", py_embedding_bwd, "tokens, dout, dtok, dpos, n_tokens, seq, cols, stream"),
       MSB_DIRECT("attention_fwd", py_attention_fwd, "qkv, out, lse, batch, seq, heads, causal, scale, status, stream"),

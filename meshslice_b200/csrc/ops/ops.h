@@ -96,6 +96,13 @@ int ce_grid(int rows);   // CTAs of ce_partial with an exchange (each counts one
 // row_loss[row] = log(sumexp) + max - target logit is written when non-null: with `exch` the three values
 // are combined from the mesh row's published partials (gmax / gsumexp / tgt_logit unused), otherwise
 // they are the arrays given.
+// Loss and gradient of whole rows on one device: logits <- (softmax - onehot) * scale, row_loss[row] = log sum exp - target logit.
+// At most ce_row_cols() columns before the padding.
+int ce_row_cols();
+cudaError_t ce_row(void* logits, int64_t ld, const int64_t* targets, int rows, int cols, int vocab, float scale, float* row_loss,
+                   cudaStream_t stream);
+// *out = (x[0] + ... + x[n - 1]) / divisor.
+cudaError_t sum_over(const float* x, int n, float divisor, float* out, cudaStream_t stream);
 cudaError_t ce_grad(void* logits, int64_t ld, const int64_t* targets, int rows, int cols,
                     int col_offset, int vocab, const float* gmax, const float* gsumexp,
                     float scale, cudaStream_t stream, float* row_loss = nullptr,

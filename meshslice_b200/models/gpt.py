@@ -206,9 +206,10 @@ class GPTModel:
             loss = ShardedTensor(m, {k0: row_loss.sum() / n_tokens_global})
         elif m.C == 1:
             # whole rows on one device: nothing to combine between the two passes
-            row_loss = {k: F.ce_grad_loss_(l, targets.shards[k], 0, cfg.vocab, *F.ce_partial(l, targets.shards[k], 0, cfg.vocab),
-                                           1.0 / n_tokens_global) for k, l in logits.shards.items()}
-            loss = ShardedTensor(m, {k: v.sum() / n_tokens_global for k, v in row_loss.items()})
+            loss = ShardedTensor(m, {})
+            for k, l in logits.shards.items():
+                row_loss = F.ce_loss_grad_(l, targets.shards[k], cfg.vocab, 1.0 / n_tokens_global)
+                loss.shards[k] = F.sum_over(row_loss, n_tokens_global)
         else:
             parts = {k: F.ce_partial(logits.shards[k], targets.shards[k], k[1] * vc, cfg.vocab) for k in m.coords()}
             mx = ShardedTensor(m, {k: v[0] for k, v in parts.items()})

@@ -299,6 +299,29 @@ def ce_grad_loss_(logits, targets, col_offset: int, vocab: int, gmax, gsum, tgt_
     return torch.log(gsum) + gmax - tgt_logit
 
 
+def ce_loss_grad_(logits, targets, vocab: int, scale: float):
+    """Whole rows: logits <- (softmax - onehot) * scale in place (padding columns get 0); returns the per-row loss
+    log(sum exp) - target logit [rows].  One launch on a GPU where a row fits into shared memory."""
+    if logits.is_cuda:
+        rows, cols = logits.shape
+        C = _C()
+        if rows > 0 and 0 < vocab and min(cols, vocab) <= C.CE_ROW_COLS:
+            row_loss = torch.empty(rows, device=logits.device, dtype=torch.float32)
+            C.ce_row_local(logits.data_ptr(), logits.stride(0), targets.data_ptr(), rows, cols, vocab, scale,
+                           row_loss.data_ptr(), _st())
+            return row_loss
+    return ce_grad_loss_(logits, targets, 0, vocab, *ce_partial(logits, targets, 0, vocab), scale)
+
+
+def sum_over(x, divisor: float):
+    """``x.sum() / divisor`` of a contiguous fp32 vector as a 0-dim tensor."""
+    if x.is_cuda:
+        out = torch.empty((), device=x.device, dtype=torch.float32)
+        _C().sum_over(x.data_ptr(), x.numel(), divisor, out.data_ptr(), _st())
+        return out
+    return x.sum() / divisor
+
+
 def ce_grad_(logits, targets, col_offset: int, vocab: int, gmax, gsum, scale: float):
     """In place: logits <- (softmax - onehot) * scale (padding columns get 0)."""
     rows, cols = logits.shape

@@ -567,3 +567,39 @@ def test_dependent_launches_stay_in_order(rows, d):
     _native.check_status()
     for i, out in enumerate(got):
         assert all(torch.equal(a, b) for a, b in zip(out, want[i % 3])), i
+
+
+@pytest.mark.parametrize("rows,cols,vocab", [(3, 8, 5), (5, 2048, 1000), (300, 1024, 1024), (7, 16392, 16385), (9, 51200, 50257),
+                                             (2, 102400, 102391), (2, 102408, 102401)])
+def test_cross_entropy_of_whole_rows(rows, cols, vocab):
+    """Loss and gradient in one launch (the last size, a vector too wide for it, in two): against 64 bits, and rows of -inf, with an
+    infinity or a NaN as the two-launch form gives them.  fp32 sums of ``vocab`` exponentials: 1e-6 relative, 2e-6 in the loss;
+    the gradient is rounded to bf16 once (2^-9, 2^-8 with the sum)."""
+    from meshslice_b200.ops import functional as F
+    g = torch.Generator(device="cuda").manual_seed(cols)
+    x = (2 * torch.randn(rows, cols, device="cuda", generator=g)).bfloat16()
+    t = torch.randint(0, vocab, (rows,), device="cuda", generator=g)
+    t[0] = vocab - 1
+    ref = x.double()
+    ref[:, vocab:] = float("-inf")
+    want = torch.softmax(ref, 1)
+    want[torch.arange(rows), t] -= 1
+    want_loss = torch.logsumexp(ref, 1) - ref.gather(1, t[:, None])[:, 0]
+    got = x.clone()
+    loss = F.ce_loss_grad_(got, t, vocab, 0.25)
+    torch.cuda.synchronize()
+    assert ((loss.double() - want_loss).abs() <= 4e-6 * (1 + want_loss.abs())).all()
+    assert ((got.double() - 0.25 * want).abs() <= 2 ** -8 * 0.25 * want.abs() + 1e-30).all()
+    assert (got[:, vocab:] == 0).all()
+    total = F.sum_over(loss, 2)
+    assert total.shape == () and abs(total.item() - 0.5 * loss.double().sum().item()) <= 1e-5 * abs(total.item())
+    odd = x.clone()
+    odd[0] = float("-inf")
+    odd[1, 3] = float("inf")
+    odd[rows - 1, vocab - 1] = float("nan")
+    odd[0, vocab:] = 7.0
+    a, b = odd.clone(), odd.clone()
+    la = F.ce_loss_grad_(a, t, vocab, 0.25)
+    lb = F.ce_grad_loss_(b, t, 0, vocab, *F.ce_partial(b, t, 0, vocab), 0.25)
+    assert torch.equal(torch.isnan(la), torch.isnan(lb)) and torch.equal(torch.isnan(a), torch.isnan(b))
+    assert torch.equal(torch.isinf(la), torch.isinf(lb))
