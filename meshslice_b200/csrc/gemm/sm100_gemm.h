@@ -217,8 +217,7 @@ struct Gemm2Problem {
   int a_map3d, b_map3d;        // the tensor map of an MN-major operand is the 3-D form of make_tensor_map_mn3d
   int c_fp32, accumulate, act;
   int tma_c;                   // C (and C_pre) leave through shared memory as TMA stores
-  int group, along_n, k_turn;  // tile order: panels of `group` blocks along M or N; every other tile of a CTA pair walks its
-                               // k-blocks backwards
+  int group, along_n;          // tile order: panels of `group` blocks along M or N
 };
 struct Gemm2Args {
   Gemm2Problem p[2];
@@ -229,7 +228,7 @@ struct Gemm2Args {
 // Columns of a cluster tile for a launch of one or two problems, the order of a problem's tiles, and its maps for that width
 // (0, or an error code).
 int gemm2_tile_n(const Gemm2Operands* o, int problems, int sms);
-struct Gemm2Order { int group, along_n, k_turn; };
+struct Gemm2Order { int group, along_n; };
 Gemm2Order gemm2_order(int64_t M, int64_t N, int64_t K, int tile_n);
 int gemm2_problem(Gemm2Problem* p, const Gemm2Operands& o, int tile_n);
 // One or two problems of the same tile width in a launch on at most `sms` SMs.

@@ -324,7 +324,6 @@ sm100_gemm2_kernel(const __grid_constant__ Gemm2Args a) {
       const uint32_t full0 = mapa_u32(smem_u32(full_bar), 0);     // the leader's barriers
       uint32_t stage = 0, phase = 0;
       bool ok = true, free = true;                                // `free`: the next stage was seen empty
-      bool back = false;                                          // this tile's k-blocks run from the last to the first
       for (int t = cluster_id; t < num_tiles && ok; t += n_clusters) {
         bool second;
         int m2, nb;
@@ -333,7 +332,6 @@ sm100_gemm2_kernel(const __grid_constant__ Gemm2Args a) {
         const CUtensorMap* map = is_a ? &p->a : &p->b;
         const bool mn_major = (is_a ? p->a_mn_major : p->b_mn_major) != 0, map3d = (is_a ? p->a_map3d : p->b_map3d) != 0;
         const int kblocks = (p->K + kBK - 1) / kBK;
-        const bool turn = p->k_turn != 0;
         // this CTA's 128 rows of A / its half of the columns of B
         const int row = is_a ? (2 * m2 + (int)rank) * kBM : nb * BN + (int)rank * (BN / 2);
         const uint32_t bytes = is_a ? kAStage2 : kBStage2;
@@ -346,7 +344,7 @@ sm100_gemm2_kernel(const __grid_constant__ Gemm2Args a) {
             break;
           }
           const uint32_t fb = full0 + stage * 8;
-          const int k0 = (back ? kblocks - 1 - kb : kb) * kBK;
+          const int k0 = kb * kBK;
           if (rank == 0) mbar_expect_tx(full_bar + stage, 2 * bytes);
           uint8_t* dst = ring + stage * bytes;
           if (!mn_major) {
@@ -359,7 +357,6 @@ sm100_gemm2_kernel(const __grid_constant__ Gemm2Args a) {
           if (++stage == kStages2) { stage = 0; phase ^= 1; }
           free = mbar_test(empty_bar + stage, phase ^ 1);
         }
-        back = !back && turn;
       }
     }
   } else if (warp == 1) {
@@ -569,16 +566,14 @@ int gemm2_tile_n(const Gemm2Operands* o, int problems, int sms) {
 // blocks along one dimension is kept in L2 (33 MB at K = 4096) while the tiles sweep the other, so the panels' operand is
 // read once and the other one once per panel: the dimension with the smaller sum.  Panels of eight / sixteen / thirty-two,
 // sustained: 8192 x 16384 x 4096 815 / 788 / 871 us (along N: 824 / 803 / 886), 4096 x 51200 x 1024 345 / 336 / 336.
-// Where a panel is more than L2 keeps, the wave before has left the end of the contraction there: every other tile walks it
-// backwards.  Panels of 8, of 16, of 16 with turns: 8192 x 4096 x 16384 833 / 840 / 822, 4096 x 16384 x 8192 added to fp32
-// 864 / 876 / 844, 4096 x 4096 x 8192 235 / 236 / 228; K = 4096 gains nothing (788 / 790 with turns).
+// Longer contractions keep panels of eight along M: 8192 x 4096 x 16384 833 / 840, 4096 x 16384 x 8192 added to fp32
+// 864 / 876, 4096 x 4096 x 8192 235 / 236.  Every tile sums its contraction from the first k-block to the last, so that a
+// result does not depend on which tiles a CTA pair had before; walking it backwards on every other tile, which finds the
+// end of the contraction in L2, would give 822, 844 and 228.
 Gemm2Order gemm2_order(int64_t M, int64_t N, int64_t K, int tile_n) {
+  if (K > 4096) return {8, 0};
   const int64_t panels_m = (M + 16 * 256 - 1) / (16 * 256), panels_n = (N + 16 * tile_n - 1) / (16 * tile_n);
-  Gemm2Order o;
-  o.group = 16;
-  o.along_n = N + panels_n * M < M + panels_m * N;
-  o.k_turn = K > 4096;
-  return o;
+  return {16, N + panels_n * M < M + panels_m * N};
 }
 
 int gemm2_problem(Gemm2Problem* p, const Gemm2Operands& o, int tile_n) {
@@ -608,10 +603,9 @@ int gemm2_problem(Gemm2Problem* p, const Gemm2Operands& o, int tile_n) {
   // which the copy engine cannot do.
   p->tma_c = !(o.accumulate && !o.c_fp32) && make_tensor_map_out(&p->c, o.C, o.N, o.M, o.ldc, o.c_fp32 != 0) == 0 &&
              (o.act != 1 || o.C_pre == nullptr || make_tensor_map_out(&p->pre, o.C_pre, o.N, o.M, o.ldc, false) == 0);
-  const Gemm2Order order = o.group > 0 ? Gemm2Order{o.group, 0, 0} : gemm2_order(o.M, o.N, o.K, tile_n);
+  const Gemm2Order order = o.group > 0 ? Gemm2Order{o.group, 0} : gemm2_order(o.M, o.N, o.K, tile_n);
   p->group = order.group;
   p->along_n = order.along_n;
-  p->k_turn = order.k_turn;
   return 0;
 }
 

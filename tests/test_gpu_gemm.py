@@ -73,8 +73,8 @@ def test_gemm_bias_gelu_epilogue():
     assert ((out.float() - ref).abs() <= 0.03 + 0.01 * ref.abs()).all()
 
 
-# Tile orders: panels of sixteen blocks along M (more than one, the last one short) and along N, contractions that are walked
-# backwards on every other tile, with an odd number of k-blocks whose last one is short.
+# Tile orders: panels of sixteen blocks along M (more than one, the last one short) and along N, panels of eight with an odd
+# number of k-blocks whose last one is short.
 @pytest.mark.parametrize("layout", ["nt", "nn", "tn"])
 @pytest.mark.parametrize("shape", [(4360, 2056, 136), (2056, 8456, 136), (8456, 1288, 4168), (4360, 4616, 4104)])
 def test_gemm_tile_orders(layout, shape):
@@ -219,7 +219,7 @@ def test_gemm_fp32_accumulation_keeps_subnormals():
 
 # Shapes (tokens, d_in, d_out) of the two gradients in one launch: fewer tiles than CTA pairs in both (narrow tiles), ragged
 # edges and rows whose pitch is no multiple of 128 bytes, one problem longer than a wave, one with a single short k-block,
-# contractions walked backwards in one of the two.
+# a panel order of its own in each.
 @pytest.mark.parametrize("dataflow", ["os", "ls", "rs"])
 @pytest.mark.parametrize("shape", [(512, 512, 1536), (1992, 1032, 4104), (264, 5128, 72), (8, 264, 520), (4360, 2048, 3080)])
 def test_gemm_pair_is_both_products(shape, dataflow):
@@ -244,6 +244,28 @@ def test_gemm_pair_is_both_products(shape, dataflow):
     _check(got[0][0], _ref(*first) + 1.0, first[0].shape[0] if first[2] == "tn" else first[0].shape[1])
     _check(got[0][1], _ref(*second), second[0].shape[1])
     assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+
+
+@pytest.mark.parametrize("layout", ["nt", "nn", "tn"])
+@pytest.mark.parametrize("K", [1032, 4104, 8192])
+def test_gemm_rows_do_not_depend_on_the_tiles_around_them(K, layout):
+    """A result's bits follow from its row of A and its column of B: more tiles than CTA pairs, the same rows in a product of one
+    block of them, and the same product as either of two in a launch."""
+    from meshslice_b200 import _native
+    from meshslice_b200.ops.gemm import gemm, gemm_pair
+    M, N = 5128, 4616
+    a, b = _operands(M, N, K, layout, seed=K)
+    whole = gemm(a, b, layout)
+    for i in (0, 256, 2048, 5120):
+        part = gemm(a[:, i:i + 256].contiguous() if layout == "tn" else a[i:i + 256], b, layout)
+        assert torch.equal(part, whole[i:i + 256]), i
+    x, y = _operands(1288, 1032, 4168, "nn")
+    want = gemm(x, y, "nn")
+    for first, second in (((a, b, layout), (x, y, "nn")), ((x, y, "nn"), (a, b, layout))):
+        outs = gemm_pair(*first, torch.empty(first[0].shape[0 if first[2] != "tn" else 1], (first[1].shape[1] if first[2] != "nt" else first[1].shape[0]),
+                                             device="cuda", dtype=torch.bfloat16), False, *second)
+        _native.check_status()
+        assert all(torch.equal(got, whole if f[0] is a else want) for got, f in zip(outs, (first, second)))
 
 
 def test_gemm_pair_refuses_what_gemm_refuses():
