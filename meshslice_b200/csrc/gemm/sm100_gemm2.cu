@@ -168,7 +168,7 @@ __device__ __forceinline__ void load32(const void* base, int64_t ld, int64_t row
   if (nvalid == 32 && aligned16(p)) {
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      const uint4 u = __ldcs(reinterpret_cast<const uint4*>(p) + i);
+      const uint4 u = ld_stream(reinterpret_cast<const uint4*>(p) + i);
       v[4 * i] = u.x; v[4 * i + 1] = u.y; v[4 * i + 2] = u.z; v[4 * i + 3] = u.w;
     }
   } else {

@@ -604,8 +604,8 @@ constexpr int kDeltaRows = 4;
 static_assert(kBlk % kDeltaRows == 0, "sequences are whole groups of rows");
 template <bool kWide>
 __global__ void __launch_bounds__(256)
-attn_delta_kernel(const uint4* __restrict__ out, const uint4* __restrict__ dout, float* __restrict__ delta,
-                  uint32_t groups, uint32_t seq, uint32_t heads, const float* __restrict__ lse, float* __restrict__ lse2,
+attn_delta_kernel(const uint4* out, const uint4* dout, float* delta,
+                  uint32_t groups, uint32_t seq, uint32_t heads, const float* lse, float* lse2,
                   float scale) {
   grid_wait();
   grid_trigger();                        // the key-major kernel may start: what it reads before its own wait is complete
@@ -621,13 +621,13 @@ attn_delta_kernel(const uint4* __restrict__ out, const uint4* __restrict__ dout,
     if (live) {
       const int64_t at = ((t0 + i) * heads + h) * 16 + sub;
       if (kWide) {
-        o[i] = __ldcs(out + at);
+        o[i] = ld_stream(out + at);
       } else {
         const uint2* p = reinterpret_cast<const uint2*>(out) + at * 2;
-        const uint2 lo = __ldcs(p), hi = __ldcs(p + 1);
+        const uint2 lo = ld_stream(p), hi = ld_stream(p + 1);
         o[i] = make_uint4(lo.x, lo.y, hi.x, hi.y);
       }
-      d[i] = __ldcs(dout + at);
+      d[i] = ld_stream(dout + at);
     }
   }
   float mine = 0.f;                      // the sum of row `sub`

@@ -341,10 +341,10 @@ __device__ __forceinline__ void add8(float* dst, const float (&v)[8]) {
 // atomic per column, so that narrow rows neither idle most of a CTA nor multiply the atomics.
 template <int MAXV, bool GROUPED>
 __global__ void __launch_bounds__(kLnBwdThreads, MAXV == 1 ? 2 : 1)
-ln_bwd_kernel(int mode, const uint4* __restrict__ dy, const uint4* __restrict__ h,
-              const uint4* __restrict__ gamma, const float* __restrict__ mean_rstd,
-              const uint4* __restrict__ dres, uint4* __restrict__ dx, float* __restrict__ stats,
-              float* __restrict__ dgamma, float* __restrict__ dbeta, int rows, int cols,
+ln_bwd_kernel(int mode, const uint4* dy, const uint4* h,
+              const uint4* gamma, const float* mean_rstd,
+              const uint4* dres, uint4* dx, float* stats,
+              float* dgamma, float* dbeta, int rows, int cols,
               int total_cols, int tpr_arg, const __grid_constant__ RowExchange ex) {
   grid_trigger();
   grid_wait();
@@ -566,8 +566,8 @@ __device__ __forceinline__ void row_sum2(float& a, float& b, float2* red) {
 
 template <int V, int W, bool RES>
 __global__ void __launch_bounds__(32 * ln_row_warps(W))
-ln_fwd_row_kernel(const uint4* __restrict__ x, const uint4* __restrict__ res, uint4* __restrict__ h_out, uint4* __restrict__ y,
-                  const uint4* __restrict__ gamma, const uint4* __restrict__ beta, float* __restrict__ mean_rstd, int rows,
+ln_fwd_row_kernel(const uint4* x, const uint4* res, uint4* h_out, uint4* y,
+                  const uint4* gamma, const uint4* beta, float* mean_rstd, int rows,
                   int cols, float eps) {
   grid_trigger();
   grid_wait();
@@ -608,6 +608,13 @@ ln_fwd_row_kernel(const uint4* __restrict__ x, const uint4* __restrict__ res, ui
       for (int i = 0; i < 8; ++i) { s += f[i]; ss += f[i] * f[i]; }
     }
   }
+  // scale and shift are asked for one vector ahead of the stores, which no later load may pass
+  uint4 gn = make_uint4(0u, 0u, 0u, 0u), bn = gn;
+  const auto affine = [&](int v) {
+    if (v < nvec && gamma != nullptr) gn = gamma[v];
+    if (v < nvec && beta != nullptr) bn = beta[v];
+  };
+  affine(t);
   row_sum2<W>(s, ss, red);
   const float mean = s / (float)cols, rstd = rsqrtf(fmaxf(ss / (float)cols - mean * mean, 0.f) + eps);
   if (t == 0 && mean_rstd != nullptr) {
@@ -625,8 +632,9 @@ ln_fwd_row_kernel(const uint4* __restrict__ x, const uint4* __restrict__ res, ui
 #pragma unroll
         for (int i = 0; i < 8; ++i) f[i] += g[i];
       }
-      if (gamma != nullptr) unpack8(gamma[v], g);
-      if (beta != nullptr) unpack8(beta[v], b);
+      unpack8(gn, g);
+      unpack8(bn, b);
+      if (k + 1 < V) affine(v + 32 * W);
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         float o = (f[i] - mean) * rstd;
@@ -642,9 +650,9 @@ ln_fwd_row_kernel(const uint4* __restrict__ x, const uint4* __restrict__ res, ui
 // dgamma += sum over the rows of dy * xhat, dbeta += sum of dy, for 32 columns and one of `slices` interleaved parts of the rows:
 // four threads with a vector each per row, T / 4 rows at a time.
 template <int T>
-__device__ __forceinline__ void ln_column_sums(const uint4* __restrict__ dy, const uint4* __restrict__ h,
-                                               const float* __restrict__ mean_rstd, int rows, int cols, float* __restrict__ dgamma,
-                                               float* __restrict__ dbeta, int block, int slice, int slices) {
+__device__ __forceinline__ void ln_column_sums(const uint4* dy, const uint4* h,
+                                               const float* mean_rstd, int rows, int cols, float* dgamma,
+                                               float* dbeta, int block, int slice, int slices) {
   __shared__ float part[T / 32][2][32];
   const int nvec = cols >> 3, sub = threadIdx.x & 3, v = block * 4 + sub;
   uint64_t g[4] = {0, 0, 0, 0}, b[4] = {0, 0, 0, 0};
@@ -706,9 +714,9 @@ __device__ __forceinline__ void ln_column_sums(const uint4* __restrict__ dy, con
 // SUMS: the first `sum_ctas` CTAs add up dgamma and dbeta, from a second look at dy and h: `slices` of the rows for every 32 columns.
 template <int V, int W, bool DRES, bool SUMS>
 __global__ void __launch_bounds__(32 * ln_row_warps(W))
-ln_bwd_row_kernel(const uint4* __restrict__ dy, const uint4* __restrict__ h, const uint4* __restrict__ gamma,
-                  const float* __restrict__ mean_rstd, const uint4* __restrict__ dres, uint4* __restrict__ dx, int rows, int cols,
-                  float* __restrict__ dgamma, float* __restrict__ dbeta, int sum_ctas, int slices) {
+ln_bwd_row_kernel(const uint4* dy, const uint4* h, const uint4* gamma,
+                  const float* mean_rstd, const uint4* dres, uint4* dx, int rows, int cols,
+                  float* dgamma, float* dbeta, int sum_ctas, int slices) {
   grid_trigger();
   grid_wait();
   if (SUMS && (int)blockIdx.x < sum_ctas) {
@@ -750,6 +758,11 @@ ln_bwd_row_kernel(const uint4* __restrict__ dy, const uint4* __restrict__ h, con
       if (DRES) r[k] = dres[base + v];
     }
   }
+  uint4 gn = make_uint4(0u, 0u, 0u, 0u);      // scale, asked for one vector ahead of the stores
+  const auto scale = [&](int v) {
+    if (v < nvec && gamma != nullptr) gn = gamma[v];
+  };
+  scale(t);
   row_sum2<W>(s1, s2, red);
   const float m1 = s1 / (float)cols, m2 = s2 / (float)cols;
 #pragma unroll
@@ -759,7 +772,8 @@ ln_bwd_row_kernel(const uint4* __restrict__ dy, const uint4* __restrict__ h, con
       float df[8], hf[8], gm[8], o[8];
       unpack8(d[k], df);
       unpack8(hv[k], hf);
-      if (gamma != nullptr) unpack8(gamma[v], gm);
+      unpack8(gn, gm);
+      if (k + 1 < V) scale(v + 32 * W);
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         const float g = gamma != nullptr ? df[i] * gm[i] : df[i];
@@ -779,7 +793,7 @@ ln_bwd_row_kernel(const uint4* __restrict__ dy, const uint4* __restrict__ h, con
 // ------------------------------------------------------------------------------------------
 // elementwise
 // ------------------------------------------------------------------------------------------
-__global__ void gelu_fwd_kernel(const uint4* __restrict__ x, uint4* __restrict__ y, int64_t nvec) {
+__global__ void gelu_fwd_kernel(const uint4* x, uint4* y, int64_t nvec) {
   grid_trigger();
   grid_wait();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nvec;
@@ -791,8 +805,8 @@ __global__ void gelu_fwd_kernel(const uint4* __restrict__ x, uint4* __restrict__
     y[i] = pack8(f);
   }
 }
-__global__ void gelu_bwd_kernel(const uint4* __restrict__ dy, const uint4* __restrict__ x,
-                                uint4* __restrict__ dx, int64_t nvec) {
+__global__ void gelu_bwd_kernel(const uint4* dy, const uint4* x,
+                                uint4* dx, int64_t nvec) {
   grid_trigger();
   grid_wait();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nvec;
@@ -805,8 +819,8 @@ __global__ void gelu_bwd_kernel(const uint4* __restrict__ dy, const uint4* __res
     dx[i] = pack8(d);
   }
 }
-__global__ void add_kernel(const uint4* __restrict__ a, const uint4* __restrict__ b,
-                           uint4* __restrict__ o, int64_t nvec) {
+__global__ void add_kernel(const uint4* a, const uint4* b,
+                           uint4* o, int64_t nvec) {
   grid_trigger();
   grid_wait();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nvec;
@@ -819,7 +833,7 @@ __global__ void add_kernel(const uint4* __restrict__ a, const uint4* __restrict_
     o[i] = pack8(f);
   }
 }
-__global__ void cast_kernel(const float4* __restrict__ in, uint2* __restrict__ out, int64_t nvec,
+__global__ void cast_kernel(const float4* in, uint2* out, int64_t nvec,
                             int accumulate) {
   grid_trigger();
   grid_wait();
@@ -843,11 +857,11 @@ __global__ void cast_kernel(const float4* __restrict__ in, uint2* __restrict__ o
 // Bound by HBM: 30 bytes an element.  One step per thread in as many CTAs as that takes: 188 M elements with their norm 1040 us
 // with 2368 CTAs that walk the arrays, 995 with 9472, 957 so (6.7 TB/s); streaming hints or the order from the last element, whose
 // gradient the norm has left in L2, to the first give nothing.
-__global__ void adamw_kernel(uint2* __restrict__ param, float4* __restrict__ master,
-                             float4* __restrict__ m, float4* __restrict__ v,
-                             const void* __restrict__ grad, int grad_fp32, int64_t nvec, float lr,
+__global__ void adamw_kernel(uint2* param, float4* master,
+                             float4* m, float4* v,
+                             const void* grad, int grad_fp32, int64_t nvec, float lr,
                              float beta1, float beta2, float eps, float wd, float bc1, float bc2,
-                             const float* __restrict__ grad_scale) {
+                             const float* grad_scale) {
   grid_trigger();
   grid_wait();
   const float gs = grad_scale != nullptr ? *grad_scale : 1.0f;
@@ -884,8 +898,8 @@ __global__ void adamw_kernel(uint2* __restrict__ param, float4* __restrict__ mas
 }
 
 // The clipping factor in one launch of one thread instead of seven of a scalar each (20 us of an optimizer step).
-__global__ void clip_scale_kernel(const float* __restrict__ sq, int n, float max_norm, float* __restrict__ norm,
-                                  float* __restrict__ scale) {
+__global__ void clip_scale_kernel(const float* sq, int n, float max_norm, float* norm,
+                                  float* scale) {
   grid_trigger();
   grid_wait();
   float s = 0.f;
@@ -899,7 +913,7 @@ __global__ void clip_scale_kernel(const float* __restrict__ sq, int n, float max
 // with one atomic: the optimizer step of 188 M elements 957 -> 948 us (eight CTAs an SM 953, 128 951).
 constexpr int kSumVec = 4;
 __global__ void __launch_bounds__(256)
-sumsq_kernel(const void* __restrict__ x, int is_fp32, int64_t nvec, float* __restrict__ out) {
+sumsq_kernel(const void* x, int is_fp32, int64_t nvec, float* out) {
   grid_trigger();
   grid_wait();
   __shared__ float red[64];
@@ -1016,10 +1030,10 @@ __device__ __forceinline__ uint4 ce_grad_vector(const uint4& u, int v, int64_t t
   return pack8(f);
 }
 __global__ void __launch_bounds__(256)
-ce_partial_kernel(const __nv_bfloat16* __restrict__ logits, int64_t ld,
-                  const int64_t* __restrict__ targets, int rows, int cols, int col_offset,
-                  int vocab, float* __restrict__ row_max, float* __restrict__ row_sumexp,
-                  float* __restrict__ tgt_logit, const __grid_constant__ RowExchange ex) {
+ce_partial_kernel(const __nv_bfloat16* logits, int64_t ld,
+                  const int64_t* targets, int rows, int cols, int col_offset,
+                  int vocab, float* row_max, float* row_sumexp,
+                  float* tgt_logit, const __grid_constant__ RowExchange ex) {
   grid_trigger();
   grid_wait();
   __shared__ float red[64];
@@ -1067,10 +1081,10 @@ ce_partial_kernel(const __nv_bfloat16* __restrict__ logits, int64_t ld,
 }
 
 __global__ void __launch_bounds__(256)
-ce_grad_kernel(__nv_bfloat16* __restrict__ logits, int64_t ld, const int64_t* __restrict__ targets,
-               int rows, int cols, int col_offset, int vocab, const float* __restrict__ gmax,
-               const float* __restrict__ gsumexp, float scale, float* __restrict__ row_loss,
-               const float* __restrict__ tgt_logit, const __grid_constant__ RowExchange ex) {
+ce_grad_kernel(__nv_bfloat16* logits, int64_t ld, const int64_t* targets,
+               int rows, int cols, int col_offset, int vocab, const float* gmax,
+               const float* gsumexp, float scale, float* row_loss,
+               const float* tgt_logit, const __grid_constant__ RowExchange ex) {
   grid_trigger();
   grid_wait();
   const int nvec = cols >> 3;
@@ -1124,8 +1138,8 @@ ce_grad_kernel(__nv_bfloat16* __restrict__ logits, int64_t ld, const int64_t* __
 constexpr int kCeAhead = 4;
 constexpr int kCeRowBytes = 200 * 1024;     // most of a row that is kept
 __global__ void __launch_bounds__(512)
-ce_row_kernel(__nv_bfloat16* __restrict__ logits, int64_t ld, const int64_t* __restrict__ targets, int cols, int vocab, float scale,
-              float* __restrict__ row_loss) {
+ce_row_kernel(__nv_bfloat16* logits, int64_t ld, const int64_t* targets, int cols, int vocab, float scale,
+              float* row_loss) {
   extern __shared__ uint4 ring[];
   __shared__ float red[64];
   grid_trigger();
@@ -1178,7 +1192,7 @@ ce_row_kernel(__nv_bfloat16* __restrict__ logits, int64_t ld, const int64_t* __r
 
 // out = sum of n values over divisor, in a fixed order, by one CTA.
 __global__ void __launch_bounds__(1024)
-sum_kernel(const float* __restrict__ x, int n, float divisor, float* __restrict__ out) {
+sum_kernel(const float* x, int n, float divisor, float* out) {
   grid_trigger();
   grid_wait();
   __shared__ float red[64];
@@ -1191,28 +1205,46 @@ sum_kernel(const float* __restrict__ x, int n, float divisor, float* __restrict_
 // ------------------------------------------------------------------------------------------
 // embedding
 // ------------------------------------------------------------------------------------------
-__global__ void embedding_fwd_kernel(const int64_t* __restrict__ tokens,
-                                     const uint4* __restrict__ tok_table,
-                                     const uint4* __restrict__ pos_table, uint4* __restrict__ out,
+// Four vectors of a row in flight before the first store: 8192 tokens of width 4096 26 us with one, 24 so.
+constexpr int kEmbVec = 4;
+__global__ void embedding_fwd_kernel(const int64_t* tokens,
+                                     const uint4* tok_table,
+                                     const uint4* pos_table, uint4* out,
                                      int n_tokens, int seq, int nvec) {
   grid_trigger();
   grid_wait();
   for (int t = blockIdx.x; t < n_tokens; t += gridDim.x) {
     const int64_t tok = tokens[t];
     const int pos = t % seq;
-    for (int v = threadIdx.x; v < nvec; v += blockDim.x) {
-      float a[8], b[8];
-      unpack8(tok_table[tok * nvec + v], a);
-      unpack8(pos_table[(int64_t)pos * nvec + v], b);
+    const uint4* row = tok_table + tok * nvec;
+    const uint4* at = pos_table + (int64_t)pos * nvec;
+    for (int v0 = threadIdx.x; v0 < nvec; v0 += kEmbVec * blockDim.x) {
+      uint4 u[kEmbVec], w[kEmbVec];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) a[i] += b[i];
-      out[(int64_t)t * nvec + v] = pack8(a);
+      for (int j = 0; j < kEmbVec; ++j) {
+        const int v = v0 + j * blockDim.x;
+        if (v < nvec) {
+          u[j] = row[v];
+          w[j] = at[v];
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < kEmbVec; ++j) {
+        const int v = v0 + j * blockDim.x;
+        if (v >= nvec) continue;
+        float a[8], b[8];
+        unpack8(u[j], a);
+        unpack8(w[j], b);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) a[i] += b[i];
+        out[(int64_t)t * nvec + v] = pack8(a);
+      }
     }
   }
 }
 // token table: scatter-add with fp32 vector atomics; position table: plain sum over the batch
-__global__ void embedding_bwd_tok_kernel(const int64_t* __restrict__ tokens,
-                                         const uint4* __restrict__ dout, float* __restrict__ dtok,
+__global__ void embedding_bwd_tok_kernel(const int64_t* tokens,
+                                         const uint4* dout, float* dtok,
                                          int n_tokens, int nvec) {
   grid_trigger();
   grid_wait();
@@ -1227,7 +1259,7 @@ __global__ void embedding_bwd_tok_kernel(const int64_t* __restrict__ tokens,
     }
   }
 }
-__global__ void embedding_bwd_pos_kernel(const uint4* __restrict__ dout, float* __restrict__ dpos,
+__global__ void embedding_bwd_pos_kernel(const uint4* dout, float* dpos,
                                          int n_tokens, int seq, int nvec) {
   grid_trigger();
   grid_wait();

@@ -345,6 +345,17 @@ def test_cross_entropy_vocab_parallel():
     assert grad[:, vocab:].abs().max() == 0
 
 
+@pytest.mark.parametrize("cols", [8, 1032, 4096, 4104, 9224])
+def test_embedding_lookup_widths(cols):
+    """Rows of one vector, of a batch of vectors per thread and of a little more: the sum of two bf16, rounded once."""
+    from meshslice_b200.ops import functional as F
+    g = torch.Generator(device="cuda").manual_seed(cols)
+    tok, pos = (torch.randn(n, cols, device="cuda", generator=g).bfloat16() for n in (50, 24))
+    ids = torch.randint(0, 50, (72,), device="cuda", generator=g)
+    out = F.embedding_fwd(ids, tok, pos, 24)
+    assert torch.equal(out, (tok[ids].float() + pos.repeat(3, 1).float()).bfloat16())
+
+
 def test_embedding_fwd_bwd():
     C, st = _C()
     vocab, seq, nb, cols = 500, 16, 4, 256
