@@ -5,8 +5,8 @@
 //   into TMEM, online softmax in the log2 domain with lazy rescaling of O (only when the running
 //   maximum grows by more than 2^8), P written back over S as packed bf16 and read by O += P V as
 //   the TMEM operand.
-// Backward (attn_bwd2_kernel<key-major>, <query-major>): dK / dV are accumulated by the CTA that works on
-//   128 keys, dQ by the CTA that works on 128 queries; both recompute S and dP, keep P and dS in TMEM,
+// Backward (attn_bwd2_kernel): dK / dV are accumulated by the CTA that works
+//   on 128 keys, dQ by the CTA that works on 128 queries; both recompute S and dP, keep P and dS in TMEM,
 //   and never add to global memory: the gradients are bit-identical from run to run.
 // All waits are bounded; a timeout records a code in `status` and the CTA leaves.
 #include "attention.h"
@@ -608,7 +608,7 @@ attn_delta_kernel(const uint4* out, const uint4* dout, float* delta,
                   uint32_t groups, uint32_t seq, uint32_t heads, const float* lse, float* lse2,
                   float scale) {
   grid_wait();
-  grid_trigger();                        // the key-major kernel may start: what it reads before its own wait is complete
+  grid_trigger();
   const uint32_t sub = threadIdx.x & 15;
   const uint32_t w = blockIdx.x * (blockDim.x >> 4) + (threadIdx.x >> 4);   // (group of tokens, head)
   const bool live = w < groups;
@@ -652,11 +652,11 @@ attn_delta_kernel(const uint4* out, const uint4* dout, float* delta,
 }
 
 // ==========================================================================================
-// backward: two deterministic kernels, P / dS stay in tensor memory
+// backward: deterministic, P / dS stay in tensor memory
 // ==========================================================================================
 // The gradient is split by who accumulates it:
-//   attn_bwd2_kernel<true>   an item is 128 KEYS, whose CTA walks the query blocks and accumulates dV, dK in TMEM
-//   attn_bwd2_kernel<false>  an item is 128 QUERIES, whose CTA walks the key blocks and accumulates dQ in TMEM
+//   key-major    an item is 128 KEYS, whose CTA walks the query blocks and accumulates dV, dK in TMEM
+//   query-major  an item is 128 QUERIES, whose CTA walks the key blocks and accumulates dQ in TMEM
 // Both recompute S and dP (7 products per block pair instead of 5), but nothing is ever added to
 // global memory: no fp32 dQ buffer, no memset, no atomics, and the result is bit-identical from run
 // to run.  P and dS are written back over S and dP as packed bf16 and feed the gradient products
@@ -694,7 +694,8 @@ constexpr int kBwdCols = kBlk * 4 / kBwdWarps;   // columns of a row per element
 constexpr int kBwdStage = 32 * kBwdCols * 2;     // output staging per element-wise warp
 constexpr int kStatBytes = kBlk * 4;        // lse2 or delta of 128 queries
 constexpr int kBwdAlignSlack = 256;
-constexpr size_t kBwd2Smem = 7 * kTile + 5 * kStatBytes + 256 + kBwdAlignSlack;
+constexpr size_t kBwdBars = 7 * kTile + 5 * kStatBytes;   // where the barriers are
+constexpr size_t kBwd2Smem = kBwdBars + 256 + kBwdAlignSlack;
 static_assert(kBwdWarps * kBwdStage == kTile, "an item's staged output takes the place of a tile");
 static_assert(kBwd2Smem <= 232448, "shared memory of a CTA");
 constexpr int kBwd2Threads = 96 + 32 * kBwdWarps;
@@ -702,6 +703,8 @@ constexpr int kBwd2Threads = 96 + 32 * kBwdWarps;
 struct Bwd2Args {
   const float* lse2;    // -lse * log2(e)          (written by attn_delta_kernel)
   const float* delta;   // -rowsum(dO * O) * scale (written by attn_delta_kernel)
+  uint32_t items;       // item i < items is key-major, items + i query-major
+  int group;            // batch-heads of a block-order group
   int batch, seq, heads, causal;
   float scale;
   uint32_t* status;
@@ -712,35 +715,30 @@ struct BwdItem {
   int b, h, blk, i0, n_it;   // sequence, head, owned block, first streamed block, streamed blocks
 };
 template <bool kKeyMajor>
-__device__ __forceinline__ BwdItem bwd_item(const Bwd2Args& a, uint32_t x, uint32_t y, uint32_t z, int group) {
+__device__ __forceinline__ BwdItem bwd_item(const Bwd2Args& a, uint32_t item) {
   BwdItem w;
-  const int bh = (int)z * group + (int)x, nblk = a.seq / kBlk;
+  const uint32_t nblk = (uint32_t)a.seq / kBlk, i = kKeyMajor ? item : item - a.items, row = i / (uint32_t)a.group;
+  const int bh = (int)(row / nblk) * a.group + (int)(i - row * (uint32_t)a.group), y = (int)(row % nblk);
   w.b = bh / a.heads;
   w.h = bh - w.b * a.heads;
   // same block order as the forward kernel: per group of batch-heads the longest tiles first (key block 0 / the
   // last query block stream the most); queries i0 .. nblk-1 for a key block, keys 0 .. blk for a query block
-  w.blk = kKeyMajor ? (int)y : (a.causal ? nblk - 1 - (int)y : (int)y);
+  w.blk = kKeyMajor || !a.causal ? y : (int)nblk - 1 - y;
   w.i0 = kKeyMajor && a.causal ? w.blk : 0;
-  w.n_it = kKeyMajor ? nblk - w.i0 : (a.causal ? w.blk + 1 : nblk);
+  w.n_it = kKeyMajor ? (int)nblk - w.i0 : (a.causal ? w.blk + 1 : (int)nblk);
   return w;
 }
 
+// A CTA's run of items of one kind, from `item` on, until cluster launch control has none left or one of the other kind (the
+// response stays in shared memory).  False after a timeout.  At its end every copy and every tcgen05 operation has arrived
+// where it was announced, so the barriers can be set up anew for the next run.
 // kKeyMajor = true:  resident tiles K, V (this item's 128 keys), streamed Q, dO; accumulators dV, dK.
 //                    TMEM lanes = keys, columns = queries: lse / delta vary along the columns.
 // kKeyMajor = false: resident tiles Q, dO (this item's 128 queries), streamed K, V; accumulator dQ.
 //                    TMEM lanes = queries, columns = keys: lse / delta are per thread.
 template <bool kKeyMajor>
-__global__ void __launch_bounds__(kBwd2Threads, 1)
-attn_bwd2_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constant__ CUtensorMap tm_do,
-                 const __grid_constant__ CUtensorMap tm_dqkv, const __grid_constant__ Bwd2Args a) {
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
-                                             ~static_cast<uintptr_t>(1023));
-  // the base is 1024-byte aligned in practice; there is no room for the full slack of an arbitrary one
-  if (smem - smem_raw > kBwdAlignSlack) {
-    if (threadIdx.x == 0) report(a.status, kErrAttn + 10, 0, 0);
-    return;
-  }
+__device__ __forceinline__ bool attn_bwd2_run(const CUtensorMap& tm_qkv, const CUtensorMap& tm_do, const CUtensorMap& tm_dqkv,
+                                              const Bwd2Args& a, uint8_t* smem, uint32_t tmem, uint32_t item) {
   uint8_t* sR0 = smem;                      // resident: K (key-major) or Q
   uint8_t* sR1 = smem + kTile;              // resident: V (key-major) or dO
   // Streamed tiles, a ring each.  Q / K is read by the first and the last product of a block, dO (key-major) by the
@@ -751,7 +749,7 @@ attn_bwd2_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_consta
   // key-major: lse2 travels with Q, delta with dO.  delta(i+2) takes the slot of delta(i): its producer waits for dS(i).
   float* sLse = reinterpret_cast<float*>(smem + 7 * kTile);   // [3][128]
   float* sDelta = sLse + 3 * kBlk;                            // [2][128]
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + 7 * kTile + 5 * kStatBytes);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kBwdBars);   // up to 30: the tensor-memory address is behind them
   uint8_t* clc_resp = reinterpret_cast<uint8_t*>(bars);   // 16 bytes
   uint64_t* clc_full = bars + 2;
   uint64_t* clc_empty = bars + 3;
@@ -768,15 +766,11 @@ attn_bwd2_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_consta
   uint64_t* p_ready = bars + 24;            // [2] key-major: the first / second 16 columns of every warp's P^T
   uint64_t* acc_done = bars + 26;           // [2] key-major: dV / dK; query-major: [1] dQ
   uint64_t* out_read = bars + 28;           // [2] the copy engine has read the output staged in a stage of ring 1
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 30);
 
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
-  const int group = gridDim.x;
   const uint64_t tmo = a.timeout_ns;
 
   if (threadIdx.x == 0) {
-    tma_prefetch_desc(&tm_qkv);
-    tma_prefetch_desc(&tm_do);
     mbar_init(clc_full, 1);
     mbar_init(clc_empty, 3 + kBwdWarps);    // producers and MMA thread, element-wise warps
     for (int i = 0; i < 3; ++i) {
@@ -798,14 +792,7 @@ attn_bwd2_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_consta
     }
     mbar_fence_init();
   }
-  if (warp == 1) {
-    tmem_alloc(tmem_slot, 512);
-    tmem_relinquish();
-  }
-  tc_fence_before_sync();
   __syncthreads();
-  tc_fence_after_sync();
-  const uint32_t tmem = *tmem_slot;
   // key-major:   S^T [0,128)  dP^T [128,256)  dV [256,384)  dK [384,512)
   // query-major: S [0,128)  dP buffers [128,256) [256,384)  dQ [384,512)
   const uint32_t t_dp = tmem + 128;
@@ -813,19 +800,21 @@ attn_bwd2_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_consta
   const auto dp_phase = [](uint32_t q) -> uint32_t { return (kKeyMajor ? q : q >> 1) & 1; };
   const uint32_t t_acc0 = tmem + (kKeyMajor ? 256 : 384), t_acc1 = tmem + 384;
 
-  BwdItem w = bwd_item<kKeyMajor>(a, blockIdx.x, blockIdx.y, blockIdx.z, group);
-  // The next item as the producer got it: false when there is none (or on a timeout).
+  BwdItem w = bwd_item<kKeyMajor>(a, item);
+  bool ok = true;
+  // The next item as the producer got it: false when there is none of this kind (or on a timeout).
   uint32_t items = 0;                       // items finished by this thread
   auto next_item = [&]() -> bool {
     uint32_t x, y, z;
     if (!mbar_wait(clc_full, items & 1, 8 * tmo)) {
       report(a.status, kErrAttn + 18, items, 0);
+      ok = false;
       return false;
     }
     ++items;
-    const bool more = clc_read(clc_resp, x, y, z);
+    const bool more = clc_read(clc_resp, x, y, z) && (x < a.items) == kKeyMajor;
     fence_proxy_async_smem();               // this read before the next response overwrites it
-    if (more) w = bwd_item<kKeyMajor>(a, x, y, z, group);
+    if (more) w = bwd_item<kKeyMajor>(a, x);
     return more;
   };
   uint32_t g = 0;                           // streamed blocks so far: stages and phases of the rings and the hand-overs
@@ -833,7 +822,7 @@ attn_bwd2_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_consta
   if (warp == 0) {
     // resident tile of S, ring of Q or K, next items
     if (elect_one()) {
-      bool ok = true, more = true;
+      bool more = true;
       while (ok && more) {
         const int colq = w.h * 3 * kD, seq0 = w.b * a.seq, rrow = seq0 + w.blk * kBlk;
         const int64_t stat0 = ((int64_t)w.b * a.heads + w.h) * a.seq;
@@ -850,13 +839,7 @@ attn_bwd2_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_consta
           if (!(ok = mbar_wait(empty0 + st, ((g / kRing0) & 1) ^ 1, 8 * tmo))) break;
           mbar_expect_tx(full0 + st, kTile + (kKeyMajor ? kStatBytes : 0));
           load_tile(sS0 + st * kTile, &tm_qkv, full0 + st, kKeyMajor ? colq : colq + kD, seq0 + srow);
-          if (kKeyMajor) {
-            if (g == 0) {
-              grid_wait();                    // the statistics are written (every read of them here comes after this or the
-              grid_trigger();                 // other producer's wait); then the query-major kernel may start on free SMs
-            }
-            bulk_g2s(sLse + st * kBlk, a.lse2 + stat0 + srow, kStatBytes, full0 + st);
-          }
+          if (kKeyMajor) bulk_g2s(sLse + st * kBlk, a.lse2 + stat0 + srow, kStatBytes, full0 + st);
           ++g;
         }
         if (ok && (ok = mbar_wait(clc_empty, (items & 1) ^ 1, 8 * tmo))) {
@@ -867,11 +850,13 @@ attn_bwd2_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_consta
         }
         if (!ok) report(a.status, kErrAttn + 11, w.blk, g);
       }
+      for (uint32_t q = g; q < g + kRing0 && ok; ++q) ok = mbar_wait(empty0 + q % kRing0, ((q / kRing0) & 1) ^ 1, 8 * tmo);
+      ok = ok && mbar_wait(res_empty, (items & 1) ^ 1, 8 * tmo);
     }
   } else if (warp == 2 + kBwdWarps) {
     // resident tile of dP, ring of dO or V: by a thread of its own, because a stage of one ring is often free long before one of the other
     if (elect_one()) {
-      bool ok = true, more = true;
+      bool more = true;
       uint32_t outs[2] = {0, 0};              // outputs staged in either stage so far
       bool staged[2] = {false, false};        // the last user of the stage was an item's output
       while (ok && more) {
@@ -892,7 +877,6 @@ attn_bwd2_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_consta
           if (kKeyMajor) {
             load_tile(sS1 + st * kTile, &tm_do, full1 + st, w.h * kD, seq0 + srow);                                // dO
             if (g > 1 && !(ok = mbar_wait(ds_ready + st, ((g - 2) >> 1) & 1, 8 * tmo))) break;
-            if (g == 0) grid_wait();
             bulk_g2s(sDelta + st * kBlk, a.delta + stat0 + srow, kStatBytes, full1 + st);
           } else {
             load_tile(sS1 + st * kTile, &tm_qkv, full1 + st, w.h * 3 * kD + 2 * kD, seq0 + srow);                  // V
@@ -910,6 +894,8 @@ attn_bwd2_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_consta
           report(a.status, kErrAttn + 11, w.blk, g);
         }
       }
+      for (uint32_t q = g; q < g + kRing1 && ok; ++q) ok = mbar_wait(empty1 + q % kRing1, ((q / kRing1) & 1) ^ 1, 8 * tmo);
+      ok = ok && mbar_wait(res_empty + 1, (items & 1) ^ 1, 8 * tmo);
     }
   } else if (warp == 1) {
     if (elect_one()) {
@@ -920,7 +906,7 @@ attn_bwd2_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_consta
       const uint64_t ds0k = desc_kmajor(smem_u32(sS0), 0), ds1k = desc_kmajor(smem_u32(sS1), 0);
       const uint64_t ds0m = desc_mnmajor(smem_u32(sS0), 0), ds1m = desc_mnmajor(smem_u32(sS1), 0);
       constexpr uint64_t kStageOff = (uint64_t)(kTile >> 4);
-      bool ok = true, more = true;
+      bool more = true;
       auto wait = [&](uint64_t* bar, uint32_t parity, uint32_t code) -> bool {
         if (mbar_wait(bar, parity, 8 * tmo)) {
           tc_fence_after_sync();
@@ -1026,7 +1012,7 @@ attn_bwd2_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_consta
     const int row = q4 * 32 + lane;                       // TMEM lane: key (key-major) or query
     const uint32_t lane_off = static_cast<uint32_t>(q4 * 32) << 16;
     const uint64_t sl2 = f32x2(a.scale * kLog2e, a.scale * kLog2e), sc2 = f32x2(a.scale, a.scale);
-    bool ok = true, more = true;
+    bool more = true;
     while (more) {
       const int me = w.blk * kBlk + row;                  // query-major: this lane's query
       const int me0 = w.blk * kBlk + q4 * 32 + (lane >> 2);   // key-major: the first of this thread's keys
@@ -1194,14 +1180,67 @@ attn_bwd2_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_consta
       __syncwarp();                              // every lane has read the response
       if (lane == 0) mbar_arrive(clc_empty);
     }
-    if (lane == 0) bulk_wait_all<0>();
+  }
+  tc_fence_before_sync();
+  const bool all = __syncthreads_and(ok) != 0;
+  tc_fence_after_sync();
+  if (threadIdx.x == 0 && all)
+    for (int i = 2; i < 30; ++i) mbar_inval(bars + i);
+  return all;
+}
+
+// A grid of key-major items, of query-major ones, or of both, all key-major items first: there query-major items, which need
+// nothing of those, take SMs as they get free, and every CTA has waited for the row sums (and so for all that came before them
+// in the stream) before it reads anything.  (Of two launches that overlap by programmatic dependence the second cannot wait for
+// the row sums alone.)  A CTA of both kinds changes when cluster launch control gives it an item of the other one, in that
+// order at most once; nothing depends on that.
+template <bool kKey, bool kQuery>
+__global__ void __launch_bounds__(kBwd2Threads, 1)
+attn_bwd2_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constant__ CUtensorMap tm_do,
+                 const __grid_constant__ CUtensorMap tm_dqkv, const __grid_constant__ Bwd2Args a) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
+                                             ~static_cast<uintptr_t>(1023));
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+  // the base is 1024-byte aligned in practice; there is no room for the full slack of an arbitrary one
+  if (smem - smem_raw > kBwdAlignSlack) {
+    grid_wait();
+    if (threadIdx.x == 0) report(a.status, kErrAttn + 10, 0, 0);
+    return;
+  }
+  uint8_t* clc_resp = smem + kBwdBars;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + kBwdBars + 30 * 8);
+  if (warp == 1) {
+    tmem_alloc(tmem_slot, 512);
+    tmem_relinquish();
+  }
+  if (threadIdx.x == 0) {
+    tma_prefetch_desc(&tm_qkv);
+    tma_prefetch_desc(&tm_do);
   }
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
+  const uint32_t tmem = *tmem_slot;
+  grid_wait();
+
+  if (kKey && kQuery) {
+    uint32_t item = blockIdx.x, y, z;
+    bool more = true;
+    while (more) {
+      const bool ok = item < a.items ? attn_bwd2_run<true>(tm_qkv, tm_do, tm_dqkv, a, smem, tmem, item)
+                                     : attn_bwd2_run<false>(tm_qkv, tm_do, tm_dqkv, a, smem, tmem, item);
+      more = ok && clc_read(clc_resp, item, y, z);
+      fence_proxy_async_smem();             // this read before the next response overwrites it
+    }
+  } else {
+    attn_bwd2_run<kKey>(tm_qkv, tm_do, tm_dqkv, a, smem, tmem, blockIdx.x);
+  }
+  if (warp >= 2 && warp < 2 + kBwdWarps && lane == 0) bulk_wait_all<0>();
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
   if (warp == 1) tmem_dealloc(tmem, 512);
-  // What follows in the stream waits for this grid alone: it ends after the key-major one, whose blocks all run or are done.
-  if (!kKeyMajor && threadIdx.x == 0) grid_wait();
 }
 
 // The shared-memory attribute is per device: set it once on every device that launches.
@@ -1213,10 +1252,10 @@ cudaError_t configure_device() {
   if (dev >= 0 && dev < 64 && configured[dev]) return cudaSuccess;
   e = cudaFuncSetAttribute(attn_fwd2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFwd2Smem);
   if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(attn_bwd2_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBwd2Smem);
-  if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(attn_bwd2_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBwd2Smem);
-  if (e != cudaSuccess) return e;
+  for (auto kernel : {attn_bwd2_kernel<true, true>, attn_bwd2_kernel<true, false>, attn_bwd2_kernel<false, true>}) {
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBwd2Smem);
+    if (e != cudaSuccess) return e;
+  }
   if (dev >= 0 && dev < 64) configured[dev] = true;
   return cudaSuccess;
 }
@@ -1282,6 +1321,8 @@ cudaError_t attention_bwd(const void* qkv, const void* out, const void* dout, co
   const auto off = [](const void* p, uintptr_t align) { return (reinterpret_cast<uintptr_t>(p) & (align - 1)) != 0; };
   if (off(qkv, 16) || off(dout, 16) || off(dqkv, 16) || off(out, 8) || off(dq_acc, 16) || off(delta, 16))
     return cudaErrorInvalidValue;
+  const int64_t items = (int64_t)batch * heads * (seq / kBlk);   // 256 KiB of tensors each
+  if (items > 1 << 29) return cudaErrorInvalidValue;
   {
     cudaError_t e0 = configure_device();
     if (e0 != cudaSuccess) return e0;
@@ -1304,21 +1345,25 @@ cudaError_t attention_bwd(const void* qkv, const void* out, const void* dout, co
                                            (uint32_t)heads, lse, dq_acc, scale);
     if (e != cudaSuccess) return e;
   }
-  // two deterministic kernels: dK / dV per key block, dQ per query block
+  // dK / dV per key block, dQ per query block
   Bwd2Args g{};
   g.lse2 = dq_acc;     // -lse * log2(e)
   g.delta = delta;     // -delta * scale
+  g.items = (uint32_t)items;
+  g.group = bh_group(batch, heads);
   g.batch = batch; g.seq = seq; g.heads = heads; g.causal = causal;
   g.scale = scale;
   g.status = status;
   g.timeout_ns = 2000000000ull;
-  const int grp = bh_group(batch, heads);
-  // Overlap of the three launches: the key-major kernel sets up and loads its first tiles while the row sums end, the
-  // query-major one, which reads nothing of it, takes SMs as they get free (batch 3 x 640, 5 heads: 75 items each).
-  const dim3 grid2(grp, seq / kBlk, batch * heads / grp);
-  cudaError_t e = launch_dependent(attn_bwd2_kernel<true>, grid2, kBwd2Threads, kBwd2Smem, stream, tq, td, tg, g);
+  // One launch of both kinds where one kind leaves SMs free, two beyond: the kernel of both is slower by 4 % (96 registers).
+  // Backward, two / one, us: batch 3 x 640, 5 heads (75 items) 35.5 / 27.5, 1 x 4096, 4 heads, causal (128) 92 / 63, 2 x 1024,
+  // 8 heads (128) 34 / 25.6; 1 x 8192, 4 heads (256) 180 / 183, 1 x 4096, 16 heads (512) 191 / 198, 4 x 2048, 32 heads (2048)
+  // 437 / 453, full 809 / 854.
+  if (items <= sm_count()) return launch_dependent(attn_bwd2_kernel<true, true>, 2 * (unsigned)items, kBwd2Threads, kBwd2Smem, stream, tq, td, tg, g);
+  const cudaError_t e = launch_dependent(attn_bwd2_kernel<true, false>, (unsigned)items, kBwd2Threads, kBwd2Smem, stream, tq, td, tg, g);
   if (e != cudaSuccess) return e;
-  return launch_dependent(attn_bwd2_kernel<false>, grid2, kBwd2Threads, kBwd2Smem, stream, tq, td, tg, g);
+  g.items = 0;
+  return launch_dependent(attn_bwd2_kernel<false, true>, (unsigned)items, kBwd2Threads, kBwd2Smem, stream, tq, td, tg, g);
 }
 
 }  // namespace msb

@@ -65,3 +65,23 @@ def test_dependent_launches_wait(path):
     assert launched or "auto kernel" in text
     for name in launched:
         assert "grid_wait()" in kernels[name][1], name
+
+
+@pytest.mark.parametrize("path", SOURCES, ids=lambda p: p.name)
+def test_dependent_kernels_wait_before_they_touch_memory(path):
+    """A grid sees the writes of the grids before it only after a wait of its own: one that every thread comes to, with no load
+    or copy in front of it and no other wait that a kernel's order could rest on."""
+    text = _code(path)
+    for name, (_, body) in functions(text, "__device__").items():
+        assert "grid_wait()" not in body, name
+    for name, (_, body) in functions(text, "__global__").items():
+        if "grid_wait()" not in body:
+            continue
+        waits = []
+        for m in re.finditer(r"grid_wait\(\);", body):
+            before = body[:m.start()]
+            leads = re.search(r"[;{}]\s*$", before) is not None          # a statement of its own, not the branch of an if
+            if leads and before.count("{") - before.count("}") == 1:
+                waits.append(before)
+        assert len(waits) == 1, name
+        assert not re.search(r"load_tile|bulk_g2s|tma_load|cp_async16|__ldcs|ld_stream", waits[0]), name

@@ -214,3 +214,23 @@ def test_attention_backward_launches_in_order(shape):
     _native.check_status()
     for i, t in enumerate(got):
         assert torch.equal(t, sets[i % 3][4]), i
+
+
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("shape", [(1, 128, 1), (2, 1152, 8), (7, 2688, 1), (37, 512, 1), (148, 128, 1)])
+def test_attention_backward_of_both_kinds_in_one_launch(shape, causal):
+    """Up to as many items as SMs, dK / dV and dQ are one launch, whose CTAs change from one kind to the other (items of one to
+    21 blocks, ring stages left at every phase); the same sequences twice are two launches.  Bits do not depend on it."""
+    from meshslice_b200 import _native
+    from meshslice_b200.ops import functional as F
+    batch, seq, heads = shape
+    g = torch.Generator(device="cuda").manual_seed(seq)
+    qkv = torch.randn(batch * seq, heads * 3 * 128, device="cuda", generator=g).bfloat16()
+    dout = torch.randn(batch * seq, heads * 128, device="cuda", generator=g).bfloat16()
+    copies = 149 // (batch * heads * (seq // 128)) + 1
+    out, lse = F.attention_fwd(qkv, batch, seq, heads, causal)
+    dqkv = F.attention_bwd(dout, qkv, out, lse, batch, seq, heads, causal)
+    many = lambda t: torch.cat([t] * copies)
+    want = F.attention_bwd(many(dout), many(qkv), many(out), many(lse), copies * batch, seq, heads, causal)
+    _native.check_status()
+    assert torch.isfinite(dqkv).all() and torch.equal(want, many(dqkv))
