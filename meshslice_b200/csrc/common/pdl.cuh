@@ -9,8 +9,10 @@
 namespace msb {
 
 // Wait until the grids before this one in the stream are complete and their writes visible / let the next grid start once every
-// block of this one has come here or left.  Without the launch attribute both do nothing.  Every block of a grid launched with
-// launch_dependent() waits, before it touches memory that an earlier grid may use: then what follows this grid follows those too.
+// block of this one has come here or left.  In a grid that was launched plainly the wait does nothing, but the trigger counts:
+// a kernel of a row exchange does not come to it, or what follows would take SMs while it waits for other GPUs.  Every block of a
+// grid launched with launch_dependent() waits, before it touches memory that an earlier grid may use: then what follows this grid
+// follows those too.
 // Such a kernel runs while its inputs are still being written, so none of its pointers is __restrict__: a const one would let
 // the compiler load through the non-coherent path, or take a load for invariant and move it over the wait.
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

@@ -346,7 +346,7 @@ ln_bwd_kernel(int mode, const uint4* dy, const uint4* h,
               const uint4* dres, uint4* dx, float* stats,
               float* dgamma, float* dbeta, int rows, int cols,
               int total_cols, int tpr_arg, const __grid_constant__ RowExchange ex) {
-  grid_trigger();
+  if (ex.n == 0) grid_trigger();
   grid_wait();
   static_assert(!GROUPED || MAXV == 1, "grouped rows are one vector per thread");
   constexpr bool kKeep = MAXV == 2;      // what both passes over a row need stays in registers where there is room for it
@@ -1034,7 +1034,7 @@ ce_partial_kernel(const __nv_bfloat16* logits, int64_t ld,
                   const int64_t* targets, int rows, int cols, int col_offset,
                   int vocab, float* row_max, float* row_sumexp,
                   float* tgt_logit, const __grid_constant__ RowExchange ex) {
-  grid_trigger();
+  if (ex.n == 0) grid_trigger();
   grid_wait();
   __shared__ float red[64];
   const int valid = max(0, min(cols, vocab - col_offset));
@@ -1085,7 +1085,7 @@ ce_grad_kernel(__nv_bfloat16* logits, int64_t ld, const int64_t* targets,
                int rows, int cols, int col_offset, int vocab, const float* gmax,
                const float* gsumexp, float scale, float* row_loss,
                const float* tgt_logit, const __grid_constant__ RowExchange ex) {
-  grid_trigger();
+  if (ex.n == 0) grid_trigger();
   grid_wait();
   const int nvec = cols >> 3;
   const int64_t valid = (int64_t)vocab - col_offset;       // columns before the padding

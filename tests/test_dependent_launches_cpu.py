@@ -85,3 +85,11 @@ def test_dependent_kernels_wait_before_they_touch_memory(path):
                 waits.append(before)
         assert len(waits) == 1, name
         assert not re.search(r"load_tile|bulk_g2s|tma_load|cp_async16|__ldcs|ld_stream", waits[0]), name
+
+
+@pytest.mark.parametrize("path", SOURCES, ids=lambda p: p.name)
+def test_kernels_of_a_row_exchange_do_not_let_the_next_one_start(path):
+    """A trigger counts in a plainly launched grid too: the next kernel would hold SMs while this one waits for other GPUs."""
+    for name, (params, body) in functions(_code(path), "__global__").items():
+        if "RowExchange" in params and "grid_trigger()" in body:
+            assert body.count("grid_trigger()") == body.count("if (ex.n == 0) grid_trigger();") == 1, name
