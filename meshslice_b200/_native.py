@@ -71,18 +71,27 @@ def _init_cuda():
     _cuda = torch._C
 
 
+def _block_here(t) -> bool:
+    """One block of memory on the current GPU, whose current stream a clear may go to."""
+    if not (t.is_cuda and t.is_contiguous()):
+        return False
+    if _cuda is None:
+        _init_cuda()
+    return t.get_device() == _cuda._cuda_getDevice()
+
+
 def zero_(t) -> None:
-    """``t.zero_()`` without the tensor library's dispatch where the memory is one block on a GPU."""
-    if t.is_cuda and t.is_contiguous():
+    """``t.zero_()`` without the tensor library's dispatch where the memory is one block on the current GPU."""
+    if _block_here(t):
         load().memset_zero(t.data_ptr(), t.numel() * t.element_size(), stream_ptr())
     else:
         t.zero_()
 
 
 def zero_both_(a, b) -> None:
-    """``zero_`` of two tensors, in one launch where ``b`` follows ``a`` without a gap in the same GPU memory block."""
+    """``zero_`` of two tensors, in one launch where ``b`` follows ``a`` without a gap in the same block of the current GPU's memory."""
     n = a.numel() * a.element_size()
-    if (a.is_cuda and b.is_cuda and a.is_contiguous() and b.is_contiguous() and b.data_ptr() == a.data_ptr() + n
+    if (_block_here(a) and _block_here(b) and b.data_ptr() == a.data_ptr() + n
             and a.untyped_storage().data_ptr() == b.untyped_storage().data_ptr()):
         load().memset_zero(a.data_ptr(), n + b.numel() * b.element_size(), stream_ptr())
     else:
