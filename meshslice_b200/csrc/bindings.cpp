@@ -365,6 +365,9 @@ void gemm_pair(const std::array<int64_t, 30>& v) {
   if (gelu_pre != 0 && (o[1].c_fp32 || o[1].accumulate)) throw std::runtime_error("gemm_pair: gelu_pre needs a plain bf16 result");
   if (!two_cta_default()) {
     if (gelu_pre != 0 && o[1].ldc != o[1].N) throw std::runtime_error("gemm_pair: gelu_pre needs a contiguous result");
+    // gelu_bwd reads and writes 16 bytes at a time
+    if (gelu_pre != 0 && ((gelu_pre | reinterpret_cast<uintptr_t>(o[1].C)) & 15))
+      throw std::runtime_error("gemm_pair: gelu_pre and the result need 16-byte aligned bases in the one-CTA form");
     for (const Gemm2Operands& p : o) run_gemm1(p, sms, status, stream);
     if (gelu_pre != 0) check(gelu_bwd(o[1].C, P<void>(gelu_pre), o[1].C, o[1].M * o[1].N, S(stream)), "gelu_bwd");
     return;

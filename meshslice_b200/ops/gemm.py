@@ -7,6 +7,8 @@ descriptors select the major-ness.
 """
 from __future__ import annotations
 
+import os
+
 import torch
 
 from .. import _native
@@ -82,6 +84,8 @@ def gemm_pair(a0, b0, layout0, out0, accumulate0, a1, b1, layout1, out1=None, ac
             if not out1.is_contiguous():
                 raise ValueError("gelu_pre needs a contiguous output")
             gelu_pre = gelu_pre.contiguous()
+        if gelu_pre.data_ptr() % 16 and os.environ.get("MSB_TWO_CTA") == "0":
+            gelu_pre = gelu_pre.clone()      # a kernel of its own reads it there, 16 bytes at a time
         pre = gelu_pre.data_ptr()
     _native.load().gemm_pair(*v0, *v1, _SM_COUNT.get(a0.device.index) or sm_count(a0.device), _native.status().dev,
                              _native.stream_ptr(), pre)

@@ -315,3 +315,25 @@ def test_gemm_pair_times_gelu_derivative(shape, dataflow, offset):
     assert torch.equal(torch.isnan(got), torch.isnan(want)) and torch.isnan(want[5]).any()
     ok = ~torch.isnan(want)
     assert ((got[ok].float() - want[ok].float()).norm() / want[ok].float().norm()).item() < 2 ** -8
+
+
+@pytest.mark.parametrize("offset", [0, 3])
+def test_gemm_pair_times_gelu_derivative_with_the_one_cta_kernel(offset, monkeypatch):
+    """MSB_TWO_CTA=0: the products one by one and the derivative by the stand-alone kernel, which reads 16 bytes at a time: a
+    pre-activation that starts elsewhere gives the same bits.  Two bf16 roundings of the result (2^-9 each)."""
+    from meshslice_b200 import _native
+    from meshslice_b200.ops.gemm import gemm_pair
+    monkeypatch.setenv("MSB_TWO_CTA", "0")
+    t, d, f = 264, 136, 520
+    g = torch.Generator(device="cuda").manual_seed(f)
+    rand = lambda *s: torch.randn(s, device="cuda", generator=g).bfloat16()
+    x, dy, w, pre = rand(t, f), rand(t, d), rand(f, d), rand(t, f) * 2
+    moved = torch.empty(t * f + offset, device="cuda", dtype=torch.bfloat16)[offset:].view(t, f).copy_(pre)
+    assert moved.data_ptr() % 16 == 2 * offset
+    both = lambda p: gemm_pair(x, dy, "tn", torch.zeros(w.shape, device="cuda"), True, dy, w, "nt", gelu_pre=p)
+    got, want = both(moved), both(pre)
+    _native.check_status()
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+    xr = pre.float().requires_grad_(True)
+    torch.nn.functional.gelu(xr, approximate="tanh").backward(_ref(dy, w, "nt"))
+    assert ((got[1].float() - xr.grad).norm() / xr.grad.norm()).item() < 2 ** -8
