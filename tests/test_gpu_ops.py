@@ -614,3 +614,16 @@ def test_cross_entropy_of_whole_rows(rows, cols, vocab):
     lb = F.ce_grad_loss_(b, t, 0, vocab, *F.ce_partial(b, t, 0, vocab), 0.25)
     assert torch.equal(torch.isnan(la), torch.isnan(lb)) and torch.equal(torch.isnan(a), torch.isnan(b))
     assert torch.equal(torch.isinf(la), torch.isinf(lb))
+
+
+def test_a_refused_launch_leaves_no_error_for_the_next_call():
+    """No rows are a launch of no blocks, which the host refuses.  The next call, launched plainly and so asking for the last
+    error behind it, is not answered with that of the one before."""
+    from meshslice_b200.ops import functional as F
+    x = torch.randn(64, 4096, device="cuda").bfloat16()
+    t = torch.zeros(0, dtype=torch.int64, device="cuda")
+    want = F.ln_stats(x, None)[1]
+    for _ in range(2):
+        with pytest.raises(RuntimeError, match="ce_partial"):
+            F.ce_partial(x[:0], t, 0, 4096)
+        assert torch.equal(F.ln_stats(x, None)[1], want)
