@@ -1492,8 +1492,13 @@ cudaError_t ln_bwd(int mode, const void* dy, const void* h, const void* gamma,
   auto DX = reinterpret_cast<uint4*>(dx);
   const LnRowShape rs = ln_bwd_row_shape(rows, cols, DR != nullptr);
   const bool sums = dgamma != nullptr;
+  // dx may be written over dy or h: the second look would find it there
+  const auto over = [&](const void* p) {
+    const uintptr_t a = reinterpret_cast<uintptr_t>(p), b = reinterpret_cast<uintptr_t>(dx), n = 2 * (uintptr_t)rows * cols;
+    return a < b + n && b < a + n;
+  };
   if (exch == nullptr && mode == 0 && total_cols == cols && (sums || dbeta == nullptr) && rs.w > 0 && rows > 0 &&
-      (!sums || ln_sums_from_second_look(rows, cols, DR != nullptr))) {
+      (!sums || (ln_sums_from_second_look(rows, cols, DR != nullptr) && !over(dy) && !over(h)))) {
     return with_row_shape(rs, [&](auto v, auto w) {
       constexpr int T = 32 * ln_row_warps(w.value), per = ln_row_warps(w.value) / w.value;
       // column sums: at least 128 CTAs, and no more than eight steps of T rows for one

@@ -627,3 +627,31 @@ def test_a_refused_launch_leaves_no_error_for_the_next_call():
         with pytest.raises(RuntimeError, match="ce_partial"):
             F.ce_partial(x[:0], t, 0, 4096)
         assert torch.equal(F.ln_stats(x, None)[1], want)
+
+
+@pytest.mark.parametrize("over", ["dy", "h"])
+@pytest.mark.parametrize("cols,rows", [(264, 4099), (2048, 4099), (4096, 3000)])
+def test_layernorm_backward_over_its_own_inputs(cols, rows, over):
+    """dx written over dy or h, as row by row it may be: the parameters' gradients are those of the inputs that were there.
+    Rows agree bit for bit with a dx of its own or, from another kernel, within a bf16 rounding; column sums are fp32 over
+    ``rows`` values."""
+    C, st = _C()
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    mk = lambda *s: torch.randn(*s, device="cuda", generator=g).bfloat16()
+    dy, h, gamma = mk(rows, cols), mk(rows, cols), mk(cols)
+    mr = torch.stack([h.float().mean(1), (h.float().var(1, unbiased=False) + 1e-5).rsqrt()], 1).contiguous()
+
+    def run(d, hh, out):
+        dg, db = torch.zeros(cols, device="cuda"), torch.zeros(cols, device="cuda")
+        C.ln_bwd(0, d.data_ptr(), hh.data_ptr(), gamma.data_ptr(), mr.data_ptr(), 0, out.data_ptr(), 0, dg.data_ptr(), db.data_ptr(),
+                 rows, cols, cols, st)
+        torch.cuda.synchronize()
+        return out, dg, db
+
+    want = run(dy, h, torch.empty_like(dy))
+    for _ in range(3):
+        d, hh = dy.clone(), h.clone()
+        got = run(d, hh, d if over == "dy" else hh)
+        assert ((got[0].float() - want[0].float()).abs() <= 2 ** -7 * want[0].float().abs() + 2 ** -7 * want[0].float().abs().mean()).all()
+        for a, b in zip(got[1:], want[1:]):
+            assert (a - b).abs().max() <= 3e-4 * rows ** 0.5
