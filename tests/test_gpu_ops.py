@@ -655,3 +655,81 @@ def test_layernorm_backward_over_its_own_inputs(cols, rows, over):
         assert ((got[0].float() - want[0].float()).abs() <= 2 ** -7 * want[0].float().abs() + 2 ** -7 * want[0].float().abs().mean()).all()
         for a, b in zip(got[1:], want[1:]):
             assert (a - b).abs().max() <= 3e-4 * rows ** 0.5
+
+
+def _steps(F, x, r, gamma, w, targets, rows, d):
+    """Dependent launches of every kind: LayerNorm, product, elementwise, loss, both gradients, attention."""
+    from meshslice_b200.ops.gemm import gemm, gemm_pair
+    h, y, mr = F.ln_full(x, r, gamma, None, 1e-5)
+    buf = gemm(y, w, "nn")
+    z = F.add(F.gelu(buf), h)
+    loss = F.sum_over(F.ce_loss_grad_(z, targets, d, 1.0 / rows), rows)
+    dw = torch.zeros(d, d, device="cuda")
+    _, dx = gemm_pair(y, z, "tn", dw, True, z, w, "nt", gelu_pre=buf)
+    dx = F.ln_bwd_full(dx, h, gamma, mr, None, None, z)
+    qkv = torch.cat([x, y, dx], 1)
+    out, lse = F.attention_fwd(qkv, 1, rows, d // 128, True)
+    return [loss, dw, dx, out, F.attention_bwd(dx, qkv, out, lse, 1, rows, d // 128, True)]
+
+
+def _step_inputs(rows, d):
+    g = torch.Generator(device="cuda").manual_seed(rows + d)
+    mk = lambda *s: torch.randn(*s, device="cuda", generator=g).bfloat16()
+    targets = torch.randint(0, d, (rows,), device="cuda", generator=g)
+    return [(mk(rows, d), mk(rows, d)) for _ in range(3)], mk(d), mk(d, d) / d ** 0.5, targets
+
+
+@pytest.mark.parametrize("rows,d", [(128, 128), (1024, 512)])
+def test_dependent_launches_behind_an_event_of_another_stream(rows, d):
+    """The first launch of a stream comes right behind its wait for an event of another one, which is still writing the inputs (a
+    large product in front of the copy), and the other stream overwrites them right behind an event of this one: the same bits
+    as with a synchronisation between all of it."""
+    from meshslice_b200 import _native
+    from meshslice_b200.ops import functional as F
+    inputs, gamma, w, targets = _step_inputs(rows, d)
+    want = [[t.clone() for t in _steps(F, x, r, gamma, w, targets, rows, d)] for x, r in inputs]
+    torch.cuda.synchronize()
+    one, two = torch.cuda.Stream(), torch.cuda.Stream()
+    x, r = torch.zeros_like(inputs[0][0]), torch.zeros_like(inputs[0][1])
+    busy = torch.randn(4096, 4096, device="cuda")
+    torch.cuda.synchronize()
+    got = []
+    for i in range(9):
+        with torch.cuda.stream(one):
+            torch.mm(busy, busy)
+            x.copy_(inputs[i % 3][0])
+            r.copy_(inputs[i % 3][1])
+            ready = one.record_event()
+        with torch.cuda.stream(two):
+            two.wait_event(ready)
+            got.append([t.clone() for t in _steps(F, x, r, gamma, w, targets, rows, d)])
+            done = two.record_event()
+        with torch.cuda.stream(one):
+            one.wait_event(done)
+            x.fill_(float("nan"))
+            r.fill_(float("nan"))
+    torch.cuda.synchronize()
+    _native.check_status()
+    for i, out in enumerate(got):
+        assert all(torch.equal(a, b) for a, b in zip(out, want[i % 3])), i
+
+
+@pytest.mark.parametrize("rows,d", [(128, 128), (1024, 512)])
+def test_dependent_launches_in_a_captured_graph(rows, d):
+    """The same steps captured and replayed on new inputs in the same buffers: the bits of the calls themselves."""
+    from meshslice_b200 import _native
+    from meshslice_b200.ops import functional as F
+    inputs, gamma, w, targets = _step_inputs(rows, d)
+    want = [[t.clone() for t in _steps(F, x, r, gamma, w, targets, rows, d)] for x, r in inputs]
+    torch.cuda.synchronize()
+    x, r = inputs[0][0].clone(), inputs[0][1].clone()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = _steps(F, x, r, gamma, w, targets, rows, d)
+    for i in range(9):
+        x.copy_(inputs[i % 3][0])
+        r.copy_(inputs[i % 3][1])
+        graph.replay()
+        got = [t.clone() for t in out]
+        assert all(torch.equal(a, b) for a, b in zip(got, want[i % 3])), i
+    _native.check_status()
