@@ -169,8 +169,8 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_gr
 // ------------------------------------------------------------------------------------------
 // LayerNorm forward in two passes (column-sharded rows: mode 1 statistics, mode 2 the rest; a row on one device is
 // ln_fwd_row_kernel's, below).  One CTA per row (grid-stride), row cached in registers.  Bound by HBM: it reads x (and res) and
-// writes h (with res) and y.  Both passes in one, 32768 x 4096 with residual: 240 us with loads of one row at a time, 172 us with
-// the row ring.  RING = false loads the row when it is due: ln_fwd_direct says where that is faster.
+// writes h (with res), or reads h and writes y.  32768 x 2048, statistics with residual: 92 us with loads of one row at a time, 64
+// with the row ring (6.3 TB/s).  RING = false loads the row when it is due: ln_fwd_direct says where that is faster.
 // (No minimum of blocks there: with one stated, of any number, the compiler takes 80 registers or spills instead of 40.)
 // ------------------------------------------------------------------------------------------
 template <int MAXV, bool RING>
@@ -243,33 +243,28 @@ ln_fwd_kernel(int mode, const uint4* __restrict__ x, const uint4* __restrict__ r
       }
     }
     stage = stage + 1 == S ? 0 : stage + 1;
-    float mean, rstd;
-    if (mode == 2) {
-      if (exchange) {
-        s = 0.f;
-        ss = 0.f;
-        for (int q = 0; q < ex.n; ++q) { s += ex_get(ex, q, row, 2, 0); ss += ex_get(ex, q, row, 2, 1); }
-      } else {
-        s = stats[2 * row];
-        ss = stats[2 * row + 1];
-      }
-    } else {
+    if (mode == 1) {
       block_sum2_alt(s, ss, red, parity);
-      if (mode == 1) {
-        if (threadIdx.x == 0) {
-          if (exchange) {
-            const float v2[2] = {s, ss};
-            ex_put<2>(ex, row, v2);
-          } else {
-            stats[2 * row] = s;
-            stats[2 * row + 1] = ss;
-          }
+      if (threadIdx.x == 0) {
+        if (exchange) {
+          const float v2[2] = {s, ss};
+          ex_put<2>(ex, row, v2);
+        } else {
+          stats[2 * row] = s;
+          stats[2 * row + 1] = ss;
         }
-        continue;
       }
+      continue;
     }
-    mean = s / (float)total_cols;
-    rstd = rsqrtf(fmaxf(ss / (float)total_cols - mean * mean, 0.f) + eps);
+    if (exchange) {
+      s = 0.f;
+      ss = 0.f;
+      for (int q = 0; q < ex.n; ++q) { s += ex_get(ex, q, row, 2, 0); ss += ex_get(ex, q, row, 2, 1); }
+    } else {
+      s = stats[2 * row];
+      ss = stats[2 * row + 1];
+    }
+    const float mean = s / (float)total_cols, rstd = rsqrtf(fmaxf(ss / (float)total_cols - mean * mean, 0.f) + eps);
     if (threadIdx.x == 0 && mean_rstd != nullptr) {
       mean_rstd[2 * row] = mean;
       mean_rstd[2 * row + 1] = rstd;
@@ -1327,12 +1322,11 @@ inline int ln_fwd_resident(int cols) {
 }
 
 // Rows of one vector per thread without the ring: while what a call moves stays in L2 there is no HBM latency to hide, and
-// the way through shared memory costs more than it gives.  Repeated calls of both passes in one, ring / direct, us: 4099 x 1544 with residual
-// (51 MB) 12.0 / 11.0, 8192 x 1024 with residual (67 MB) 12.8 / 11.5, 8192 x 2048 without (67 MB) 20.8 / 18.0; beyond L2 the
-// ring wins: 12000 x 1024 with residual (98 MB) 18.8 / 18.9, 16384 x 1024 (134 MB) 26.3 / 28.9; and below 8 MB, where a CTA
-// has one row, by 0.1 us (512 x 512 with residual 2.5 / 2.7).  With inputs from HBM the two differ by little up to the
-// line (8192 x 2048 26.6 / 26.6, 4099 x 1544 with residual 18.4 / 20.5).  Wider rows keep the ring: direct loads are faster
-// there only on inputs in L2, and slower from HBM (1024 x 12288: 21 / 17 and 27 / 33).
+// the way through shared memory costs more than it gives.  Repeated calls, ring / direct, us: statistics of 16384 x 1024 (32 MB)
+// 14.5 / 12.4, with residual 12000 x 1024 (70 MB) 14.5 / 13.2, rows of 8192 x 2048 (64 MB) 18.6 / 16.5; beyond L2 the ring wins:
+// statistics with residual of 8192 x 2048 (96 MB) 20.5 / 24.0, rows of 16384 x 2048 (128 MB) 35.8 / 36.9; below 8 MB there is
+// nothing between them.  With inputs from HBM the ring is ahead by 0 to 2 us on most sizes, 4 with a residual (12000 x 1024 20.4 / 24.5).
+// Wider rows keep the ring.
 constexpr int64_t kLnDirectMin = 8 << 20, kLnDirectMax = 80 << 20;
 inline bool ln_fwd_direct(int rows, int cols, int tensors) {
   const int64_t bytes = 2 * (int64_t)rows * cols * tensors;
@@ -1349,19 +1343,15 @@ inline bool ln_fwd_direct(int rows, int cols, int tensors) {
 //   with dres          65536 x 512 46 / 53 / 92, 32768 x 1024 52 / 41 / 56, x 3072 - / 132 / 145, x 4096 - / 192 / 172 (persistent 183),
 //                      8192 x 8192 - / 125 / 110 (persistent 96): three tensors in registers beyond three vectors each are too many
 struct LnRowShape { int v, w; };
-inline LnRowShape ln_row_shape(int rows, int cols, int max1, int max4, int max8) {
+struct LnRowMost { int w1, w4, w8; };     // most vectors per thread of a row of one, four, eight warps
+constexpr LnRowMost kLnFwdMost{8, 8, 8}, kLnFwdResMost{7, 5, 8}, kLnBwdMost{8, 8, 8}, kLnBwdDresMost{2, 3, 3};
+constexpr LnRowShape ln_row_shape(int rows, int cols, LnRowMost most) {
   const int nvec = cols / 8;
   const auto vectors = [&](int w) { return (nvec + 32 * w - 1) / (32 * w); };
-  int w = vectors(1) <= max1 ? 1 : vectors(4) <= max4 ? 4 : vectors(8) <= max8 ? 8 : 0;
+  int w = vectors(1) <= most.w1 ? 1 : vectors(4) <= most.w4 ? 4 : vectors(8) <= most.w8 ? 8 : 0;
   if (w == 0) return {0, 0};
   while (w < 8 && vectors(w) > 1 && (int64_t)rows * w < 1024) w = w == 1 ? 4 : 8;
   return {vectors(w), w};
-}
-inline LnRowShape ln_fwd_row_shape(int rows, int cols, bool res) {
-  return res ? ln_row_shape(rows, cols, 7, 5, 8) : ln_row_shape(rows, cols, 8, 8, 8);
-}
-inline LnRowShape ln_bwd_row_shape(int rows, int cols, bool dres) {
-  return dres ? ln_row_shape(rows, cols, 2, 3, 3) : ln_row_shape(rows, cols, 8, 8, 8);
 }
 // dgamma and dbeta from a second look at dy and h, in CTAs of the same launch, instead of the persistent kernel's registers: that
 // kernel ends with atomics of every CTA to the same addresses (5 us and more), and rows of up to 2048 columns wait there at a
@@ -1374,12 +1364,14 @@ inline bool ln_sums_from_second_look(int rows, int cols, bool dres) {
   if (cols <= kLnGroupedMaxCols) return !dres || mb <= 64;
   return mb <= (dres ? 25 : 34);
 }
-// f(vectors, warps) as integral constants
-template <class F>
+// f(vectors, warps) as integral constants, for the shapes that ln_row_shape gives with `w1`, `w4`, `w8` and no others.
+template <int w1, int w4, int w8, class F>
 cudaError_t with_row_shape(LnRowShape s, F&& f) {
-#define MSB_ROW(V, W) if (s.v == V && s.w == W) return f(std::integral_constant<int, V>{}, std::integral_constant<int, W>{});
-#define MSB_ROWS(W) MSB_ROW(1, W) MSB_ROW(2, W) MSB_ROW(3, W) MSB_ROW(4, W) MSB_ROW(5, W) MSB_ROW(6, W) MSB_ROW(7, W) MSB_ROW(8, W)
-  MSB_ROWS(1) MSB_ROWS(4) MSB_ROWS(8)
+#define MSB_ROW(V, W, MOST) \
+  if constexpr (V <= MOST)  \
+    if (s.v == V && s.w == W) return f(std::integral_constant<int, V>{}, std::integral_constant<int, W>{});
+#define MSB_ROWS(W, M) MSB_ROW(1, W, M) MSB_ROW(2, W, M) MSB_ROW(3, W, M) MSB_ROW(4, W, M) MSB_ROW(5, W, M) MSB_ROW(6, W, M) MSB_ROW(7, W, M) MSB_ROW(8, W, M)
+  MSB_ROWS(1, w1) MSB_ROWS(4, w4) MSB_ROWS(8, w8)
 #undef MSB_ROWS
 #undef MSB_ROW
   return cudaErrorInvalidValue;
@@ -1438,7 +1430,7 @@ cudaError_t ln_fwd(int mode, const void* x, const void* res, void* h_out, void* 
                    int cols, int total_cols, float eps, cudaStream_t stream, const RowExchange* exch) {
   if (cols % 8 != 0 || cols > 8 * kLnThreads * 8) return cudaErrorInvalidValue;
   if (exch != nullptr && mode != 1 && mode != 2) return cudaErrorInvalidValue;
-  if (rows <= 0) return cudaErrorInvalidValue;
+  if (rows <= 0 || (mode == 0 && total_cols != cols)) return cudaErrorInvalidValue;
   const int grid = exch != nullptr ? ln_grid(0, rows, cols) : ln_local_grid(0, rows, cols);
   RowExchange ex;
   if (exch != nullptr) ex = *exch; else memset(&ex, 0, sizeof(ex));
@@ -1451,12 +1443,16 @@ cudaError_t ln_fwd(int mode, const void* x, const void* res, void* h_out, void* 
   const int threads = ln_threads(cols), maxv = ln_fwd_maxv(cols);
   const int inputs = mode != 2 && res != nullptr ? 2 : 1;
   const int tensors = inputs + (mode != 2 && h_out != nullptr ? 1 : 0) + (mode != 1 ? 1 : 0);
-  if (exch == nullptr && mode == 0 && total_cols == cols) {
-    return with_row_shape(ln_fwd_row_shape(rows, cols, R != nullptr), [&](auto v, auto w) {
-      constexpr int per = ln_row_warps(w.value) / w.value;
-      auto kernel = R != nullptr ? ln_fwd_row_kernel<v.value, w.value, true> : ln_fwd_row_kernel<v.value, w.value, false>;
-      return launch_dependent(kernel, (rows + per - 1) / per, 32 * ln_row_warps(w.value), 0, stream, X, R, H, Y, G, B, mean_rstd, rows,
-                              cols, eps);
+  if (mode == 0) {
+    auto run = [&](auto kernel, int w) {
+      const int per = ln_row_warps(w) / w;
+      return launch_dependent(kernel, (rows + per - 1) / per, 32 * ln_row_warps(w), 0, stream, X, R, H, Y, G, B, mean_rstd, rows, cols, eps);
+    };
+    constexpr LnRowMost a = kLnFwdMost, b = kLnFwdResMost;
+    return R == nullptr ? with_row_shape<a.w1, a.w4, a.w8>(ln_row_shape(rows, cols, a), [&](auto v, auto w) {
+      return run(ln_fwd_row_kernel<v.value, w.value, false>, w.value);
+    }) : with_row_shape<b.w1, b.w4, b.w8>(ln_row_shape(rows, cols, b), [&](auto v, auto w) {
+      return run(ln_fwd_row_kernel<v.value, w.value, true>, w.value);
     });
   }
   if (exch == nullptr && ln_fwd_direct(rows, cols, tensors)) {
@@ -1490,7 +1486,7 @@ cudaError_t ln_bwd(int mode, const void* dy, const void* h, const void* gamma,
   auto G = reinterpret_cast<const uint4*>(gamma);
   auto DR = reinterpret_cast<const uint4*>(dres);
   auto DX = reinterpret_cast<uint4*>(dx);
-  const LnRowShape rs = ln_bwd_row_shape(rows, cols, DR != nullptr);
+  const LnRowShape rs = ln_row_shape(rows, cols, DR != nullptr ? kLnBwdDresMost : kLnBwdMost);
   const bool sums = dgamma != nullptr;
   // dx may be written over dy or h: the second look would find it there
   const auto over = [&](const void* p) {
@@ -1499,17 +1495,19 @@ cudaError_t ln_bwd(int mode, const void* dy, const void* h, const void* gamma,
   };
   if (exch == nullptr && mode == 0 && total_cols == cols && (sums || dbeta == nullptr) && rs.w > 0 && rows > 0 &&
       (!sums || (ln_sums_from_second_look(rows, cols, DR != nullptr) && !over(dy) && !over(h)))) {
-    return with_row_shape(rs, [&](auto v, auto w) {
-      constexpr int T = 32 * ln_row_warps(w.value), per = ln_row_warps(w.value) / w.value;
+    auto run = [&](auto kernel, int w) {
       // column sums: at least 128 CTAs, and no more than eight steps of T rows for one
+      const int T = 32 * ln_row_warps(w), per = ln_row_warps(w) / w;
       const int blocks = (cols + 31) / 32, most = (rows + T - 1) / T, few = (128 + blocks - 1) / blocks, deep = rows / (8 * T);
       const int want = few > deep ? few : deep, slices = !sums ? 1 : want < most ? want : most, sum_ctas = sums ? blocks * slices : 0;
-      auto run = [&](auto kernel) {
-        return launch_dependent(kernel, sum_ctas + (rows + per - 1) / per, T, 0, stream, DY, H, G, mean_rstd, DR, DX, rows, cols, dgamma,
-                                dbeta, sum_ctas, slices);
-      };
-      if (sums) return DR != nullptr ? run(ln_bwd_row_kernel<v.value, w.value, true, true>) : run(ln_bwd_row_kernel<v.value, w.value, false, true>);
-      return DR != nullptr ? run(ln_bwd_row_kernel<v.value, w.value, true, false>) : run(ln_bwd_row_kernel<v.value, w.value, false, false>);
+      return launch_dependent(kernel, sum_ctas + (rows + per - 1) / per, T, 0, stream, DY, H, G, mean_rstd, DR, DX, rows, cols, dgamma,
+                              dbeta, sum_ctas, slices);
+    };
+    constexpr LnRowMost a = kLnBwdMost, b = kLnBwdDresMost;
+    return DR == nullptr ? with_row_shape<a.w1, a.w4, a.w8>(rs, [&](auto v, auto w) {
+      return sums ? run(ln_bwd_row_kernel<v.value, w.value, false, true>, w.value) : run(ln_bwd_row_kernel<v.value, w.value, false, false>, w.value);
+    }) : with_row_shape<b.w1, b.w4, b.w8>(rs, [&](auto v, auto w) {
+      return sums ? run(ln_bwd_row_kernel<v.value, w.value, true, true>, w.value) : run(ln_bwd_row_kernel<v.value, w.value, true, false>, w.value);
     });
   }
   const LnBwdShape sh = ln_bwd_shape(cols);

@@ -733,3 +733,48 @@ def test_dependent_launches_in_a_captured_graph(rows, d):
         got = [t.clone() for t in out]
         assert all(torch.equal(a, b) for a, b in zip(got, want[i % 3])), i
     _native.check_status()
+
+
+@pytest.mark.parametrize("cols,rows,residual", [(264, 125000, True), (1024, 33000, True), (2048, 16500, True), (4096, 3300, True),
+                                                (4096, 4300, False), (3080, 4200, True), (12288, 1500, True)])
+def test_layernorm_persistent_backward_in_one_pass(cols, rows, residual):
+    """Calls beyond the rule for the second look: the persistent kernel with several rows per CTA (widths up to 2048, the last CTA
+    partly empty) and with a row each, with the parameters' gradients, which it adds to what is there.  Rows are rounded to bf16
+    once (2^-8 of the value, 2^-7 with the statistics); fp32 sums of ``rows`` products of normal values: 1e-5 sqrt(rows) times
+    thirty."""
+    from meshslice_b200.ops import functional as F
+    g = torch.Generator(device="cuda").manual_seed(cols + rows)
+    mk = lambda *s: torch.randn(*s, device="cuda", generator=g).bfloat16()
+    h, dy, dres, gamma = mk(rows, cols) + 1, mk(rows, cols), mk(rows, cols), mk(cols)
+    _, _, mr = F.ln_full(h, None, None, None, 1e-5)
+    dg, db = torch.ones(cols, device="cuda"), torch.ones(cols, device="cuda")
+    dx = F.ln_bwd_full(dy, h, gamma, mr, dg, db, dres if residual else None)
+    torch.cuda.synchronize()
+    hd, gd, bd = h.double().requires_grad_(True), gamma.double().requires_grad_(True), torch.zeros(cols, device="cuda", dtype=torch.double).requires_grad_(True)
+    torch.nn.functional.layer_norm(hd, (cols,), gd, bd, 1e-5).backward(dy.double())
+    want = hd.grad + dres.double() if residual else hd.grad
+    assert ((dx.double() - want).abs() <= 2 ** -7 * want.abs() + 2 ** -7 * want.abs().mean()).all()
+    tol = 3e-4 * rows ** 0.5
+    assert (dg.double() - 1 - gd.grad).abs().max() <= tol and (db.double() - 1 - bd.grad).abs().max() <= tol
+
+
+@pytest.mark.parametrize("residual", [True, False])
+@pytest.mark.parametrize("cols,rows", [(2048, 9001), (2056, 1300), (4096, 1187), (4104, 700), (8192, 600), (8200, 333), (16384, 300)])
+def test_layernorm_two_passes_of_wide_shards(cols, rows, residual):
+    """Every number of vectors per thread of the two-pass forward kernel (shards of up to 16384 columns), with fewer and with more
+    rows than a CTA's ring holds: statistics in fp32 over ``cols`` values (1e-5 of the sum of their sizes), rows rounded to
+    bf16 once (2^-8 of the value, 2^-7 with the statistics)."""
+    from meshslice_b200.ops import functional as F
+    g = torch.Generator(device="cuda").manual_seed(cols + rows)
+    mk = lambda *s: torch.randn(*s, device="cuda", generator=g).bfloat16()
+    x, res, gamma, beta = mk(rows, cols), mk(rows, cols), mk(cols), mk(cols)
+    h, stats = F.ln_stats(x, res if residual else None)
+    y, mr = F.ln_apply(h, stats, gamma, beta, cols, 1e-5)
+    torch.cuda.synchronize()
+    assert torch.equal(h, (x.float() + res.float()).bfloat16() if residual else x)
+    hd = h.double()
+    want = torch.stack([hd.sum(1), (hd * hd).sum(1)], 1)
+    assert ((stats.double() - want).abs() <= 1e-5 * torch.stack([hd.abs().sum(1), want[:, 1]], 1)).all()
+    ref = torch.nn.functional.layer_norm(hd, (cols,), gamma.double(), beta.double(), 1e-5)
+    assert ((y.double() - ref).abs() <= 2 ** -7 * ref.abs() + 2 ** -7 * ref.abs().mean()).all()
+    assert (mr[:, 0].double() - hd.mean(1)).abs().max() <= 1e-5 and ((mr[:, 1].double() - (hd.var(1, unbiased=False) + 1e-5).rsqrt()).abs() <= 1e-5).all()
