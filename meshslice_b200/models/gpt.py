@@ -12,8 +12,6 @@ the optimizer is one kernel launch per buffer; gradients mirror them.
 """
 from __future__ import annotations
 
-import os
-
 from dataclasses import dataclass, field
 from typing import List, Optional, Tuple
 
@@ -22,10 +20,8 @@ import torch
 from ..ops import functional as F
 from ..parallel.mesh import Mesh, ShardedTensor
 from ..parallel.tensor_parallel import init_block
+from . import sharded_layers
 from .sharded_layers import GeLU, ShardedAttention, ShardedFFLayer, ShardedLayerNorm, _add
-
-# GeLU inside the ff1 GEMM epilogue (MSB_FUSED_GELU=0 runs the stand-alone kernel instead)
-_FUSE_GELU = os.environ.get("MSB_FUSED_GELU", "1") != "0"
 
 
 @dataclass
@@ -104,7 +100,7 @@ class GPTBlock:
         a = self._lin(self.out_proj, self.attn.forward(self._lin(self.in_proj, y)))
         y = self.ln2.forward(a, x)                # h = x + a
         h = self.ln2.h
-        if self.ff1._fused and self.ff1.dataflow == "os" and _FUSE_GELU:
+        if self.ff1._fused and self.ff1.dataflow == "os" and sharded_layers.FUSE_GELU:
             g, pre = self.ff1.forward_gelu(y)          # GeLU in the GEMM epilogue
             self.gelu.remember(pre)
         else:
@@ -115,7 +111,7 @@ class GPTBlock:
     def backward(self, dh: ShardedTensor, dm: ShardedTensor):
         """dh: gradient of the residual stream after this block, dm: gradient of the MLP output.
         Returns (dx, ddelta) for the block below."""
-        if _FUSE_GELU and self.ff2.dataflow != "rs":
+        if self.ff2.dataflow != "rs":
             d = self.ff2.backward_gelu(dm, self.gelu)     # GeLU's derivative in the GEMM epilogue
         else:
             d = self.gelu.backward(self._lin_bwd(self.ff2, dm))

@@ -19,6 +19,7 @@ Gloo/NCCL ``DistMesh`` and, through the mesh's fused engine, on the tcgen05 kern
 """
 from __future__ import annotations
 
+import os
 from typing import Callable, List, Optional
 
 import torch
@@ -27,6 +28,9 @@ from .._native import zero_, zero_both_
 from ..ops import functional as F
 from ..parallel.mesh import Mesh, ShardedTensor
 from ..parallel.tensor_parallel import SPMD, createMultihostMatrix
+
+# GeLU and its derivative in the epilogues of the products next to them (MSB_FUSED_GELU=0 runs the stand-alone kernels instead)
+FUSE_GELU = os.environ.get("MSB_FUSED_GELU", "1") != "0"
 
 
 def _default_alloc(shape, dtype, device):
@@ -119,8 +123,8 @@ class ShardedFFLayer:
 
     def backward_gelu(self, dy: ShardedTensor, gelu: "GeLU") -> Optional[ShardedTensor]:
         """``gelu.backward(self.backward(dy))`` for a layer whose input is the output of ``gelu``: on a 1 x 1 mesh in the
-        epilogue of the input's gradient, without a pass of its own."""
-        if self._dw_dx is None or self.dataflow == "rs" or not gelu.fits(self._x):
+        epilogue of the input's gradient, without a pass of its own (with ``FUSE_GELU``)."""
+        if not FUSE_GELU or self._dw_dx is None or self.dataflow == "rs" or not gelu.fits(self._x):
             return gelu.backward(self.backward(dy))
         x, self._x = self._x, None
         return self._both(x, dy, gelu.take())

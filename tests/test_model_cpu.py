@@ -229,3 +229,40 @@ def test_mesh_transpose_is_the_global_transpose():
         mesh = EmuMesh(*shape)
         X = torch.arange(24 * 48, dtype=torch.float32).reshape(24, 48)
         assert torch.equal(mesh.unshard(mesh.transpose(mesh.shard(X))), X.t())
+
+
+@pytest.mark.parametrize("fuse", [True, False])
+def test_every_block_obeys_the_switch_of_the_fused_gelu(fuse, monkeypatch):
+    """With the switch off no block hands its pre-activation to the launch of both gradients (a stand-in on the CPU): the derivative
+    is GeLU's own."""
+    from meshslice_b200.models import sharded_layers
+    from meshslice_b200.models.gpt import GPTBlock
+    monkeypatch.setattr(sharded_layers, "FUSE_GELU", fuse)
+    monkeypatch.setattr(sharded_layers.GeLU, "fits", lambda self, y: True)
+    mesh = EmuMesh(1, 1)
+    S, H, D = 16, 2, 16
+    block = TransformerBlock(mesh, S, H, D, ["os", "os", "os", "ls"], ksplits=(1, 1, 1, 1), dtype=torch.float32, std=0.05)
+    gpt = GPTBlock(mesh, GPTConfig(n_layers=1, d_model=H * D, n_heads=H, ffn=4 * H * D, vocab=64, seq=S, ksplits=(1, 1, 1, 1),
+                                   dtype=torch.float32), 0, None, None, None, None)
+    x = ShardedTensor(mesh, {(0, 0): torch.randn(S, H * D, generator=torch.Generator().manual_seed(0))})
+    for b in (block, gpt):
+        handed = []
+
+        def both(dataflow, x, dy, w, grad, pre=None):
+            x, dy, w = (t.local() for t in (x, dy, w))
+            assert dataflow == "ls"
+            grad += dy.t() @ x
+            dx = dy @ w
+            if pre is None:
+                return dx
+            handed.append(1)
+            return sharded_layers.F.gelu_bwd(dx, pre.local())
+
+        b.ff2._dw_dx = both
+        if b is block:
+            b.forward(x)
+            d = b.backward(x)
+        else:
+            b.forward(x, None)
+            d, _ = b.backward(x, x)
+        assert len(handed) == fuse and torch.isfinite(d.local()).all()
