@@ -686,7 +686,8 @@ attn_delta_kernel(const uint4* out, const uint4* dout, float* delta,
 // became 490), and two exponentials of eight run on the FMA pipe (none of eight 363 -> 381 us, two 350, three 390 thousand
 // cycles for the first case below).
 // With one producer, rings of two stages each and a staging area: batch 4 x 2048, 32 heads, causal, 217 (key-major) and
-// 173 us (query-major), now 219 and 165 (429 -> 421 us with the row sums); full 737 -> 719, 16 heads x 8192 causal 709 -> 684.
+// 173 us (query-major), now 219 and 165 (429 -> 421 us with the row sums); full 737 -> 716, 16 heads x 8192 causal 709 -> 671.
+// Items of one or two blocks pay for the shared stage: batch 64 x 128, 32 heads 147 -> 157, 64 x 256 causal 295 -> 314.
 // P^T through shared memory, so that S(i+1) need not wait for dV(i): no faster (3500 cycles; Q's ring has two stages then).
 constexpr int kBwdPoly = 2;                 // key-major: exponentials of every eight that run on the FMA pipe
 constexpr int kBwdWarps = 16;               // element-wise warps

@@ -10,6 +10,8 @@ def _C():
     return _native.load(), _native.stream_ptr()
 
 
+# Whole rows take the row kernels forward and, where the second look at dy and h is the faster one, backward.  The ring and the
+# vectors per thread of the kernels behind them: test_layernorm_two_passes_of_wide_shards, test_layernorm_persistent_backward_in_one_pass.
 @pytest.mark.parametrize("residual", [True, False])
 @pytest.mark.parametrize("cols,rows", [(8, 1), (264, 5000), (2048, 9001), (2056, 1300), (4096, 1187), (8192, 600), (8200, 333),
                                        (12288, 450), (12296, 301), (16384, 300)])
@@ -75,6 +77,7 @@ def test_layernorm_of_whole_rows(cols, rows, residual):
     assert torch.isnan(yb[~keep]).any(1).all() and torch.equal(yb[keep], y[keep]) and torch.equal(mb[keep], mr[keep])
 
 
+# Every size here is on the near side of the rule; test_layernorm_persistent_backward_in_one_pass has the far one.
 @pytest.mark.parametrize("residual", [True, False])
 @pytest.mark.parametrize("cols,rows", [(8, 1), (40, 3000), (264, 129), (1544, 127), (1800, 4099), (2048, 513), (2056, 1025), (3080, 4100),
                                        (6152, 33), (16384, 20), (1024, 31500), (4096, 3052)])
@@ -103,6 +106,7 @@ def test_layernorm_parameter_gradients(cols, rows, residual):
     assert sums[0] == 1 and sums[-1] == 1
 
 
+# The ring is the two-pass kernel's; in one pass both sizes take the row kernel, whose bits do not depend on the number of rows here.
 @pytest.mark.parametrize("residual", [True, False])
 @pytest.mark.parametrize("cols", [264, 1024, 2048])
 def test_layernorm_forward_with_and_without_the_ring(cols, residual):
@@ -129,6 +133,8 @@ def test_layernorm_forward_with_and_without_the_ring(cols, residual):
         assert all(torch.equal(p, cut(w)) for p, w in zip(F.ln_apply(hp, sp, gamma, beta, cols, 1e-5), two))
 
 
+# Several rows per CTA and a row per CTA of the persistent kernel: test_layernorm_persistent_backward_in_one_pass; these sizes take
+# the row kernels but for the widest.
 @pytest.mark.parametrize("cols,rows", [(1024, 301), (768, 43), (64, 1000), (2048, 300), (4096, 300), (12288, 300)])
 def test_layernorm_fwd_bwd_single_pass(cols, rows):
     """Widths up to 2048 run several rows per CTA in the backward kernel (row counts that leave the last CTA
