@@ -849,10 +849,11 @@ __device__ __forceinline__ bool attn_bwd2_run(const CUtensorMap& tm_qkv, const C
           more = next_item();
           mbar_arrive(clc_empty);
         }
-        if (!ok) report(a.status, kErrAttn + 11, w.blk, g);
       }
+      // what is still under way (a timeout above is reported here too)
       for (uint32_t q = g; q < g + kRing0 && ok; ++q) ok = mbar_wait(empty0 + q % kRing0, ((q / kRing0) & 1) ^ 1, 8 * tmo);
       ok = ok && mbar_wait(res_empty, (items & 1) ^ 1, 8 * tmo);
+      if (!ok) report(a.status, kErrAttn + 11, w.blk, g);
     }
   } else if (warp == 2 + kBwdWarps) {
     // resident tile of dP, ring of dO or V: by a thread of its own, because a stage of one ring is often free long before one of the other
@@ -891,12 +892,11 @@ __device__ __forceinline__ bool attn_bwd2_run(const CUtensorMap& tm_qkv, const C
         if (ok) {
           more = next_item();
           mbar_arrive(clc_empty);
-        } else {
-          report(a.status, kErrAttn + 11, w.blk, g);
         }
       }
       for (uint32_t q = g; q < g + kRing1 && ok; ++q) ok = mbar_wait(empty1 + q % kRing1, ((q / kRing1) & 1) ^ 1, 8 * tmo);
       ok = ok && mbar_wait(res_empty + 1, (items & 1) ^ 1, 8 * tmo);
+      if (!ok) report(a.status, kErrAttn + 11, w.blk, g);
     }
   } else if (warp == 1) {
     if (elect_one()) {
@@ -1183,6 +1183,7 @@ __device__ __forceinline__ bool attn_bwd2_run(const CUtensorMap& tm_qkv, const C
     }
   }
   tc_fence_before_sync();
+  __syncwarp();
   const bool all = __syncthreads_and(ok) != 0;
   tc_fence_after_sync();
   if (threadIdx.x == 0 && all)
