@@ -687,7 +687,8 @@ attn_delta_kernel(const uint4* out, const uint4* dout, float* delta,
 // cycles for the first case below).
 // With one producer, rings of two stages each and a staging area: batch 4 x 2048, 32 heads, causal, 217 (key-major) and
 // 173 us (query-major), now 219 and 165 (429 -> 421 us with the row sums); full 737 -> 716, 16 heads x 8192 causal 709 -> 671.
-// Items of one or two blocks pay for the shared stage: batch 64 x 128, 32 heads 147 -> 157, 64 x 256 causal 295 -> 314.
+// The response is given back before the output leaves, not behind its copy: batch 64 x 128, 32 heads, full, forward and backward
+// 206 -> 192 us (194 with the staging area).
 // P^T through shared memory, so that S(i+1) need not wait for dV(i): no faster (3500 cycles; Q's ring has two stages then).
 constexpr int kBwdPoly = 2;                 // key-major: exponentials of every eight that run on the FMA pipe
 constexpr int kBwdWarps = 16;               // element-wise warps
@@ -1148,6 +1149,8 @@ __device__ __forceinline__ bool attn_bwd2_run(const CUtensorMap& tm_qkv, const C
       const uint32_t out_st = (g - 1) & 1;
       uint8_t* stage = sS1 + out_st * kTile + (warp - 2) * kBwdStage;   // where the item's last dO or V was
       more = next_item();                        // w is the next item's from here on
+      __syncwarp();                              // every lane has read the response: the one after may be asked for now
+      if (lane == 0) mbar_arrive(clc_empty);
 #pragma unroll 1
       for (int which = kKeyMajor ? 0 : 1; which < 2; ++which) {
         if (!warp_wait(acc_done + which, phase, 8 * tmo)) {
@@ -1178,8 +1181,7 @@ __device__ __forceinline__ bool attn_bwd2_run(const CUtensorMap& tm_qkv, const C
         mbar_arrive(out_read + out_st);          // the stage may take a tile again
       }
       tc_fence_before_sync();                    // the accumulators are read before the next P / dS is announced
-      __syncwarp();                              // every lane has read the response
-      if (lane == 0) mbar_arrive(clc_empty);
+      __syncwarp();
     }
   }
   tc_fence_before_sync();
